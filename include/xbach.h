@@ -157,9 +157,8 @@ int xb_ctx_set_params(xb_ctx* ctx, const xb_params* p);
  * "rank_candidates" (0..16, default 0 = every candidate): score and reorder
  * only the first n candidates of each stamp (the reference's brightest
  * first); the others keep their places after them.
- * "ldl_panel" (0/1, default 1, mixed mode): let the tuner choose among the
- * column LDL^T kernel and its panel variants (identical factors); 0 keeps
- * the column kernel.
+ * "ldl_panel" (0/1, default 1, mixed mode): accepted and without effect (one
+ * LDL^T kernel serves every system).
  * "ldl_cluster" (16 or 8, default 16, mixed mode): CTAs of the LDL^T cluster
  * (identical factors).
  * "gram_fp64" (0/1, mixed mode): compute the per-stamp Gram matrices with

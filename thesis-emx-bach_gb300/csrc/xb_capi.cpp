@@ -255,7 +255,7 @@ int xb_set_option(xb_ctx* c, const char* name, long long value) {
   } else if(n == "test_wait_timeout") {
     c->testWaitTimeout = value != 0;
   } else if(n == "ldl_panel") {
-    c->ldlPanel = value != 0;
+    // one LDL^T kernel serves every system
   } else if(n == "ldl_cluster") {
     if(value != 8 && value != 16) return XB_ERR_ARG;
     c->ldlCluster = (int)value;

@@ -267,7 +267,6 @@ std::string shapeKey(const xb_ctx* c, int w, int h) {
   put(p.convPerPixel);
   put(p.fitWeighted);
   put(c->gramFp64);
-  put(c->ldlPanel);
   put(c->ldlCluster);
   put(c->fillGram);
   put(c->fillGramTma);

@@ -1,5 +1,5 @@
 // xb_ldl.cu — the global normal system of the mixed path: LDL^T factorisation
-// on a thread-block cluster and a refined solve.
+// and a refined solve on one thread-block cluster.
 //
 // The global matrix built by createMatrix (src/cdkscUtil.cpp:307-402) is a
 // sum of Gram blocks weighted by outer products of the spatial terms, so it
@@ -8,27 +8,10 @@
 // The mixed path factors it as L D L^T instead (half the arithmetic, no
 // pivot search); a non-positive or non-finite pivot raises a flag and the
 // pivoted LU of xb_mixed.cu redoes the system, so singular systems end exactly
-// as in the reference.
-//
-// Factorisation.  Columns are dealt cyclically over the CL CTAs of a cluster
-// and live in shared memory.  Step j (1-based) is owned by CTA (j-1) % CL: it
-// sends the finished column j (unscaled) and r_j = 1/d_j to every other CTA
-// with one bulk shared-to-shared copy per receiver that completes on an
-// mbarrier in the receiver; each CTA then applies a_ik -= a_ij * (a_kj * r_j)
-// to its own columns k > j, rows i >= k.  The owner of column j+1 applies step j to that column first,
-// factors it and sends it before touching its other columns, so the critical
-// path per step is one shared-memory hop plus one column update.  Receive
-// buffers form a ring of LDL_RING slots per CTA; a slot is refilled only
-// after every receiver has released it (an "empty" mbarrier in the CTA that
-// sends the step that reuses the slot).  Every wait is bounded by a global
-// timer deadline; on expiry the kernel records a timeout and runs to the end
-// without waiting, so the launch always terminates.
-//
-// Solve.  One cluster: the CTAs invert the 32x32 diagonal blocks of L, CTA 0
-// runs the blocked triangular solves (a block = one small product with its
-// inverse, then the rows below/above it), all CTAs compute the FP64 residual
-// r = b - A x of the original matrix, and CTA 0 solves for the correction,
-// which is added once.
+// as in the reference.  One step of iterative refinement (FP64 residual of the
+// original matrix, corrected with the same factors) follows, which brings the
+// rounding of the factorisation back to the accuracy of the residual; the
+// correction is added once.
 
 #include <cooperative_groups.h>
 
@@ -42,681 +25,517 @@ namespace xb {
 
 namespace {
 
-constexpr int LDL_THREADS = 256;
-constexpr int LDL_RING = 8;  // receive slots per CTA
-constexpr unsigned long long LDL_WAIT_NS = 2000000000ull;  // deadline per launch
+// Factorisation and refined solve in one cluster launch (below).  Rows are
+// dealt cyclically: row i (0-based) lives in CTA i % CL, packed to its lower
+// part, so that every panel of 16 columns has its diagonal rows spread evenly
+// over the cluster and the trailing work stays balanced.
+constexpr int LS_THREADS = 512;
+constexpr int LS_BG = 4;          // warps that update while a panel is factored
+constexpr int LS_P = 16;          // panel width
+constexpr int LS_OWN = 64;         // own rows of a panel step: eight warps of eight
+constexpr int LS_SB = LS_P + 2;   // row stride of the exchanged 16-vectors
+constexpr int LS_TC = LS_P + 1;   // row stride of the factored diagonal block's columns
 
-// ------------------------------------------------------------ PTX helpers --
-__device__ __forceinline__ uint32_t smemAddr(const void* p) {
-  return (uint32_t)__cvta_generic_to_shared(p);
-}
-__device__ __forceinline__ uint32_t mapaRank(uint32_t a, int rank) {
-  uint32_t r;
-  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(rank));
-  return r;
-}
-__device__ __forceinline__ void mbarInit(uint32_t bar, int count) {
-  asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(bar), "r"(count) : "memory");
-}
-__device__ __forceinline__ void mbarArriveExpect(uint32_t bar, uint32_t bytes) {
-  asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes)
-               : "memory");
-}
-__device__ __forceinline__ void mbarArriveCluster(uint32_t clusterBar) {
-  asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(clusterBar)
-               : "memory");
-}
-__device__ __forceinline__ bool mbarTryWait(uint32_t bar, uint32_t parity) {
-  uint32_t ok;
-  asm volatile(
-      "{\n\t.reg .pred p;\n\t"
-      "mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n\t"
-      "selp.u32 %0, 1, 0, p;\n\t}"
-      : "=r"(ok)
-      : "r"(bar), "r"(parity)
-      : "memory");
-  return ok != 0;
-}
-// Bulk copy of `bytes` from this CTA's shared memory to another CTA's,
-// completing `bytes` of transactions on that CTA's mbarrier.
-__device__ __forceinline__ void bulkCopyCluster(uint32_t dstCluster, uint32_t srcCta,
-                                                uint32_t bytes, uint32_t barCluster) {
-  asm volatile(
-      "cp.async.bulk.shared::cluster.shared::cta.mbarrier::complete_tx::bytes [%0], [%1], %2, "
-      "[%3];" ::"r"(dstCluster),
-      "r"(srcCta), "r"(bytes), "r"(barCluster)
-      : "memory");
-}
-// Orders this thread's earlier shared-memory writes before later reads of the
-// async proxy (the bulk copies).
-__device__ __forceinline__ void fenceProxyAsync() {
-  asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-}
-__device__ __forceinline__ unsigned long long globalTimer() {
-  unsigned long long t;
-  asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
-  return t;
+struct LsLayout {
+  int nP, nPad;        // panels, padded order
+  int nr;              // rows per CTA (the right-hand side is one more row of CTA 0)
+  size_t rows, y, vec, small;  // doubles of each part of shared memory
+  __host__ __device__ size_t doubles() const { return rows + y + vec + small; }
+};
+__host__ __device__ inline LsLayout lsLayout(int n, int CL) {
+  LsLayout l;
+  l.nP = (n + LS_P - 1) / LS_P;
+  l.nPad = l.nP * LS_P;
+  l.nr = l.nPad / CL;  // CL is 8 or 16
+  l.rows = (size_t)CL * l.nr * (l.nr + 1) / 2 + l.nPad;
+  l.y = (size_t)l.nP * LS_P * LS_P;
+  l.vec = (size_t)(5 + LS_P / CL) * l.nPad;
+  // kept factors of diagonal blocks, the rows' right-hand sides
+  l.small = (size_t)((l.nP + CL - 1) / CL) * LS_P * LS_P + ((l.nr + 1) & ~1);
+  return l;
 }
 
-// 1/d to about one ulp: a single-precision reciprocal as the start value,
-// then one third-order Newton-Raphson step, x1 = x0 (1 + e + e^2) with
-// e = 1 - d x0 (the truncated series of 1/(1 - e)); |e| <= 2^-22 leaves a
-// truncation error below 2^-66.  Outside the float range, plain division.
-__device__ __forceinline__ double recipFast(double d) {
-  const double ad = fabs(d);
-  if(!(ad > 1e-30 && ad < 1e30)) return 1.0 / d;
-  const double x0 = (double)__frcp_rn((float)d);
-  const double e = fma(-d, x0, 1.0);
-  return fma(x0, fma(e, e, e), x0);
+// x > 0 and finite by its bits (an FP64 compare costs as much as a product)
+__device__ __forceinline__ bool positiveFinite(double x) {
+  const long long b = __double_as_longlong(x);
+  return b > 0 && b < 0x7FF0000000000000ll;
 }
 
-// Bytes step j sends to one receiver: entries [i0-2, LC) of the column, i0
-// the even row at or below j+1 (entry i0-2 carries r_j; LC is even, so the
-// size is a multiple of 16 bytes and both ends are 16-byte aligned).
-__device__ __forceinline__ uint32_t stepBytes(int j, int LC) {
-  return 8u * (uint32_t)(LC - ((j + 1) & ~1) + 2);
+__device__ __forceinline__ void clusterArrive() {
+  asm volatile("barrier.cluster.arrive.release;" ::: "memory");
+}
+__device__ __forceinline__ void clusterWait() {
+  asm volatile("barrier.cluster.wait.acquire;" ::: "memory");
+}
+// Barrier 1 over the first warps of a phase (count threads).
+__device__ __forceinline__ void barSome(int count) {
+  asm volatile("bar.sync 1, %0;" ::"r"(count) : "memory");
 }
 
-// Bounded wait on a local mbarrier phase; false (and the timeout flags set)
-// once the launch deadline has passed.
-__device__ __forceinline__ bool waitPhase(uint32_t bar, uint32_t parity,
-                                          unsigned long long deadline, volatile int* sErr,
-                                          int* status) {
-  if(*sErr) return false;
-  while(!mbarTryWait(bar, parity)) {
-    if(globalTimer() > deadline) {
-      *sErr = 1;
-      atomicOr(status + 1, 1);
-      return false;
-    }
-  }
-  return true;
-}
-
-}  // namespace
-
-// status[0] bit 0: a pivot was not positive and finite (LU fallback);
-// status[1] bit 0: a wait ran out of time.  F receives d_k on the diagonal and
-// l_ik (i > k) in both triangles (F[k][i] and F[i][k]); rinv[k] = 1/d_k.
+// M x = rhs by L D L^T and one step of iterative refinement with the FP64
+// residual of M, rhs <- x, on one cluster; status[0] bit 0 and rhs untouched
+// when a pivot is not positive and finite (the pivoted LU solves it then).
+//
+// Per panel of 16 columns: every CTA holds the panel's updated diagonal
+// block, gathered by remote shared-memory stores, and factors it redundantly
+// together with the panel columns of its own rows (four threads per row, four
+// columns each in registers; one barrier per column).  A pivot's reciprocal is
+// the 20-bit estimate x0 (PTX rcp.approx.ftz.f64) times 1 + e + e^2 with
+// e = 1 - d x0, the truncated series of 1/(1 - e): its error is e^3 < 2^-60.
+// (A conversion to or from FP32 takes as long as an FP64 product here.)  The
+// unscaled panel columns Y = L D go through global memory (each CTA writes its
+// rows, reads all): pushing them into 15 CTAs' shared memory took 4.2k cycles
+// per panel, the store, barrier and L2 reads ~3.5k.  Then the next panel's
+// diagonal rows are updated first and sent, the other rows of its columns
+// while that exchange runs, and the rest by LS_BG warps under the next panel's
+// factorisation and by all under the exchange after it.  The right-hand side
+// rides along as one more row, which is the forward substitution.
+//
+// The triangular passes exchange one 16-vector per panel: a pass applies the
+// inverse of the panel's diagonal block to it and every CTA updates its own
+// part.  Partial sums are kept per residue of the row modulo 16, so 8- and
+// 16-CTA clusters give the same bits.  No wait depends on anything but the
+// hardware cluster barrier.
+//
+// Bound by FP64: one warp instruction per 19 cycles per SM (62 in a chain), so
+// the n^3/6 products alone take 74 us on 16 SMs at n = 292 and the chains of
+// the n pivots ~65 us.  Alone on a GB300: 309 us at n = 292 and 1.01 ms at
+// n = 587; a column-by-column factorisation followed by block inverses, two
+// one-CTA triangular solves and a residual kernel took 640 us and 2.0 ms.
 template <int CL>
-__global__ void __launch_bounds__(LDL_THREADS)
-    k_global_ldl(const double* __restrict__ M, double* __restrict__ F, double* __restrict__ rinv,
-                 int n, int* __restrict__ status) {
-  extern __shared__ __align__(16) double ldl_s[];
+__global__ void __launch_bounds__(LS_THREADS)
+    k_ldl_factor_solve(const double* __restrict__ M, double* __restrict__ rhs, int n,
+                       double* __restrict__ Yg, int* __restrict__ status) {
+  extern __shared__ __align__(16) double ls_s[];
   cg::cluster_group cluster = cg::this_cluster();
+  constexpr int G = LS_P / CL;  // rows of a panel per CTA
   const int rank = (int)cluster.block_rank(), tid = threadIdx.x;
   const int lane = tid & 31, warp = tid >> 5;
-  constexpr int NW = LDL_THREADS / 32;
-  const int ld = n + 1;
-  const int LC = (n + 3) & ~1;  // even, >= n + 2
-  const int ncol = (n + CL - 1) / CL;
-  double* col = ldl_s;                               // ncol x LC
-  double* slot = col + (size_t)ncol * LC;            // LDL_RING x LC
-  double* rvec = slot + (size_t)LDL_RING * LC;       // LC
-  unsigned long long* bars = (unsigned long long*)(rvec + LC);
-  // bars[0..LDL_RING) full (receive) barriers, bars[LDL_RING] the empty barrier
-  __shared__ int sErr;
-  const unsigned long long deadline = globalTimer() + LDL_WAIT_NS;
+  const LsLayout lay = lsLayout(n, CL);
+  const int nP = lay.nP, nPad = lay.nPad, nr = lay.nr, ld = n + 1;
+  double* A = ls_s;                          // own rows, packed
+  double* Y = A + lay.rows;                  // [16][nPad]; later the inverses [nP][16][16]
+  double* wv = Y + lay.y;                    // nPad
+  double* xg = wv + nPad;                    // nPad
+  double* x1 = xg + nPad;                    // nPad
+  double* dinv = x1 + nPad;                  // nPad
+  double* yv = dinv + nPad;                  // nPad
+  double* sPart = yv + nPad;                 // G x nPad
+  double* keep = sPart + (size_t)G * nPad;   // slots x 16 x 16: L of diagonal blocks kept here
+  double* accv = keep + (size_t)((nP + CL - 1) / CL) * LS_P * LS_P;  // nr: the rows' right-hand sides
+  __shared__ __align__(16) double Tg[LS_P * LS_P];      // gathered diagonal block
+  __shared__ __align__(16) double Tc[LS_P * LS_TC];     // its column q at step q
+  __shared__ __align__(16) double Rq[LS_P];             // reciprocal pivots of the panel
+  __shared__ __align__(16) double SB[2 * LS_P * LS_SB]; // exchanged partial sums
+  __shared__ __align__(16) double FB[2 * LS_P];         // exchanged right-hand sides
+  __shared__ __align__(16) double tv[2 * LS_P];         // own values to send
+  __shared__ int sFlag, sNext, sPanel;
+  auto rowPtr = [&](int lr) { return A + (size_t)CL * lr * (lr + 1) / 2; };
+  double* rhsRow = rowPtr(nr);  // CTA 0
 
-  for(int lc = 0; lc < ncol; lc++) {
-    const int k = lc * CL + rank + 1;
-    double* ck = col + (size_t)lc * LC;
-    for(int i = tid; i < LC; i += LDL_THREADS)
-      ck[i] = (k <= n && i <= n) ? M[(size_t)k * ld + i] : 0.0;  // row k = column k
+  // own rows (lower part; identity past n) and the right-hand side
+  for(int lr = warp; lr < nr; lr += LS_THREADS / 32) {
+    const int i = lr * CL + rank;
+    double* a = rowPtr(lr);
+    for(int j = lane; j < (lr + 1) * CL; j += 32)
+      a[j] = (i < n && j <= i) ? M[(size_t)(i + 1) * ld + j + 1] : (i == j ? 1.0 : 0.0);
   }
-  for(int i = tid; i < LC; i += LDL_THREADS) rvec[i] = 0.0;
-  if(tid == 0) {
-    sErr = 0;
-    for(int r = 0; r < LDL_RING; r++) mbarInit(smemAddr(&bars[r]), 1);
-    mbarInit(smemAddr(&bars[LDL_RING]), CL - 1);
-    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-    // arm each slot for the first step this CTA receives through it
-    for(int r = 0; r < LDL_RING; r++)
-      for(int j = r + 1; j <= n - 1; j += LDL_RING)
-        if((j - 1) % CL != rank) {
-          mbarArriveExpect(smemAddr(&bars[r]), stepBytes(j, LC));
-          break;
-        }
-  }
-  __syncthreads();
-  cluster.sync();
+  if(rank == 0)
+    for(int j = tid; j < nPad; j += LS_THREADS) rhsRow[j] = j < n ? rhs[j + 1] : 0.0;
+  if(tid == 0) sFlag = sNext = sPanel = 0;
+  cluster.sync();  // every CTA runs: its shared memory may be written
 
-  uint32_t phaseBits = 0;  // receive-slot parities
-  uint32_t emptyPhase = 0;
-  volatile int* vErr = &sErr;
-
-  // Pivot of the finished column jp (owned here): r = 1/d is stored in rvec
-  // and at entry i0-2 of the column (a row above the diagonal, never used
-  // again), where it travels with the column.  One thread.
-  auto pivotStore = [&](int jp) {
-    double* cp = col + (size_t)((jp - 1) / CL) * LC;
-    const double d = cp[jp];
-    double r = recipFast(d);
-    if(!(d > 0.0) || !isfinite(r)) {
-      atomicOr(status, 1);
-      r = 0.0;
-    }
-    rvec[jp] = r;
-    cp[((jp + 1) & ~1) - 2] = r;
+  // The G rows of 16 values in `rows` to row g * CL + rank of `dst` (row
+  // stride ldd) in every CTA, one 16-byte store per thread.
+  auto push = [&](const double* rows, double* dst, int ldd) {
+    if(tid >= 128 * CL / 16 * G) return;
+    const int k = tid & 7, d = (tid >> 3) % CL, g = (tid >> 3) / CL;
+    ((double2*)(cluster.map_shared_rank(dst, d) + (size_t)(g * CL + rank) * ldd))[k] =
+        ((const double2*)(rows + g * LS_P))[k];
   };
-  // Copy column jp, entries [i0-2, LC), to the same place in every other
-  // CTA's receive slot, completing on that CTA's full barrier.  Called by all
-  // threads after the column's writes were fenced for the async proxy and
-  // the CTA synchronised; thread 0 waits for the slot and issues the copies.
-  auto sendColumn = [&](int jp) {
-    if(tid == 0) {
-      if(jp > LDL_RING) waitPhase(smemAddr(&bars[LDL_RING]), emptyPhase, deadline, vErr, status);
-      const int rs = (jp - 1) % LDL_RING;
-      const uint32_t off = (uint32_t)(((jp + 1) & ~1) - 2) * 8u;
-      const uint32_t src = smemAddr(col + (size_t)((jp - 1) / CL) * LC) + off;
-      const uint32_t dstSlot = smemAddr(slot + (size_t)rs * LC) + off;
-      const uint32_t fullA = smemAddr(&bars[rs]);
-      const uint32_t bytes = stepBytes(jp, LC);
-      for(int q = 0; q < CL; q++)
-        if(q != rank) bulkCopyCluster(mapaRank(dstSlot, q), src, bytes, mapaRank(fullA, q));
-    }
-    if(jp > LDL_RING) emptyPhase ^= 1u;
-  };
-
-  if(rank == 0) {
-    if(tid == 0) pivotStore(1);
-    fenceProxyAsync();
-    __syncthreads();
-    if(n > 1) sendColumn(1);
-  }
-  for(int j = 1; j < n; j++) {
-    const int rs = (j - 1) % LDL_RING;
-    const bool own = (j - 1) % CL == rank;
-    const double* a;
-    if(own) {
-      a = col + (size_t)((j - 1) / CL) * LC;
-    } else {
-      a = slot + (size_t)rs * LC;
-      waitPhase(smemAddr(&bars[rs]), (phaseBits >> rs) & 1u, deadline, vErr, status);
-      phaseBits ^= 1u << rs;
-    }
-    const double r = own ? rvec[j] : a[((j + 1) & ~1) - 2];
-    if(!own && tid == 0) rvec[j] = r;
-    const int lcStart = (j - rank + CL - 1) / CL;  // first local column k > j
-    const bool ahead = j % CL == rank;             // this CTA owns column j + 1
-    if(ahead) {
-      double* c1 = col + (size_t)lcStart * LC;
-      const double cf = a[j + 1] * r;
-      for(int i = j + 1 + tid; i <= n; i += LDL_THREADS) c1[i] = fma(-a[i], cf, c1[i]);
-      if(tid == 0) pivotStore(j + 1);  // row j+1 was this thread's first
-      fenceProxyAsync();
-      __syncthreads();
-      if(j + 1 < n) sendColumn(j + 1);
-    }
-    for(int lc = lcStart + (ahead ? 1 : 0) + warp; lc < ncol; lc += NW) {
-      const int k = lc * CL + rank + 1;
-      if(k > n) break;
-      double* ck = col + (size_t)lc * LC;
-      const double cf = a[k] * r;
-      for(int i = k + lane; i <= n; i += 32) ck[i] = fma(-a[i], cf, ck[i]);
-    }
-    __syncthreads();
-    if(!own && tid == 0) {
-      for(int jn = j + LDL_RING; jn <= n - 1; jn += LDL_RING)
-        if((jn - 1) % CL != rank) {
-          mbarArriveExpect(smemAddr(&bars[rs]), stepBytes(jn, LC));
-          break;
-        }
-      if(j + LDL_RING <= n - 1)
-        mbarArriveCluster(mapaRank(smemAddr(&bars[LDL_RING]), (j + LDL_RING - 1) % CL));
-    }
-  }
-  __syncthreads();
-  for(int lc = 0; lc < ncol; lc++) {
-    const int k = lc * CL + rank + 1;
-    if(k > n) break;
-    const double* ck = col + (size_t)lc * LC;
-    const double rk = rvec[k];
-    for(int i = k + tid; i <= n; i += LDL_THREADS) {
-      const double v = i == k ? ck[k] : ck[i] * rk;
-      F[(size_t)k * ld + i] = v;  // row k: l_ik, i > k
-      F[(size_t)i * ld + k] = v;  // row i: l_ik, k < i
-    }
-    if(tid == 0) rinv[k] = rk;
-  }
-  cluster.sync();  // no CTA leaves while another may still address its shared memory
-}
-
-// Panel variant (same factors, bit for bit): panels of P columns, panel p
-// owned by CTA p % CL, which applies every earlier panel to it, factors it
-// locally (pivot, then the updates inside the panel, in column order) and
-// copies the P columns to ring slot p % ring of every other CTA with one
-// bulk copy per receiver.  Every column receives the same updates, in the same
-// order, with the same FMAs as in the column kernel above; only the number
-// of cluster-wide exchanges drops (n/P instead of n).  Receivers arm a slot
-// before its copy can come and release it to the sender of panel p + ring
-// (ring <= CL keeps the empty-barrier phases in order).  The protocol is
-// modelled on the CPU in tests/test_ldl_panel_protocol.py.
-template <int CL, int P>
-__global__ void __launch_bounds__(LDL_THREADS)
-    k_global_ldl_panel(const double* __restrict__ M, double* __restrict__ F,
-                       double* __restrict__ rinv, int n, int ring, int* __restrict__ status) {
-  extern __shared__ __align__(16) double ldl_s[];
-  cg::cluster_group cluster = cg::this_cluster();
-  const int rank = (int)cluster.block_rank(), tid = threadIdx.x;
-  const int lane = tid & 31, warp = tid >> 5;
-  constexpr int NW = LDL_THREADS / 32;
-  const int ld = n + 1;
-  const int LC = (n + 3) & ~1;
-  const int nP = (n + P - 1) / P, lpn = (nP + CL - 1) / CL, lastSent = nP - 2;
-  double* col = ldl_s;                                // lpn * P x LC (panel lp = p / CL)
-  double* slot = col + (size_t)lpn * P * LC;          // ring x P x LC
-  double* rvec = slot + (size_t)ring * P * LC;        // LC
-  unsigned long long* bars = (unsigned long long*)(rvec + LC);  // ring full + 1 empty
-  __shared__ int sErr;
-  const unsigned long long deadline = globalTimer() + LDL_WAIT_NS;
-  const uint32_t panelBytes = (uint32_t)P * (uint32_t)LC * 8u;
-  auto ownerOf = [](int p) { return p % CL; };
-  auto localCol = [&](int k) {  // column k (1-based) of a panel owned here
-    const int p = (k - 1) / P;
-    return col + (size_t)((p / CL) * P + (k - 1) % P) * LC;
-  };
-
-  for(int lp = 0; lp < lpn; lp++) {
-    const int p = lp * CL + rank;
-    for(int q = 0; q < P; q++) {
-      const int k = 1 + p * P + q;
-      double* ck = col + (size_t)(lp * P + q) * LC;
-      for(int i = tid; i < LC; i += LDL_THREADS)
-        ck[i] = (p < nP && k <= n && i <= n) ? M[(size_t)k * ld + i] : 0.0;
-    }
-  }
-  for(int i = tid; i < LC; i += LDL_THREADS) rvec[i] = 0.0;
-  if(tid == 0) {
-    sErr = 0;
-    for(int r = 0; r < ring; r++) mbarInit(smemAddr(&bars[r]), 1);
-    mbarInit(smemAddr(&bars[ring]), CL - 1);
-    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-    for(int r = 0; r < ring; r++)
-      for(int p = r; p <= lastSent; p += ring)
-        if(ownerOf(p) != rank) {
-          mbarArriveExpect(smemAddr(&bars[r]), panelBytes);
-          break;
-        }
-  }
-  __syncthreads();
-  cluster.sync();
-
-  uint32_t phaseBits = 0, emptyPhase = 0;
-  volatile int* vErr = &sErr;
-
-  // pivots and in-panel updates of panel p (owned, earlier panels applied)
-  auto factorPanel = [&](int p) {
-    const int first = 1 + p * P, last = min(n, first + P - 1);
-    for(int j = first; j <= last; j++) {
-      double* cj = localCol(j);
-      if(tid == 0) {
-        const double d = cj[j];
-        double r = recipFast(d);
-        if(!(d > 0.0) || !isfinite(r)) {
-          atomicOr(status, 1);
-          r = 0.0;
-        }
-        rvec[j] = r;
-        cj[((j + 1) & ~1) - 2] = r;  // travels with the column, above its diagonal
+  // Diagonal rows of panel p, the columns of panel p - 1 applied: group g of
+  // 64 threads has row p*16 + g*CL + rank, four threads per column, which
+  // split the 16 products.
+  auto diagRows = [&](int p) {
+    if(tid < 64 * G) {
+      const int g = tid >> 6, c = (tid >> 2) & 15, part = tid & 3;
+      const int lr = p * G + g, i = lr * CL + rank, j = p * LS_P + c;
+      double* a = rowPtr(lr);
+      double s = 0.0;
+      if(p > 0 && j <= i) {
+        const double* l = a + (p - 1) * LS_P + 4 * part;
+        const double* y = Y + (size_t)4 * part * nPad + j;
+#pragma unroll
+        for(int q = 0; q < 4; q++) s = fma(l[q], y[(size_t)q * nPad], s);
       }
-      __syncthreads();
-      const double r = rvec[j];
-      for(int k = j + 1 + warp; k <= last; k += NW) {
-        double* ck = localCol(k);
-        const double cf = cj[k] * r;
-        for(int i = k + lane; i <= n; i += 32) ck[i] = fma(-cj[i], cf, ck[i]);
-      }
-      __syncthreads();
+      s += __shfl_xor_sync(0xffffffffu, s, 1);
+      s += __shfl_xor_sync(0xffffffffu, s, 2);
+      if(part == 0) tv[g * LS_P + c] = j <= i ? a[j] - s : 0.0;
+    }
+    if(tid < 128) {
+      barSome(128);
+      push(tv, Tg, LS_P);
     }
   };
-  // panel p (base: its P columns) applied to the local columns of the panels
-  // [pFrom, pTo]: per entry, the panel's columns in order
-  auto applyPanel = [&](const double* base, int p, int pFrom, int pTo) {
-    const int first = 1 + p * P, w = min(P, n - first + 1);
-    double rq[P];
+
+  // Columns of panel p applied to one entry of an own row.
+  auto update = [&](double* a, int p, int j) {
+    double v = a[j];
+    const double* l = a + p * LS_P;
+    const double* y = Y + j;
 #pragma unroll
-    for(int q = 0; q < P; q++) rq[q] = q < w ? base[(size_t)q * LC + ((first + q + 1) & ~1) - 2] : 0.0;
-    const int lp0 = (pFrom - rank + CL - 1) / CL;  // first local panel >= pFrom
-    for(int e = warp; ; e += NW) {
-      const int lp = lp0 + e / P, q = e % P, pk = lp * CL + rank, k = 1 + pk * P + q;
-      if(pk > pTo || pk >= nP || k > n) break;
-      double* ck = col + (size_t)(lp * P + q) * LC;
-      double cf[P];
+    for(int q = 0; q < LS_P; q++) v = fma(-l[q], y[(size_t)q * nPad], v);
+    a[j] = v;
+  };
+  // What is left of a panel's trailing update, the columns past the next
+  // panel, flattened over (row, column); warps take 32 entries at a time.
+  struct Rest {
+    int p, lrA, nRow, c0, nTri, tot, j0;
+    float b;
+    __device__ void set(int p_, int rank, int nr, int nPad) {
+      p = p_;
+      lrA = (p + 2) * G;
+      j0 = (p + 2) * LS_P;
+      nRow = nr - lrA;
+      c0 = lrA * CL + rank - j0 + 1;  // columns of the first row
+      nTri = nRow > 0 ? nRow * c0 + CL * (nRow * (nRow - 1) / 2) : 0;
+      tot = p < 0 ? 0 : nTri + (rank == 0 ? nPad - j0 : 0);
+      b = (float)c0 - 0.5f * CL;
+    }
+  } rest;
+  rest.set(-1, rank, nr, nPad);
+  auto restStep = [&]() -> bool {
+    int e = 0;
+    if(lane == 0) e = atomicAdd(&sNext, 32);
+    e = __shfl_sync(0xffffffffu, e, 0);
+    if(e >= rest.tot) return false;
+    e += lane;
+    if(e < rest.nTri) {
+      int t = (int)((sqrtf(rest.b * rest.b + 2.f * CL * (float)e) - rest.b) * (1.f / CL));
+      t = max(0, min(t, rest.nRow - 1));
+      while(t > 0 && t * rest.c0 + CL * (t * (t - 1) / 2) > e) t--;
+      while(t + 1 < rest.nRow && (t + 1) * rest.c0 + CL * ((t + 1) * t / 2) <= e) t++;
+      update(rowPtr(rest.lrA + t), rest.p, rest.j0 + e - (t * rest.c0 + CL * (t * (t - 1) / 2)));
+    } else if(e < rest.tot) {
+      update(rhsRow, rest.p, rest.j0 + e - rest.nTri);
+    }
+    __syncwarp();
+    return true;
+  };
+
+  diagRows(0);
+  clusterArrive();
+  clusterWait();
+  for(int p = 0; p < nP; p++) {
+    const int K = p * LS_P;
+    // ---- the panel: diagonal block (warps 0, 1) and own rows below it
+    // (warps 2, 3, 6, 7, ...: the other two schedulers)
+    const int lr0 = (p + 1) * G;                          // first own row below the panel
+    const int nOwn = nr - lr0 + (rank == 0 ? 1 : 0);      // CTA 0: the right-hand side too
+    const int nOwnW = (nOwn + 7) >> 3, nBar = 32 * (3 + nOwnW);
+    const bool isT = warp < 2, isR = warp == 4;  // the block; its pivots' reciprocals
+    const int ow = (warp >> 2) * 2 + (warp & 1);          // own-row warp index
+    __syncthreads();  // the panel's columns are up to date
+    if(isT || isR || ((warp & 2) && ow < nOwnW)) {
+      const int u = lane & 3;
+      const int t = isT ? tid >> 2 : ow * 8 + (lane >> 2);
+      const bool live = isT || (!isR && t < nOwn);
+      double* a = isT ? nullptr : (lr0 + t < nr ? rowPtr(lr0 + t) : rhsRow) + K;
+      double z[4], l[4];
 #pragma unroll
-      for(int u = 0; u < P; u++) cf[u] = u < w ? base[(size_t)u * LC + k] * rq[u] : 0.0;
-      for(int i = k + lane; i <= n; i += 32) {
-        double v = ck[i];
+      for(int m = 0; m < 4; m++) {
+        const int c = 4 * m + u;
+        l[m] = 0.0;
+        z[m] = isT ? (c <= t ? Tg[t * LS_P + c] : 0.0) : (live ? a[c] : 0.0);
+      }
+      if(isT && u == 0) Tc[t] = z[0];
+      double dl = 0.0, dc[4];  // the block's updates of a step that its chain does not wait for
 #pragma unroll
-        for(int u = 0; u < P; u++)
-          if(u < w) v = fma(-base[(size_t)u * LC + i], cf[u], v);
-        ck[i] = v;
+      for(int m = 0; m < 4; m++) dc[m] = 0.0;
+#pragma unroll
+      for(int q = 0; q < LS_P; q++) {
+        barSome(nBar);
+        if(isT) {
+          if(q > 7 && warp == 0) continue;  // its rows 0..7 are done
+          const double* tc = Tc + q * LS_TC;
+          const double d = tc[q];
+          double x0;
+          asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(x0) : "d"(d));
+          if(q > 0) {  // step q - 1 of the columns beyond q
+#pragma unroll
+            for(int m = (q >> 2) + 1; m < 4; m++) z[m] = fma(-dl, dc[m], z[m]);
+          }
+          const double zq = __shfl_sync(0xffffffffu, z[q >> 2], (lane & ~3) | (q & 3));
+          const double e = fma(-d, x0, 1.0), v = zq * x0;
+          const double lq = fma(v, fma(e, e, e), v);
+          if(u == (q & 3)) l[q >> 2] = lq;
+          if(q + 1 < LS_P) {
+            const int m0 = (q + 1) >> 2;
+#pragma unroll
+            for(int m = m0; m < 4; m++) dc[m] = tc[4 * m + u];
+            if(4 * m0 + u > q) z[m0] = fma(-lq, dc[m0], z[m0]);
+            if(u == ((q + 1) & 3)) Tc[(q + 1) * LS_TC + t] = z[m0];
+            dl = lq;
+          }
+        } else if(isR) {
+          // the pivot's reciprocal, its check and its copy
+          const double d = Tc[q * LS_TC + q];
+          double x0;
+          asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(x0) : "d"(d));
+          const double e = fma(-d, x0, 1.0);
+          double r = fma(x0, fma(e, e, e), x0);
+          if(!positiveFinite(d) || !positiveFinite(r)) {
+            if(lane == 0) sFlag = 1;
+            r = 0.0;
+          }
+          if(lane == 0) {
+            Rq[q] = r;
+            dinv[K + q] = r;
+          }
+        } else if(q > 0) {
+          // own rows run one step behind: the reciprocal of step q - 1 was
+          // stored before this step's barrier
+          const double* tp = Tc + (q - 1) * LS_TC;
+          const double zp = __shfl_sync(0xffffffffu, z[(q - 1) >> 2], (lane & ~3) | ((q - 1) & 3));
+          const double lp = zp * Rq[q - 1];
+#pragma unroll
+          for(int m = q >> 2; m < 4; m++) {
+            const int c = 4 * m + u;
+            if(c >= q) z[m] = fma(-lp, tp[c], z[m]);
+          }
+          if(u == ((q - 1) & 3)) l[(q - 1) >> 2] = lp;
+        }
+      }
+      barSome(nBar);
+      if(isT) {
+        if(p % CL == rank) {
+          double* kp = keep + (size_t)(p / CL) * LS_P * LS_P + t * LS_P;
+#pragma unroll
+          for(int m = 0; m < 4; m++) kp[4 * m + u] = 4 * m + u < t ? l[m] : 0.0;
+        }
+      } else if(!isR) {
+        const double zp = __shfl_sync(0xffffffffu, z[3], lane | 3);
+        if(u == 3) l[3] = zp * Rq[LS_P - 1];
+        if(live) {
+          const int i = (lr0 + t) * CL + rank;
+#pragma unroll
+          for(int m = 0; m < 4; m++) {
+            a[4 * m + u] = l[m];
+            if(lr0 + t < nr) Yg[(size_t)(4 * m + u) * nPad + i] = z[m];
+          }
+        }
       }
     }
-  };
-  auto sendPanel = [&](int p) {
-    if(tid == 0) {
-      if(p >= ring) waitPhase(smemAddr(&bars[ring]), emptyPhase, deadline, vErr, status);
-      const int sl = p % ring;
-      const uint32_t src = smemAddr(localCol(1 + p * P));
-      const uint32_t dst = smemAddr(slot + (size_t)sl * P * LC);
-      const uint32_t fullA = smemAddr(&bars[sl]);
-      for(int q = 0; q < CL; q++)
-        if(q != rank) bulkCopyCluster(mapaRank(dst, q), src, panelBytes, mapaRank(fullA, q));
-    }
-    if(p >= ring) emptyPhase ^= 1u;
-  };
-
-  if(ownerOf(0) == rank) {
-    factorPanel(0);
-    fenceProxyAsync();
-    __syncthreads();
-    if(0 <= lastSent) sendPanel(0);
-  }
-  for(int p = 0; p < nP - 1; p++) {
-    const int sl = p % ring;
-    const bool own = ownerOf(p) == rank;
-    const double* base;
-    if(own) {
-      base = localCol(1 + p * P);
-    } else {
-      base = slot + (size_t)sl * P * LC;
-      waitPhase(smemAddr(&bars[sl]), (phaseBits >> sl) & 1u, deadline, vErr, status);
-      phaseBits ^= 1u << sl;
-    }
-    const bool ahead = ownerOf(p + 1) == rank;
-    if(ahead) {  // look-ahead: the next panel first, factored and sent
-      applyPanel(base, p, p + 1, p + 1);
-      __syncthreads();
-      factorPanel(p + 1);
-      fenceProxyAsync();
-      __syncthreads();
-      if(p + 1 <= lastSent) sendPanel(p + 1);
-    }
-    applyPanel(base, p, ahead ? p + 2 : p + 1, nP - 1);
-    __syncthreads();
-    if(!own && tid == 0) {
-      for(int pn = p + ring; pn <= lastSent; pn += ring)
-        if(ownerOf(pn) != rank) {
-          mbarArriveExpect(smemAddr(&bars[sl]), panelBytes);
-          break;
-        }
-      if(p + ring <= lastSent) mbarArriveCluster(mapaRank(smemAddr(&bars[ring]), ownerOf(p + ring)));
-    }
-  }
-  __syncthreads();
-  for(int lp = 0; lp < lpn; lp++)
-    for(int q = 0; q < P; q++) {
-      const int k = 1 + (lp * CL + rank) * P + q;
-      if(k > n) break;
-      const double* ck = col + (size_t)(lp * P + q) * LC;
-      const double rk = rvec[k];
-      for(int i = k + tid; i <= n; i += LDL_THREADS) {
-        const double v = i == k ? ck[k] : ck[i] * rk;
-        F[(size_t)k * ld + i] = v;
-        F[(size_t)i * ld + k] = v;
+    // the other warps: LS_BG of them work on the panel before's update
+    // meanwhile, the rest wait
+    else if(warp >= LS_THREADS / 32 - LS_BG) {
+      while(*(volatile int*)&sPanel <= p && restStep()) {
       }
-      if(tid == 0) rinv[k] = rk;
     }
-  cluster.sync();  // no CTA leaves while another may still address its shared memory
-}
-
-// ------------------------------------------------------------------ solve --
-namespace {
-
-constexpr int SV_THREADS = 512;
-constexpr int SV_NB = 32;  // diagonal block size
-constexpr int SV_AW = 4;   // warps of a 32x32 block product (8 terms each)
-
-// Inverse of the unit lower-triangular diagonal block q of L (rows/cols
-// [1 + 32q, 1 + 32q + 32), padded with the identity past n) into Linv
-// (32 x 32, row-major), by recursive doubling: for a 2m block
-// [[A, 0], [C, B]] the inverse's lower-left part is -B^-1 (C A^-1).
-// CTA-wide; X is 32 x 33, T 256 doubles of shared memory.
-__device__ void invertDiagBlock(const double* __restrict__ F, int n, int q, double* X, double* T,
-                                double* __restrict__ Linv) {
-  const int tid = threadIdx.x, ld = n + 1, s = 1 + q * SV_NB;
-  constexpr int XL = SV_NB + 1;
-  for(int e = tid; e < SV_NB * SV_NB; e += SV_THREADS) {
-    const int t = e / SV_NB, u = e % SV_NB;
-    double v = t == u ? 1.0 : 0.0;
-    if(t > u && s + t <= n) v = F[(size_t)(s + t) * ld + s + u];  // L[t][u] (kept in X's lower part)
-    X[t * XL + u] = v;
-  }
-  __syncthreads();
-  // X's strictly lower part holds L until each level overwrites its blocks
-  for(int m = 1; m < SV_NB; m *= 2) {
-    const int nPair = SV_NB / (2 * m), cnt = nPair * m * m;
-    // T = C A^-1 for every pair block
-    for(int e = tid; e < cnt; e += SV_THREADS) {
-      const int p = e / (m * m), a = (e / m) % m, b = e % m, o = p * 2 * m;
-      double acc = 0.0;
-      for(int c = b; c < m; c++)  // A^-1 is unit lower: entries c >= b
-        acc = fma(X[(o + m + a) * XL + o + c], c == b ? 1.0 : X[(o + c) * XL + o + b], acc);
-      T[e] = acc;
-    }
+    if(isR && lane == 0) *(volatile int*)&sPanel = p + 1;
     __syncthreads();
-    // lower-left <- -B^-1 T
-    for(int e = tid; e < cnt; e += SV_THREADS) {
-      const int p = e / (m * m), a = (e / m) % m, b = e % m, o = p * 2 * m;
-      double acc = T[e];  // the unit diagonal of B^-1
-      for(int c = 0; c < a; c++) acc = fma(X[(o + m + a) * XL + o + m + c], T[p * m * m + c * m + b], acc);
-      X[(o + m + a) * XL + o + b] = -acc;
+    if(p + 1 == nP) break;
+    clusterArrive();
+    while(restStep()) {
     }
-    __syncthreads();
-  }
-  for(int e = tid; e < SV_NB * SV_NB; e += SV_THREADS)
-    Linv[(size_t)q * SV_NB * SV_NB + e] = X[(e / SV_NB) * XL + e % SV_NB];
-  __syncthreads();
-}
-
-// x <- L^-T D^-1 L^-1 x on x[1..n] (shared), CTA-wide, with the inverses of
-// the diagonal blocks in Li (shared, nB x 32 x 32).  Per block: the 32x32
-// product with the inverse (warps 0-3, eight terms each), then the next
-// block's rows (warps 0-3) and, at the same time, the rows beyond it
-// (warps 4-15, one row per thread; each loads its row's 32 entries of L at
-// once, since the chain is bound by L2 latency).  part: SV_AW x 32 doubles.
-// sum_t F[s + t][i] x[s + t] over the nb (<= 32) rows of a block: four
-// accumulators over t in steps of four, the remainder into the first; the 32
-// loads are issued before the products.
-__device__ __forceinline__ double rowDot(const double* __restrict__ F, int ld, int s, int nb,
-                                         int i, const double* x) {
-  double f[SV_NB];
-#pragma unroll
-  for(int t = 0; t < SV_NB; t++) f[t] = t < nb ? F[(size_t)(s + t) * ld + i] : 0.0;
-  double a0 = 0.0, a1 = 0.0, a2 = 0.0, a3 = 0.0;
-#pragma unroll
-  for(int t = 0; t < SV_NB; t += 4)
-    if(t + 4 <= nb) {
-      a0 = fma(f[t], x[s + t], a0);
-      a1 = fma(f[t + 1], x[s + t + 1], a1);
-      a2 = fma(f[t + 2], x[s + t + 2], a2);
-      a3 = fma(f[t + 3], x[s + t + 3], a3);
-    }
-#pragma unroll
-  for(int t = 0; t < SV_NB; t++)
-    if(t >= (nb & ~3) && t < nb) a0 = fma(f[t], x[s + t], a0);
-  return (a0 + a1) + (a2 + a3);
-}
-
-__device__ void ldlSolveCta(const double* __restrict__ F, const double* __restrict__ rinv, int n,
-                            const double* Li, double* x, double* part) {
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, ld = n + 1;
-  const int nB = (n + SV_NB - 1) / SV_NB;
-  // ---- forward: L y = x
-  for(int K = 0; K < nB; K++) {
-    const int s = 1 + K * SV_NB, nb = min(SV_NB, n + 1 - s);
-    const double* Lk = Li + (size_t)K * SV_NB * SV_NB;
-    if(warp < SV_AW) {  // y_K = Linv_K x_K
-      double acc = 0.0;
-#pragma unroll
-      for(int u = 0; u < SV_NB / SV_AW; u++) {
-        const int t = warp * (SV_NB / SV_AW) + u;
-        if(t < nb) acc = fma(Lk[lane * SV_NB + t], x[s + t], acc);
+    __syncthreads();  // Y of the panel before is read
+    clusterWait();
+    // ---- all rows' Y of this panel into shared memory
+    {
+      const int j0 = K + LS_P, half = (nPad - j0) / 2, tot = LS_P * half;
+      for(int e = tid; e < tot; e += LS_THREADS) {
+        const int q = e / half, j = j0 + 2 * (e - q * half);
+        *(double2*)(Y + (size_t)q * nPad + j) = __ldcg((const double2*)(Yg + (size_t)q * nPad + j));
       }
-      part[warp * 32 + lane] = acc;
     }
     __syncthreads();
-    if(warp == 0 && lane < nb)
-      x[s + lane] = (part[lane] + part[32 + lane]) + (part[64 + lane] + part[96 + lane]);
-    __syncthreads();
-    const int s2 = s + SV_NB, nb2 = min(SV_NB, n + 1 - s2);  // next block
-    if(warp < SV_AW) {
-      if(nb2 > 0) {
+    diagRows(p + 1);
+    clusterArrive();
+    // ---- the next panel's columns of the other own rows
+    {
+      const int lrA = (p + 2) * G, nRow = nr - lrA + (rank == 0 ? 1 : 0);
+      for(int e = tid; e < nRow * LS_P; e += LS_THREADS) {
+        const int lr = lrA + (e >> 4);
+        update(lr < nr ? rowPtr(lr) : rhsRow, p, K + LS_P + (e & 15));
+      }
+    }
+    rest.set(p + 2 < nP ? p : -1, rank, nr, nPad);
+    if(tid == 0) sNext = 0;
+    clusterWait();
+  }
+  __syncthreads();
+  if(sFlag) {  // the same in every CTA: the block was factored from the same bits
+    if(rank == 0 && tid == 0) atomicOr(status, 1);
+    cluster.sync();  // remote stores into this CTA are done
+    return;
+  }
+
+  // ---- inverses of the unit lower diagonal blocks: CTA p % CL inverts block
+  // p by recursive doubling (a 2m block [[A, 0], [C, B]] has the inverse's
+  // lower left -B^-1 (C A^-1)), then all CTAs get all of them
+  {
+    const int slot = tid >> 7, h = tid & 127, nSlot = (nP - rank + CL - 1) / CL;
+    for(int s0 = 0; s0 < (nP + CL - 1) / CL; s0 += 4) {
+      const bool on = s0 + slot < nSlot;
+      double* X = keep + (size_t)(s0 + slot) * LS_P * LS_P;
+      if(on && h < LS_P) X[h * LS_P + h] = 1.0;
+      __syncthreads();
+#pragma unroll
+      for(int m = 1; m < LS_P; m *= 2) {
+        const int cnt = (LS_P / (2 * m)) * m * m;  // 8, 16, 32, 64
+        const int pr = h / (m * m), r = (h / m) % m, cc = h % m, o = pr * 2 * m;
         double acc = 0.0;
-#pragma unroll
-        for(int u = 0; u < SV_NB / SV_AW; u++) {
-          const int t = warp * (SV_NB / SV_AW) + u;
-          if(t < nb && lane < nb2) acc = fma(F[(size_t)(s + t) * ld + s2 + lane], x[s + t], acc);
+        if(on && h < cnt)
+          for(int k = cc; k < m; k++)
+            acc = fma(X[(o + m + r) * LS_P + o + k], X[(o + k) * LS_P + o + cc], acc);
+        __syncthreads();
+        if(on && h < cnt) X[(o + m + r) * LS_P + o + cc] = acc;
+        __syncthreads();
+        acc = 0.0;
+        if(on && h < cnt)
+          for(int k = 0; k <= r; k++)
+            acc = fma(X[(o + m + r) * LS_P + o + m + k], X[(o + m + k) * LS_P + o + cc], acc);
+        __syncthreads();
+        if(on && h < cnt) X[(o + m + r) * LS_P + o + cc] = -acc;
+        __syncthreads();
+      }
+    }
+    for(int e = tid; e < nSlot * 128; e += LS_THREADS)
+      __stcg((double2*)(Yg + (size_t)((e >> 7) * CL + rank) * 256) + (e & 127),
+             ((const double2*)(keep + (size_t)(e >> 7) * 256))[e & 127]);
+    if(rank == 0)  // D^-1 L^-1 rhs: the right-hand side's scaled row
+      for(int k = tid; k < nPad; k += LS_THREADS) __stcg(Yg + (size_t)LS_P * nPad + k, rhsRow[k]);
+    cluster.sync();
+    for(int e = tid; e < nP * 128; e += LS_THREADS) ((double2*)Y)[e] = __ldcg((const double2*)Yg + e);
+    for(int k = tid; k < nPad; k += LS_THREADS) wv[k] = __ldcg(Yg + (size_t)LS_P * nPad + k);
+    __syncthreads();
+  }
+  const double* Li = Y;
+
+  // A 16 x 16 product in 128 threads (warps 0-3): out[c] = sum_k m(c, k) v[k],
+  // eight threads per c with two terms each.
+  auto block16 = [&](auto mat, const double* v) -> double {
+    const int c = tid >> 3, k = tid & 7;
+    double s = mat(c, k) * v[k];
+    s = fma(mat(c, k + 8), v[k + 8], s);
+    s += __shfl_xor_sync(0xffffffffu, s, 4);
+    s += __shfl_xor_sync(0xffffffffu, s, 2);
+    s += __shfl_xor_sync(0xffffffffu, s, 1);
+    return s;
+  };
+
+  // L^T x = wv into xg, panels from the bottom.
+  auto backward = [&]() {
+    for(int k = tid; k < G * nPad; k += LS_THREADS) sPart[k] = 0.0;
+    __syncthreads();
+    for(int p = nP - 1; p >= 0; p--) {
+      const int K = p * LS_P;
+      double* sb = SB + (p & 1) * LS_P * LS_SB;
+      // this panel's partial sums, the panel below applied, to every CTA
+      if(tid < 128) {
+        if(tid < LS_P * G) {
+          const int g = tid >> 4, c = tid & 15;
+          double v = sPart[g * nPad + K + c];
+          if(p + 1 < nP) {
+            const int lr = (p + 1) * G + g;
+            v = fma(rowPtr(lr)[K + c], xg[lr * CL + rank], v);
+          }
+          tv[tid] = v;
         }
-        part[warp * 32 + lane] = acc;
+        barSome(128);
+        push(tv, sb, LS_SB);
       }
-    } else {
-      for(int i = s2 + SV_NB + (tid - SV_AW * 32); i <= n; i += SV_THREADS - SV_AW * 32)
-        x[i] -= rowDot(F, ld, s, nb, i, x);
-    }
-    __syncthreads();
-    if(warp == 0 && nb2 > 0 && lane < nb2)
-      x[s2 + lane] -= (part[lane] + part[32 + lane]) + (part[64 + lane] + part[96 + lane]);
-    __syncthreads();
-  }
-  for(int i = 1 + tid; i <= n; i += SV_THREADS) x[i] *= rinv[i];
-  __syncthreads();
-  // ---- backward: L^T x = z, blocks from the bottom; (Linv_K)^T on the block
-  for(int K = nB - 1; K >= 0; K--) {
-    const int s = 1 + K * SV_NB, nb = min(SV_NB, n + 1 - s);
-    const double* Lk = Li + (size_t)K * SV_NB * SV_NB;
-    if(warp < SV_AW) {
-      double acc = 0.0;
-#pragma unroll
-      for(int u = 0; u < SV_NB / SV_AW; u++) {
-        const int t = warp * (SV_NB / SV_AW) + u;
-        if(t < nb) acc = fma(Lk[t * SV_NB + lane], x[s + t], acc);
-      }
-      part[warp * 32 + lane] = acc;
-    }
-    __syncthreads();
-    if(warp == 0 && lane < nb)
-      x[s + lane] = (part[lane] + part[32 + lane]) + (part[64 + lane] + part[96 + lane]);
-    __syncthreads();
-    const int s2 = s - SV_NB;  // previous block (full size)
-    if(warp < SV_AW) {
-      if(K > 0) {
-        double acc = 0.0;
-#pragma unroll
-        for(int u = 0; u < SV_NB / SV_AW; u++) {
-          const int t = warp * (SV_NB / SV_AW) + u;  // row s+t of L, column s2+lane
-          if(t < nb) acc = fma(F[(size_t)(s + t) * ld + s2 + lane], x[s + t], acc);
+      clusterArrive();
+      if(p + 1 < nP)
+        for(int k = tid; k < G * K; k += LS_THREADS) {  // the panels further up
+          const int g = G == 1 ? 0 : k / K, j = G == 1 ? k : k - g * K;
+          const int lr = (p + 1) * G + g;
+          sPart[g * nPad + j] = fma(rowPtr(lr)[j], xg[lr * CL + rank], sPart[g * nPad + j]);
         }
-        part[warp * 32 + lane] = acc;
+      clusterWait();
+      if(tid < 128) {
+        const int c = tid >> 3, k = tid & 7;
+        double s = sb[k * LS_SB + c] + sb[(k + 8) * LS_SB + c];
+        s += __shfl_xor_sync(0xffffffffu, s, 4);
+        s += __shfl_xor_sync(0xffffffffu, s, 2);
+        s += __shfl_xor_sync(0xffffffffu, s, 1);
+        if(k == 0) tv[c] = wv[K + c] - s;
+        barSome(128);
+        const double* L = Li + (size_t)p * 256;
+        const double x = block16([&](int cc, int kk) { return L[kk * LS_P + cc]; }, tv);
+        if(k == 0) xg[K + c] = x;
       }
-    } else {
-      for(int k = 1 + (tid - SV_AW * 32); k < s2; k += SV_THREADS - SV_AW * 32)
-        x[k] -= rowDot(F, ld, s, nb, k, x);
+      __syncthreads();
     }
-    __syncthreads();
-    if(warp == 0 && K > 0)
-      x[s2 + lane] -= (part[lane] + part[32 + lane]) + (part[64 + lane] + part[96 + lane]);
-    __syncthreads();
-  }
-}
+  };
+  // L y = (own parts in accv) and wv <- D^-1 y, panels from the top.
+  auto forward = [&]() {
+    for(int p = 0; p < nP; p++) {
+      const int K = p * LS_P;
+      double* fb = FB + (p & 1) * LS_P;
+      if(tid < CL * G) {
+        const int g = tid / CL, d = tid % CL;
+        cluster.map_shared_rank(fb, d)[g * CL + rank] = accv[p * G + g];
+      }
+      clusterArrive();
+      clusterWait();
+      if(tid < 128) {
+        const double* L = Li + (size_t)p * 256;
+        const double y = block16([&](int cc, int kk) { return L[cc * LS_P + kk]; }, fb);
+        if((tid & 7) == 0) {
+          yv[K + (tid >> 3)] = y;
+          wv[K + (tid >> 3)] = y * dinv[K + (tid >> 3)];
+        }
+      }
+      __syncthreads();
+      // own rows below the panel, eight threads per row
+      const int lr0 = (p + 1) * G;
+      for(int r0 = lr0; r0 < nr; r0 += LS_THREADS / 8) {
+        const int lr = r0 + (tid >> 3), k = tid & 7;
+        double s = 0.0;
+        if(lr < nr) {
+          const double* l = rowPtr(lr) + K;
+          s = l[k] * yv[K + k];
+          s = fma(l[k + 8], yv[K + k + 8], s);
+        }
+        s += __shfl_xor_sync(0xffffffffu, s, 4);
+        s += __shfl_xor_sync(0xffffffffu, s, 2);
+        s += __shfl_xor_sync(0xffffffffu, s, 1);
+        if(lr < nr && k == 0) accv[lr] -= s;
+      }
+      __syncthreads();
+    }
+  };
 
-}  // namespace
-
-// Inverses of the diagonal blocks of L, one CTA per block (Linv: global,
-// ceil(n/32) x 32 x 32).  With status bit 0 set the pivoted LU solves the
-// system instead and the kernel returns at once.
-__global__ void __launch_bounds__(SV_THREADS)
-    k_ldl_block_inv(const double* __restrict__ F, int n, const int* __restrict__ status,
-                    double* __restrict__ Linv) {
-  __shared__ double X[SV_NB * (SV_NB + 1)];
-  __shared__ double T[256];
-  if(status[0] & 1) return;
-  invertDiagBlock(F, n, blockIdx.x, X, T, Linv);
-}
-
-// One triangular-solve pass of the refined solve, on one CTA (the pivot
-// chain is sequential; no other SM waits on it).  first = 1: x1 = (L D L^T)^-1
-// rhs into x1g.  first = 0: x2 = (L D L^T)^-1 res and rhs <- x1g + x2.
-// With status bit 0 set the pivoted LU solves the system instead.
-__global__ void __launch_bounds__(SV_THREADS)
-    k_ldl_solve(const double* __restrict__ F, const double* __restrict__ rinv, int n,
-                double* __restrict__ rhs, const double* __restrict__ res,
-                double* __restrict__ x1g, const int* __restrict__ status,
-                const double* __restrict__ Linv, int first) {
-  extern __shared__ __align__(16) double sv_s[];
-  const int tid = threadIdx.x;
-  const int LX = (n + 2) & ~1, nB = (n + SV_NB - 1) / SV_NB;
-  double* x = sv_s;                  // LX
-  double* part = x + LX;             // SV_AW x 32
-  double* Li = part + SV_AW * 32;    // nB x 32 x 32
-  if(status[0] & 1) return;  // the LU fallback solves this system
-  for(int e = tid; e < nB * SV_NB * SV_NB; e += SV_THREADS) Li[e] = Linv[e];
-  const double* src = first ? rhs : res;
-  for(int i = tid; i < LX; i += SV_THREADS) x[i] = i >= 1 && i <= n ? src[i] : 0.0;
+  backward();
+  for(int k = tid; k < nPad; k += LS_THREADS) x1[k] = xg[k];
   __syncthreads();
-  ldlSolveCta(F, rinv, n, Li, x, part);
-  if(first) {
-    for(int i = tid; i < LX; i += SV_THREADS) x1g[i] = x[i];
-  } else {
-    for(int i = 1 + tid; i <= n; i += SV_THREADS) rhs[i] = x1g[i] + x[i];
-  }
-}
-
-// Residual of the first pass, res_i = rhs_i - A_i . x1, one row per warp
-// (lane-strided FMA chain, loads issued ahead, xor-shuffle sum) over
-// ceil(n / 16) CTAs: FP64 runs at ~1.7 FMA per clock per SM on this part, so
-// the n^2 products are spread over SMs.
-__global__ void __launch_bounds__(SV_THREADS)
-    k_ldl_residual(const double* __restrict__ A, int n, const double* __restrict__ rhs,
-                   const double* __restrict__ x1g, const int* __restrict__ status,
-                   double* __restrict__ res) {
-  if(status[0] & 1) return;
-  constexpr int NW = SV_THREADS / 32, RU = 8;
-  const int lane = threadIdx.x & 31, ld = n + 1;
-  const int i = 1 + blockIdx.x * NW + (threadIdx.x >> 5);
-  if(i > n) return;
-  double a = 0.0;
-  for(int j0 = 1 + lane; j0 <= n; j0 += 32 * RU) {
-    double av[RU], xv[RU];
+  // residual of the own rows against M, one warp per row
+  for(int lr = warp; lr < nr; lr += LS_THREADS / 32) {
+    const int i = lr * CL + rank;
+    double s = 0.0;
+    if(i < n) {
+      const double* row = M + (size_t)(i + 1) * ld + 1;
+      constexpr int RU = 10;
+      for(int j0 = lane; j0 < n; j0 += 32 * RU) {
+        double av[RU];
 #pragma unroll
-    for(int u = 0; u < RU; u++) {
-      const int j = j0 + 32 * u;
-      av[u] = j <= n ? A[(size_t)i * ld + j] : 0.0;
-      xv[u] = j <= n ? x1g[j] : 0.0;
+        for(int u = 0; u < RU; u++) av[u] = j0 + 32 * u < n ? row[j0 + 32 * u] : 0.0;
+#pragma unroll
+        for(int u = 0; u < RU; u++)
+          if(j0 + 32 * u < n) s = fma(av[u], x1[j0 + 32 * u], s);
+      }
     }
 #pragma unroll
-    for(int u = 0; u < RU; u++)
-      if(j0 + 32 * u <= n) a = fma(av[u], xv[u], a);
+    for(int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+    if(lane == 0) accv[lr] = i < n ? rhs[i + 1] - s : 0.0;
   }
-#pragma unroll
-  for(int o = 16; o > 0; o >>= 1) a += __shfl_xor_sync(0xffffffffu, a, o);
-  if(lane == 0) res[i] = rhs[i] - a;
-}
-
-template __global__ void k_global_ldl<8>(const double*, double*, double*, int, int*);
-template __global__ void k_global_ldl_panel<16, 2>(const double*, double*, double*, int, int, int*);
-template __global__ void k_global_ldl_panel<16, 4>(const double*, double*, double*, int, int, int*);
-template __global__ void k_global_ldl_panel<16, 8>(const double*, double*, double*, int, int, int*);
-template __global__ void k_global_ldl_panel<8, 2>(const double*, double*, double*, int, int, int*);
-template __global__ void k_global_ldl_panel<8, 4>(const double*, double*, double*, int, int, int*);
-template __global__ void k_global_ldl_panel<8, 8>(const double*, double*, double*, int, int, int*);
-template __global__ void k_global_ldl<16>(const double*, double*, double*, int, int*);
-
-namespace {
-
-size_t ldlSmemBytes(int n, int CL) {
-  const int LC = (n + 3) & ~1, ncol = (n + CL - 1) / CL;
-  return ((size_t)ncol * LC + (size_t)LDL_RING * LC + LC) * sizeof(double) +
-         (LDL_RING + 1) * sizeof(unsigned long long);
-}
-
-// Shared memory of the panel kernel: the owned panels, the receive ring, the
-// pivots and the barriers.
-size_t ldlPanelSmemBytes(int n, int CL, int P, int ring) {
-  const int LC = (n + 3) & ~1, nP = (n + P - 1) / P, lpn = (nP + CL - 1) / CL;
-  return ((size_t)lpn * P * LC + (size_t)ring * P * LC + LC) * sizeof(double) +
-         (size_t)(ring + 1) * sizeof(unsigned long long);
+  __syncthreads();
+  forward();
+  backward();
+  cluster.sync();  // every CTA has read rhs, and no remote store is pending
+  if(rank == 0)
+    for(int k = tid; k < n; k += LS_THREADS) rhs[k + 1] = x1[k] + xg[k];
 }
 
 template <class Kern, class... Args>
@@ -761,89 +580,31 @@ void globalSolveMixed(xb_ctx* c, const double* M, int n, double* rhs, int* piv, 
   const int ld = n + 1;
   int* status = deviceStatus(c);
   XB_CUDA(cudaMemsetAsync(status, 0, sizeof(int), c->stream));
-  double* F = buf<double>(c, "ldl_F", (size_t)ld * ld);
-  double* rinv = buf<double>(c, "ldl_rinv", ld);
-  // 16-CTA clusters where the device allows them, else 8
+  // 16-CTA clusters where the device allows them and the context asks for
+  // them, else 8 (the same bits)
   static std::atomic<int> clusterSize{0};
   {
-    // Variants with the same factors bit for bit: the column kernel (0) and
-    // panels of 2, 4 or 8 columns (1-3), where shared memory holds a receive
-    // ring of at least two panels.  Wider panels need fewer cluster-wide
-    // exchanges but put more FP64 work on the owner of the next panel (the
-    // look-ahead), so the autotuner times them.
-    int maxSmem = 0;
-    XB_CUDA(cudaDeviceGetAttribute(&maxSmem, cudaDevAttrMaxSharedMemoryPerBlockOptin, c->device));
-    auto ringFor = [&](int CL, int P) {
-      for(int rg = std::min(4, CL); rg >= 2; rg--)
-        if(ldlPanelSmemBytes(n, CL, P, rg) <= (size_t)maxSmem) return rg;
-      return 0;
-    };
-    auto launchVariant = [&](int v, int CL) -> cudaError_t {
-      const int P = v == 1 ? 2 : v == 2 ? 4 : 8;
-      const int rg = v > 0 ? ringFor(CL, P) : 0;
-      if(v == 0 || rg == 0)
-        return CL == 16 ? launchCluster(c, k_global_ldl<16>, 16, LDL_THREADS, ldlSmemBytes(n, 16),
-                                        M, F, rinv, n, status)
-                        : launchCluster(c, k_global_ldl<8>, 8, LDL_THREADS, ldlSmemBytes(n, 8), M,
-                                        F, rinv, n, status);
-      const size_t sm = ldlPanelSmemBytes(n, CL, P, rg);
-      if(CL == 16)
-        return P == 2 ? launchCluster(c, k_global_ldl_panel<16, 2>, 16, LDL_THREADS, sm, M, F, rinv,
-                                      n, rg, status)
-             : P == 4 ? launchCluster(c, k_global_ldl_panel<16, 4>, 16, LDL_THREADS, sm, M, F, rinv,
-                                      n, rg, status)
-                      : launchCluster(c, k_global_ldl_panel<16, 8>, 16, LDL_THREADS, sm, M, F, rinv,
-                                      n, rg, status);
-      return P == 2 ? launchCluster(c, k_global_ldl_panel<8, 2>, 8, LDL_THREADS, sm, M, F, rinv, n,
-                                    rg, status)
-           : P == 4 ? launchCluster(c, k_global_ldl_panel<8, 4>, 8, LDL_THREADS, sm, M, F, rinv, n,
-                                    rg, status)
-                    : launchCluster(c, k_global_ldl_panel<8, 8>, 8, LDL_THREADS, sm, M, F, rinv, n,
-                                    rg, status);
-    };
-    // 16-CTA clusters where the device allows them and the context asks for
-    // them, else 8
-    auto launch = [&](int v) {
-      cudaError_t e = cudaErrorUnknown;
-      if(clusterSize.load() != 8 && c->ldlCluster == 16) {
-        e = launchVariant(v, 16);
-        if(e == cudaSuccess) clusterSize = 16;
-        else cudaGetLastError();
-      }
-      if(e != cudaSuccess) {
-        XB_CUDA(launchVariant(v, 8));
-        if(c->ldlCluster == 16) clusterSize = 8;
-      }
-      XB_LAUNCHED(c);
-    };
-    const int v = c->ldlPanel ? tunedVariant(c, "global_ldl", (long long)n * 32 + c->ldlCluster, 4,
-                                             launch)
-                              : 0;
     KT_SCOPE(c, "global_ldl");
-    launch(v);
-  }
-  luFallbackSolve(c, M, F, n, rhs, piv, singular, status);
-  {
-    KT_SCOPE(c, "global_solve");
-    const int nB = (n + SV_NB - 1) / SV_NB;
-    double* Linv = buf<double>(c, "ldl_linv", (size_t)nB * SV_NB * SV_NB);
-    const size_t smem =
-        ((size_t)((n + 2) & ~1) + SV_AW * 32 + (size_t)nB * SV_NB * SV_NB) * sizeof(double);
-    double* x1g = buf<double>(c, "ldl_x1", (size_t)n + 2);
-    double* res = buf<double>(c, "ldl_res", (size_t)n + 2);
-    k_ldl_block_inv<<<nB, SV_THREADS, 0, c->stream>>>((const double*)F, n, (const int*)status, Linv);
-    XB_LAUNCHED(c);
-    XB_CUDA(allowMaxDynamicSmem((const void*)k_ldl_solve, c->device));
-    k_ldl_solve<<<1, SV_THREADS, smem, c->stream>>>((const double*)F, (const double*)rinv, n, rhs,
-                                                    res, x1g, (const int*)status, Linv, 1);
-    XB_LAUNCHED(c);
-    k_ldl_residual<<<(n + SV_THREADS / 32 - 1) / (SV_THREADS / 32), SV_THREADS, 0, c->stream>>>(
-        (const double*)M, n, rhs, x1g, (const int*)status, res);
-    XB_LAUNCHED(c);
-    k_ldl_solve<<<1, SV_THREADS, smem, c->stream>>>((const double*)F, (const double*)rinv, n, rhs,
-                                                    res, x1g, (const int*)status, Linv, 0);
+    double* Yg = buf<double>(c, "ldl_y", (size_t)(LS_P + 1) * lsLayout(n, 16).nPad);
+    auto launch = [&](auto kernel, int CL) -> cudaError_t {
+      const LsLayout lay = lsLayout(n, CL);
+      if(lay.nr + 1 > LS_OWN) return cudaErrorInvalidConfiguration;
+      return launchCluster(c, kernel, CL, LS_THREADS, lay.doubles() * sizeof(double), M, rhs, n, Yg,
+                           status);
+    };
+    cudaError_t e = cudaErrorUnknown;
+    if(clusterSize.load() != 8 && c->ldlCluster == 16) {
+      e = launch(k_ldl_factor_solve<16>, 16);
+      if(e == cudaSuccess) clusterSize = 16;
+      else cudaGetLastError();
+    }
+    if(e != cudaSuccess) {
+      XB_CUDA(launch(k_ldl_factor_solve<8>, 8));
+      if(c->ldlCluster == 16) clusterSize = 8;
+    }
     XB_LAUNCHED(c);
   }
+  luFallbackSolve(c, M, buf<double>(c, "ldl_F", (size_t)ld * ld), n, rhs, piv, singular, status);
 }
 
 void checkSolveTimeout(xb_ctx* c) {
