@@ -22,7 +22,7 @@
 //   head  [pool 8, mlp 32] -> 1 logit (accept probability = sigmoid)
 // Training: binary cross-entropy with per-sample weights; one CTA computes
 // the forward pass, the loss and the gradient of one sample; the gradients
-// are summed over the batch in sample order (deterministic) and Adam updates
+// are summed over the batch in a fixed order (deterministic) and Adam updates
 // the parameters.  Everything runs on the GPU from the C ABI.
 
 #include <algorithm>
@@ -39,7 +39,7 @@ namespace xb {
 
 namespace {
 
-constexpr int RK_T = 128;  // threads per sample
+constexpr int RK_T = 128;  // threads per candidate (features)
 constexpr int RK_WIN = 31, RK_HWIN = 15, RK_NS = 16, RK_C = 8, RK_H = 32;
 constexpr int RK_S1 = 14, RK_S2 = 6, RK_S3 = 4;
 constexpr int RK_PIX = 2 * RK_WIN * RK_WIN;
@@ -57,248 +57,511 @@ __device__ __forceinline__ float rkWeight(const float* W, int q) {
 }
 __device__ __forceinline__ float rkWeight(const __nv_bfloat16* W, int q) { return __bfloat162float(W[q]); }
 
-// Activations of one sample (shared memory).
-struct RkAct {
-  float in[RK_PIX];
-  float a1[RK_C * RK_S1 * RK_S1];  // post-ReLU
-  float a2[RK_C * RK_S2 * RK_S2];
-  float a3[RK_C * RK_S3 * RK_S3];
-  float st[RK_NS];
-  float hid[RK_C + RK_H];          // [pool, mlp] (post-ReLU)
-  float logit;
-};
+// ------------------------------------------------------------------ forward --
+// Two warps per sample.  The 109k multiply-adds of a sample are bound by the
+// FP32 pipe only where each value read from shared memory feeds several of
+// them: conv1 keeps 7 outputs of a row x 4 channels per lane (140 FMAs per 17
+// window values and 5 broadcast float4 of weights), conv2 6 outputs of one
+// channel, conv3 2.  Every output is summed in the order bias, input channel,
+// row, column, so the logits are those of one thread per output (whose two
+// shared reads per FMA took 101 us for 2000 samples on a GB300; this form takes
+// 27 us).  24 warps per SM hide the latencies of the short layers; one warp
+// per sample with all 8 channels had half of them and took 53 us.
+constexpr int RF_SAMPLES = 4;           // samples per CTA
+constexpr int RF_T = 64 * RF_SAMPLES;
+constexpr int RF_LD = 35;               // window row: columns 0..16, then 14..30, and a pad
+constexpr int RF_IN = RK_WIN * RF_LD;   // one image of the pair
+constexpr int RF_A2 = RK_C * RK_S2 * RK_S2, RF_A3 = RK_C * RK_S3 * RK_S3;
+constexpr int RF_A1 = RK_C * RK_S1 * RK_S1;
+constexpr int RF_BUF = 2 * RF_IN + RF_A1 + 2;  // floats per sample
+static_assert(RF_BUF % 4 == 0, "16-byte rows");
+// weights with the output channel innermost
+constexpr int RW_1 = 0, RW_2 = RW_1 + 400, RW_3 = RW_2 + 576, RW_M = RW_3 + 576,
+              RW_B1 = RW_M + RK_H * RK_NS, RW_B2 = RW_B1 + 8, RW_B3 = RW_B2 + 8,
+              RW_BM = RW_B3 + 8, RW_H = RW_BM + RK_H, RW_HB = RW_H + RK_C + RK_H, RW_N = RW_HB + 4;
+constexpr size_t RF_SMEM = (size_t)(RW_N + RF_SAMPLES * RF_BUF) * sizeof(float);
 
-__device__ float rkForward(const float* __restrict__ W, RkAct& A) {
-  const int tid = threadIdx.x;
-  for(int o = tid; o < RK_C * RK_S1 * RK_S1; o += RK_T) {
-    const int c = o / (RK_S1 * RK_S1), y = (o / RK_S1) % RK_S1, x = o % RK_S1;
-    float v = W[O_C1B + c];
-    for(int ci = 0; ci < 2; ci++)
-      for(int ky = 0; ky < 5; ky++)
-        for(int kx = 0; kx < 5; kx++)
-          v = fmaf(W[O_C1W + ((c * 2 + ci) * 5 + ky) * 5 + kx],
-                   A.in[(ci * RK_WIN + 2 * y + ky) * RK_WIN + 2 * x + kx], v);
-    A.a1[o] = fmaxf(v, 0.f);
-  }
-  __syncthreads();
-  for(int o = tid; o < RK_C * RK_S2 * RK_S2; o += RK_T) {
-    const int c = o / (RK_S2 * RK_S2), y = (o / RK_S2) % RK_S2, x = o % RK_S2;
-    float v = W[O_C2B + c];
-    for(int ci = 0; ci < RK_C; ci++)
-      for(int ky = 0; ky < 3; ky++)
-        for(int kx = 0; kx < 3; kx++)
-          v = fmaf(W[O_C2W + ((c * RK_C + ci) * 3 + ky) * 3 + kx],
-                   A.a1[(ci * RK_S1 + 2 * y + ky) * RK_S1 + 2 * x + kx], v);
-    A.a2[o] = fmaxf(v, 0.f);
-  }
-  __syncthreads();
-  for(int o = tid; o < RK_C * RK_S3 * RK_S3; o += RK_T) {
-    const int c = o / (RK_S3 * RK_S3), y = (o / RK_S3) % RK_S3, x = o % RK_S3;
-    float v = W[O_C3B + c];
-    for(int ci = 0; ci < RK_C; ci++)
-      for(int ky = 0; ky < 3; ky++)
-        for(int kx = 0; kx < 3; kx++)
-          v = fmaf(W[O_C3W + ((c * RK_C + ci) * 3 + ky) * 3 + kx],
-                   A.a2[(ci * RK_S2 + y + ky) * RK_S2 + x + kx], v);
-    A.a3[o] = fmaxf(v, 0.f);
-  }
-  for(int j = tid; j < RK_H; j += RK_T) {
-    float v = W[O_M1B + j];
-    for(int i = 0; i < RK_NS; i++) v = fmaf(W[O_M1W + j * RK_NS + i], A.st[i], v);
-    A.hid[RK_C + j] = fmaxf(v, 0.f);
-  }
-  __syncthreads();
-  if(tid < RK_C) {
-    float v = 0.f;
-    for(int p = 0; p < RK_S3 * RK_S3; p++) v += A.a3[tid * RK_S3 * RK_S3 + p];
-    A.hid[tid] = v * (1.f / (RK_S3 * RK_S3));
-  }
-  __syncthreads();
-  if(tid == 0) {
-    float z = W[O_HB];
-    for(int i = 0; i < RK_C + RK_H; i++) z = fmaf(W[O_HW + i], A.hid[i], z);
-    A.logit = z;
-  }
-  __syncthreads();
-  return A.logit;
+__device__ __forceinline__ int rwIndex(int q) {
+  if(q < O_C1B) return RW_1 + (q % 50) * 8 + q / 50;
+  if(q < O_C2W) return RW_B1 + q - O_C1B;
+  if(q < O_C2B) return RW_2 + ((q - O_C2W) % 72) * 8 + (q - O_C2W) / 72;
+  if(q < O_C3W) return RW_B2 + q - O_C2B;
+  if(q < O_C3B) return RW_3 + ((q - O_C3W) % 72) * 8 + (q - O_C3W) / 72;
+  if(q < O_M1W) return RW_B3 + q - O_C3B;
+  if(q < O_M1B) return RW_M + ((q - O_M1W) % RK_NS) * RK_H + (q - O_M1W) / RK_NS;
+  if(q < O_HW) return RW_BM + q - O_M1B;
+  return RW_H + q - O_HW;  // head weights, then its bias
 }
 
-// Gradient of loss = sw * BCE(sigmoid(z), y) with respect to every
-// parameter, written to g (RK_NP floats).  Uses the activations of rkForward.
-struct RkGrad {
-  float dz;
-  float dh[RK_C + RK_H];
-  float d3[RK_C * RK_S3 * RK_S3];  // dL/d(conv3 pre-activation)
-  float d2[RK_C * RK_S2 * RK_S2];  // dL/d(conv2 pre-activation)
-  float d1[RK_C * RK_S1 * RK_S1];  // dL/d(conv1 pre-activation)
-};
-
-__device__ void rkBackward(const float* __restrict__ W, const RkAct& A, RkGrad& D, float y,
-                           float sw, float* __restrict__ g) {
-  const int tid = threadIdx.x;
-  if(tid == 0) {
-    const float p = 1.f / (1.f + expf(-A.logit));
-    D.dz = sw * (p - y);
-  }
-  __syncthreads();
-  const float dz = D.dz;
-  for(int i = tid; i < RK_C + RK_H; i += RK_T) {
-    g[O_HW + i] = dz * A.hid[i];
-    D.dh[i] = dz * W[O_HW + i];
-  }
-  if(tid == 0) g[O_HB] = dz;
-  __syncthreads();
-  // mlp
-  for(int j = tid; j < RK_H; j += RK_T) {
-    const float dp = A.hid[RK_C + j] > 0.f ? D.dh[RK_C + j] : 0.f;
-    g[O_M1B + j] = dp;
-    for(int i = 0; i < RK_NS; i++) g[O_M1W + j * RK_NS + i] = dp * A.st[i];
-  }
-  // pool -> conv3 pre-activation
-  for(int o = tid; o < RK_C * RK_S3 * RK_S3; o += RK_T) {
-    const int c = o / (RK_S3 * RK_S3);
-    D.d3[o] = A.a3[o] > 0.f ? D.dh[c] * (1.f / (RK_S3 * RK_S3)) : 0.f;
-  }
-  __syncthreads();
-  // conv3 weights / bias
-  for(int q = tid; q < RK_C * RK_C * 9 + RK_C; q += RK_T) {
-    if(q < RK_C * RK_C * 9) {
-      const int c = q / (RK_C * 9), ci = (q / 9) % RK_C, ky = (q / 3) % 3, kx = q % 3;
-      float v = 0.f;
-      for(int y = 0; y < RK_S3; y++)
-        for(int x = 0; x < RK_S3; x++)
-          v = fmaf(D.d3[(c * RK_S3 + y) * RK_S3 + x], A.a2[(ci * RK_S2 + y + ky) * RK_S2 + x + kx], v);
-      g[O_C3W + q] = v;
-    } else {
-      const int c = q - RK_C * RK_C * 9;
-      float v = 0.f;
-      for(int p = 0; p < RK_S3 * RK_S3; p++) v += D.d3[c * RK_S3 * RK_S3 + p];
-      g[O_C3B + c] = v;
-    }
-  }
-  // conv2 pre-activation
-  for(int o = tid; o < RK_C * RK_S2 * RK_S2; o += RK_T) {
-    const int ci = o / (RK_S2 * RK_S2), yy = (o / RK_S2) % RK_S2, xx = o % RK_S2;
-    float v = 0.f;
-    if(A.a2[o] > 0.f)
-      for(int c = 0; c < RK_C; c++)
-        for(int ky = 0; ky < 3; ky++)
-          for(int kx = 0; kx < 3; kx++) {
-            const int y = yy - ky, x = xx - kx;
-            if(y < 0 || y >= RK_S3 || x < 0 || x >= RK_S3) continue;
-            v = fmaf(D.d3[(c * RK_S3 + y) * RK_S3 + x], W[O_C3W + ((c * RK_C + ci) * 3 + ky) * 3 + kx], v);
-          }
-    D.d2[o] = v;
-  }
-  __syncthreads();
-  for(int q = tid; q < RK_C * RK_C * 9 + RK_C; q += RK_T) {
-    if(q < RK_C * RK_C * 9) {
-      const int c = q / (RK_C * 9), ci = (q / 9) % RK_C, ky = (q / 3) % 3, kx = q % 3;
-      float v = 0.f;
-      for(int y = 0; y < RK_S2; y++)
-        for(int x = 0; x < RK_S2; x++)
-          v = fmaf(D.d2[(c * RK_S2 + y) * RK_S2 + x],
-                   A.a1[(ci * RK_S1 + 2 * y + ky) * RK_S1 + 2 * x + kx], v);
-      g[O_C2W + q] = v;
-    } else {
-      const int c = q - RK_C * RK_C * 9;
-      float v = 0.f;
-      for(int p = 0; p < RK_S2 * RK_S2; p++) v += D.d2[c * RK_S2 * RK_S2 + p];
-      g[O_C2B + c] = v;
-    }
-  }
-  // conv1 pre-activation
-  for(int o = tid; o < RK_C * RK_S1 * RK_S1; o += RK_T) {
-    const int ci = o / (RK_S1 * RK_S1), yy = (o / RK_S1) % RK_S1, xx = o % RK_S1;
-    float v = 0.f;
-    if(A.a1[o] > 0.f)
-      for(int c = 0; c < RK_C; c++)
-        for(int ky = 0; ky < 3; ky++)
-          for(int kx = 0; kx < 3; kx++) {
-            const int ty = yy - ky, tx = xx - kx;  // = 2y, 2x
-            if(ty < 0 || tx < 0 || (ty & 1) || (tx & 1)) continue;
-            const int y = ty >> 1, x = tx >> 1;
-            if(y >= RK_S2 || x >= RK_S2) continue;
-            v = fmaf(D.d2[(c * RK_S2 + y) * RK_S2 + x], W[O_C2W + ((c * RK_C + ci) * 3 + ky) * 3 + kx], v);
-          }
-    D.d1[o] = v;
-  }
-  __syncthreads();
-  for(int q = tid; q < RK_C * 2 * 25 + RK_C; q += RK_T) {
-    if(q < RK_C * 2 * 25) {
-      const int c = q / 50, ci = (q / 25) % 2, ky = (q / 5) % 5, kx = q % 5;
-      float v = 0.f;
-      for(int y = 0; y < RK_S1; y++)
-        for(int x = 0; x < RK_S1; x++)
-          v = fmaf(D.d1[(c * RK_S1 + y) * RK_S1 + x], A.in[(ci * RK_WIN + 2 * y + ky) * RK_WIN + 2 * x + kx], v);
-      g[O_C1W + q] = v;
-    } else {
-      const int c = q - RK_C * 2 * 25;
-      float v = 0.f;
-      for(int p = 0; p < RK_S1 * RK_S1; p++) v += D.d1[c * RK_S1 * RK_S1 + p];
-      g[O_C1B + c] = v;
-    }
-  }
+__device__ __forceinline__ void cpAsync4(float* dst, const float* src) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(
+                   (unsigned)__cvta_generic_to_shared(dst)),
+               "l"(src)
+               : "memory");
+}
+__device__ __forceinline__ void cpAsyncWait() {
+  asm volatile("cp.async.wait_all;" ::: "memory");
+}
+// Barrier of the two warps of sample slot s.
+__device__ __forceinline__ void pairSync(int s) {
+  asm volatile("bar.sync %0, 64;" ::"r"(s + 1) : "memory");
 }
 
-__device__ __forceinline__ void rkLoad(const float* __restrict__ stats, const float* __restrict__ pix,
-                                       int i, RkAct& A) {
-  for(int q = threadIdx.x; q < RK_PIX; q += RK_T) A.in[q] = pix[(size_t)i * RK_PIX + q];
-  for(int q = threadIdx.x; q < RK_NS; q += RK_T) A.st[q] = stats[(size_t)i * RK_NS + q];
+// Logit of one sample by the two warps (half 0 and 1) of slot s; the lanes of
+// half 0 return it.
+__device__ float rfSample(const float* __restrict__ Wt, const float* __restrict__ stats,
+                          const float* __restrict__ pix, float* __restrict__ buf, int s, int half) {
+  const int lane = threadIdx.x & 31;
+  float* in = buf;
+  float* a1 = buf + 2 * RF_IN;
+  float* a2 = buf;                // over the window, which is spent after conv1
+  float* a3 = buf + RF_A2;
+  float* hid = a3 + RF_A3;
+  pairSync(s);  // the sample before is done
+  if(lane < RK_WIN) {
+    const float* src = pix + half * RK_WIN * RK_WIN + lane;
+    float* dst = in + half * RF_IN + lane;
+#pragma unroll 4
+    for(int r = 0; r < RK_WIN; r++) {  // four-byte copies: any alignment of the caller's array
+      if(lane < 17) cpAsync4(dst + r * RF_LD, src + r * RK_WIN);
+      if(lane >= 14) cpAsync4(dst + r * RF_LD + 3, src + r * RK_WIN);
+    }
+  }
+  const float st = lane < RK_NS ? stats[lane] : 0.f;
+  cpAsyncWait();
+  pairSync(s);
+  if(lane < 2 * RK_S1) {
+    const int y = lane >> 1, h = lane & 1;
+    float acc[7][4];
+#pragma unroll
+    for(int c = 0; c < 4; c++)
+#pragma unroll
+      for(int k = 0; k < 7; k++) acc[k][c] = Wt[RW_B1 + 4 * half + c];
+#pragma unroll 1
+    for(int r = 0; r < 10; r++) {
+      const int ci = r / 5, ky = r - 5 * ci;
+      const float* row = in + ci * RF_IN + (2 * y + ky) * RF_LD + 17 * h;
+      float x[17];
+#pragma unroll
+      for(int k = 0; k < 17; k++) x[k] = row[k];
+      const float4* w4 = (const float4*)(Wt + RW_1 + r * 40) + half;
+#pragma unroll
+      for(int kx = 0; kx < 5; kx++) {
+        const float4 wv = w4[2 * kx];
+        const float w[4] = {wv.x, wv.y, wv.z, wv.w};
+#pragma unroll
+        for(int k = 0; k < 7; k++)
+#pragma unroll
+          for(int c = 0; c < 4; c++) acc[k][c] = fmaf(w[c], x[2 * k + kx], acc[k][c]);
+      }
+    }
+#pragma unroll
+    for(int c = 0; c < 4; c++)
+#pragma unroll
+      for(int k = 0; k < 7; k++)
+        a1[((4 * half + c) * RK_S1 + y) * RK_S1 + 7 * h + k] = fmaxf(acc[k][c], 0.f);
+  }
+  pairSync(s);
+  if(lane < 4 * RK_S2) {
+    const int y = lane >> 2, c = 4 * half + (lane & 3);
+    float acc[RK_S2];
+#pragma unroll
+    for(int k = 0; k < RK_S2; k++) acc[k] = Wt[RW_B2 + c];
+#pragma unroll 2
+    for(int r = 0; r < 24; r++) {
+      const int ci = r / 3, ky = r - 3 * ci;
+      const float* row = a1 + (ci * RK_S1 + 2 * y + ky) * RK_S1;
+      float x[13];
+#pragma unroll
+      for(int k = 0; k < 13; k++) x[k] = row[k];
+#pragma unroll
+      for(int kx = 0; kx < 3; kx++) {
+        const float w = Wt[RW_2 + (r * 3 + kx) * 8 + c];
+#pragma unroll
+        for(int k = 0; k < RK_S2; k++) acc[k] = fmaf(w, x[2 * k + kx], acc[k]);
+      }
+    }
+#pragma unroll
+    for(int k = 0; k < RK_S2; k++) a2[(c * RK_S2 + y) * RK_S2 + k] = fmaxf(acc[k], 0.f);
+  }
+  pairSync(s);
+  {
+    const int y = lane >> 3, c = lane & 7, x0 = 2 * half;
+    float v0 = Wt[RW_B3 + c], v1 = v0;
+#pragma unroll 3
+    for(int r = 0; r < 24; r++) {
+      const int ci = r / 3, ky = r - 3 * ci;
+      const float* row = a2 + (ci * RK_S2 + y + ky) * RK_S2 + x0;
+      float x[4];
+#pragma unroll
+      for(int k = 0; k < 4; k++) x[k] = row[k];
+#pragma unroll
+      for(int kx = 0; kx < 3; kx++) {
+        const float w = Wt[RW_3 + (r * 3 + kx) * 8 + c];
+        v0 = fmaf(w, x[kx], v0);
+        v1 = fmaf(w, x[1 + kx], v1);
+      }
+    }
+    a3[(c * RK_S3 + y) * RK_S3 + x0] = fmaxf(v0, 0.f);
+    a3[(c * RK_S3 + y) * RK_S3 + x0 + 1] = fmaxf(v1, 0.f);
+  }
+  if(half) {
+    float v = Wt[RW_BM + lane];
+#pragma unroll
+    for(int i = 0; i < RK_NS; i++)
+      v = fmaf(Wt[RW_M + i * RK_H + lane], __shfl_sync(0xffffffffu, st, i), v);
+    hid[RK_C + lane] = fmaxf(v, 0.f);
+  }
+  pairSync(s);
+  float z = 0.f;
+  if(!half) {
+    if(lane < RK_C) {
+      float v = 0.f;
+#pragma unroll
+      for(int p = 0; p < RK_S3 * RK_S3; p++) v += a3[lane * RK_S3 * RK_S3 + p];
+      hid[lane] = v * (1.f / (RK_S3 * RK_S3));
+    }
+    __syncwarp();
+    z = Wt[RW_HB];
+#pragma unroll
+    for(int i = 0; i < RK_C + RK_H; i++) z = fmaf(Wt[RW_H + i], hid[i], z);
+  }
+  return z;
 }
 
 // slots (optional): the candidate slots of the stamps, maxSS per stamp; a
 // slot that is empty, past nRank in its stamp or in a stamp past *liveN
 // gets no score (k_rank_order reads none for it).
 template <class WT>
-__global__ void __launch_bounds__(RK_T)
+__global__ void __launch_bounds__(RF_T, 3)
     k_rank_forward(const WT* __restrict__ W, const float* __restrict__ stats,
                    const float* __restrict__ pix, int n, float* __restrict__ logit,
                    const int2* __restrict__ slots = nullptr, int maxSS = 1, int nRank = 1,
                    const int* __restrict__ liveN = nullptr) {
-  __shared__ float Ws[RK_NP];
-  __shared__ RkAct A;
-  for(int q = threadIdx.x; q < RK_NP; q += RK_T) Ws[q] = rkWeight(W, q);
-  for(int i = blockIdx.x; i < n; i += gridDim.x) {
+  extern __shared__ __align__(16) float rf_s[];
+#pragma unroll 4
+  for(int q = threadIdx.x; q < RK_NP; q += RF_T) rf_s[rwIndex(q)] = rkWeight(W, q);
+  __syncthreads();
+  const int s = threadIdx.x >> 6, half = (threadIdx.x >> 5) & 1;
+  float* buf = rf_s + RW_N + s * RF_BUF;
+  for(int i = blockIdx.x * RF_SAMPLES + s; i < n; i += gridDim.x * RF_SAMPLES) {
     if(slots && ((liveN && i / maxSS >= *liveN) || i % maxSS >= nRank || slots[i].x == INT_MAX))
-      continue;  // uniform over the CTA
-    __syncthreads();
-    rkLoad(stats, pix, i, A);
-    __syncthreads();
-    const float z = rkForward(Ws, A);
-    if(threadIdx.x == 0) logit[i] = z;
+      continue;  // uniform over the two warps
+    const float z = rfSample(rf_s, stats + (size_t)i * RK_NS, pix + (size_t)i * RK_PIX, buf, s, half);
+    if((threadIdx.x & 63) == 0) logit[i] = z;
   }
 }
 
-__global__ void __launch_bounds__(RK_T)
+// ----------------------------------------------------------------- gradient --
+// One CTA of eight warps per sample: forward, loss and the gradient of every
+// parameter (loss = sw * BCE(sigmoid(z), y)) into the sample's row of gPer.
+// A warp owns one output channel; a lane keeps a row segment of outputs, or
+// the three or five weights of one kernel row, in registers, so that a row
+// read from shared memory feeds several products (one thread per output or
+// weight, two shared reads per product, took 123 us for 512 samples on a GB300;
+// this form takes 44 us).  The gradients at the pre-activations of conv2
+// and conv3 are stored with a border of zeros, which the gathers of the layer
+// below read in the place of bounds checks.
+constexpr int RG_T = 256;
+constexpr int RG_LD = 33;             // window rows
+constexpr int RG_P = 8;               // rows of the padded gradient maps
+struct RkSample {
+  float in[2 * RK_WIN * RG_LD];
+  float a1[RK_C * RK_S1 * RK_S1];     // post-ReLU activations
+  float a2[RK_C * RK_S2 * RK_S2];
+  float a3[RK_C * RK_S3 * RK_S3];
+  float st[RK_NS];
+  float hid[RK_C + RK_H];
+  float dh[RK_C + RK_H];
+  float z;
+  float d3[RK_C * RG_P * RG_P];       // (y, x) at [y + 2][x + 2]
+  float d2[RK_C * RG_P * RG_P];       // (y, x) at [y + 1][x + 1]
+  float d1[RK_C * RK_S1 * RK_S1];
+};
+
+__device__ __forceinline__ float warpSum(float v) {
+#pragma unroll
+  for(int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+  return v;
+}
+
+__device__ void rgForward(const float* __restrict__ W, RkSample& A) {
+  const int tid = threadIdx.x, lane = tid & 31, c = tid >> 5;
+  if(lane < 2 * RK_S1) {
+    const int y = lane >> 1, h = lane & 1;
+    float acc[7];
+#pragma unroll
+    for(int k = 0; k < 7; k++) acc[k] = W[O_C1B + c];
+#pragma unroll 2
+    for(int r = 0; r < 10; r++) {
+      const int ci = r / 5, ky = r - 5 * ci;
+      const float* row = A.in + (ci * RK_WIN + 2 * y + ky) * RG_LD + 14 * h;
+      const float* w = W + O_C1W + (c * 2 + ci) * 25 + ky * 5;
+      float x[17];
+#pragma unroll
+      for(int k = 0; k < 17; k++) x[k] = row[k];
+#pragma unroll
+      for(int kx = 0; kx < 5; kx++)
+#pragma unroll
+        for(int k = 0; k < 7; k++) acc[k] = fmaf(w[kx], x[2 * k + kx], acc[k]);
+    }
+#pragma unroll
+    for(int k = 0; k < 7; k++) A.a1[(c * RK_S1 + y) * RK_S1 + 7 * h + k] = fmaxf(acc[k], 0.f);
+  }
+  __syncthreads();
+  if(lane < 3 * RK_S2) {
+    const int y = lane / 3, x0 = 2 * (lane % 3);
+    float v0 = W[O_C2B + c], v1 = v0;
+#pragma unroll 4
+    for(int r = 0; r < 24; r++) {
+      const int ci = r / 3, ky = r - 3 * ci;
+      const float* row = A.a1 + (ci * RK_S1 + 2 * y + ky) * RK_S1 + 2 * x0;
+      const float* w = W + O_C2W + (c * RK_C + ci) * 9 + ky * 3;
+      float x[5];
+#pragma unroll
+      for(int k = 0; k < 5; k++) x[k] = row[k];
+#pragma unroll
+      for(int kx = 0; kx < 3; kx++) {
+        v0 = fmaf(w[kx], x[kx], v0);
+        v1 = fmaf(w[kx], x[2 + kx], v1);
+      }
+    }
+    A.a2[(c * RK_S2 + y) * RK_S2 + x0] = fmaxf(v0, 0.f);
+    A.a2[(c * RK_S2 + y) * RK_S2 + x0 + 1] = fmaxf(v1, 0.f);
+  }
+  __syncthreads();
+  {
+    const int y = (lane >> 2) & 3, x = lane & 3, half = lane >> 4;
+    float v = half ? 0.f : W[O_C3B + c];
+#pragma unroll
+    for(int q = 0; q < 4; q++) {
+      const int ci = 4 * half + q;
+      const float* w = W + O_C3W + (c * RK_C + ci) * 9;
+#pragma unroll
+      for(int k = 0; k < 9; k++)
+        v = fmaf(w[k], A.a2[(ci * RK_S2 + y + k / 3) * RK_S2 + x + k % 3], v);
+    }
+    v += __shfl_xor_sync(0xffffffffu, v, 16);
+    v = fmaxf(v, 0.f);
+    if(!half) A.a3[c * 16 + lane] = v;
+    v = half ? 0.f : v;
+    v = warpSum(v);
+    if(lane == 0) A.hid[c] = v * (1.f / (RK_S3 * RK_S3));
+  }
+  if(c == 0) {
+    float v = W[O_M1B + lane];
+#pragma unroll
+    for(int i = 0; i < RK_NS; i++) v = fmaf(W[O_M1W + lane * RK_NS + i], A.st[i], v);
+    A.hid[RK_C + lane] = fmaxf(v, 0.f);
+  }
+  __syncthreads();
+  if(c == 0) {
+    float v = W[O_HW + lane] * A.hid[lane];
+    if(lane < RK_C) v = fmaf(W[O_HW + 32 + lane], A.hid[32 + lane], v);
+    v = warpSum(v);
+    if(lane == 0) A.z = v + W[O_HB];
+  }
+  __syncthreads();
+}
+
+__device__ void rgBackward(const float* __restrict__ W, RkSample& A, float dz,
+                           float* __restrict__ g) {
+  const int tid = threadIdx.x, lane = tid & 31, c = tid >> 5;
+  if(tid < RK_C + RK_H) {
+    g[O_HW + tid] = dz * A.hid[tid];
+    A.dh[tid] = dz * W[O_HW + tid];
+  }
+  if(tid == RK_C + RK_H) g[O_HB] = dz;
+  __syncthreads();
+  for(int q = tid; q < RK_H * RK_NS; q += RG_T) {
+    const int j = q / RK_NS;
+    g[O_M1W + q] = A.hid[RK_C + j] > 0.f ? A.dh[RK_C + j] * A.st[q % RK_NS] : 0.f;
+  }
+  if(tid < RK_H) g[O_M1B + tid] = A.hid[RK_C + tid] > 0.f ? A.dh[RK_C + tid] : 0.f;
+  // pool -> conv3 pre-activation
+  float v3 = 0.f;
+  if(lane < 16) {
+    v3 = A.a3[c * 16 + lane] > 0.f ? A.dh[c] * (1.f / (RK_S3 * RK_S3)) : 0.f;
+    A.d3[(c * RG_P + 2 + (lane >> 2)) * RG_P + 2 + (lane & 3)] = v3;
+  }
+  v3 = warpSum(v3);
+  if(lane == 0) g[O_C3B + c] = v3;
+  __syncthreads();
+  // conv3 weights: lane = (input channel, kernel row)
+  if(lane < 24) {
+    const int ci = lane / 3, ky = lane % 3;
+    float acc[3] = {0.f, 0.f, 0.f};
+#pragma unroll
+    for(int y = 0; y < RK_S3; y++) {
+      const float* d = A.d3 + (c * RG_P + 2 + y) * RG_P + 2;
+      const float* row = A.a2 + (ci * RK_S2 + y + ky) * RK_S2;
+      float x[6];
+#pragma unroll
+      for(int k = 0; k < 6; k++) x[k] = row[k];
+#pragma unroll
+      for(int k = 0; k < RK_S3; k++) {
+        const float dv = d[k];
+#pragma unroll
+        for(int kx = 0; kx < 3; kx++) acc[kx] = fmaf(dv, x[k + kx], acc[kx]);
+      }
+    }
+#pragma unroll
+    for(int kx = 0; kx < 3; kx++) g[O_C3W + (c * RK_C + ci) * 9 + ky * 3 + kx] = acc[kx];
+  }
+  // conv2 pre-activation
+  for(int o = tid; o < RK_C * RK_S2 * RK_S2; o += RG_T) {
+    const int ci = o / (RK_S2 * RK_S2), yy = (o / RK_S2) % RK_S2, xx = o % RK_S2;
+    float v = 0.f;
+    if(A.a2[o] > 0.f)
+#pragma unroll 2
+      for(int cc = 0; cc < RK_C; cc++) {
+        const float* w = W + O_C3W + (cc * RK_C + ci) * 9;
+        const float* d = A.d3 + (cc * RG_P + 2 + yy) * RG_P + 2 + xx;
+#pragma unroll
+        for(int k = 0; k < 9; k++) v = fmaf(d[-(k / 3) * RG_P - k % 3], w[k], v);
+      }
+    A.d2[(ci * RG_P + 1 + yy) * RG_P + 1 + xx] = v;
+  }
+  __syncthreads();
+  // conv2 weights and bias
+  {
+    float v = A.d2[(c * RG_P + 1 + lane / RK_S2) * RG_P + 1 + lane % RK_S2];
+    if(lane < 4) v += A.d2[(c * RG_P + 6) * RG_P + 3 + lane];
+    v = warpSum(v);
+    if(lane == 0) g[O_C2B + c] = v;
+  }
+  if(lane < 24) {
+    const int ci = lane / 3, ky = lane % 3;
+    float acc[3] = {0.f, 0.f, 0.f};
+#pragma unroll 2
+    for(int y = 0; y < RK_S2; y++) {
+      const float* d = A.d2 + (c * RG_P + 1 + y) * RG_P + 1;
+      const float* row = A.a1 + (ci * RK_S1 + 2 * y + ky) * RK_S1;
+      float x[13];
+#pragma unroll
+      for(int k = 0; k < 13; k++) x[k] = row[k];
+#pragma unroll
+      for(int k = 0; k < RK_S2; k++) {
+        const float dv = d[k];
+#pragma unroll
+        for(int kx = 0; kx < 3; kx++) acc[kx] = fmaf(dv, x[2 * k + kx], acc[kx]);
+      }
+    }
+#pragma unroll
+    for(int kx = 0; kx < 3; kx++) g[O_C2W + (c * RK_C + ci) * 9 + ky * 3 + kx] = acc[kx];
+  }
+  // conv1 pre-activation, 2 x 2 outputs per thread: with stride 2 an even row
+  // (column) takes kernel rows 0 and 2, an odd one row 1
+  for(int o = tid; o < RK_C * 49; o += RG_T) {
+    const int ci = o / 49, by = (o / 7) % 7, bx = o % 7;
+    float v00 = 0.f, v01 = 0.f, v10 = 0.f, v11 = 0.f;
+#pragma unroll 2
+    for(int cc = 0; cc < RK_C; cc++) {
+      const float* d = A.d2 + (cc * RG_P + 1 + by) * RG_P + 1 + bx;
+      const float* w = W + O_C2W + (cc * RK_C + ci) * 9;
+      const float a = d[0], up = d[-RG_P], le = d[-1], ul = d[-RG_P - 1];
+      v00 = fmaf(a, w[0], fmaf(up, w[6], fmaf(le, w[2], fmaf(ul, w[8], v00))));
+      v01 = fmaf(a, w[1], fmaf(up, w[7], v01));
+      v10 = fmaf(a, w[3], fmaf(le, w[5], v10));
+      v11 = fmaf(a, w[4], v11);
+    }
+    const int e = (ci * RK_S1 + 2 * by) * RK_S1 + 2 * bx;
+    A.d1[e] = A.a1[e] > 0.f ? v00 : 0.f;
+    A.d1[e + 1] = A.a1[e + 1] > 0.f ? v01 : 0.f;
+    A.d1[e + RK_S1] = A.a1[e + RK_S1] > 0.f ? v10 : 0.f;
+    A.d1[e + RK_S1 + 1] = A.a1[e + RK_S1 + 1] > 0.f ? v11 : 0.f;
+  }
+  __syncthreads();
+  // conv1 weights and bias: lane = (input channel, kernel row, third of the
+  // output rows), summed over the thirds at the end
+  {
+    float v = 0.f;
+    for(int p = lane; p < RK_S1 * RK_S1; p += 32) v += A.d1[c * RK_S1 * RK_S1 + p];
+    v = warpSum(v);
+    if(lane == 0) g[O_C1B + c] = v;
+    const int part = lane % 3, ck = lane / 3, ci = ck / 5, ky = ck % 5;
+    float acc[5] = {0.f, 0.f, 0.f, 0.f, 0.f};
+    if(lane < 30)
+#pragma unroll 1
+      for(int y = 5 * part; y < min(5 * part + 5, RK_S1); y++) {
+        const float* d = A.d1 + (c * RK_S1 + y) * RK_S1;
+        const float* row = A.in + (ci * RK_WIN + 2 * y + ky) * RG_LD;
+        float x[RK_WIN];
+#pragma unroll
+        for(int k = 0; k < RK_WIN; k++) x[k] = row[k];
+#pragma unroll
+        for(int k = 0; k < RK_S1; k++) {
+          const float dv = d[k];
+#pragma unroll
+          for(int kx = 0; kx < 5; kx++) acc[kx] = fmaf(dv, x[2 * k + kx], acc[kx]);
+        }
+      }
+#pragma unroll
+    for(int kx = 0; kx < 5; kx++) {
+      const float s1 = __shfl_down_sync(0xffffffffu, acc[kx], 1);
+      const float s2 = __shfl_down_sync(0xffffffffu, acc[kx], 2);
+      if(lane < 30 && part == 0) g[O_C1W + (c * 2 + ci) * 25 + ky * 5 + kx] = acc[kx] + s1 + s2;
+    }
+  }
+}
+
+__global__ void __launch_bounds__(RG_T, 4)
     k_rank_grad(const float* __restrict__ W, const float* __restrict__ stats,
                 const float* __restrict__ pix, const float* __restrict__ label,
                 const float* __restrict__ sweight, int n, float* __restrict__ gPer,
                 float* __restrict__ loss) {
   __shared__ float Ws[RK_NP];
-  __shared__ RkAct A;
-  __shared__ RkGrad D;
-  for(int q = threadIdx.x; q < RK_NP; q += RK_T) Ws[q] = rkWeight(W, q);
+  __shared__ RkSample A;
+  const int tid = threadIdx.x;
+#pragma unroll 9
+  for(int q = tid; q < RK_NP; q += RG_T) Ws[q] = rkWeight(W, q);
+  for(int q = tid; q < RK_C * RG_P * RG_P; q += RG_T) A.d3[q] = A.d2[q] = 0.f;
   for(int i = blockIdx.x; i < n; i += gridDim.x) {
     __syncthreads();
-    rkLoad(stats, pix, i, A);
+#pragma unroll 8
+    for(int q = tid; q < RK_PIX; q += RG_T) {
+      const int r = q / RK_WIN;
+      A.in[r * RG_LD + q - r * RK_WIN] = pix[(size_t)i * RK_PIX + q];
+    }
+    if(tid < RK_NS) A.st[tid] = stats[(size_t)i * RK_NS + tid];
     __syncthreads();
-    const float z = rkForward(Ws, A);
-    const float y = label[i], sw = sweight ? sweight[i] : 1.f;
-    if(threadIdx.x == 0)  // sw * BCE with logits, stable form
+    rgForward(Ws, A);
+    const float z = A.z, y = label[i], sw = sweight ? sweight[i] : 1.f;
+    if(tid == 0)  // sw * BCE with logits, stable form
       loss[i] = sw * (fmaxf(z, 0.f) - z * y + log1pf(expf(-fabsf(z))));
-    rkBackward(Ws, A, D, y, sw, gPer + (size_t)i * RK_NP);
+    rgBackward(Ws, A, sw * (1.f / (1.f + expf(-z)) - y), gPer + (size_t)i * RK_NP);
   }
 }
 
-// g[p] = (sum over samples in order of gPer[s][p]) * scale
-__global__ void k_rank_reduce(const float* __restrict__ gPer, int n, float scale,
-                              float* __restrict__ g) {
-  const int p = blockIdx.x * blockDim.x + threadIdx.x;
-  if(p >= RK_NP) return;
+// g[p] = (sum over the samples of gPer[s][p]) * scale: 32 parameters per CTA,
+// warp w sums the samples w, w + 16, ... in order and the 16 partial sums are
+// added in order (one thread per parameter over all samples was bound by the
+// latency of its loads: 22 us for 512 samples against 4.1 us).
+constexpr int RR_W = 16;
+__global__ void __launch_bounds__(32 * RR_W)
+    k_rank_reduce(const float* __restrict__ gPer, int n, float scale, float* __restrict__ g) {
+  __shared__ float part[RR_W][32];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, p = blockIdx.x * 32 + lane;
   float v = 0.f;
-  for(int s = 0; s < n; s++) v += gPer[(size_t)s * RK_NP + p];
-  g[p] = v * scale;
+  if(p < RK_NP) {
+    int s = warp;
+    for(; s + 7 * RR_W < n; s += 8 * RR_W) {
+      float x[8];
+#pragma unroll
+      for(int k = 0; k < 8; k++) x[k] = gPer[(size_t)(s + k * RR_W) * RK_NP + p];
+#pragma unroll
+      for(int k = 0; k < 8; k++) v += x[k];
+    }
+    for(; s < n; s += RR_W) v += gPer[(size_t)s * RK_NP + p];
+  }
+  part[warp][lane] = v;
+  __syncthreads();
+  if(warp == 0 && p < RK_NP) {
+    v = 0.f;
+#pragma unroll
+    for(int k = 0; k < RR_W; k++) v += part[k][lane];
+    g[p] = v * scale;
+  }
 }
 
 __global__ void k_rank_adam(float* __restrict__ W, const float* __restrict__ g,
@@ -583,8 +846,11 @@ void rankSubstamps(xb_ctx* c) {
     XB_LAUNCHED(c);
     {
       KT_SCOPE(c, "rank_score");
-      k_rank_forward<__nv_bfloat16><<<std::min(n, c->smCount * 8), RK_T, 0, c->stream>>>(
-          (const __nv_bfloat16*)c->rankW, dStats, dPix, n, dLogit, S.ssxy, g.maxSS, nRank, S.dN);
+      XB_CUDA(allowMaxDynamicSmem((const void*)k_rank_forward<__nv_bfloat16>, c->device));
+      k_rank_forward<__nv_bfloat16>
+          <<<std::min((n + RF_SAMPLES - 1) / RF_SAMPLES, c->smCount * 3), RF_T, RF_SMEM,
+             c->stream>>>((const __nv_bfloat16*)c->rankW, dStats, dPix, n, dLogit, S.ssxy, g.maxSS,
+                          nRank, S.dN);
       XB_LAUNCHED(c);
     }
     k_rank_order<<<(S.n + 127) / 128, 128, 0, c->stream>>>(S.ssxy, S.ssval, dLogit, S.n, S.dN,
@@ -670,8 +936,13 @@ int xb_ranker_forward(const float* dW, const float* dStats, const float* dPix, i
                       float* dLogit, void* stream) {
   if(n < 0 || (n > 0 && (!dW || !dStats || !dPix || !dLogit))) return XB_ERR_ARG;
   if(n == 0) return XB_OK;
-  k_rank_forward<float><<<std::min(n, 4096), RK_T, 0, (cudaStream_t)stream>>>(dW, dStats, dPix, n,
-                                                                              dLogit);
+  int device = 0, sms = 0;
+  if(cudaGetDevice(&device) != cudaSuccess ||
+     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device) != cudaSuccess ||
+     allowMaxDynamicSmem((const void*)k_rank_forward<float>, device) != cudaSuccess)
+    return XB_ERR_CUDA;
+  k_rank_forward<float><<<std::min((n + RF_SAMPLES - 1) / RF_SAMPLES, sms * 3), RF_T, RF_SMEM,
+                          (cudaStream_t)stream>>>(dW, dStats, dPix, n, dLogit);
   return rkLaunched() == cudaSuccess ? XB_OK : XB_ERR_CUDA;
 }
 
@@ -681,10 +952,10 @@ int xb_ranker_grad(const float* dW, const float* dStats, const float* dPix, cons
   if(n <= 0 || !dW || !dStats || !dPix || !dLabel || !dGradPerSample || !dGrad || !dLoss)
     return XB_ERR_ARG;
   cudaStream_t st = (cudaStream_t)stream;
-  k_rank_grad<<<std::min(n, 4096), RK_T, 0, st>>>(dW, dStats, dPix, dLabel, dWeight, n,
+  k_rank_grad<<<std::min(n, 4096), RG_T, 0, st>>>(dW, dStats, dPix, dLabel, dWeight, n,
                                                   dGradPerSample, dLoss);
   if(rkLaunched() != cudaSuccess) return XB_ERR_CUDA;
-  k_rank_reduce<<<(RK_NP + 127) / 128, 128, 0, st>>>(dGradPerSample, n, 1.f / n, dGrad);
+  k_rank_reduce<<<(RK_NP + 31) / 32, 32 * RR_W, 0, st>>>(dGradPerSample, n, 1.f / n, dGrad);
   return rkLaunched() == cudaSuccess ? XB_OK : XB_ERR_CUDA;
 }
 
