@@ -12,6 +12,7 @@
 #include <cooperative_groups.h>
 
 #include <algorithm>
+#include <atomic>
 #include <climits>
 
 #include "xb_device.cuh"
@@ -467,205 +468,307 @@ __global__ void k_build_rhs(const int* __restrict__ list, int nList, const int* 
 }
 
 // ------------------------------------------------------ global LU ---------
-// CPU ludcmp (bachUtil.cpp:319-384) on the (matSize)^2 system, distributed
-// over a thread-block cluster: CTA r owns the columns j with (j-1) % CL == r
-// in shared memory.  Per step the owner of column j finds the pivot, scales
-// the L column and publishes both; every CTA then swaps the pivot rows and
-// updates its own trailing columns.  Right-looking elimination gives the
-// same products in the same order as the reference's Crout loops.
+// CPU ludcmp and the forward half of lubksb (bachUtil.cpp:319-411) on the
+// matSize^2 system, distributed over a thread-block cluster: CTA r owns the
+// columns j with (j-1) % CL == r in shared memory, the right-hand side being
+// column n + 1.  Right-looking elimination gives every entry the same products
+// in the same order as the reference's Crout loops, and the right-hand side's
+// column the ones of its forward substitution (the rows a leading zero of b
+// skips there only subtract zeros here).
+//
+// Step j: every CTA copies the scaled column j and its pivot row from the
+// owner, swaps the pivot rows of its columns and updates them.  The owner of
+// column j + 1 updates that column first, finds its pivot and publishes it
+// before its other columns, so that chain (two products, the pivot search, a
+// reciprocal, one exchange) runs while the others update.  The pivot search
+// compares the bits of the nonnegative scaled values: an FP64 compare takes
+// as long as a product (62 cycles).  Bound by that chain and by FP64 (a
+// product and a subtraction per entry, one warp instruction per 19 cycles per
+// SM): 0.77 ms at n = 292 on 16 CTAs; 8 CTAs with the search between the
+// exchange and the update took 2.0 ms.
+constexpr int GLU_T = 512;
+inline size_t gluDoubles(int n, int CL) {
+  const size_t ld = n + 1;
+  return (size_t)((n + CL) / CL) * ld + 4 * ld + 4;
+}
+
+// Larger (value, row) of nonnegative values by their bits; row < 0 never wins.
+struct PivotKey {
+  long long v;
+  int i;
+};
+__device__ __forceinline__ void pivotMax(PivotKey& a, const PivotKey& b) {
+  if(b.v > a.v || (b.v == a.v && b.i > a.i)) a = b;
+}
+__device__ __forceinline__ PivotKey pivotWarpMax(PivotKey k) {
+#pragma unroll
+  for(int o = 16; o > 0; o >>= 1) {
+    PivotKey b;
+    b.v = __shfl_xor_sync(0xffffffffu, k.v, o);
+    b.i = __shfl_xor_sync(0xffffffffu, k.i, o);
+    pivotMax(k, b);
+  }
+  return k;
+}
+
 template <int CL>
-__global__ void __launch_bounds__(256)
-    k_global_lu(double* __restrict__ M, int n, int* __restrict__ idxOut,
-                int* __restrict__ singular) {
+__global__ void __launch_bounds__(GLU_T)
+    k_global_lu(double* __restrict__ M, int n, double* __restrict__ b, int* __restrict__ singular) {
   extern __shared__ double glu_s[];
   cg::cluster_group cluster = cg::this_cluster();
-  const int rank = (int)cluster.block_rank(), tid = threadIdx.x, nt = blockDim.x;
+  const int rank = (int)cluster.block_rank(), tid = threadIdx.x;
+  const int lane = tid & 31, warp = tid >> 5;
   const int ld = n + 1;
-  const int ncol = (n + CL - 1) / CL;  // local columns (some may be past n)
+  const int ncol = (n + CL) / CL;               // local columns of the n + 1 (some may be past it)
   double* col = glu_s;                          // ncol * ld (column-major)
   double* vv = col + (size_t)ncol * ld;         // ld
-  double* bc = vv + ld;                         // 2 * (ld + 1) broadcast buffers
-  double* L = bc + 2 * (ld + 1);                // ld
-  __shared__ double rv[8];
-  __shared__ int ri[8];
-  __shared__ int sP, sMaxI, sSing;
+  double* bc = vv + ld;                         // 2 x ld: published columns; entry 0 the pivot row
+  double* L = bc + 2 * ld;                      // ld
+  __shared__ PivotKey wk[GLU_T / 32];
+  __shared__ double sRecip;
+  __shared__ int sSing;
   // row scaling (CPU form: a zero row aborts before the elimination)
   if(tid == 0) sSing = 0;
   __syncthreads();
-  for(int i = 1 + tid; i <= n; i += nt) {
-    double big = 0.0;
-    for(int j = 1; j <= n; j++) {
-      double t = fabs(M[(size_t)i * ld + j]);
+  for(int i = 1 + warp; i <= n; i += GLU_T / 32) {
+    long long big = 0;
+    for(int j = 1 + lane; j <= n; j += 32) {
+      const double t = fabs(M[(size_t)i * ld + j]);
+      const long long tb = __double_as_longlong(t);
+      if(tb <= 0x7FF0000000000000ll && tb > big) big = tb;  // a NaN is never larger
+    }
+#pragma unroll
+    for(int o = 16; o > 0; o >>= 1) {
+      const long long t = __shfl_xor_sync(0xffffffffu, big, o);
       if(t > big) big = t;
     }
-    if(big == 0.0) sSing = 1;
-    vv[i] = 1.0 / big;
+    if(lane == 0) {
+      if(big == 0) sSing = 1;
+      vv[i] = 1.0 / __longlong_as_double(big);
+    }
   }
   __syncthreads();
   if(sSing) {
     if(rank == 0 && tid == 0) *singular = 1;
-    for(int i = tid; i <= n; i += nt)
-      if(rank == 0) idxOut[i] = 0;
     cluster.sync();
     return;
   }
   for(int lc = 0; lc < ncol; lc++) {
     const int j = lc * CL + rank + 1;
-    for(int i = tid; i <= n; i += nt) col[(size_t)lc * ld + i] = j <= n ? M[(size_t)i * ld + j] : 0.0;
+    for(int i = tid; i <= n; i += GLU_T)
+      col[(size_t)lc * ld + i] = i == 0 || j > n + 1 ? 0.0 : j <= n ? M[(size_t)i * ld + j] : b[i];
   }
-  if(tid == 0) sMaxI = 0;
   __syncthreads();
   cluster.sync();
+
+  int lastPivot = 0;
+  // Pivot of column j (owned here, updated through step j - 1), its scaling
+  // and its publication.
+  auto publish = [&](int j) {
+    double* c = col + (size_t)((j - 1) / CL) * ld;
+    double* my = bc + (j & 1) * ld;
+    PivotKey k = {-1, -1};
+    for(int i = j + tid; i <= n; i += GLU_T) {
+      const double v = vv[i] * fabs(c[i]);
+      const long long vb = __double_as_longlong(v);
+      if(vb >= 0 && vb <= 0x7FF0000000000000ll) pivotMax(k, PivotKey{vb, i});
+    }
+    k = pivotWarpMax(k);
+    if(lane == 0) wk[warp] = k;
+    __syncthreads();
+    k = wk[lane & (GLU_T / 32 - 1)];
+    k = pivotWarpMax(k);
+    const int p = k.i >= 0 ? k.i : lastPivot;
+    double cj = c[j], d = c[p];
+    if(d == 0.0) d = 1.0e-20;
+    if(warp == 0) {
+      const double r = 1.0 / d;
+      if(lane == 0) sRecip = r;
+    }
+    __syncthreads();
+    const double r = sRecip;
+    for(int i = j + 1 + tid; i <= n; i += GLU_T) {
+      const double l = (i == p ? cj : c[i]) * r;
+      c[i] = l;
+      my[i] = l;
+    }
+    if(tid == 0) {
+      c[j] = d;
+      my[0] = (double)p;
+    }
+  };
+  if(rank == 0) publish(1);
+  asm volatile("barrier.cluster.arrive.release;" ::: "memory");
   for(int j = 1; j <= n; j++) {
     const int owner = (j - 1) % CL, lcj = (j - 1) / CL;
-    double* myBc = bc + (j & 1) * (ld + 1);
-    if(rank == owner) {
-      double* cj = col + (size_t)lcj * ld;
-      double bv = 0.0;
-      int bi = -1;
-      for(int i = j + tid; i <= n; i += nt) {
-        double dum = vv[i] * fabs(cj[i]);
-        if(dum >= 0.0) pivotCombine(bv, bi, dum, i);
-      }
-#pragma unroll
-      for(int o = 16; o > 0; o >>= 1) {
-        double ov = __shfl_down_sync(0xffffffffu, bv, o);
-        int oi = __shfl_down_sync(0xffffffffu, bi, o);
-        pivotCombine(bv, bi, ov, oi);
-      }
-      if((tid & 31) == 0) {
-        rv[tid >> 5] = bv;
-        ri[tid >> 5] = bi;
-      }
-      __syncthreads();
-      if(tid == 0) {
-        double v = rv[0];
-        int i0 = ri[0];
-        for(int w = 1; w < nt / 32; w++) pivotCombine(v, i0, rv[w], ri[w]);
-        int p = i0 >= 0 ? i0 : sMaxI;
-        if(p != j) {
-          double t = cj[p];
-          cj[p] = cj[j];
-          cj[j] = t;
-        }
-        if(cj[j] == 0.0) cj[j] = 1.0e-20;
-        myBc[0] = (double)p;
-      }
-      __syncthreads();
-      if(j != n) {
-        const double dum = 1.0 / cj[j];
-        for(int i = j + 1 + tid; i <= n; i += nt) cj[i] *= dum;
-      }
-      __syncthreads();
-      for(int i = j + 1 + tid; i <= n; i += nt) myBc[i] = cj[i];
-    }
-    cluster.sync();
-    const double* src = cluster.map_shared_rank(myBc, owner);
-    if(tid == 0) {
-      sP = (int)src[0];
-      sMaxI = sP;
-    }
-    for(int i = j + 1 + tid; i <= n; i += nt) L[i] = src[i];
-    __syncthreads();
-    const int p = sP;
-    if(rank == 0 && tid == 0) idxOut[j] = p;
+    asm volatile("barrier.cluster.wait.acquire;" ::: "memory");
+    const double* src = cluster.map_shared_rank(bc + (j & 1) * ld, owner);
+    const int p = (int)src[0];
+    lastPivot = p;
+    for(int i = j + 1 + tid; i <= n; i += GLU_T) L[i] = src[i];
+    const bool ahead = j < n && j % CL == rank;  // this CTA owns column j + 1
+    if(!ahead) asm volatile("barrier.cluster.arrive.release;" ::: "memory");
     if(p != j) {
-      for(int lc = tid; lc < ncol; lc += nt) {
-        if(rank == owner && lc == lcj) continue;  // already swapped by the owner
+      for(int lc = tid; lc < ncol; lc += GLU_T) {
+        if(rank == owner && lc == lcj) continue;  // swapped by its publication
         double* c = col + (size_t)lc * ld;
-        double t = c[p];
+        const double t = c[p];
         c[p] = c[j];
         c[j] = t;
       }
       if(tid == 0) vv[p] = vv[j];
     }
     __syncthreads();
-    // trailing update of the local columns k > j
     const int lcStart = (j - rank + CL - 1) / CL;  // first lc with lc*CL + rank + 1 > j
-    const int nLoc = ncol - lcStart, m = n - j;
-    for(int e = tid; e < nLoc * m; e += nt) {
-      const int lc = lcStart + e / m, i = j + 1 + e % m;
-      if(lc * CL + rank + 1 > n) continue;
-      double* c = col + (size_t)lc * ld;
+    int lcA = lcStart;
+    if(ahead) {
+      double* c = col + (size_t)lcStart * ld;
+      const double cj = c[j];
+      for(int i = j + 1 + tid; i <= n; i += GLU_T) c[i] -= L[i] * cj;
+      __syncthreads();
+      publish(j + 1);
+      asm volatile("barrier.cluster.arrive.release;" ::: "memory");
+      lcA++;
+    }
+    // the other local columns k > j, flattened over (column, row)
+    const int lcEnd = min(ncol, (n - rank) / CL + 1);  // columns past n + 1 do not exist
+    const int m = n - j, tot = (lcEnd - lcA) * m;
+    const float im = 1.f / (float)max(m, 1);
+    for(int e = tid; e < tot; e += GLU_T) {
+      int q = (int)((float)e * im);
+      q -= q * m > e;
+      q += (q + 1) * m <= e;
+      double* c = col + (size_t)(lcA + q) * ld;
+      const int i = j + 1 + e - q * m;
       c[i] -= L[i] * c[j];
     }
     __syncthreads();
   }
-  cluster.sync();
+  asm volatile("barrier.cluster.wait.acquire;" ::: "memory");
   for(int lc = 0; lc < ncol; lc++) {
     const int j = lc * CL + rank + 1;
-    if(j > n) break;
-    for(int i = tid; i <= n; i += nt) M[(size_t)i * ld + j] = col[(size_t)lc * ld + i];
+    const double* c = col + (size_t)lc * ld;
+    if(j <= n)
+      for(int i = 1 + tid; i <= j; i += GLU_T) M[(size_t)i * ld + j] = c[i];  // U
+    else if(j == n + 1)
+      for(int i = 1 + tid; i <= n; i += GLU_T) b[i] = c[i];  // L^-1 P b
   }
-  if(rank == 0 && tid == 0) idxOut[0] = 0;
+  cluster.sync();  // no CTA leaves while another may still read its columns
 }
 
-// lubksb of the global system (bachUtil.cpp:380-411) on two warps: lane 0 of
-// warp 0 runs each row's sequential chain `sum -= a[i][j] * b[j]` (the
-// reference's order and roundings), while warp 1 forms the next row's
-// products a[i'][j] * b[j] for the b[j] already final; lane 0 forms the one
-// product that needs the row it just finished, from a value it loaded before
-// its chain.  One 64-thread barrier per row.
-constexpr int LUB_THREADS = 64;
+// x / y for the correctly rounded r = 1 / y.  A q within one ulp of the
+// quotient has an exact remainder x - q y (one FMA), and RN(q + (x - q y) r) is
+// then the correctly rounded quotient (P. Markstein, IBM J. Res. Dev. 34,
+// 1990).  RN(x r) can be 1.5 ulp off, so one such step brings q there and a
+// second one rounds.  Exponents that could over- or underflow take the
+// division.
+__device__ __forceinline__ double quotient(double x, double y, double r) {
+  const int ex = (int)((__double_as_longlong(x) >> 52) & 0x7FF);
+  const int ey = (int)((__double_as_longlong(y) >> 52) & 0x7FF);
+  if(ex < 400 || ex > 1600 || ey < 700 || ey > 1350) return x / y;
+  double q = x * r;
+  q = fma(fma(-q, y, x), r, q);
+  return fma(fma(-q, y, x), r, q);
+}
+
+// Back half of lubksb (bachUtil.cpp:399-409): U x = y, b <- x.  Warp 0 runs each
+// row's chain `sum -= a[i][j] * b[j]` in the reference's order and roundings
+// while warps 1 and 2 form the next row's products a[i'][j] * b[j] of the b[j]
+// already final; the one product that needs the row just finished is formed by
+// warp 0.  One barrier per row.  The n^2/2 subtractions of the chains are one
+// dependent sequence (every row starts from the unknown before it), 62 cycles
+// each: 1.67 ms at n = 292, of which 1.3 ms the chain alone (half of the
+// 3.43 ms that one lane took for both halves; warp steps on the integer grid of
+// the running sum, as in the stamp statistics, took 3.1 ms: these sums of mixed
+// signs leave a binade every two or three terms).
+//
+// With *singular set (a zero row) the matrix is as built and the reference
+// runs lubksb on it with the pivot indices it has, zeros: lane 0 does the same.
+constexpr int LUB_THREADS = 96;
+constexpr int LUB_PAD = 16;  // terms past n that the chain may read
 __global__ void __launch_bounds__(LUB_THREADS)
-    k_global_lubksb(const double* __restrict__ M, int n, const int* __restrict__ idx,
-                    double* __restrict__ b) {
+    k_global_backsub(const double* __restrict__ M, int n, const int* __restrict__ singular,
+                     double* __restrict__ b) {
   extern __shared__ double sol_s[];
-  double* bs = sol_s;          // n + 1
-  double* pA = bs + n + 1;     // n + 1: products of the current row
-  double* pB = pA + n + 1;     // n + 1: products of the next row
-  int* is = (int*)(pB + n + 1);
-  __shared__ int iiS[2];  // ii for row i in slot i & 1 (written one row ahead)
+  const int len = n + LUB_PAD;
+  double* bs = sol_s;        // len
+  double* pA = bs + len;     // len: products of the current row, zeros past n
+  double* pB = pA + len;     // len: products of the next row
+  double* dg = pB + len;     // len: diagonal
+  double* rd = dg + len;     // len: its reciprocals
+  double* sup = rd + len;    // len: entries right of the diagonal
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, ld = n + 1;
   for(int i = tid; i <= n; i += LUB_THREADS) {
     bs[i] = b[i];
-    is[i] = idx[i];
+    dg[i] = i > 0 ? M[(size_t)i * ld + i] : 1.0;
+    sup[i] = i > 0 && i < n ? M[(size_t)i * ld + i + 1] : 0.0;
   }
-  if(tid == 0) iiS[0] = iiS[1] = 0;
+  __syncthreads();
+  if(*singular) {
+    if(tid == 0) {
+      int ii = 0;
+      for(int i = 1; i <= n; i++) {
+        double sum = bs[0];
+        bs[0] = bs[i];
+        if(ii != 0)
+          for(int j = ii; j < i; j++) sum -= M[(size_t)i * ld + j] * bs[j];
+        else if(sum != 0.0)
+          ii = i;
+        bs[i] = sum;
+      }
+      for(int i = n; i >= 1; i--) {
+        double sum = bs[i];
+        for(int j = i + 1; j <= n; j++) sum -= M[(size_t)i * ld + j] * bs[j];
+        bs[i] = sum / dg[i];
+      }
+    }
+    __syncthreads();
+    for(int i = tid; i <= n; i += LUB_THREADS) b[i] = bs[i];
+    return;
+  }
+  for(int i = tid; i <= n; i += LUB_THREADS) rd[i] = 1.0 / dg[i];
+  for(int i = tid; i < len; i += LUB_THREADS) pA[i] = pB[i] = 0.0;
   __syncthreads();
   double* cur = pA;
   double* nxt = pB;
-  // forward: L y = P b
-  for(int i = 1; i <= n; i++) {
-    const int ii0 = iiS[i & 1];
-    if(tid == 0) {
-      const double aNext = i < n ? M[(size_t)(i + 1) * ld + i] : 0.0;
-      const int ip = is[i];
-      double sum = bs[ip];
-      bs[ip] = bs[i];
-      int ii = ii0;
-      if(ii0 != 0) {
-#pragma unroll 8
-        for(int j = ii0; j < i; j++) sum -= cur[j];
-      } else if(sum != 0.0) {
-        ii = i;
-      }
-      iiS[(i + 1) & 1] = ii;
-      bs[i] = sum;
-      if(i < n && ii != 0) nxt[i] = aNext * sum;
-    } else if(warp == 1 && ii0 != 0 && i < n) {
-      for(int j = ii0 + lane; j < i; j += 32) nxt[j] = M[(size_t)(i + 1) * ld + j] * bs[j];
-    }
-    __syncthreads();
-    double* t = cur;
-    cur = nxt;
-    nxt = t;
-  }
-  // backward: U x = y (row n has no products)
+  double x = 0.0;  // warp 0: the row before
   for(int i = n; i >= 1; i--) {
-    if(tid == 0) {
-      const double aii = M[(size_t)i * ld + i];
-      const double aPrev = i > 1 ? M[(size_t)(i - 1) * ld + i] : 0.0;
-      double sum = bs[i];
+    if(warp == 0) {
+      double s = bs[i];
       if(i < n) {
-#pragma unroll 8
-        for(int j = i + 1; j <= n; j++) sum -= cur[j];
+        // terms in fours, the next four loaded meanwhile; subtracting the
+        // zeros past n leaves the sum as it is
+        const double* c = cur + i + 2;
+        double a0 = c[0], a1 = c[1], a2 = c[2], a3 = c[3];
+        s -= sup[i] * x;
+#pragma unroll 2
+        for(int m = n - i - 1; m > 0; m -= 4) {
+          c += 4;
+          const double b0 = c[0], b1 = c[1], b2 = c[2], b3 = c[3];
+          s -= a0;
+          s -= a1;
+          s -= a2;
+          s -= a3;
+          a0 = b0;
+          a1 = b1;
+          a2 = b2;
+          a3 = b3;
+        }
       }
-      const double xi = sum / aii;
-      bs[i] = xi;
-      if(i > 1) nxt[i] = aPrev * xi;
-    } else if(warp == 1 && i > 1) {
-      for(int j = i + 1 + lane; j <= n; j += 32) nxt[j] = M[(size_t)(i - 1) * ld + j] * bs[j];
+      x = quotient(s, dg[i], rd[i]);
+      if(lane == 0) bs[i] = x;
+    } else if(i > 1) {  // row i - 1, columns past i
+      const double* row = M + (size_t)(i - 1) * ld;
+      constexpr int W = LUB_THREADS - 32;
+      int j = i + 1 + tid - 32;
+      for(; j + 3 * W <= n; j += 4 * W) {
+        double a[4];
+#pragma unroll
+        for(int u = 0; u < 4; u++) a[u] = row[j + u * W];
+#pragma unroll
+        for(int u = 0; u < 4; u++) nxt[j + u * W] = a[u] * bs[j + u * W];
+      }
+      for(; j <= n; j += W) nxt[j] = row[j] * bs[j];
     }
     __syncthreads();
     double* t = cur;
@@ -1075,44 +1178,51 @@ static void solveGlobal(xb_ctx* c, int si, const FitBuffers& f, const int* list,
       c->put(cpuRhs ? "ksc_matrix0" : key, toHost(c, f.M, (size_t)ld * ld));
   }
   // LU on a thread-block cluster
-  const int n = g.matSize, ld = n + 1;
+  const int n = g.matSize;
   k_zero_ints<<<1, 32, 0, c->stream>>>(f.singular, 1);
   XB_LAUNCHED(c);
   if(mixed) {
     globalSolveMixed(c, f.M, n, dSol, f.piv, f.singular);
     return;
   }
-  // 8 CTAs, or 16 when 8 cannot hold the columns (the same products in the
-  // same order either way)
-  int maxSmem = 0;
-  XB_CUDA(cudaDeviceGetAttribute(&maxSmem, cudaDevAttrMaxSharedMemoryPerBlockOptin, c->device));
-  auto luSmem = [&](int cl) {
-    return ((size_t)((n + cl - 1) / cl) * ld + ld + 2 * (ld + 1) + ld) * sizeof(double);
+  // 16 CTAs where the device allows that cluster, else 8 (the same products
+  // in the same order either way)
+  static std::atomic<int> clusterSize{0};
+  auto launchLu = [&](auto kernel, int CL) -> cudaError_t {
+    cudaError_t e = allowMaxDynamicSmem((const void*)kernel, c->device);
+    if(e == cudaSuccess && CL > 8)
+      e = cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+    if(e != cudaSuccess) return e;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(CL);
+    cfg.blockDim = dim3(GLU_T);
+    cfg.dynamicSmemBytes = gluDoubles(n, CL) * sizeof(double);
+    cfg.stream = c->stream;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = CL;
+    attr[0].val.clusterDim.y = 1;
+    attr[0].val.clusterDim.z = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, kernel, f.M, n, dSol, f.singular);
   };
-  const int CL = luSmem(8) <= (size_t)maxSmem ? 8 : 16;
-  const size_t smem = luSmem(CL);
-  auto luKernel = CL == 8 ? k_global_lu<8> : k_global_lu<16>;
-  XB_CUDA(allowMaxDynamicSmem((const void*)luKernel, c->device));
-  if(CL > 8) XB_CUDA(cudaFuncSetAttribute(luKernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(CL);
-  cfg.blockDim = dim3(256);
-  cfg.dynamicSmemBytes = smem;
-  cfg.stream = c->stream;
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeClusterDimension;
-  attr[0].val.clusterDim.x = CL;
-  attr[0].val.clusterDim.y = 1;
-  attr[0].val.clusterDim.z = 1;
-  cfg.attrs = attr;
-  cfg.numAttrs = 1;
   { KT_SCOPE(c, "global_lu");
-  XB_CUDA(cudaLaunchKernelEx(&cfg, luKernel, f.M, n, f.piv, f.singular));
+  cudaError_t e = cudaErrorUnknown;
+  if(clusterSize.load() != 8) {
+    e = launchLu(k_global_lu<16>, 16);
+    if(e == cudaSuccess) clusterSize = 16;
+    else cudaGetLastError();
+  }
+  if(e != cudaSuccess) {
+    XB_CUDA(launchLu(k_global_lu<8>, 8));
+    clusterSize = 8;
+  }
   XB_LAUNCHED(c);
   }
-  const size_t smemS = (size_t)(3 * (n + 1)) * sizeof(double) + (size_t)(n + 1) * sizeof(int);
   { KT_SCOPE(c, "global_lubksb");
-  k_global_lubksb<<<1, LUB_THREADS, smemS, c->stream>>>(f.M, n, f.piv, dSol);
+  k_global_backsub<<<1, LUB_THREADS, (size_t)(6 * (n + LUB_PAD)) * sizeof(double), c->stream>>>(
+      f.M, n, f.singular, dSol);
   XB_LAUNCHED(c);
   }
 }
