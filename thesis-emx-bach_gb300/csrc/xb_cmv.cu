@@ -11,6 +11,7 @@
 
 #include <algorithm>
 
+#include "xb_device.cuh"
 #include "xb_internal.h"
 
 namespace xb {
@@ -31,7 +32,13 @@ __device__ __forceinline__ double ipow(double x, int n) {
   return r;
 }
 
-// Y then X pass for one (stamp, Y-filter group).
+// Y then X pass for one (stamp, Y-filter group).  The window and the Y outputs
+// are held as doubles (exact), so that a tap is one product and one sum, the
+// Y accumulator's rounding to float on its bits: bound by FP64, which issues
+// one warp instruction per 19 cycles per SM, conversions included (with a
+// conversion of the window, one of the accumulator to float and one back per
+// Y tap, and one of the Y output per X tap, 256 stamps took 3.15 ms; now
+// 2.37 ms).
 template <class T>
 __global__ void __launch_bounds__(FILL_THREADS)
     k_fill_w(const T* __restrict__ img, int w, int h, const int* __restrict__ list,
@@ -40,7 +47,7 @@ __global__ void __launch_bounds__(FILL_THREADS)
              const double* __restrict__ fY, const int* __restrict__ gStart,
              const int* __restrict__ gMembers, int hSS, int hK, int wRows,
              double* __restrict__ W) {
-  extern __shared__ unsigned char fill_s[];
+  extern __shared__ double fill_s[];
   const int s = list[blockIdx.x], gi = blockIdx.y, tid = threadIdx.x;
   const int fK = 2 * hK + 1, fSS = 2 * hSS + 1, wCols = fSS * fSS;
   const int xHalf = hSS + hK, tw = 2 * xHalf + 1, th = fSS;
@@ -55,13 +62,13 @@ __global__ void __launch_bounds__(FILL_THREADS)
     return;
   }
   const int2 c = ssxy[(size_t)s * maxSS + cur[s]];
-  float* win = (float*)fill_s;                 // tw x tw, rows y, cols x
-  float* tmp = win + tw * tw;                  // th x tw
-  const int off = tw * tw + th * tw;
-  double* fy = (double*)(win + off + (off & 1));  // 8-byte aligned
+  double* win = fill_s;                        // tw x tw, rows y, cols x
+  double* tmp = win + tw * tw;                 // th x tw
+  double* fy = tmp + th * tw;
   double* fx = fy + fK;
   const int n0 = gMembers[m0];
-  for(int i = tid; i < fK; i += FILL_THREADS) fy[i] = fY[(size_t)n0 * fK + i];
+  // reversed, so that a tap and its filter value run in the same direction
+  for(int i = tid; i < fK; i += FILL_THREADS) fy[i] = fY[(size_t)n0 * fK + fK - 1 - i];
   // input window: x in [ssx - xHalf, ssx + xHalf], y in [ssy - xHalf, ssy + xHalf]
   for(int i = tid; i < tw * tw; i += FILL_THREADS) {
     int lx = i % tw, ly = i / tw;
@@ -69,68 +76,81 @@ __global__ void __launch_bounds__(FILL_THREADS)
     // maskInput); the clamp only guards the address
     int gx = min(max(c.x - xHalf + lx, 0), w - 1);
     int gy = min(max(c.y - xHalf + ly, 0), h - 1);
-    win[i] = (float)img[(size_t)gx + (size_t)gy * w];
+    win[i] = (double)(float)img[(size_t)gx + (size_t)gy * w];
   }
   __syncthreads();
   // Y pass (cmv.cl:70-106): v accumulates in float, products in double
   for(int p = tid; p < th * tw; p += FILL_THREADS) {
     const int row = p / tw, col = p % tw;
-    float v = 0.0f;
-    for(int y = -hK; y <= hK; y++)
-      v = (float)((double)v + (double)win[(row + hK + y) * tw + col] * fy[hK - y]);
+    const double* wc = win + row * tw + col;
+    double v = 0.0;
+#pragma unroll 7
+    for(int y = 0; y < fK; y++) v = roundToFloat(v + wc[y * tw] * fy[y]);
     tmp[p] = v;
   }
   __syncthreads();
   for(int m = m0; m < m1; m++) {
     const int n = gMembers[m];
-    for(int i = tid; i < fK; i += FILL_THREADS) fx[i] = fX[(size_t)n * fK + i];
+    for(int i = tid; i < fK; i += FILL_THREADS) fx[i] = fX[(size_t)n * fK + fK - 1 - i];
     __syncthreads();
     // X pass (cmv.cl:108-135)
     for(int p = tid; p < wCols; p += FILL_THREADS) {
       const int row = p / fSS, ii = p % fSS;
+      const double* tr = tmp + row * tw + ii;
       double w0 = 0.0;
-      for(int x = -hK; x <= hK; x++) w0 += (double)tmp[row * tw + ii + x + hK] * fx[hK - x];
+#pragma unroll 7
+      for(int x = 0; x < fK; x++) w0 += tr[x] * fx[x];
       Ws[(size_t)n * wCols + p] = w0;
     }
     __syncthreads();
   }
 }
 
-// convStampOdd (cmv.cl:137-154) and convStampBg (:156-193).
+// convStampOdd (cmv.cl:137-154) and convStampBg (:156-193), one row of W per
+// CTA (one CTA per stamp, row after row, took 44 us for its dependent loads).
 __global__ void __launch_bounds__(FILL_THREADS)
     k_fill_finish(const int* __restrict__ list, const int* __restrict__ count,
                   const int* __restrict__ cur, const int2* __restrict__ ssxy, int maxSS,
                   const int* __restrict__ kx, const int* __restrict__ ky, int nPSF,
                   const int2* __restrict__ bgXY, int nBG, int hSS, int w, int h,
                   int wRows, double* __restrict__ W) {
-  const int s = list[blockIdx.x], tid = threadIdx.x;
+  const int s = list[blockIdx.x], n = 1 + blockIdx.y, tid = threadIdx.x;
   const int fSS = 2 * hSS + 1, wCols = fSS * fSS;
   double* Ws = W + (size_t)s * wRows * wCols;
-  const bool live = cur[s] < count[s];
-  for(int n = 1; n < nPSF; n++) {
-    if(kx[n] % 2 != 0 || ky[n] % 2 != 0) continue;
+  if(n < nPSF) {
+    if(kx[n] % 2 != 0 || ky[n] % 2 != 0) return;
+#pragma unroll 4
     for(int p = tid; p < wCols; p += FILL_THREADS) Ws[(size_t)n * wCols + p] -= Ws[p];
+    return;
   }
+  const int b = n - nPSF;
+  const bool live = cur[s] < count[s];
   int2 c = make_int2(0, 0);
   if(live) c = ssxy[(size_t)s * maxSS + cur[s]];
-  for(int b = 0; b < nBG; b++)
-    for(int p = tid; p < wCols; p += FILL_THREADS) {
-      double a = 0.0;
-      if(live) {
-        int x = c.x - hSS + p % fSS, y = c.y - hSS + p / fSS;
-        double xf = floatNorm(x, w), yf = floatNorm(y, h);
-        a = ipow(xf, bgXY[b].x) * ipow(yf, bgXY[b].y);
-      }
-      Ws[(size_t)(nPSF + b) * wCols + p] = a;
+  for(int p = tid; p < wCols; p += FILL_THREADS) {
+    double a = 0.0;
+    if(live) {
+      int x = c.x - hSS + p % fSS, y = c.y - hSS + p / fSS;
+      double xf = floatNorm(x, w), yf = floatNorm(y, h);
+      a = ipow(xf, bgXY[b].x) * ipow(yf, bgXY[b].y);
     }
+    Ws[(size_t)(nPSF + b) * wCols + p] = a;
+  }
 }
 
-// createQ (cmv.cl:195-215) and createB (:217-248) for one stamp per CTA.
-// Q: each thread owns up to GQ_E lower-triangle entries and accumulates them
-// over K in ascending order while W tiles stream through shared memory.
-constexpr int GQ_KT = 32, GQ_E = 8;
-template <class T>
-__global__ void __launch_bounds__(FILL_THREADS)
+// createQ (cmv.cl:195-215) and createB (:217-248).  A CTA of NT threads owns NT
+// entries of a stamp's lower triangle, row after row, each accumulated over the
+// pixels in ascending order by one thread while the rows of W it needs stream
+// through two shared-memory tiles; the last CTA of a stamp (blockIdx.y) makes
+// B and the zeros of Q.  A product and a sum per entry and pixel, so bound by
+// FP64 (19 cycles per warp instruction and SM) where the list fills the GPU and
+// by one entry's chain of 961 sums (62 cycles each) where it does not: 64
+// threads per CTA then spread a stamp over 21 SMs.  One CTA per stamp took
+// 1.62 ms for 256 stamps and 0.80 ms for a single one; now 1.37 and 0.09 ms.
+constexpr int GQ_KT = 32;
+constexpr int GQ_MAXENT = 2048;  // entries of the triangle (host check)
+template <class T, int NT>
+__global__ void __launch_bounds__(NT)
     k_gram_qb(const T* __restrict__ other, const T* __restrict__ conv, int w, int h,
               const int* __restrict__ list,
               const int* __restrict__ count, const int* __restrict__ cur,
@@ -145,14 +165,13 @@ __global__ void __launch_bounds__(FILL_THREADS)
   const double* Ws = W + (size_t)s * wRows * wCols;
   double* Qs = Q + (size_t)s * qCount * qCount;
   double* Bs = B + (size_t)s * qCount;
-  double* tile = gq_s;                      // R x (GQ_KT + 1)
-  double* sub = gq_s + R * (GQ_KT + 1);     // fSS * fSS image values
-  double* om = sub + wCols;                 // fSS * fSS pixel weights (weighted fit)
+  double* om = gq_s;                                // fSS * fSS pixel weights (weighted fit)
+  double* tile = om + (omega ? wCols : 0);          // 2 x (rows x (GQ_KT + 1)), or the image values
   const bool live = cur[s] < count[s];
+  const int2 c = live ? ssxy[(size_t)s * maxSS + cur[s]] : make_int2(0, 0);
   if(omega) {
     // weights of the current substamp's pixels (exhausted stamps: zero)
-    const int2 c = live ? ssxy[(size_t)s * maxSS + cur[s]] : make_int2(0, 0);
-    for(int i = tid; i < wCols; i += FILL_THREADS) {
+    for(int i = tid; i < wCols; i += NT) {
       double v = 0.0;
       if(live) {
         const int gx = min(max(i % fSS - hSS + c.x, 0), w - 1);
@@ -161,76 +180,219 @@ __global__ void __launch_bounds__(FILL_THREADS)
         v = fitWeight((double)conv[id], (double)other[id], invGain, rn2x2);
       }
       om[i] = v;
-      omega[(size_t)s * wCols + i] = v;
+      if(blockIdx.y == 0) omega[(size_t)s * wCols + i] = v;
     }
   }
-  int ei[GQ_E], ej[GQ_E];
-  double acc[GQ_E];
-#pragma unroll
-  for(int e = 0; e < GQ_E; e++) {
-    int idx = tid + e * FILL_THREADS;
-    acc[e] = 0.0;
-    ei[e] = -1;
-    ej[e] = 0;
-    if(idx < nEnt) {
-      // idx -> (i, j), i >= j, row-major lower triangle
-      int i = (int)((sqrt(8.0 * idx + 1.0) - 1.0) * 0.5);
-      while((i + 1) * (i + 2) / 2 <= idx) i++;
-      while(i * (i + 1) / 2 > idx) i--;
-      ei[e] = i;
-      ej[e] = idx - i * (i + 1) / 2;
-    }
-  }
-  for(int k0 = 0; k0 < wCols; k0 += GQ_KT) {
-    const int kt = min(GQ_KT, wCols - k0);
-    for(int i = tid; i < R * GQ_KT; i += FILL_THREADS) {
-      int r = i / GQ_KT, kk = i % GQ_KT;
-      tile[r * (GQ_KT + 1) + kk] = kk < kt ? Ws[(size_t)r * wCols + k0 + kk] : 0.0;
-    }
-    __syncthreads();
-#pragma unroll
-    for(int e = 0; e < GQ_E; e++) {
-      if(ei[e] < 0) continue;
-      const double* a = tile + ei[e] * (GQ_KT + 1);
-      const double* b = tile + ej[e] * (GQ_KT + 1);
-      double q = acc[e];
-      if(omega) {
-        for(int kk = 0; kk < kt; kk++) q += a[kk] * (b[kk] * om[k0 + kk]);
-      } else {
-        for(int kk = 0; kk < kt; kk++) q += a[kk] * b[kk];
+  if(blockIdx.y == gridDim.y - 1) {
+    // zeros of the Q buffer: row 0, column 0 and above the diagonal
+    for(int i = tid; i < qCount * qCount; i += NT)
+      if(i % qCount > i / qCount || i % qCount == 0) Qs[i] = 0.0;
+    // B: W[i-1] . other image, x outer / y inner (column-major)
+    double* sub = tile;
+    if(live)
+      for(int i = tid; i < wCols; i += NT) {
+        int x = i % fSS - hSS, y = i / fSS - hSS;
+        int gx = min(max(x + c.x, 0), w - 1), gy = min(max(y + c.y, 0), h - 1);
+        sub[i] = (double)other[(size_t)gx + (size_t)gy * w];
       }
-      acc[e] = q;
+    __syncthreads();
+    for(int i = tid; i < qCount; i += NT) {
+      double p0 = 0.0;
+      if(live && i > 0) {
+        const double* wr = Ws + (size_t)(i - 1) * wCols;
+        for(int x = 0; x < fSS; x++) {
+          const double* wx = wr + x;
+          const double* sx = sub + x;
+          const double* ox = om + x;
+#pragma unroll 8
+          for(int y = 0; y < fSS; y++)
+            p0 += omega ? wx[(size_t)fSS * y] * (sx[fSS * y] * ox[fSS * y])
+                        : wx[(size_t)fSS * y] * sx[fSS * y];
+        }
+      }
+      Bs[i] = p0;
+    }
+    return;
+  }
+  // idx -> (i, j), i >= j, row-major lower triangle
+  auto rowOf = [](int idx) {
+    int i = (int)((sqrtf(8.f * (float)idx + 1.f) - 1.f) * 0.5f);
+    while((i + 1) * (i + 2) / 2 <= idx) i++;
+    while(i * (i + 1) / 2 > idx) i--;
+    return i;
+  };
+  const int idx = blockIdx.y * NT + tid;
+  const int rows = rowOf(min((int)(blockIdx.y + 1) * NT, nEnt) - 1) + 1;  // rows of W needed
+  const int ei = idx < nEnt ? rowOf(idx) : 0, ej = idx < nEnt ? idx - ei * (ei + 1) / 2 : 0;
+  const int tileLen = rows * (GQ_KT + 1), nT = (wCols + GQ_KT - 1) / GQ_KT;
+  auto load = [&](int t) {
+    const int k = t * GQ_KT + (tid & 31);
+    double* dst = tile + (t & 1) * tileLen + (tid & 31);
+    if(k < wCols)
+      for(int r = tid >> 5; r < rows; r += NT / 32)
+        cpAsync8(dst + r * (GQ_KT + 1), Ws + (size_t)r * wCols + k);
+    cpAsyncCommit();
+  };
+  load(0);
+  double q = 0.0;
+  for(int t = 0; t < nT; t++) {
+    if(t + 1 < nT) {
+      load(t + 1);
+      cpAsyncWaitGroup<1>();
+    } else {
+      cpAsyncWaitGroup<0>();
+    }
+    __syncthreads();
+    const double* a = tile + (t & 1) * tileLen + ei * (GQ_KT + 1);
+    const double* b = tile + (t & 1) * tileLen + ej * (GQ_KT + 1);
+    const int kt = min(GQ_KT, wCols - t * GQ_KT);
+    if(omega) {
+      const double* o = om + t * GQ_KT;
+#pragma unroll 4
+      for(int kk = 0; kk < kt; kk++) q += a[kk] * (b[kk] * o[kk]);
+    } else if(kt == GQ_KT) {
+#pragma unroll 8
+      for(int kk = 0; kk < GQ_KT; kk++) q += a[kk] * b[kk];
+    } else {
+      for(int kk = 0; kk < kt; kk++) q += a[kk] * b[kk];
     }
     __syncthreads();
   }
-  // Q buffer: entry (i+1, j+1) for the triangle, zero elsewhere
-  for(int i = tid; i < qCount * qCount; i += FILL_THREADS) Qs[i] = 0.0;
-  __syncthreads();
-#pragma unroll
-  for(int e = 0; e < GQ_E; e++)
-    if(ei[e] >= 0) Qs[(size_t)(ei[e] + 1) * qCount + (ej[e] + 1)] = acc[e];
-  // B: W[i-1] . other image, x outer / y inner (column-major)
-  if(live) {
-    const int2 c = ssxy[(size_t)s * maxSS + cur[s]];
-    for(int i = tid; i < wCols; i += FILL_THREADS) {
-      int x = i % fSS - hSS, y = i / fSS - hSS;
-      int gx = min(max(x + c.x, 0), w - 1), gy = min(max(y + c.y, 0), h - 1);
-      sub[i] = (double)other[(size_t)gx + (size_t)gy * w];
+  if(idx < nEnt) Qs[(size_t)(ei + 1) * qCount + (ej + 1)] = q;
+}
+
+// ------------------------------------------------------- per-stamp dots ---
+// The W dot products the global matrix needs (cd.cl:199-261,
+// cdkscUtil.cpp:363-392) and the background projections of both RHS forms:
+//   dots[s][0 .. nC1*nBG)            W[i1] . W[bg]       (i1 = 1..nC1)
+//   dots[s][nC1*nBG + ib]            W[0]  . W[bg ib]
+//   dots[s][.. + nBG + ib*nBG + jb]  W[bg ib] . W[bg jb]  (jb <= ib)
+//   dots[s][.. + nBG*nBG + ib]       W[bg ib] . O, row-major, FP64 (cd.cl:331-339)
+//   dots[s][.. + nBG + ib]           W[bg ib] . float(O), column-major
+//                                    (cdkscUtil.cpp:459-469)
+// Every dot runs in ascending pixel order (or the stated order) per thread.
+// Made when a stamp is filled: they change only with its substamp, so a refit
+// makes those of the refilled stamps only.
+// A CTA owns DOT_THREADS products of a stamp, whose rows of W stream through
+// two shared-memory tiles, the last CTA of a stamp (blockIdx.y) the background
+// projections: 961 chained sums of 62 cycles, so spreading a stamp over CTAs is
+// what shortens it (one CTA per stamp, the projections after the products and
+// from dependent global loads, took 0.46 ms for 256 stamps; now 0.27 ms, 0.09 ms for one stamp).
+constexpr int DOT_THREADS = 64, DOT_KT = 32, DOT_MAX = 1024;
+struct DotPair {
+  int ra, rb, oi;  // rows of W and output index; ra < 0: none
+};
+__device__ __forceinline__ DotPair dotPair(int pi, int nC1, int nPSF, int nBG) {
+  const int nKB = nC1 * nBG;
+  if(pi < nKB) return {1 + pi / nBG, nPSF + pi % nBG, pi};
+  if(pi < nKB + nBG) return {0, nPSF + (pi - nKB), pi};
+  const int e = pi - nKB - nBG, ib = e / nBG, jb = e % nBG;
+  if(ib < nBG && jb <= ib) return {nPSF + ib, nPSF + jb, nKB + nBG + ib * nBG + jb};
+  return {-1, -1, -1};
+}
+template <class T>
+__global__ void __launch_bounds__(DOT_THREADS)
+    k_stamp_dots(const int* __restrict__ list, const int* __restrict__ count,
+                 const int* __restrict__ cur, const int2* __restrict__ ssxy, int maxSS,
+                 const double* __restrict__ W, int wRows, int hSS, int nPSF, int nBG,
+                 const T* __restrict__ O, int w, int h, double* __restrict__ dots, int stride,
+                 int rowsAt, const double* __restrict__ omega) {
+  extern __shared__ double dot_s[];
+  const int s = list[blockIdx.x], tid = threadIdx.x;
+  const int fSS = 2 * hSS + 1, wCols = fSS * fSS, nC1 = nPSF - 1;
+  const double* Ws = W + (size_t)s * wRows * wCols;
+  double* out = dots + (size_t)s * stride;
+  const int nKB = nC1 * nBG, nPairs = nKB + nBG + nBG * nBG;
+  double* om = dot_s;                         // wCols pixel weights (weighted fit)
+  double* tile = om + (omega ? wCols : 0);    // 2 x rows x (DOT_KT+1), or the image values
+  if(omega)
+    for(int i = tid; i < wCols; i += DOT_THREADS) om[i] = omega[(size_t)s * wCols + i];
+  if(blockIdx.y == gridDim.y - 1) {
+    // background projections on the other image, as many background rows at a
+    // time as `rowsAt` says fit behind the image values (and those as floats)
+    const bool live = cur[s] < count[s];
+    double* sub = tile;
+    double* subF = sub + wCols;
+    double* bg = subF + wCols;
+    if(live) {
+      const int2 c = ssxy[(size_t)s * maxSS + cur[s]];
+      for(int i = tid; i < wCols; i += DOT_THREADS) {
+        int x = i % fSS - hSS, y = i / fSS - hSS;
+        int gx = min(max(x + c.x, 0), w - 1), gy = min(max(y + c.y, 0), h - 1);
+        sub[i] = (double)O[(size_t)gx + (size_t)gy * w];
+        subF[i] = (double)(float)sub[i];
+      }
     }
-  }
-  __syncthreads();
-  for(int i = tid; i < qCount; i += FILL_THREADS) {
-    double p0 = 0.0;
-    if(live && i > 0) {
-      const double* wr = Ws + (size_t)(i - 1) * wCols;
-      for(int x = 0; x < fSS; x++)
-        for(int y = 0; y < fSS; y++) {
-          int k = x + fSS * y;
-          p0 += omega ? wr[k] * (sub[k] * om[k]) : wr[k] * sub[k];
-        }
+    for(int b0 = 0; b0 < nBG; b0 += rowsAt) {
+      const int nb = min(rowsAt, nBG - b0);
+      __syncthreads();
+#pragma unroll 8
+      for(int i = tid; i < nb * wCols; i += DOT_THREADS) bg[i] = Ws[(size_t)(nPSF + b0) * wCols + i];
+      __syncthreads();
+      // lanes 0..nb-1 row-major, the next nb column-major
+      for(int e = tid; e < 2 * nb; e += DOT_THREADS) {
+        const bool byCol = e >= nb;
+        const double* wb = bg + (size_t)(e % nb) * wCols;
+        const double* o = byCol ? subF : sub;
+        double q = 0.0;
+        if(live)
+          for(int a = 0; a < fSS; a++) {
+            const int k0 = byCol ? a : a * fSS, dk = byCol ? fSS : 1;
+#pragma unroll 8
+            for(int i = 0; i < fSS; i++) {
+              const int k = k0 + i * dk;
+              q += omega ? wb[k] * (o[k] * om[k]) : wb[k] * o[k];
+            }
+          }
+        out[nPairs + (byCol ? nBG : 0) + b0 + e % nb] = q;
+      }
     }
-    Bs[i] = p0;
+    return;
   }
+  // rows of this CTA's products: the background rows, row 0 and, while it has
+  // products of kernel rows, those from rLo on
+  const int p0 = blockIdx.y * DOT_THREADS, pi = p0 + tid;
+  const int rLo = min(1 + p0 / nBG, nC1 + 1), rHi = min(1 + (p0 + DOT_THREADS - 1) / nBG, nC1);
+  const int rows = 1 + nBG + max(rHi - rLo + 1, 0);
+  auto rowAt = [&](int slot) { return slot == 0 ? 0 : slot <= nBG ? nPSF + slot - 1 : rLo + slot - 1 - nBG; };
+  auto slotOf = [&](int r) { return r == 0 ? 0 : r >= nPSF ? 1 + r - nPSF : 1 + nBG + r - rLo; };
+  const DotPair dp = pi < nPairs ? dotPair(pi, nC1, nPSF, nBG) : DotPair{-1, -1, -1};
+  const int sa = dp.ra < 0 ? 0 : slotOf(dp.ra), sb = dp.ra < 0 ? 0 : slotOf(dp.rb);
+  const int tileLen = rows * (DOT_KT + 1), nT = (wCols + DOT_KT - 1) / DOT_KT;
+  auto load = [&](int kt) {
+    const int k = kt * DOT_KT + (tid & 31);
+    double* dst = tile + (kt & 1) * tileLen + (tid & 31);
+    if(k < wCols)
+      for(int r = tid >> 5; r < rows; r += DOT_THREADS / 32)
+        cpAsync8(dst + r * (DOT_KT + 1), Ws + (size_t)rowAt(r) * wCols + k);
+    cpAsyncCommit();
+  };
+  load(0);
+  double acc = 0.0;
+  for(int kt = 0; kt < nT; kt++) {
+    if(kt + 1 < nT) {
+      load(kt + 1);
+      cpAsyncWaitGroup<1>();
+    } else {
+      cpAsyncWaitGroup<0>();
+    }
+    __syncthreads();
+    const double* a = tile + (kt & 1) * tileLen + sa * (DOT_KT + 1);
+    const double* b = tile + (kt & 1) * tileLen + sb * (DOT_KT + 1);
+    const int len = min(DOT_KT, wCols - kt * DOT_KT);
+    if(omega) {
+      const double* o = om + kt * DOT_KT;
+#pragma unroll 4
+      for(int kk = 0; kk < len; kk++) acc += a[kk] * (b[kk] * o[kk]);
+    } else if(len == DOT_KT) {
+#pragma unroll 8
+      for(int kk = 0; kk < DOT_KT; kk++) acc += a[kk] * b[kk];
+    } else {
+      for(int kk = 0; kk < len; kk++) acc += a[kk] * b[kk];
+    }
+    __syncthreads();
+  }
+  if(dp.ra >= 0) out[dp.oi] = acc;
 }
 
 }  // namespace
@@ -249,9 +411,11 @@ void fillStamps(xb_ctx* c, int si, const int* dList, int nList, int imgConv, con
   StampSetDev& S = c->set[si];
   const int nGroups = (int)c->basis.yGroupStart.size() - 1;
   const int tw = 2 * (g.hSS + g.hK) + 1, th = g.fSS;
-  size_t smemFill = (size_t)(tw * tw + th * tw + 2) * sizeof(float) + 2 * g.fK * sizeof(double);
+  const size_t smemFill = ((size_t)tw * tw + (size_t)th * tw + 2 * g.fK) * sizeof(double);
   dim3 grid(nList, nGroups);
   double* W = (double*)S.W;
+  XB_CUDA(allowMaxDynamicSmem((const void*)k_fill_w<double>, c->device));
+  XB_CUDA(allowMaxDynamicSmem((const void*)k_fill_w<float>, c->device));
   { KT_SCOPE(c, "fill_w");
   if(c->imgIsF64)
     k_fill_w<double><<<grid, FILL_THREADS, smemFill, c->stream>>>(
@@ -265,32 +429,60 @@ void fillStamps(xb_ctx* c, int si, const int* dList, int nList, int imgConv, con
   }
   int2* bgXY = buf<int2>(c, "bgXY", g.nBG);
   { KT_SCOPE(c, "fill_finish");
-  k_fill_finish<<<nList, FILL_THREADS, 0, c->stream>>>(dList, S.count, S.cur, S.ssxy, g.maxSS,
+  k_fill_finish<<<dim3(nList, g.nPSF - 1 + g.nBG), FILL_THREADS, 0, c->stream>>>(dList, S.count, S.cur, S.ssxy, g.maxSS,
                                                        c->dKx, c->dKy, g.nPSF, bgXY, g.nBG,
                                                        g.hSS, c->w, c->h, g.wRows, W);
   XB_LAUNCHED(c);
   }
-  size_t smemGram = ((size_t)(g.qCount - 1) * (GQ_KT + 1) + 2 * (size_t)g.wCols) * sizeof(double);
   const double invGain = noiseInvGain(c->p), rn2x2 = noiseRn2x2(c->p);
   double* omega = c->p.fitWeighted ? S.omega : nullptr;
   const int other = 1 - imgConv;
+  const size_t smemGram = (std::max((size_t)2 * (g.qCount - 1) * (GQ_KT + 1), (size_t)g.wCols) +
+                           (omega ? (size_t)g.wCols : 0)) * sizeof(double);
+  const int nEnt = (g.qCount - 1) * g.qCount / 2;
+  // 128 entries per CTA where the list fills the SMs, else 64
+  auto gram = [&](auto* img, auto kernel, int nt) {
+    XB_CUDA(allowMaxDynamicSmem((const void*)kernel, c->device));
+    kernel<<<dim3(nList, (nEnt + nt - 1) / nt + 1), nt, smemGram, c->stream>>>(
+        img, (decltype(img))c->img[imgConv], c->w, c->h, dList, S.count, S.cur, S.ssxy, g.maxSS,
+        g.hSS, g.wRows, g.qCount, W, S.Q, S.B, invGain, rn2x2, omega);
+  };
+  const bool wide = (long long)nList * nEnt > 2ll * 256 * c->smCount;
   { KT_SCOPE(c, "gram_qb");
-  if(c->imgIsF64)
-    k_gram_qb<double><<<nList, FILL_THREADS, smemGram, c->stream>>>(
-        (const double*)c->img[other], (const double*)c->img[imgConv], c->w, c->h, dList, S.count,
-        S.cur, S.ssxy, g.maxSS, g.hSS, g.wRows, g.qCount, W, S.Q, S.B, invGain, rn2x2, omega);
-  else
-    k_gram_qb<float><<<nList, FILL_THREADS, smemGram, c->stream>>>(
-        (const float*)c->img[other], (const float*)c->img[imgConv], c->w, c->h, dList, S.count,
-        S.cur, S.ssxy, g.maxSS, g.hSS, g.wRows, g.qCount, W, S.Q, S.B, invGain, rn2x2, omega);
+  if(c->imgIsF64) {
+    if(wide) gram((const double*)c->img[other], k_gram_qb<double, 128>, 128);
+    else gram((const double*)c->img[other], k_gram_qb<double, 64>, 64);
+  } else {
+    if(wide) gram((const float*)c->img[other], k_gram_qb<float, 128>, 128);
+    else gram((const float*)c->img[other], k_gram_qb<float, 64>, 64);
+  }
+  XB_LAUNCHED(c);
+  }
+  const int nPairs = g.nComp1 * g.nBG + g.nBG + g.nBG * g.nBG;
+  const int maxRows = 1 + g.nBG + std::min(g.nComp1, DOT_THREADS / g.nBG + 2);
+  // background rows staged at a time: all of them, or what 96 KB hold
+  const int rowsAt = std::max(1, std::min(g.nBG, (int)((96 << 10) / (g.wCols * sizeof(double)))));
+  const size_t smemDots = (std::max((size_t)2 * maxRows * (DOT_KT + 1), (size_t)(2 + rowsAt) * g.wCols) +
+                           (omega ? (size_t)g.wCols : 0)) * sizeof(double);
+  auto dots = [&](auto* img, auto kernel) {
+    XB_CUDA(allowMaxDynamicSmem((const void*)kernel, c->device));
+    kernel<<<dim3(nList, (nPairs + DOT_THREADS - 1) / DOT_THREADS + 1), DOT_THREADS, smemDots,
+             c->stream>>>(dList, S.count, S.cur, S.ssxy, g.maxSS, W, g.wRows, g.hSS, g.nPSF, g.nBG,
+                          img, c->w, c->h, S.dots, plainDotStride(g), rowsAt, omega);
+  };
+  { KT_SCOPE(c, "stamp_dots");
+  if(c->imgIsF64) dots((const double*)c->img[other], k_stamp_dots<double>);
+  else dots((const float*)c->img[other], k_stamp_dots<float>);
   XB_LAUNCHED(c);
   }
 }
 
 void stageCmv(xb_ctx* c) {
   const Geo& g = c->g;
-  if((g.qCount - 1) * (g.qCount) / 2 > GQ_E * FILL_THREADS)
+  if((g.qCount - 1) * (g.qCount) / 2 > GQ_MAXENT)
     throw XbError{XB_ERR_UNSUPPORTED, "too many basis functions for the Gram kernel"};
+  if(!mixedMode(c) && g.nComp1 * g.nBG + g.nBG + g.nBG * g.nBG > DOT_MAX)
+    throw XbError{XB_ERR_UNSUPPORTED, "too many basis and background terms for the dot kernel"};
   // basis tables (host-built once per context) and background exponents
   std::vector<int2> bg(g.nBG);
   for(int b = 0; b < g.nBG; b++) bg[b] = make_int2(c->basis.bgX[b], c->basis.bgY[b]);
@@ -304,6 +496,7 @@ void stageCmv(xb_ctx* c) {
       S.dots = buf<double>(c, "dots" + sfx, (size_t)std::max(S.n, 1) * mixedDotStride(g));
     } else {
       S.W = buf<double>(c, "W" + sfx, (size_t)std::max(S.n, 1) * g.wRows * g.wCols);
+      S.dots = buf<double>(c, "dots" + sfx, (size_t)std::max(S.n, 1) * plainDotStride(g));
       S.omega = c->p.fitWeighted ? buf<double>(c, "omega" + sfx, (size_t)std::max(S.n, 1) * g.wCols)
                                  : nullptr;
     }

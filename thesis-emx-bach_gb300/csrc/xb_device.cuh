@@ -48,6 +48,29 @@ __device__ __forceinline__ double ipowD(double x, int n) {
   return r;
 }
 
+// (double)(float)t without the two conversions (each takes an FP64 issue slot
+// here): round the bits to 24 significant ones, ties to even.  Values whose
+// float is subnormal, zero, infinite or NaN, or could overflow, convert.
+__device__ __forceinline__ double roundToFloat(double t) {
+  const long long b = __double_as_longlong(t);
+  const unsigned e = (unsigned)(b >> 52) & 0x7FFu;
+  if(e - 897u >= 253u) return (double)(float)t;  // below 2^-126 or from 2^127 up
+  return __longlong_as_double((b + 0x0FFFFFFFll + ((b >> 29) & 1)) & ~0x1FFFFFFFll);
+}
+
+// Copies of 8 bytes to shared memory that complete asynchronously, in groups.
+__device__ __forceinline__ void cpAsync8(void* dst, const void* src) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(
+                   (unsigned)__cvta_generic_to_shared(dst)),
+               "l"(src)
+               : "memory");
+}
+__device__ __forceinline__ void cpAsyncCommit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+template <int N>
+__device__ __forceinline__ void cpAsyncWaitGroup() {
+  asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
+}
+
 // OR `bits` into the 16-bit mask entry i with a 32-bit atomic on its
 // aligned word (the mask buffer carries two spare entries at the end).
 __device__ __forceinline__ void maskOr(uint16_t* m, size_t i, uint16_t bits) {

@@ -259,212 +259,135 @@ __global__ void __launch_bounds__(256)
 
 // ---------------------------------------------------- spatial weights -----
 // createMatrixWeights (cd.cl:152-180) = the weight loop of CPU createMatrix
-// (cdkscUtil.cpp:331-342).
-__global__ void k_weights(const int* __restrict__ list, int nList, const int* __restrict__ liveN,
-                          const int* __restrict__ count, const int* __restrict__ cur,
-                          const int2* __restrict__ ssxy, int maxSS, const int2* __restrict__ kp,
-                          int nC2, int w, int h, double* __restrict__ wts) {
-  if(liveN) nList = min(nList, *liveN);
-  int e = blockIdx.x * blockDim.x + threadIdx.x;
-  if(e >= nList * nC2) return;
-  int t = e / nC2, k = e % nC2, s = list[t];
-  double a = 0.0;
-  if(cur[s] < count[s]) {
-    int2 c = ssxy[(size_t)s * maxSS + cur[s]];
-    a = ipowD(floatNormD(c.x, w), kp[k].x) * ipowD(floatNormD(c.y, h), kp[k].y);
-  }
-  wts[e] = a;
-}
-
-// ------------------------------------------------------- per-stamp dots ---
-// The W dot products the global matrix needs (cd.cl:199-261,
-// cdkscUtil.cpp:363-392) and the background projections of both RHS forms:
-//   dots[t][0 .. nC1*nBG)            W[i1] . W[bg]       (i1 = 1..nC1)
-//   dots[t][nC1*nBG + ib]            W[0]  . W[bg ib]
-//   dots[t][.. + nBG + ib*nBG + jb]  W[bg ib] . W[bg jb]  (jb <= ib)
-//   dots[t][.. + nBG*nBG + ib]       W[bg ib] . O, row-major, FP64 (cd.cl:331-339)
-//   dots[t][.. + nBG + ib]           W[bg ib] . float(O), column-major
-//                                    (cdkscUtil.cpp:459-469)
-// Every dot runs in ascending pixel order (or the stated order) per thread.
-constexpr int DOT_THREADS = 256, DOT_KT = 32, DOT_PAIRS = 4;
-template <class T>
-__global__ void __launch_bounds__(DOT_THREADS)
-    k_stamp_dots(const int* __restrict__ list, const int* __restrict__ count,
-                 const int* __restrict__ cur, const int2* __restrict__ ssxy, int maxSS,
-                 const double* __restrict__ W, int wRows, int hSS, int nPSF, int nBG,
-                 const T* __restrict__ O, int w, int h, double* __restrict__ dots, int stride,
-                 const double* __restrict__ omega) {
-  extern __shared__ double dot_s[];
-  const int t = blockIdx.x, s = list[t], tid = threadIdx.x;
-  const int fSS = 2 * hSS + 1, wCols = fSS * fSS, nC1 = nPSF - 1;
-  const double* Ws = W + (size_t)s * wRows * wCols;
-  double* out = dots + (size_t)t * stride;
-  const bool live = cur[s] < count[s];
-  double* tile = dot_s;                       // wRows x (DOT_KT+1)
-  double* sub = dot_s + wRows * (DOT_KT + 1); // wCols (image) values
-  double* om = sub + wCols;                   // wCols pixel weights (weighted fit)
-  if(omega)
-    for(int i = tid; i < wCols; i += DOT_THREADS) om[i] = omega[(size_t)s * wCols + i];
-  // products: the (rowA, rowB) pairs tid, tid + DOT_THREADS, ... (up to
-  // DOT_PAIRS per thread; the host checks the bound), each summed over the
-  // pixels in ascending order
-  const int nKB = nC1 * nBG, nPairs = nKB + nBG + nBG * nBG;
-  int ra[DOT_PAIRS], rb[DOT_PAIRS], oi[DOT_PAIRS];
-  double acc[DOT_PAIRS];
-#pragma unroll
-  for(int q = 0; q < DOT_PAIRS; q++) {
-    const int pi = tid + q * DOT_THREADS;
-    ra[q] = rb[q] = oi[q] = -1;
-    acc[q] = 0.0;
-    if(pi >= nPairs) continue;
-    if(pi < nKB) {
-      ra[q] = 1 + pi / nBG;
-      rb[q] = nPSF + pi % nBG;
-      oi[q] = pi;
-    } else if(pi < nKB + nBG) {
-      ra[q] = 0;
-      rb[q] = nPSF + (pi - nKB);
-      oi[q] = pi;
-    } else {
-      int e = pi - nKB - nBG, ib = e / nBG, jb = e % nBG;
-      if(jb <= ib) {
-        ra[q] = nPSF + ib;
-        rb[q] = nPSF + jb;
-        oi[q] = nKB + nBG + ib * nBG + jb;
-      }
+// (cdkscUtil.cpp:331-342), as the table of products the matrix entries use:
+// pw[t][a][b] = w_a w_b over the nC2 weights and, at index nC2, a one; and the
+// listed stamps, exhausted ones with bit 31 set.
+__global__ void __launch_bounds__(128)
+    k_weights(const int* __restrict__ list, const int* __restrict__ count,
+              const int* __restrict__ cur, const int2* __restrict__ ssxy, int maxSS,
+              const int2* __restrict__ kp, int nC2, int w, int h, double* __restrict__ pw,
+              int* __restrict__ stamps) {
+  extern __shared__ double wt_s[];
+  const int t = blockIdx.x, s = list[t], tid = threadIdx.x, n1 = nC2 + 1;
+  if(tid == 0) stamps[t] = cur[s] < count[s] ? s : s | INT_MIN;
+  for(int k = tid; k < n1; k += 128) {
+    double a = k == nC2 ? 1.0 : 0.0;
+    if(k < nC2 && cur[s] < count[s]) {
+      int2 c = ssxy[(size_t)s * maxSS + cur[s]];
+      a = ipowD(floatNormD(c.x, w), kp[k].x) * ipowD(floatNormD(c.y, h), kp[k].y);
     }
-  }
-  for(int k0 = 0; k0 < wCols; k0 += DOT_KT) {
-    const int kt = min(DOT_KT, wCols - k0);
-    for(int i = tid; i < wRows * DOT_KT; i += DOT_THREADS) {
-      int r = i / DOT_KT, kk = i % DOT_KT;
-      tile[r * (DOT_KT + 1) + kk] = kk < kt ? Ws[(size_t)r * wCols + k0 + kk] : 0.0;
-    }
-    __syncthreads();
-#pragma unroll
-    for(int q = 0; q < DOT_PAIRS; q++) {
-      if(ra[q] < 0) continue;
-      const double* pa = tile + ra[q] * (DOT_KT + 1);
-      const double* pb = tile + rb[q] * (DOT_KT + 1);
-      double a = acc[q];
-      if(omega) {
-        for(int kk = 0; kk < kt; kk++) a += pa[kk] * (pb[kk] * om[k0 + kk]);
-      } else {
-        for(int kk = 0; kk < kt; kk++) a += pa[kk] * pb[kk];
-      }
-      acc[q] = a;
-    }
-    __syncthreads();
-  }
-#pragma unroll
-  for(int q = 0; q < DOT_PAIRS; q++)
-    if(ra[q] >= 0) out[oi[q]] = acc[q];
-  // background projections on the other image
-  const int base = nKB + nBG + nBG * nBG;
-  if(live) {
-    const int2 c = ssxy[(size_t)s * maxSS + cur[s]];
-    for(int i = tid; i < wCols; i += DOT_THREADS) {
-      int x = i % fSS - hSS, y = i / fSS - hSS;
-      int gx = min(max(x + c.x, 0), w - 1), gy = min(max(y + c.y, 0), h - 1);
-      sub[i] = (double)O[(size_t)gx + (size_t)gy * w];
-    }
+    wt_s[k] = a;
   }
   __syncthreads();
-  if(tid < 2 * nBG) {
-    const int ib = tid % nBG;
-    const double* wb = Ws + (size_t)(nPSF + ib) * wCols;
-    double q = 0.0;
-    if(live) {
-      if(tid < nBG) {
-        for(int k = 0; k < wCols; k++) q += omega ? wb[k] * (sub[k] * om[k]) : wb[k] * sub[k];
-      } else {
-        for(int x = 0; x < fSS; x++)
-          for(int y = 0; y < fSS; y++) {
-            int k = x + fSS * y;
-            q += omega ? wb[k] * ((double)(float)sub[k] * om[k]) : wb[k] * (double)(float)sub[k];
-          }
-      }
-    }
-    out[base + tid] = q;
-  }
+  for(int e = tid; e < n1 * n1; e += 128)
+    pw[(size_t)t * n1 * n1 + e] = wt_s[e / n1] * wt_s[e % n1];
 }
 
 // ------------------------------------------------------ global matrix ------
 // Lower triangle of createMatrix (cd.cl:182-295 == cdkscUtil.cpp:307-402),
-// each entry summed over the listed stamps in order, then mirrored.
+// each entry summed over the listed stamps in order, then mirrored, and
+// createScProd: kernel terms and the constant term are common to both RHS
+// forms, the background terms come from the stamps' dots (bgBase selects the form).
+// Every term is a table weight (a product of two spatial weights, of which one
+// or both may be the one) times one number of the stamp; multiplying by one is
+// exact, so all entries run the same loop, eight stamps' loads ahead of its two
+// FP64 instructions (a chain of dependent loads per stamp took 340 us for 256
+// stamps and 190 us for the right-hand side; now 138 us for both).
 __global__ void __launch_bounds__(256)
-    k_build_matrix(const int* __restrict__ list, int nList, const int* __restrict__ count,
-                   const int* __restrict__ cur, const double* __restrict__ Q, int qc,
-                   const double* __restrict__ wts, const double* __restrict__ dots, int stride,
-                   int byStamp, int nC1, int nC2, int nBG, int matSize, double* __restrict__ M) {
-  const int ld = matSize + 1, nComp = nC1 * nC2;
+    k_build_system(const int* __restrict__ stamps, int nList, const double* __restrict__ Q,
+                   const double* __restrict__ B, int qc, const double* __restrict__ pw,
+                   const double* __restrict__ dots, int stride, int bgBase, int nC1, int nC2,
+                   int nBG, int matSize, int nSol, double* __restrict__ M,
+                   double* __restrict__ res) {
+  const int ld = matSize + 1, nComp = nC1 * nC2, n1 = nC2 + 1, one = nC2;
   const long long nTri = (long long)matSize * (matSize + 1) / 2;
-  for(long long e = (long long)blockIdx.x * blockDim.x + threadIdx.x; e < nTri;
+  for(long long e = (long long)blockIdx.x * blockDim.x + threadIdx.x; e < nTri + nSol;
       e += (long long)gridDim.x * blockDim.x) {
-    // e -> (r, c) with 1 <= c <= r <= matSize
-    int r = (int)((sqrt(8.0 * (double)e + 1.0) - 1.0) * 0.5);
-    while((long long)(r + 1) * (r + 2) / 2 <= e) r++;
-    while((long long)r * (r + 1) / 2 > e) r--;
-    const int row = r + 1, col = (int)(e - (long long)r * (r + 1) / 2) + 1;
-    double m0 = 0.0;
-    for(int t = 0; t < nList; t++) {
-      const int s = list[t];
-      const double* Qs = Q + (size_t)s * qc * qc;
-      const double* wt = wts + (size_t)t * nC2;
-      const double* dt = dots + (size_t)(byStamp ? s : t) * stride;
-      if(row == 1 && col == 1) {
-        m0 += Qs[1 * qc + 1];
-      } else if(row > nComp + 1 && col > nComp + 1) {
-        m0 += dt[nC1 * nBG + nBG + (row - (nComp + 2)) * nBG + (col - (nComp + 2))];
-      } else if(col == 1 && row > nComp + 1) {
-        m0 += dt[nC1 * nBG + (row - (nComp + 2))];
-      } else if(row > nComp + 1 && col >= 2) {
-        int ib = row - (nComp + 2), i1 = (col - 2) / nC2 + 1, i2 = (col - 2) % nC2;
-        m0 += dt[(i1 - 1) * nBG + ib] * wt[i2];
-      } else if(col == 1 && row >= 2) {
-        int i = row - 2, i1 = i / nC2, i2 = i - i1 * nC2;
-        m0 += wt[i2] * Qs[(i1 + 2) * qc + 1];
+    const double* base;  // the stamp's number: base[stamp * stampStride]
+    size_t stampStride = stride;
+    int wa = one, wb = one, row = 0, col = 0;
+    const bool rhs = e >= nTri;
+    if(!rhs) {
+      // e -> (r, c) with 1 <= c <= r <= matSize
+      int r = (int)((sqrtf(8.f * (float)e + 1.f) - 1.f) * 0.5f);
+      while((long long)(r + 1) * (r + 2) / 2 <= e) r++;
+      while((long long)r * (r + 1) / 2 > e) r--;
+      row = r + 1;
+      col = (int)(e - (long long)r * (r + 1) / 2) + 1;
+      const int ib = row - (nComp + 2);
+      if(ib >= 0) {
+        if(col > nComp + 1) {
+          base = dots + nC1 * nBG + nBG + ib * nBG + (col - (nComp + 2));
+        } else if(col == 1) {
+          base = dots + nC1 * nBG + ib;
+        } else {
+          base = dots + ((col - 2) / nC2) * nBG + ib;
+          wa = (col - 2) % nC2;
+        }
       } else {
-        int i = row - 2, j = col - 2;
-        int i1 = i / nC2, i2 = i - i1 * nC2, j1 = j / nC2, j2 = j - j1 * nC2;
-        m0 += wt[i2] * wt[j2] * Qs[(i1 + 2) * qc + (j1 + 2)];
+        stampStride = (size_t)qc * qc;
+        int qi = 1, qj = 1;
+        if(row >= 2) {
+          qi = (row - 2) / nC2 + 2;
+          wa = (row - 2) % nC2;
+        }
+        if(col >= 2) {
+          qj = (col - 2) / nC2 + 2;
+          wb = (col - 2) % nC2;
+        }
+        base = Q + (size_t)qi * qc + qj;
+      }
+    } else {
+      const int id = (int)(e - nTri);
+      base = nullptr;
+      if(id == 1) {
+        base = B + 1;
+        stampStride = qc;
+      } else if(id >= 2 && id < nComp + 2) {
+        base = B + (id - 2) / nC2 + 2;
+        stampStride = qc;
+        wa = (id - 2) % nC2;
+      } else if(id >= nComp + 2 && id < nComp + 2 + nBG) {
+        base = dots + bgBase + (id - (nComp + 2));
+      }
+      if(!base) {
+        res[id] = 0.0;
+        continue;
       }
     }
-    M[(size_t)row * ld + col] = m0;
-    M[(size_t)col * ld + row] = m0;
+    const double* pwe = pw + wa * n1 + wb;
+    const size_t pwS = (size_t)n1 * n1;
+    double m0 = 0.0;
+    int t = 0;
+    for(; t + 8 <= nList; t += 8) {
+      double v[8], f[8];
+#pragma unroll
+      for(int u = 0; u < 8; u++) {
+        const int s = stamps[t + u];
+        v[u] = base[(size_t)(s & INT_MAX) * stampStride];
+        f[u] = pwe[(t + u) * pwS];
+        if(rhs && s < 0) v[u] = f[u] = 0.0;  // createScProd skips exhausted stamps
+      }
+#pragma unroll
+      for(int u = 0; u < 8; u++) m0 += f[u] * v[u];
+    }
+    for(; t < nList; t++) {
+      const int s = stamps[t];
+      if(rhs && s < 0) continue;
+      m0 += pwe[t * pwS] * base[(size_t)(s & INT_MAX) * stampStride];
+    }
+    if(rhs) {
+      res[e - nTri] = m0;
+    } else {
+      M[(size_t)row * ld + col] = m0;
+      M[(size_t)col * ld + row] = m0;
+    }
   }
   // row 0 / column 0 stay zero
   for(int i = blockIdx.x * blockDim.x + threadIdx.x; i < ld; i += gridDim.x * blockDim.x) {
     M[i] = 0.0;
     M[(size_t)i * ld] = 0.0;
   }
-}
-
-// createScProd: kernel terms and the constant term are common to both forms;
-// the background terms come from k_stamp_dots (form selects the column).
-__global__ void k_build_rhs(const int* __restrict__ list, int nList, const int* __restrict__ count,
-                            const int* __restrict__ cur, const double* __restrict__ B, int qc,
-                            const double* __restrict__ wts, const double* __restrict__ dots,
-                            int stride, int byStamp, int bgBase, int nC1, int nC2, int nBG,
-                            int nSol, double* __restrict__ res) {
-  const int id = blockIdx.x * blockDim.x + threadIdx.x;
-  if(id >= nSol) return;
-  const int nComp = nC1 * nC2;
-  double r0 = 0.0;
-  for(int t = 0; t < nList; t++) {
-    const int s = list[t];
-    if(cur[s] >= count[s]) continue;
-    const double* Bs = B + (size_t)s * qc;
-    if(id == 1) {
-      r0 += Bs[1];
-    } else if(id >= 2 && id < nComp + 2) {
-      int i = (id - 2) / nC2 + 1, j = (id - 2) % nC2;
-      r0 += Bs[i + 1] * wts[(size_t)t * nC2 + j];
-    } else if(id >= nComp + 2 && id < nComp + 2 + nBG) {
-      r0 += dots[(size_t)(byStamp ? s : t) * stride + bgBase + (id - (nComp + 2))];
-    }
-  }
-  res[id] = r0;
 }
 
 // ------------------------------------------------------ global LU ---------
@@ -905,11 +828,13 @@ __global__ void __launch_bounds__(SIG_THREADS)
     int ok = 0;
     if(live && gy < fSS) {
       const int j = gx + gy * fSS;
-      float m0 = (float)(sol1 * Ws[j]);
-      for(int i = 1; i < nPSF; i++) m0 = (float)((double)m0 + coeff[i] * Ws[(size_t)i * pix + j]);
+      // the model accumulates in float (cd.cl:489-531)
+      double m0 = roundToFloat(sol1 * Ws[j]);
+#pragma unroll 8
+      for(int i = 1; i < nPSF; i++) m0 = roundToFloat(m0 + coeff[i] * Ws[(size_t)i * pix + j]);
       const int ax = gx - fSS / 2 + c.x, ay = gy - fSS / 2 + c.y;
       const size_t ai = (size_t)min(max(ax, 0), w - 1) + (size_t)min(max(ay, 0), h - 1) * w;
-      const double tD = (double)m0, sD = (double)sImg[ai];
+      const double tD = m0, sD = (double)sImg[ai];
       const double diff = tD - sD + bg;
       if((mask[ai] & BAD_INPUT) == 0 && fabs(sD) > 1e-10) {
         if(isnan(tD) || isnan(sD)) {
@@ -1075,7 +1000,6 @@ __global__ void k_zero_ints(int* p, int n) {
 struct FitBuffers {
   int* list;
   double* wts;
-  double* dots;
   int stride;
   double* M;
   double* rhs;
@@ -1093,9 +1017,8 @@ static FitBuffers fitBuffers(xb_ctx* c, int nMax) {
   FitBuffers f{};
   const int ld = g.matSize + 1;
   f.list = buf<int>(c, "fit_list", std::max(nMax, 1));
-  f.wts = buf<double>(c, "fit_wts", (size_t)std::max(nMax, 1) * g.nComp2);
-  f.stride = g.nComp1 * g.nBG + g.nBG + g.nBG * g.nBG + 2 * g.nBG;
-  f.dots = buf<double>(c, "fit_dots", (size_t)std::max(nMax, 1) * f.stride);
+  f.wts = buf<double>(c, "fit_wts", mixedMode(c) ? 1 : (size_t)std::max(nMax, 1) * (g.nComp2 + 1) * (g.nComp2 + 1));
+  f.stride = plainDotStride(g);
   f.M = buf<double>(c, "fit_M", (size_t)ld * ld);
   f.rhs = buf<double>(c, "fit_rhs", std::max(g.nSol, ld));
   f.piv = buf<int>(c, "fit_piv", ld);
@@ -1125,51 +1048,25 @@ static void solveGlobal(xb_ctx* c, int si, const FitBuffers& f, const int* list,
   const Geo& g = c->g;
   StampSetDev& S = c->set[si];
   const bool mixed = mixedMode(c);
-  if(!mixed) {  // the mixed build forms its spatial weights itself
-  const int2* kp = kernelPowers(c);
-  const int nW = nList * g.nComp2;
-  { KT_SCOPE(c, "weights");
-  k_weights<<<(nW + 255) / 256, 256, 0, c->stream>>>(list, nList, liveN, S.count, S.cur, S.ssxy,
-                                                    g.maxSS, kp, g.nComp2, c->w, c->h, f.wts);
-  XB_LAUNCHED(c);
-  }
-  }
-  const double* dots = mixed ? S.dots : f.dots;  // mixed: filled per stamp by the Gram kernel
-  if(nList > 0 && !mixed) {
-    if(g.nComp1 * g.nBG + g.nBG + g.nBG * g.nBG > DOT_PAIRS * DOT_THREADS)
-      throw XbError{XB_ERR_UNSUPPORTED, "too many basis and background terms for the dot kernel"};
-    const size_t smem = ((size_t)g.wRows * (DOT_KT + 1) + 2 * (size_t)g.wCols) * sizeof(double);
-    const double* omega = c->p.fitWeighted ? S.omega : nullptr;
-    { KT_SCOPE(c, "stamp_dots");
-    if(c->imgIsF64)
-      k_stamp_dots<double><<<nList, DOT_THREADS, smem, c->stream>>>(
-          list, S.count, S.cur, S.ssxy, g.maxSS, (const double*)S.W, g.wRows, g.hSS, g.nPSF,
-          g.nBG, (const double*)c->img[other], c->w, c->h, f.dots, f.stride, omega);
-    else
-      k_stamp_dots<float><<<nList, DOT_THREADS, smem, c->stream>>>(
-          list, S.count, S.cur, S.ssxy, g.maxSS, (const double*)S.W, g.wRows, g.hSS, g.nPSF,
-          g.nBG, (const float*)c->img[other], c->w, c->h, f.dots, f.stride, omega);
-    XB_LAUNCHED(c);
-    }
-  }
   const int bgBase = g.nComp1 * g.nBG + g.nBG + g.nBG * g.nBG + (cpuRhs ? g.nBG : 0);
-  const long long nTri = (long long)g.matSize * (g.matSize + 1) / 2;
-  if(mixed) {
+  if(mixed) {  // forms its spatial weights itself; its dots are filled by the Gram kernel
     buildSystemMixed(c, si, list, nList, bgBase, f.M, dSol, liveN);
   } else {
-  { KT_SCOPE(c, "build_matrix");
-  k_build_matrix<<<(int)std::min<long long>((nTri + 255) / 256, c->smCount * 8), 256, 0, c->stream>>>(
-      list, nList, S.count, S.cur, S.Q, g.qCount, f.wts, dots, f.stride, mixed ? 1 : 0, g.nComp1,
-      g.nComp2, g.nBG, g.matSize, f.M);
-  XB_LAUNCHED(c);
-  }
-  { KT_SCOPE(c, "build_rhs");
-  k_build_rhs<<<(g.nSol + 127) / 128, 128, 0, c->stream>>>(list, nList, S.count, S.cur, S.B,
-                                                          g.qCount, f.wts, dots, f.stride,
-                                                          mixed ? 1 : 0, bgBase, g.nComp1,
-                                                          g.nComp2, g.nBG, g.nSol, dSol);
-  XB_LAUNCHED(c);
-  }
+    const int2* kp = kernelPowers(c);
+    const int n1 = g.nComp2 + 1;
+    { KT_SCOPE(c, "weights");
+    k_weights<<<nList, 128, n1 * sizeof(double), c->stream>>>(
+        list, S.count, S.cur, S.ssxy, g.maxSS, kp, g.nComp2, c->w, c->h, f.wts, f.list);
+    XB_LAUNCHED(c);
+    }
+    const long long nEnt = (long long)g.matSize * (g.matSize + 1) / 2 + g.nSol;
+    { KT_SCOPE(c, "build_matrix");
+    k_build_system<<<(int)std::min<long long>((nEnt + 255) / 256, c->smCount * 8), 256,
+                     0, c->stream>>>(f.list, nList, S.Q, S.B, g.qCount, f.wts, S.dots, f.stride,
+                                     bgBase, g.nComp1, g.nComp2, g.nBG, g.matSize, g.nSol, f.M,
+                                     dSol);
+    XB_LAUNCHED(c);
+    }
   }
   if(c->trace) {
     const int ld = g.matSize + 1;

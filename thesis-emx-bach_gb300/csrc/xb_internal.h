@@ -78,7 +78,7 @@ struct StampSetDev {
   double* B = nullptr;       // n * bCount
   float* Wf = nullptr;       // mixed mode: W [n][wRows][ld] as hi + lo floats, ld = wCols
   float* Wlo = nullptr;      //   padded to 32 (Wf the hi parts, Wlo the lo parts)
-  double* dots = nullptr;    // mixed mode: per-stamp dot table of the global matrix
+  double* dots = nullptr;    // per-stamp dot table of the global matrix
   double* omega = nullptr;   // plain mode, weighted fit: n * wCols pixel weights 1 / sigma^2
   const int* dN = nullptr;   // frame graphs: the kept count on the device (n is its bound)
 };
@@ -308,6 +308,10 @@ void stageConvSub(xb_ctx* c, bool doSub);
 // mixed-precision stages (xb_mixed.cu)
 int mixedLd(const Geo& g);
 int mixedDotStride(const Geo& g);
+// doubles per stamp of the plain path's dot table (k_stamp_dots, xb_cmv.cu)
+inline int plainDotStride(const Geo& g) {
+  return g.nComp1 * g.nBG + g.nBG + g.nBG * g.nBG + 2 * g.nBG;
+}
 void fillStampsMixed(xb_ctx* c, int si, const int* dList, int nList, int imgConv,
                      const int* liveN = nullptr);
 void sigsMixed(xb_ctx* c, int si, const int* dList, int nList, const double* dSol, int convImg,
