@@ -796,10 +796,14 @@ __device__ void fmInit(const T* img, const uint16_t* mask, int w, int cx, int cy
 }
 
 // Window maps over the columns [x0, x1] of the rows [k0, k1] (row maps) and
-// [r0, r1] (column maps), by the block scans of k_find_substamps_sm (van
-// Herk / Gil-Werman: prefix and suffix argmax / OR within blocks of the window
-// width; ties keep the smaller index), with 16-bit indices for stamps up to
-// 2048 pixels wide.
+// [r0, r1] (column maps), by block scans (van Herk / Gil-Werman): split the
+// line into blocks of the window width W, scan each forwards (prefix) and
+// backwards (suffix); the window [a, b] is then suffix(a) with prefix(b) when
+// they lie in different blocks, prefix(b) when a starts its block, suffix(a)
+// otherwise (b is then the line's end).  Ties keep the smaller index: the
+// prefix updates on a larger key, the suffix on a larger or equal one, and
+// prefix(b) wins only with a larger key.  16-bit indices for stamps up to 2048
+// pixels wide.
 __device__ void fmMaps(int n, int sx, int sy, int hSS, const uint8_t* flags, const uint8_t* bad,
                        const unsigned long long* key, unsigned short* hx, uint8_t* rowf, int* arg,
                        uint8_t* okw, unsigned short* tPA, unsigned short* tSA, uint8_t* tPO,
@@ -1117,16 +1121,31 @@ __global__ void __launch_bounds__(FM_THREADS)
 }
 
 // ------------------------------------------- substamp search in shared memory --
-// The decisions of k_find_substamps_maps for FP32 images, with the stamp's
-// pixels and every map in shared memory (15 B per pixel, one CTA per SM):
-// keys are the float bit patterns (ordered like the doubles of the reference
-// for positive values), the bad map is updated in place after an acceptance
-// (the skip bit it sets is part of this image's bad mask, and no other CTA
-// touches this image's bits of the stamp), and the two static predicates
-// (v - sky) / fwhm > tKF and !((v - sky) * (1/fwhm) < tKF), monotone in v,
-// become compares against their exact thresholds, found once per stamp by a
-// warp search over the ordered doubles; so does the pass threshold v > lim.
+// The decisions of k_find_substamps_maps for FP32 images, with the stamp in
+// shared memory at 6.4 bytes per pixel (pixel, flags, row winner, two bit
+// maps), so that stamps up to ~190 px fit and two 107-px ones share an SM:
+//   * a candidate's window maximum (the largest key, ties to the first in
+//     raster order) is found when the scan reaches the candidate, by one warp:
+//     a lane per row of the window reads that row's winner (hx, the maximum
+//     over the 2 hSS + 1 columns around the candidate's) and one reduction
+//     finds the first largest;
+//   * the window conditions "holds a bad pixel" and "holds a pixel above the
+//     stamp's threshold" are bit maps dilated by the window, so a lookup each;
+//     an acceptance turns its window bad, which ORs one rectangle into the
+//     first and can change hx only in the window's rows within hSS of it in x.
+// Keys are the float bit patterns (ordered like the doubles of the reference
+// for positive values); the two static predicates (v - sky) / fwhm > tKF and
+// !((v - sky) * (1/fwhm) < tKF), monotone in v, become compares against their
+// exact thresholds, found once per stamp by a warp search over the ordered
+// doubles; so does the pass threshold v > lim.
+// Two-dimensional maps of the winners and conditions by block scans, rebuilt
+// around every acceptance (15 bytes per pixel, one CTA per SM, stamps above
+// 123 px from global memory), took 0.55 ms for 2 x 256 stamps of 107 px and
+// 3.77 ms for 2 x 400 of 183; now FIND_MS.
 constexpr int FS_T = 512;
+constexpr uint8_t FS_BAD = 0x80;  // in the flags byte
+constexpr int FS_MAXN = 255;      // row winners are bytes, 0xFF none
+constexpr int FS_SEG = 8;         // columns per task of the row winners
 
 // One warp: smallest key in (lo, hi] at which pred turns true, given
 // pred(lo) false and pred(hi) true (pred monotone between them).
@@ -1157,9 +1176,31 @@ __device__ unsigned long long warpFirstTrue(unsigned long long lo, unsigned long
   return hi;
 }
 
-size_t fsSmemBytes(int n) { return (size_t)n * n * 15 + 64; }
+inline int fsWords(int n) { return (n + 31) / 32; }
+size_t fsSmemBytes(int n) {
+  return (((size_t)n * n * 6 + 3) & ~(size_t)3) + (size_t)3 * n * fsWords(n) * 4;
+}
 
-__global__ void __launch_bounds__(FS_T, 1)
+// Dilation of bit rows by r columns each way, in place, one thread per row
+// (at most 8 words, r < 64).
+__device__ void dilateRow(uint32_t* row, int nw, int r) {
+  uint32_t up[8], dn[8];
+#pragma unroll
+  for(int j = 0; j < 8; j++) up[j] = dn[j] = j < nw ? row[j] : 0u;
+  for(int len = 1; len < r + 1;) {
+    const int sh = min(min(len, r + 1 - len), 31);
+#pragma unroll
+    for(int j = 7; j >= 0; j--) up[j] |= (up[j] << sh) | (j > 0 ? up[j - 1] >> (32 - sh) : 0u);
+#pragma unroll
+    for(int j = 0; j < 8; j++) dn[j] |= (dn[j] >> sh) | (j < 7 ? dn[j + 1] << (32 - sh) : 0u);
+    len += sh;
+  }
+#pragma unroll
+  for(int j = 0; j < 8; j++)
+    if(j < nw) row[j] = up[j] | dn[j];
+}
+
+__global__ void __launch_bounds__(FS_T, 2)
     k_find_substamps_sm(const float* __restrict__ img0, const float* __restrict__ img1,
                         uint16_t* __restrict__ mask, const int4* __restrict__ geom,
                         const double* __restrict__ sky0, const double* __restrict__ fwhm0,
@@ -1179,38 +1220,38 @@ __global__ void __launch_bounds__(FS_T, 1)
       (uint16_t)((MASK_ALL & ~OK_CONV) & ~(im == 0 ? (BAD_PIXEL_S | SKIP_S) : (BAD_PIXEL_T | SKIP_T)));
   const uint16_t skipMask = im == 0 ? SKIP_T : SKIP_S;
   const int4 gm = geom[s];
-  const int cx = gm.x, cy = gm.y, sx = gm.z, sy = gm.w, n = fSW, N = n * n;
+  const int cx = gm.x, cy = gm.y, sx = gm.z, sy = gm.w, n = fSW, N = n * n, nw = (n + 31) / 32;
   const double invFwhm = 1.0 / fwhm;
   float* V = (float*)fs_s;                 // N pixel values
-  uint16_t* arg = (uint16_t*)(V + N);      // N (0xFFFF: none)
-  uint8_t* flags = (uint8_t*)(arg + N);    // N
-  uint8_t* bad = flags + N;                // N
-  uint8_t* hx = bad + N;                   // N (0xFF: none)
-  uint8_t* rowf = hx + N;                  // N
-  uint8_t* okw = rowf + N;                 // N
-  // block scans of the map build: prefix / suffix argmax (index in the row
-  // or column, 0xFF: none) and prefix / suffix OR within blocks of the window
-  // width
-  uint8_t* tPA = okw + N;                  // N
-  uint8_t* tSA = tPA + N;                  // N
-  uint8_t* tPO = tSA + N;                  // N
-  uint8_t* tSO = tPO + N;                  // N
+  uint8_t* F = (uint8_t*)(V + N);          // N flags
+  uint8_t* hx = F + N;                     // N row winners (0xFF: none)
+  uint32_t* dBad = (uint32_t*)(fs_s + (((size_t)N * 6 + 3) & ~(size_t)3));  // n x nw bit rows
+  uint32_t* dTmp = dBad + n * nw;
+  uint32_t* dPred = dTmp + n * nw;
   __shared__ int2 locXY[MAX_MAXSS];
   __shared__ double locVal[MAX_MAXSS];
-  __shared__ int sBest;
+  __shared__ int sBest, sM;
   __shared__ double rA[NW], rB[NW];
   __shared__ double sSum;
   __shared__ float sfP, sfK, sfLim;
   __shared__ int sDirect;
 
   // warps 2.. load the stamp while warps 0 and 1 search the exact
-  // thresholds of the two static predicates
+  // thresholds of the two static predicates; the window conditions cover
+  // the pixels inside the frame (x < sx, y < sy)
   if(warp >= 2)
     for(int ly = warp - 2; ly < n; ly += NW - 2)
-      for(int lx = lane; lx < n; lx += 32) {
-        const size_t a = (size_t)(cx + lx) + (size_t)(cy + ly) * w;
-        V[ly * n + lx] = img[a];
-        bad[ly * n + lx] = (ldMask(mask, a) & badMask) ? 1 : 0;
+      for(int j = 0; j < nw; j++) {
+        const int lx = 32 * j + lane;
+        bool b = false;
+        if(lx < n) {
+          const size_t a = (size_t)(cx + lx) + (size_t)(cy + ly) * w;
+          V[ly * n + lx] = img[a];
+          b = (ldMask(mask, a) & badMask) != 0;
+          F[ly * n + lx] = b ? FS_BAD : 0;
+        }
+        const uint32_t m = __ballot_sync(0xffffffffu, b && lx < sx && ly < sy);
+        if(lane == 0) dTmp[ly * nw + j] = m;
       }
   if(warp < 2) {
     auto pr = [&](double v) { return (v - sky) / fwhm > tKF; };
@@ -1232,172 +1273,151 @@ __global__ void __launch_bounds__(FS_T, 1)
   __syncthreads();
   const bool direct = sDirect != 0;
   const float fP = sfP, fK = sfK;
-  for(int p = tid; p < N; p += FS_T) {
-    const float f = V[p];
-    bool pr, kq;
-    if(direct) {
-      pr = ((double)f - sky) / fwhm > tKF;
-      kq = !(((double)f - sky) * invFwhm < tKF);
-    } else {
-      pr = f >= fP;
-      kq = isnan(f) || f >= fK;
+  for(int ly = warp; ly < n; ly += NW)
+    for(int j = 0; j < nw; j++) {
+      const int lx = 32 * j + lane;
+      bool pr = false;
+      if(lx < n) {
+        const int p = ly * n + lx;
+        const float f = V[p];
+        bool kq;
+        if(direct) {
+          pr = ((double)f - sky) / fwhm > tKF;
+          kq = !(((double)f - sky) * invFwhm < tKF);
+        } else {
+          pr = f >= fP;
+          kq = isnan(f) || f >= fK;
+        }
+        const bool vpos = f > 0.f;
+        uint8_t fl = F[p];
+        if(pr) fl |= FL_PRED;
+        if(pr && !vpos) fl |= FL_NONPOS;
+        if(kq) fl |= FL_KFQ;
+        if(vpos) fl |= FL_VPOS;
+        F[p] = fl;
+      }
+      const uint32_t m = __ballot_sync(0xffffffffu, pr && lx < sx && ly < sy);
+      if(lane == 0) dPred[ly * nw + j] = m;
     }
-    const bool vpos = f > 0.f;
-    uint8_t fl = 0;
-    if(pr) fl |= FL_PRED;
-    if(pr && !vpos) fl |= FL_NONPOS;
-    if(kq) fl |= FL_KFQ;
-    if(vpos) fl |= FL_VPOS;
-    flags[p] = fl;
-  }
   __syncthreads();
-  // maps of the current bad state (window argmax of the keys, window ORs)
-  // over the columns [x0, x1] of the rows [k0, k1] (row maps) and [r0, r1]
-  // (column maps); the full build covers the stamp.  After an acceptance
-  // only the accepted window's bad bits change, so only row maps within hSS
-  // of it in x and column maps within hSS of it in x and y can change:
-  // rebuilding that region gives the maps of a full rebuild.
-  // A key is the float bit pattern of a qualifying pixel (0: none).  Window
-  // argmax and OR use the van Herk / Gil-Werman scheme: split the line into
-  // blocks of the window width W, scan each block forwards (prefix) and
-  // backwards (suffix); the window [a, b] is then suffix(a) with prefix(b)
-  // when they lie in different blocks, prefix(b) when a starts its block,
-  // suffix(a) otherwise (b is then the line's end).  Ties keep the smaller
-  // index: the prefix updates on a larger key, the suffix on a larger or
-  // equal one, and prefix(b) wins only with a larger key.
-  const int W = 2 * hSS + 1;
+  // window conditions: rows, then columns (bad: dTmp -> dBad, pred: dPred ->
+  // dTmp, which is the final map)
+  if(tid < n) dilateRow(dTmp + tid * nw, nw, hSS);
+  else if(tid - 256 >= 0 && tid - 256 < n) dilateRow(dPred + (tid - 256) * nw, nw, hSS);
+  __syncthreads();
+  auto dilateColumns = [&](const uint32_t* src, uint32_t* dst) {
+    for(int e = tid; e < n * nw; e += FS_T) {
+      const int y = e / nw, j = e - y * nw;
+      uint32_t o = 0;
+      for(int yy = max(y - hSS, 0); yy <= min(y + hSS, n - 1); yy++) o |= src[yy * nw + j];
+      dst[e] = o;
+    }
+    __syncthreads();
+  };
+  dilateColumns(dTmp, dBad);
+  dilateColumns(dPred, dTmp);
+  const uint32_t* dOk = dTmp;
+  auto bitAt = [&](const uint32_t* d, int y, int x) { return (d[y * nw + (x >> 5)] >> (x & 31)) & 1u; };
+
+  // A key is the float bit pattern of a qualifying pixel (0: none).
   auto keyAt = [&](int p) -> uint32_t {
-    const uint8_t fl = flags[p];
-    return (!bad[p] && (fl & FL_KFQ) && (fl & FL_VPOS)) ? __float_as_uint(V[p]) : 0u;
+    const uint8_t fl = F[p];
+    return (fl & (FS_BAD | FL_KFQ | FL_VPOS)) == (FL_KFQ | FL_VPOS) ? __float_as_uint(V[p]) : 0u;
   };
-  auto orAt = [&](int p) -> uint8_t {
-    const uint8_t fl = flags[p];
-    return (bad[p] ? OK_BAD : 0) | ((fl & FL_PRED) ? OK_PRED : 0) | ((fl & FL_NONPOS) ? OK_NONPOS : 0);
-  };
-  auto build = [&](int x0, int x1, int k0, int k1, int r0, int r1) {
-    // ---- rows [k0, k1]: block scans along x over the blocks under the windows
-    {
-      const int ba = max(x0 - hSS, 0) / W, bb = min(x1 + hSS, n - 1) / W;
-      const int nr = k1 - k0 + 1, nTask = nr * (bb - ba + 1);
-      for(int t = tid; t < 2 * nTask; t += FS_T) {  // prefix and suffix on separate threads
-        const bool suffix = t >= nTask;
-        const int tt = suffix ? t - nTask : t;
-        const int ly = k0 + tt % nr, blk = ba + tt / nr, row = ly * n;
-        const int b0 = blk * W, b1 = min(b0 + W - 1, n - 1);
-        uint32_t bk = 0;
-        int bi = 0xFF;
-        uint8_t o = 0;
-        if(!suffix) {
-          for(int x = b0; x <= b1; x++) {
-            const int p = row + x;
-            const uint32_t k = keyAt(p);
+  // Row winners of the columns [x0, x1] of the rows [k0, k1], FS_SEG columns
+  // per task: their windows share the middle, so each is the best of a suffix
+  // of the columns left of it, the middle, and a prefix of those right of it
+  // (ties keep the smaller column).  Neighbouring lanes take neighbouring rows.
+  auto rowWinners = [&](int x0, int x1, int k0, int k1) {
+    const int s0 = x0 / FS_SEG, s1 = x1 / FS_SEG, nr = k1 - k0 + 1;
+    for(int t = tid; t < nr * (s1 - s0 + 1); t += FS_T) {
+      const int q = t / nr, xs = (s0 + q) * FS_SEG, row = (k0 + t - q * nr) * n;
+      if(hSS < FS_SEG / 2) {  // windows without a shared middle
+        for(int i = 0; i < FS_SEG && xs + i < n; i++) {
+          uint32_t bk = 0;
+          int bi = 0xFF;
+          for(int x = max(xs + i - hSS, 0); x <= min(xs + i + hSS, n - 1); x++) {
+            const uint32_t k = keyAt(row + x);
             if(k > bk) {
               bk = k;
               bi = x;
             }
-            if(x < sx) o |= orAt(p);
-            tPA[p] = (uint8_t)bi;
-            tPO[p] = o;
           }
-        } else {
-          for(int x = b1; x >= b0; x--) {
-            const int p = row + x;
-            const uint32_t k = keyAt(p);
-            if(k != 0 && k >= bk) {
-              bk = k;
-              bi = x;
-            }
-            if(x < sx) o |= orAt(p);
-            tSA[p] = (uint8_t)bi;
-            tSO[p] = o;
-          }
+          hx[row + xs + i] = (uint8_t)bi;
+        }
+        continue;
+      }
+      uint32_t lk[FS_SEG - 1], mk = 0, bk = 0;
+      int li[FS_SEG - 1], mi = 0xFF, bi = 0xFF;
+#pragma unroll
+      for(int i = FS_SEG - 2; i >= 0; i--) {
+        const int x = xs - hSS + i;
+        const uint32_t k = x >= 0 && x < n ? keyAt(row + x) : 0u;
+        if(k != 0 && k >= bk) {
+          bk = k;
+          bi = x;
+        }
+        lk[i] = bk;
+        li[i] = bi;
+      }
+      for(int x = max(xs - hSS + FS_SEG - 1, 0); x <= min(xs + hSS, n - 1); x++) {
+        const uint32_t k = keyAt(row + x);
+        if(k > mk) {
+          mk = k;
+          mi = x;
         }
       }
-    }
-    __syncthreads();
-    const int kw = x1 - x0 + 1;
-    for(int i = tid; i < (k1 - k0 + 1) * kw; i += FS_T) {
-      const int ly = k0 + i / kw, lx = x0 + i % kw, row = ly * n;
-      const int a = max(lx - hSS, 0), b = min(lx + hSS, n - 1);
-      uint8_t h, o;
-      if(a / W != b / W) {
-        const uint8_t L = tSA[row + a], R = tPA[row + b];
-        h = L == 0xFF ? R : R == 0xFF ? L : (keyAt(row + R) > keyAt(row + L) ? R : L);
-        o = tSO[row + a] | tPO[row + b];
-      } else if(a % W == 0) {
-        h = tPA[row + b];
-        o = tPO[row + b];
-      } else {
-        h = tSA[row + a];
-        o = tSO[row + a];
-      }
-      hx[row + lx] = h;
-      rowf[row + lx] = o;
-    }
-    __syncthreads();
-    // ---- columns [x0, x1]: block scans along y of the row winners
-    {
-      const int ba = max(r0 - hSS, 0) / W, bb = min(r1 + hSS, n - 1) / W;
-      const int nTask = kw * (bb - ba + 1);
-      auto candKey = [&](int y, int lx) -> uint32_t {
-        const uint8_t xx = hx[y * n + lx];
-        return xx == 0xFF ? 0u : keyAt(y * n + xx);
-      };
-      for(int t = tid; t < 2 * nTask; t += FS_T) {
-        const bool suffix = t >= nTask;
-        const int tt = suffix ? t - nTask : t;
-        const int lx = x0 + tt % kw, blk = ba + tt / kw;
-        const int b0 = blk * W, b1 = min(b0 + W - 1, n - 1);
-        uint32_t bk = 0;
-        int bi = 0xFF;
-        uint8_t o = 0;
-        if(!suffix) {
-          for(int y = b0; y <= b1; y++) {
-            const uint32_t k = candKey(y, lx);
-            if(k > bk) {
-              bk = k;
-              bi = y;
-            }
-            if(y < sy) o |= rowf[y * n + lx];
-            tPA[y * n + lx] = (uint8_t)bi;
-            tPO[y * n + lx] = o;
-          }
-        } else {
-          for(int y = b1; y >= b0; y--) {
-            const uint32_t k = candKey(y, lx);
-            if(k != 0 && k >= bk) {
-              bk = k;
-              bi = y;
-            }
-            if(y < sy) o |= rowf[y * n + lx];
-            tSA[y * n + lx] = (uint8_t)bi;
-            tSO[y * n + lx] = o;
+      uint32_t rk = 0;
+      int ri = 0xFF;
+#pragma unroll
+      for(int i = 0; i < FS_SEG; i++) {
+        uint32_t k = i < FS_SEG - 1 ? lk[i < FS_SEG - 1 ? i : 0] : 0u;
+        int o = i < FS_SEG - 1 ? li[i < FS_SEG - 1 ? i : 0] : 0xFF;
+        if(mk > k) {
+          k = mk;
+          o = mi;
+        }
+        if(i > 0) {
+          const int x = xs + hSS + i;
+          const uint32_t kx = x < n ? keyAt(row + x) : 0u;
+          if(kx > rk) {
+            rk = kx;
+            ri = x;
           }
         }
-      }
-      __syncthreads();
-      for(int i = tid; i < (r1 - r0 + 1) * kw; i += FS_T) {
-        const int ly = r0 + i / kw, lx = x0 + i % kw;
-        const int a = max(ly - hSS, 0), b = min(ly + hSS, n - 1);
-        uint8_t yb, o;
-        if(a / W != b / W) {
-          const uint8_t L = tSA[a * n + lx], R = tPA[b * n + lx];
-          yb = L == 0xFF ? R : R == 0xFF ? L : (candKey(R, lx) > candKey(L, lx) ? R : L);
-          o = tSO[a * n + lx] | tPO[b * n + lx];
-        } else if(a % W == 0) {
-          yb = tPA[b * n + lx];
-          o = tPO[b * n + lx];
-        } else {
-          yb = tSA[a * n + lx];
-          o = tSO[a * n + lx];
-        }
-        arg[ly * n + lx] = yb == 0xFF ? (uint16_t)0xFFFF : (uint16_t)(yb * n + hx[yb * n + lx]);
-        okw[ly * n + lx] = o;
+        if(rk > k) o = ri;
+        if(xs + i < n) hx[row + xs + i] = (uint8_t)o;
       }
     }
     __syncthreads();
   };
-  build(0, n - 1, 0, n - 1, 0, n - 1);
+  rowWinners(0, n - 1, 0, n - 1);
+  const int W = 2 * hSS + 1;
+  // The pixel a candidate stands for: its window's first largest key, or
+  // itself where the window has none.  One warp.
+  auto windowMax = [&](int p) -> int {
+    const int ly = p / n, lx = p - ly * n;
+    uint32_t bk = 0;
+    int m = p;
+    for(int b = 0; b < W; b += 32) {
+      const int y = ly - hSS + b + lane;
+      uint32_t k = 0;
+      int q = p;
+      if(b + lane < W && y >= 0 && y < n) {
+        const int h = hx[y * n + lx];
+        if(h != 0xFF) {
+          q = y * n + h;
+          k = __float_as_uint(V[q]);
+        }
+      }
+      const uint32_t kb = __reduce_max_sync(0xffffffffu, k);
+      if(kb > bk) {
+        bk = kb;
+        m = __shfl_sync(0xffffffffu, q, __ffs(__ballot_sync(0xffffffffu, k == kb)) - 1);
+      }
+    }
+    return m;
+  };
   const double floorV = sky + tKF * fwhm;
   double dfrac = 0.9;
   int cnt = 0, passes = 0;
@@ -1410,30 +1430,31 @@ __global__ void __launch_bounds__(FS_T, 1)
     const float fLim = sfLim;
     int start = 0;
     while(cnt < maxSS && start < N) {
-      int mine = INT_MAX;
+      int mine = INT_MAX, mineM = 0;
       for(int p0 = start; p0 < N && mine == INT_MAX; p0 += 4 * FS_T) {
-        for(int k = 0; k < 4; k++) {
-          const int p = p0 + k * FS_T + tid;
-          if(p >= N || p >= mine) break;
-          if(bad[p] || !(flags[p] & FL_KFQ)) continue;
-          if(!(V[p] > fLim)) continue;
-          const int m = arg[p] != 0xFFFF ? arg[p] : p;
-          const uint8_t o = okw[m];
-          if(!(o & OK_BAD) && (o & OK_PRED)) {
-            mine = p;
-            break;
+        for(int k = 0; k < 4 && mine == INT_MAX; k++) {
+          const int pw = p0 + k * FS_T + warp * 32, p = pw + lane;
+          const bool cand = p < N && (F[p] & (FS_BAD | FL_KFQ)) == FL_KFQ && V[p] > fLim;
+          for(unsigned c = __ballot_sync(0xffffffffu, cand); c; c &= c - 1) {
+            const int pc = pw + __ffs(c) - 1, m = windowMax(pc);
+            const int my = m / n, mx = m - my * n;
+            if(!bitAt(dBad, my, mx) && bitAt(dOk, my, mx)) {
+              mine = pc;
+              mineM = m;
+              break;
+            }
           }
         }
-        mine = __reduce_min_sync(0xffffffffu, mine);
         if(tid == 0) sBest = INT_MAX;
         __syncthreads();
         if(lane == 0 && mine != INT_MAX) atomicMin(&sBest, mine);
         __syncthreads();
+        if(lane == 0 && mine != INT_MAX && mine == sBest) sM = mineM;
         mine = sBest;
         __syncthreads();
       }
       if(mine == INT_MAX) break;
-      const int p = mine, m = arg[p] != 0xFFFF ? arg[p] : p;
+      const int p = mine, m = sM;
       const int mx = cx + m % n, my = cy + m / n;
       const int u0 = max(mx - hSS, cx), v0 = max(my - hSS, cy);
       const int u1 = min(mx + hSS, cx + sx - 1), v1 = min(my + hSS, cy + sy - 1);
@@ -1444,25 +1465,28 @@ __global__ void __launch_bounds__(FS_T, 1)
       // (every pixel is a multiple of that quantum), no partial sum rounds in
       // any order; otherwise warp 0 forms the serial sum bit for bit (osum;
       // a pixel below the threshold adds +0.0, which changes nothing).
-      double part = 0.0, amin = INFINITY;
+      double part = 0.0;
+      float amin = INFINITY;
+      bool nonpos = false;
       for(int i = tid; i < un; i += FS_T) {
         const int q = (v0 + i / uw - cy) * n + (u0 + i % uw - cx);
-        if(flags[q] & FL_PRED) {
-          const double v = (double)V[q];
-          part += v;
-          amin = fmin(amin, fabs(v));
+        const uint8_t fl = F[q];
+        if(fl & FL_PRED) {
+          part += (double)V[q];
+          amin = fminf(amin, fabsf(V[q]));
+          nonpos |= (fl & FL_NONPOS) != 0;
         }
       }
 #pragma unroll
       for(int o = 16; o > 0; o >>= 1) {
         part += __shfl_xor_sync(0xffffffffu, part, o);
-        amin = fmin(amin, __shfl_xor_sync(0xffffffffu, amin, o));
+        amin = fminf(amin, __shfl_xor_sync(0xffffffffu, amin, o));
       }
       if(lane == 0) {
         rA[warp] = part;
-        rB[warp] = amin;
+        rB[warp] = (double)amin;
       }
-      __syncthreads();
+      nonpos = __syncthreads_or(nonpos);
       if(warp == 0) {
         double t = lane < NW ? rA[lane] : 0.0, mn = lane < NW ? rB[lane] : INFINITY;
 #pragma unroll
@@ -1471,7 +1495,7 @@ __global__ void __launch_bounds__(FS_T, 1)
           mn = fmin(mn, __shfl_xor_sync(0xffffffffu, mn, o));
         }
         bool exact = false;
-        if(!(okw[m] & OK_NONPOS) && mn > 0.0 && mn < INFINITY) {
+        if(!nonpos && mn > 0.0 && mn < INFINITY) {
           int e;
           frexp(mn, &e);  // mn in [2^(e-1), 2^e)
           exact = t < ldexp(1.0, e - 1 - 23 + 52);
@@ -1479,7 +1503,7 @@ __global__ void __launch_bounds__(FS_T, 1)
         if(!exact)
           t = osum::warpOrderedSumOf(un, [&](int i) {
             const int q = (v0 + i / uw - cy) * n + (u0 + i % uw - cx);
-            return (flags[q] & FL_PRED) ? V[q] : 0.f;
+            return (F[q] & FL_PRED) ? V[q] : 0.f;
           });
         if(lane == 0) sSum = t;
       }
@@ -1492,17 +1516,22 @@ __global__ void __launch_bounds__(FS_T, 1)
         locVal[cnt] = ret;
       }
       cnt++;
+      // the window turns bad (skipMask is part of badMask)
       for(int i = tid; i < un; i += FS_T) {
         const int gx = u0 + i % uw, gy = v0 + i / uw;
         orMask(mask, (size_t)gx + (size_t)gy * w, skipMask);
-        bad[(gy - cy) * n + (gx - cx)] = 1;  // skipMask is part of badMask
+        F[(gy - cy) * n + (gx - cx)] |= FS_BAD;
       }
-      __syncthreads();
       if(cnt < maxSS) {
-        // keys change inside the window only; maps within hSS of it
-        const int a0 = u0 - cx, a1 = u1 - cx, b0 = v0 - cy, b1 = v1 - cy;
-        build(max(a0 - hSS, 0), min(a1 + hSS, n - 1), b0, b1, max(b0 - hSS, 0),
-              min(b1 + hSS, n - 1));
+        const int a0 = max(u0 - cx - hSS, 0), a1 = min(u1 - cx + hSS, n - 1);
+        const int b0 = max(v0 - cy - hSS, 0), b1 = min(v1 - cy + hSS, n - 1);
+        for(int e = tid; e < (b1 - b0 + 1) * nw; e += FS_T) {
+          const int y = b0 + e / nw, j = e % nw;
+          const int l = max(a0 - 32 * j, 0), h = min(a1 - 32 * j, 31);  // bits l..h of word j
+          if(l <= h) dBad[y * nw + j] |= (0xFFFFFFFFu >> (31 - h)) & (0xFFFFFFFFu << l);
+        }
+        __syncthreads();
+        rowWinners(a0, a1, v0 - cy, v1 - cy);
       }
     }
     if(cnt >= maxSS || lim == floorV) break;
@@ -1622,7 +1651,11 @@ static void sssPass(xb_ctx* c, int* nKept) {
   { KT_SCOPE(c, "find_substamps");
   const size_t perCta = ((size_t)fSW * fSW * 24 + 255) / 256 * 256;
   const size_t fsSmem = fsSmemBytes(fSW);
-  const bool inShared = !c->imgIsF64 && fSW <= 120;
+  // stamps that fit in shared memory with byte row winners, of FP32 images;
+  // else maps in global memory
+  int optin = 0;
+  XB_CUDA(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, c->device));
+  const bool inShared = !c->imgIsF64 && fSW <= FS_MAXN && fsSmem + 1024 <= (size_t)optin;
   // global-memory maps only for the kernel that uses them
   unsigned char* scratch =
       inShared ? nullptr : buf<unsigned char>(c, "fm_scratch", (size_t)2 * nAll * perCta);
