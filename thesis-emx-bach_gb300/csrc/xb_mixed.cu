@@ -941,144 +941,457 @@ __global__ void __launch_bounds__(BX * 21, BX == 8 ? 2 : 1)
 // dP_t = P_t(x, y) - P_t(xc, yc): the block kernel is evaluated in FP64 and
 // rounded once (as k_conv_sub_f32 does), and the FP32 rounding of the
 // term images only scales the small dP_t (|dP| <= ~fK / frame size), so
-// fits whose spatial terms cancel keep the block kernel's accuracy.  Seven
-// pixels of one row per thread, the window in registers, one pass over the
-// tile per term.
-template <int FK, int CV_BX>
-__global__ void __launch_bounds__(CV_BX * FK * (FK / 7))
-    k_conv_sub_pp_f32(const float* __restrict__ I, const float* __restrict__ O,
-                      const double* __restrict__ sol, const double* __restrict__ Kt,
-                      const double* __restrict__ kernSumPtr, ConvArgsF a,
-                      const uint8_t* __restrict__ inMask, uint16_t* __restrict__ mask,
-                      float* __restrict__ convF, float* __restrict__ diffF) {
-  constexpr int HK = FK / 2, NK = FK * FK, PX = 7, TPR = FK / PX;
-  constexpr int TH = FK + 2 * HK, TW = CV_BX * FK + 2 * HK;
-  constexpr int MAXT = (MAX_KORDER + 1) * (MAX_KORDER + 2) / 2;
-  __shared__ float tile[TH][TW + 1];
-  __shared__ unsigned char bad[TH][TW + 1];
-  __shared__ unsigned char rowBad[TH][CV_BX * FK];
-  __shared__ float kern[CV_BX][NK];
-  __shared__ double poly[CV_BX][MAXT];
-  __shared__ float bgc[16];
-  extern __shared__ float ktf[];  // nC2 * NK, term 0 unused
-  const int tid = threadIdx.x, nthr = blockDim.x;
-  const int xB0 = blockIdx.x * CV_BX, yB = blockIdx.y;
-  const int x0 = xB0 * FK, y0 = yB * FK;
-  const int nC2 = (a.kOrder + 1) * (a.kOrder + 2) / 2;
-  const double hx = 0.5 * a.w, hy = 0.5 * a.h;
-  if(tid < CV_BX) {
-    // spatial terms at the block centre (conv(), src/bach.cpp:339-350)
-    const double xf = ((xB0 + tid) * FK + 2 * HK - hx) / hx, yf = (yB * FK + 2 * HK - hy) / hy;
-    double ax = 1.0;
-    int t = 0;
-    for(int i = 0; i <= a.kOrder; i++) {
-      double ay = 1.0;
-      for(int j = 0; j <= a.kOrder - i; j++) {
-        poly[tid][t++] = ax * ay;
-        ay *= yf;
+// fits whose spatial terms cancel keep the block kernel's accuracy.
+//
+// One convolution per spatial term, two at a time over the same 7 x 3 pixel
+// tile per thread as k_conv_sub_f32: a row of 27 window values feeds three
+// rows of two kernels, 882 FMAs per 27 + 36 shared loads (the term kernels are
+// the same for every block).  Bound by FP32 (0.28 ms at 2048^2 for six terms);
+// seven pixels of one row per thread and, for every pixel with a bad one under
+// its window, its own kernel tap by tap took 5.2 ms, this form 0.94 ms.
+//
+// The 0.99 |kernel| rule of such a pixel: with E = sum_t max|dP_t| |Kt[t]| the
+// largest change of a tap's kernel within the block, the bad taps' sum is
+// within sum(E) of that of the block kernel and the whole sum within the
+// total of E, which decides most pixels; the others take their own kernel's
+// bad taps and the whole sum to first order in dP.  Those whose bounds still
+// straddle 0.99 (with 1e-4 for the rounding of the FP32 sums) sum their own
+// kernel, a warp per pixel.  (All of them a lane per pixel: 2.3 ms, the CTA
+// waiting for it; the first bound alone before that sum: 1.3 ms.)
+template <int FK, int BX>
+struct ConvTilePP {
+  using L = ConvTileF<FK, BX>;
+  static constexpr int KMAX = 3;                  // spatial order bound of the mixed conv
+  static constexpr int TMAX = (KMAX + 1) * (KMAX + 2) / 2;
+  static constexpr size_t OFF_XP = (L::BYTES + 15) / 16 * 16;      // column powers
+  static constexpr size_t OFF_YP = OFF_XP + (size_t)(KMAX + 1) * BX * FK * 8;
+  static constexpr size_t OFF_POLY = OFF_YP + (size_t)(KMAX + 1) * FK * 8;
+  static constexpr size_t OFF_DMAX = OFF_POLY + (size_t)BX * TMAX * 8;  // max |dP_t| per block
+  static constexpr size_t OFF_E = OFF_DMAX + (size_t)BX * TMAX * 4;     // E per block and tap
+  static constexpr size_t OFF_ETOT = OFF_E + (size_t)BX * L::NK * 4;
+  static constexpr size_t OFF_TERM = (OFF_ETOT + (size_t)(BX + 4) * 4 + 15) / 16 * 16;
+  static constexpr size_t bytes(int nC2) { return OFF_TERM + (size_t)(nC2 - 1) * FK * L::KS * 4; }
+};
+
+template <int FK, int BX, bool TWO>
+__device__ __forceinline__ void convTilePair(const float* trow, int S, const float* kA,
+                                             const float* kB, float (&a)[3][7], float (&b)[3][7]) {
+  constexpr int KS = 24;
+#pragma unroll
+  for(int o = 0; o < 3; o++)
+#pragma unroll
+    for(int q = 0; q < 7; q++) a[o][q] = b[o][q] = 0.f;
+#pragma unroll 1
+  for(int R = 0; R < FK + 2; R++, trow += S) {
+    float win[27];
+#pragma unroll
+    for(int q = 0; q < 27; q++) win[q] = trow[q];
+#pragma unroll
+    for(int o = 0; o < 3; o++) {
+      const int jj = R - o;
+      if(jj < 0 || jj >= FK) continue;
+#pragma unroll
+      for(int u = 0; u < (TWO ? 2 : 1); u++) {
+        const float4* kr4 = (const float4*)((u == 0 ? kA : kB) + (FK - 1 - jj) * KS);
+        float kf[24];
+#pragma unroll
+        for(int m = 0; m < 6; m++) {
+          const float4 v = kr4[m];
+          kf[4 * m] = v.x;
+          kf[4 * m + 1] = v.y;
+          kf[4 * m + 2] = v.z;
+          kf[4 * m + 3] = v.w;
+        }
+#pragma unroll
+        for(int ii = 0; ii < FK; ii++) {
+          const float kk = kf[FK - 1 - ii];
+#pragma unroll
+          for(int q = 0; q < 7; q++) {
+            if(u == 0) a[o][q] = fmaf(kk, win[q + ii], a[o][q]);
+            else b[o][q] = fmaf(kk, win[q + ii], b[o][q]);
+          }
+        }
       }
-      ax *= xf;
     }
   }
-  for(int e = tid; e < nC2 * NK; e += nthr) ktf[e] = (float)Kt[e];
-  for(int i = tid; i < TH * TW; i += nthr) {
-    const int ly = i / TW, lx = i % TW;
+}
+
+template <int FK, int BX>
+__global__ void __launch_bounds__(BX * 21, 3)
+    k_conv_sub_pp_f32(const float* __restrict__ I, const float* __restrict__ O,
+                      const double* __restrict__ sol, const double* __restrict__ Kt,
+                      const double* __restrict__ blockXY, const double* __restrict__ kernSumPtr,
+                      ConvArgsF a, const uint8_t* __restrict__ inMask, uint16_t* __restrict__ mask,
+                      float* __restrict__ convF, float* __restrict__ diffF) {
+  using L = ConvTileF<FK, BX>;
+  using P = ConvTilePP<FK, BX>;
+  constexpr int HK = L::HK, NK = L::NK, S = L::S, TW = L::TW, TH = L::TH, NW = L::NW, KS = L::KS;
+  constexpr int NT = L::NT, NFULL = NT / 32, TMAX = P::TMAX, RW = BX * FK;
+  extern __shared__ __align__(16) unsigned char cv_smem[];
+  float* tile = (float*)cv_smem;
+  float* kern = (float*)(cv_smem + L::OFF_KERN);
+  uint32_t* bits = (uint32_t*)(cv_smem + L::OFF_BITS);
+  float* aks = (float*)(cv_smem + L::OFF_AKS);
+  float* bgc = aks + BX;  // background coefficients (getBackground), FP32
+  double* xpow = (double*)(cv_smem + P::OFF_XP);    // [power][column]
+  double* ypow = (double*)(cv_smem + P::OFF_YP);    // [power][row]
+  double* poly = (double*)(cv_smem + P::OFF_POLY);  // [block][term] at the block centre
+  float* dMax = (float*)(cv_smem + P::OFF_DMAX);
+  float* E = (float*)(cv_smem + P::OFF_E);
+  float* eTot = (float*)(cv_smem + P::OFF_ETOT);
+  float* term = (float*)(cv_smem + P::OFF_TERM);    // Kt[t], t >= 1, rows of KS floats
+  __shared__ int sAny;
+  __shared__ float sDP[(NT + 31) / 32][TMAX];
+  __shared__ float gTerm[BX][TMAX], cTot[BX], sTot[BX];
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int xB0 = blockIdx.x * BX, yB = blockIdx.y;
+  const int x0 = xB0 * FK, y0 = yB * FK;  // tile origin; block pixels start at +HK
+  const int K = a.kOrder, nC2 = (K + 1) * (K + 2) / 2;
+  const double hx = 0.5 * a.w, hy = 0.5 * a.h;
+  if(tid == 0) sAny = 0;
+  for(int i = tid; i < TH * TW; i += NT) {
+    const int ly = i / TW, lx = i - ly * TW;
     const int gx = min(x0 + lx, a.w - 1), gy = min(y0 + ly, a.h - 1);
-    const float v = I[(size_t)gx + (size_t)gy * a.w];
-    tile[ly][lx] = v;
-    bad[ly][lx] = ((convMaskF(v, a.tH, a.tL) & BAD_INPUT) ||
-                   (inMask && inMask[(size_t)gx + (size_t)gy * a.w])) ? 1 : 0;
+    tile[ly * S + lx] = I[(size_t)gx + (size_t)gy * a.w];
+  }
+  {
+    const double yf = blockXY[a.xSteps + yB];
+    switch(K) {
+      case 0: convBlockKernels<0, FK, BX, NT>(Kt, blockXY, yf, xB0, kern); break;
+      case 1: convBlockKernels<1, FK, BX, NT>(Kt, blockXY, yf, xB0, kern); break;
+      case 2: convBlockKernels<2, FK, BX, NT>(Kt, blockXY, yf, xB0, kern); break;
+      default: convBlockKernels<3, FK, BX, NT>(Kt, blockXY, yf, xB0, kern); break;
+    }
+    for(int e = tid; e < (nC2 - 1) * NK; e += NT) {
+      const int t = e / NK, p = e - t * NK;
+      term[(t * FK + p / FK) * KS + p % FK] = (float)Kt[NK + e];
+    }
+    // powers of the pixel coordinates, by repeated products
+    if(tid < RW) {
+      const double xf = ((double)(x0 + HK + tid) - hx) / hx;
+      double xp = 1.0;
+      for(int i = 0; i <= K; i++, xp *= xf) xpow[i * RW + tid] = xp;
+    }
+    if(tid < FK) {
+      const double py = ((double)(y0 + HK + tid) - hy) / hy;
+      double yp = 1.0;
+      for(int j = 0; j <= K; j++, yp *= py) ypow[j * FK + tid] = yp;
+    }
+    if(tid < BX) {
+      const double xf = blockXY[xB0 + tid];
+      double ax = 1.0;
+      int t = 0;
+      for(int i = 0; i <= K; i++, ax *= xf) {
+        double ay = 1.0;
+        for(int j = 0; j <= K - i; j++, ay *= yf) poly[tid * TMAX + t++] = ax * ay;
+      }
+    }
+  }
+  __syncthreads();
+  if(warp < NFULL) {
+    uint32_t any = 0;
+    for(int ly = warp; ly < TH; ly += NFULL) {
+      const int gy = min(y0 + ly, a.h - 1);
+#pragma unroll
+      for(int wc = 0; wc < NW; wc++) {
+        const int c = wc * 32 + lane;
+        bool bd = false;
+        if(c < TW) {
+          bd = convMaskF(tile[ly * S + c], a.tH, a.tL) & BAD_INPUT;
+          if(inMask) bd |= inMask[(size_t)min(x0 + c, a.w - 1) + (size_t)gy * a.w] != 0;
+        }
+        const unsigned m = __ballot_sync(0xffffffffu, bd);
+        any |= m;
+        if(lane == 0) bits[ly * NW + wc] = m;
+      }
+    }
+    if(lane == 0 && any) sAny = 1;
   }
   const int nBgC = (a.bgOrder + 1) * (a.bgOrder + 2) / 2;
-  if(tid < nBgC && tid < 16) bgc[tid] = (float)sol[a.nComp + 2 + tid];
-  __syncthreads();
-  for(int e = tid; e < CV_BX * NK; e += nthr) {
-    const int b = e / NK, p = e % NK;
-    double k0 = 0.0;
-    for(int t = 0; t < nC2; t++) k0 = fma(poly[b][t], Kt[(size_t)t * NK + p], k0);
-    kern[b][p] = (float)k0;
+  if(tid < nBgC) bgc[tid] = (float)sol[a.nComp + 2 + tid];
+  // largest |dP_t| of each block: a product of powers, so at a corner pixel,
+  // or (even powers) where a coordinate crosses zero: the bound of the
+  // coordinates' largest magnitudes covers both
+  for(int e = tid; e < BX * nC2; e += NT) {
+    const int b = e / nC2, t = e - b * nC2;
+    int i = 0, t0 = 0;
+    while(t - t0 > K - i) t0 += K - i++ + 1;
+    const int jj = t - t0;
+    const double c = poly[b * TMAX + t];
+    const double xa = xpow[i * RW + b * FK], xb = xpow[i * RW + b * FK + FK - 1];
+    const double ya = ypow[jj * FK], yb = ypow[jj * FK + FK - 1];
+    double m = fmax(fmax(fabs(xa * ya - c), fabs(xa * yb - c)),
+                    fmax(fabs(xb * ya - c), fabs(xb * yb - c)));
+    const bool xZero = K > 0 && xpow[RW + b * FK] * xpow[RW + b * FK + FK - 1] <= 0.0;
+    const bool yZero = K > 0 && ypow[FK] * ypow[FK + FK - 1] <= 0.0;
+    if(xZero || yZero)
+      m = fmax(m, fabs(c) + fmax(fabs(xa), fabs(xb)) * fmax(fabs(ya), fabs(yb)));
+    dMax[b * TMAX + t] = (float)(m * (1.0 + 1e-6));
   }
-  for(int e = tid; e < TH * CV_BX * FK; e += nthr) {
-    const int ly = e / (CV_BX * FK), lx = e % (CV_BX * FK);
-    unsigned char o = 0;
+  __syncthreads();
+  const bool anyBad = sAny != 0;
+  if(anyBad) {
+    for(int e = tid; e < BX * NK; e += NT) {
+      const int b = e / NK, p = e - b * NK, at = (p / FK) * KS + p % FK;
+      float s = 0.f;
+      for(int t = 1; t < nC2; t++) s = fmaf(dMax[b * TMAX + t], fabsf(term[(t - 1) * FK * KS + at]), s);
+      E[e] = s;
+    }
+    __syncthreads();
+    if(warp < NFULL)
+      for(int b = warp; b < BX; b += NFULL) {
+        // the sums of |k| and E, what E can add where it exceeds |k|, and per
+        // term the sums of sign(k) Kt and |Kt|
+        float s = 0.f, se = 0.f, sc = 0.f, gt[TMAX], at[TMAX];
 #pragma unroll
-    for(int d = 0; d < FK; d++) o |= bad[ly][lx + d];
-    rowBad[ly][lx] = o;
+        for(int t = 0; t < TMAX; t++) gt[t] = at[t] = 0.f;
+        for(int p = lane; p < NK; p += 32) {
+          const int o = (p / FK) * KS + p % FK;
+          const float k = kern[b * FK * KS + o], e = E[b * NK + p];
+          s += fabsf(k);
+          se += e;
+          sc += fmaxf(e - fabsf(k), 0.f);
+#pragma unroll
+          for(int t = 1; t < TMAX; t++)
+            if(t < nC2) {
+              const float kt = term[(t - 1) * FK * KS + o];
+              gt[t] += k < 0.f ? -kt : kt;
+              at[t] += fabsf(kt);
+            }
+        }
+        auto sum = [](float v) {
+#pragma unroll
+          for(int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+          return v;
+        };
+        s = sum(s);
+        se = sum(se);
+        sc = sum(sc);
+        float sa = 0.f;
+#pragma unroll
+        for(int t = 1; t < TMAX; t++)
+          if(t < nC2) {
+            const float g = sum(gt[t]);
+            sa += sum(at[t]);
+            if(lane == 0) gTerm[b][t] = g;
+          }
+        if(lane == 0) {
+          aks[b] = s;
+          eTot[b] = se;
+          cTot[b] = 2.f * sc;
+          sTot[b] = 2e-7f * sa;
+        }
+      }
+    __syncthreads();
   }
+  // thread -> (block b, column group k, row group g): 7 columns x 3 rows
+  const int b = tid / L::TPB, r = tid - b * L::TPB, kq = r / 7, g = r - kq * 7;
+  const int ly0 = L::RY * g, lx0 = b * FK + L::PX * kq;
+  const float* kb = kern + b * FK * KS;
+  const float* tr = tile + ly0 * S + lx0;
+  float base[3][7], corr[3][7];
+  // corr += dP_t * ct of term t (powers i, j)
+  auto addTerm = [&](int t, int i, int jj, const float (&ct)[3][7]) {
+    const double c = poly[b * TMAX + t];
+#pragma unroll
+    for(int o = 0; o < 3; o++) {
+      const double yp = ypow[jj * FK + ly0 + o];
+#pragma unroll
+      for(int q = 0; q < 7; q++)
+        corr[o][q] = fmaf((float)(xpow[i * RW + lx0 + q] * yp - c), ct[o][q], corr[o][q]);
+    }
+  };
+#pragma unroll
+  for(int o = 0; o < 3; o++)
+#pragma unroll
+    for(int q = 0; q < 7; q++) corr[o][q] = 0.f;
+  {
+    int t = 1, i = 0, jj = 1;  // term t has powers i, jj (x power outer)
+    auto next = [&]() {
+      t++;
+      if(++jj > K - i) {
+        i++;
+        jj = 0;
+      }
+    };
+    if(K == 0) {
+      convTilePair<FK, BX, false>(tr, S, kb, kb, base, corr);
+    } else {
+      float ct[3][7];
+      convTilePair<FK, BX, true>(tr, S, kb, term, base, ct);
+      addTerm(t, i, jj, ct);
+      next();
+      while(t < nC2) {
+        float c2[3][7];
+        const bool two = t + 1 < nC2;
+        const float* kA = term + (t - 1) * FK * KS;
+        if(two) convTilePair<FK, BX, true>(tr, S, kA, kA + FK * KS, ct, c2);
+        else convTilePair<FK, BX, false>(tr, S, kA, kA, ct, c2);
+        addTerm(t, i, jj, ct);
+        next();
+        if(two) {
+          addTerm(t, i, jj, c2);
+          next();
+        }
+      }
+    }
+  }
+  // The 0.99 rule (2: BAD_CONV, 1: OK_CONV) of the pixels with a bad one under
+  // their window
+  unsigned char flag[3][7];
+#pragma unroll
+  for(int o = 0; o < 3; o++)
+#pragma unroll
+    for(int q = 0; q < 7; q++) flag[o][q] = 0;
+  if(anyBad) {
+    constexpr unsigned long long WIN = (1ull << FK) - 1, COLS = (1ull << 27) - 1;
+    // each bad pixel's |k| and E, added to every pixel of this thread whose
+    // window covers it
+    unsigned long long orw[3] = {0ull, 0ull, 0ull};
+    float sk[3][7], se[3][7];
+#pragma unroll
+    for(int o = 0; o < 3; o++)
+#pragma unroll
+      for(int q = 0; q < 7; q++) sk[o][q] = se[o][q] = 0.f;
+#pragma unroll 1
+    for(int R = 0; R < FK + 2; R++) {
+      const uint32_t* br = bits + (ly0 + R) * NW + (lx0 >> 5);
+      unsigned long long wb =
+          (((unsigned long long)br[0] | ((unsigned long long)br[1] << 32)) >> (lx0 & 31)) & COLS;
+      if(wb == 0ull) continue;
+#pragma unroll
+      for(int o = 0; o < 3; o++)
+        if(R - o >= 0 && R - o < FK) orw[o] |= wb;
+      while(wb != 0ull) {
+        const int cI = __ffsll((long long)wb) - 1;  // window column of a bad pixel
+        wb &= wb - 1ull;
+#pragma unroll
+        for(int o = 0; o < 3; o++) {
+          const int jj = R - o;
+          if(jj < 0 || jj >= FK) continue;
+          const float* krow = kb + (FK - 1 - jj) * KS + (FK - 1);
+          const float* erow = E + b * NK + (FK - 1 - jj) * FK + (FK - 1);
+#pragma unroll
+          for(int q = 0; q < 7; q++) {
+            const int ii = cI - q;
+            if(ii >= 0 && ii < FK) {
+              sk[o][q] += fabsf(krow[-ii]);
+              se[o][q] += erow[-ii];
+            }
+          }
+        }
+      }
+    }
+    const float ak = aks[b], et = eTot[b];
+    const unsigned lanes = (warp + 1) * 32 <= NT ? 0xffffffffu : (1u << (NT & 31)) - 1u;
+#pragma unroll
+    for(int o = 0; o < 3; o++)
+#pragma unroll
+      for(int q = 0; q < 7; q++) {
+        const bool hit = ((orw[o] >> q) & WIN) != 0ull;
+        int f = 0;
+        if(hit) {
+          if((sk[o][q] + se[o][q]) < (0.01f - 1e-4f) * (ak - et)) f = 1;
+          else if((sk[o][q] - se[o][q]) > (0.01f + 1e-4f) * (ak + et)) f = 2;
+          else {
+            // this pixel's dP_t in FP32 (within 2e-7 of |Kt| each), its bad
+            // taps' sum, and its |kernel| sum: that of the block with the
+            // signs of its taps kept, more where a change exceeds the tap
+            float dP[TMAX], lin = ak;
+            int t = 0;
+#pragma unroll
+            for(int i = 0; i <= P::KMAX; i++)
+#pragma unroll
+              for(int j = 0; j <= P::KMAX - i; j++)
+                if(i <= K && j <= K - i) {
+                  const float d = fmaf((float)xpow[i * RW + lx0 + q], (float)ypow[j * FK + ly0 + o],
+                                       -(float)poly[b * TMAX + t]);
+                  if(t > 0) lin = fmaf(d, gTerm[b][t], lin);
+                  dP[t++] = d;
+                }
+            float bs = 0.f;
+            for(int jj = 0; jj < FK; jj++) {
+              const uint32_t* br = bits + (ly0 + o + jj) * NW + (lx0 >> 5);
+              unsigned long long m =
+                  ((((unsigned long long)br[0] | ((unsigned long long)br[1] << 32)) >> (lx0 & 31)) >> q) & WIN;
+              for(; m; m &= m - 1) {
+                const int at = (FK - 1 - jj) * KS + FK - __ffsll((long long)m);
+                float kv = kb[at];
+                for(int tt = 1; tt < nC2; tt++) kv = fmaf(dP[tt], term[(tt - 1) * FK * KS + at], kv);
+                bs += fabsf(kv);
+              }
+            }
+            const float eps = sTot[b];
+            if((bs + eps) < (0.01f - 1e-4f) * (lin - eps)) f = 1;
+            else if((bs - eps) > (0.01f + 1e-4f) * (lin + cTot[b] + eps)) f = 2;
+          }
+        }
+        // undecided: the warp sums that pixel's own kernel, 14 taps per lane
+        for(unsigned u = __ballot_sync(lanes, hit && f == 0); u; u &= u - 1) {
+          const int src = __ffs(u) - 1, st = warp * 32 + src;
+          const int sb = st / L::TPB, sr = st - sb * L::TPB, sk7 = sr / 7;
+          const int py = L::RY * (sr - sk7 * 7) + o, px = sb * FK + L::PX * sk7 + q;
+          if(lane < nC2) {
+            int i = 0, t0 = 0;
+            while(lane - t0 > K - i) t0 += K - i++ + 1;
+            sDP[warp][lane] =
+                (float)(xpow[i * RW + px] * ypow[(lane - t0) * FK + py] - poly[sb * TMAX + lane]);
+          }
+          __syncwarp(lanes);
+          float av = 0.f, uv = 0.f;
+          for(int p = lane; p < NK; p += __popc(lanes)) {
+            const int jj = p / FK, ii = p - jj * FK;
+            const int at = (FK - 1 - jj) * KS + FK - 1 - ii;
+            float kv = kern[sb * FK * KS + at];
+            for(int tt = 1; tt < nC2; tt++)
+              kv = fmaf(sDP[warp][tt], term[(tt - 1) * FK * KS + at], kv);
+            av += fabsf(kv);
+            if(!((bits[(py + jj) * NW + ((px + ii) >> 5)] >> ((px + ii) & 31)) & 1u)) uv += fabsf(kv);
+          }
+#pragma unroll
+          for(int d = 16; d > 0; d >>= 1) {
+            const float a2 = __shfl_down_sync(lanes, av, d), u2 = __shfl_down_sync(lanes, uv, d);
+            if(lane + d < 32 && ((lanes >> (lane + d)) & 1u)) {
+              av += a2;
+              uv += u2;
+            }
+          }
+          const int fs = (__shfl_sync(lanes, uv, 0) / __shfl_sync(lanes, av, 0)) < 0.99f ? 2 : 1;
+          if(lane == src) f = fs;
+          __syncwarp(lanes);
+        }
+        flag[o][q] = (unsigned char)f;
+      }
+  }
+  __syncthreads();  // every thread is done with the kernel rows
+  float* sv = kern;  // conv sums of the CTA's pixels, row-major (FK rows x BX*FK)
+  unsigned char* cflag = cv_smem + L::OFF_FLAG;
+#pragma unroll
+  for(int o = 0; o < 3; o++)
+#pragma unroll
+    for(int q = 0; q < 7; q++) {
+      const int e = (ly0 + o) * RW + lx0 + q;
+      sv[e] = base[o][q] + corr[o][q];
+      cflag[e] = flag[o][q];
+    }
   __syncthreads();
+  // one output column per thread, consecutive x across the CTA: coalesced
+  // reads of the other image and writes of mask, conv and difference
+  const float hxF = 0.5f * (float)a.w, hyF = 0.5f * (float)a.h;
+  const float ihxF = 1.f / hxF, ihyF = 1.f / hyF;
   const float kernSum = (float)*kernSumPtr;
   const float invKernMult = a.scaleConv ? 1.f / kernSum : 1.f;
   const float convFactor = a.scaleConv ? kernSum : 1.f;
   const float finalFactor = a.scaleConv ? -(1.f / kernSum) : 1.f;
-  const int perBlock = FK * TPR;
-  if(tid >= CV_BX * perBlock) return;
-  const int b = tid / perBlock, r = tid % perBlock, ly = r / TPR, lx0 = b * FK + (r % TPR) * PX;
-  const double yf = ((double)(y0 + HK + ly) - hy) / hy;
-  double xf[PX], xp[PX];
-  float base[PX], corr[PX];
-#pragma unroll
-  for(int q = 0; q < PX; q++) {
-    xf[q] = ((double)(x0 + HK + lx0 + q) - hx) / hx;
-    xp[q] = 1.0;
-    corr[q] = 0.f;
-  }
-  // t = 0 pass: the block kernel
-  {
-#pragma unroll
-    for(int q = 0; q < PX; q++) base[q] = 0.f;
-    for(int jj = 0; jj < FK; jj++) {
-      float win[PX + FK - 1];
-#pragma unroll
-      for(int q = 0; q < PX + FK - 1; q++) win[q] = tile[ly + jj][lx0 + q];
-      const float* krow = kern[b] + (FK - 1 - jj) * FK;
-#pragma unroll
-      for(int ii = 0; ii < FK; ii++) {
-        const float kk = krow[FK - 1 - ii];
-#pragma unroll
-        for(int q = 0; q < PX; q++) base[q] = fmaf(kk, win[q + ii], base[q]);
-      }
-    }
-  }
-  // t >= 1 passes: the spatial-term images weighted by dP_t
-  int t = 0;
-  for(int i = 0; i <= a.kOrder; i++) {
-    double yp = 1.0;
-    for(int j = 0; j <= a.kOrder - i; j++, t++) {
-      if(t > 0) {
-        const float* kb = ktf + t * NK;
-        float ct[PX];
-#pragma unroll
-        for(int q = 0; q < PX; q++) ct[q] = 0.f;
-        for(int jj = 0; jj < FK; jj++) {
-          float win[PX + FK - 1];
-#pragma unroll
-          for(int q = 0; q < PX + FK - 1; q++) win[q] = tile[ly + jj][lx0 + q];
-          const float* krow = kb + (FK - 1 - jj) * FK;
-#pragma unroll
-          for(int ii = 0; ii < FK; ii++) {
-            const float kk = krow[FK - 1 - ii];
-#pragma unroll
-            for(int q = 0; q < PX; q++) ct[q] = fmaf(kk, win[q + ii], ct[q]);
-          }
-        }
-#pragma unroll
-        for(int q = 0; q < PX; q++)
-          corr[q] = fmaf((float)(xp[q] * yp - poly[b][t]), ct[q], corr[q]);
-      }
-      yp *= yf;
-    }
-#pragma unroll
-    for(int q = 0; q < PX; q++) xp[q] *= xf[q];
-  }
-  const float hxF = 0.5f * (float)a.w, hyF = 0.5f * (float)a.h;
-  const float ihxF = 1.f / hxF, ihyF = 1.f / hyF;
-#pragma unroll
-  for(int q = 0; q < PX; q++) {
-    const int x = x0 + HK + lx0 + q, y = y0 + HK + ly;
-    if(x >= a.w - HK || y >= a.h - HK) continue;
-    unsigned char any = 0;
-    for(int jj = 0; jj < FK; jj++) any |= rowBad[ly + jj][lx0 + q];
-    const float bxf = ((float)x - hxF) * ihxF, byf = ((float)y - hyF) * ihyF;
+  static_assert(NT == RW, "one output column per thread");
+  const int x = x0 + HK + tid;
+  if(x >= a.w - HK) return;
+  const float bxf = ((float)x - hxF) * ihxF;
+  for(int ly = 0; ly < FK; ly++) {
+    const int y = y0 + HK + ly;
+    if(y >= a.h - HK) break;
+    const int e = ly * RW + tid;
+    const float byf = ((float)y - hyF) * ihyF;
     float bgv = 0.f, ax = 1.f;
     int k = 0;
     for(int i = 0; i <= a.bgOrder; i++) {
@@ -1089,45 +1402,20 @@ __global__ void __launch_bounds__(CV_BX * FK * (FK / 7))
       }
       ax *= bxf;
     }
-    const float v = (base[q] + corr[q] + bgv) * invKernMult;
+    const float v = (sv[e] + bgv) * invKernMult;
     const size_t id = (size_t)x + (size_t)y * a.w;
-    const float tc = tile[ly + HK][lx0 + q + HK];
-    uint16_t cm = convMaskF(tc, a.tH, a.tL);
-    if(inMask && inMask[id]) cm |= INPUT_MASK | BAD_INPUT;
-    uint16_t nm = cm;
-    if(cm & BAD_INPUT) nm |= BAD_OUTPUT;
-    if(any) {
-      // this pixel's kernel tap by tap, for the 0.99 |kernel| rule
-      float dP[MAXT];
-      {
-        double xpw = 1.0;
-        int tt = 0;
-        for(int i = 0; i <= a.kOrder; i++) {
-          double ypw = 1.0;
-          for(int j = 0; j <= a.kOrder - i; j++, tt++) {
-            dP[tt] = (float)(xpw * ypw - poly[b][tt]);
-            ypw *= yf;
-          }
-          xpw *= xf[q];
-        }
-      }
-      float aks = 0.f, uks = 0.f;
-      for(int jj = 0; jj < FK; jj++)
-        for(int ii = 0; ii < FK; ii++) {
-          const int tap = (FK - 1 - ii) + (FK - 1 - jj) * FK;
-          float kv = kern[b][tap];
-          for(int tt = 1; tt < nC2; tt++) kv = fmaf(dP[tt], ktf[tt * NK + tap], kv);
-          aks += fabsf(kv);
-          if(!bad[ly + jj][lx0 + q + ii]) uks += fabsf(kv);
-        }
-      if((uks / aks) < 0.99f) nm |= BAD_OUTPUT | BAD_CONV;
-      else nm |= OK_CONV;
-    }
-    const float o = O[id];
-    nm |= afterMaskF(o, a.tH, a.tL);
+    const float tc = tile[(ly + HK) * S + tid + HK];
+    uint16_t nm = convMaskF(tc, a.tH, a.tL);
+    if(inMask && inMask[id]) nm |= INPUT_MASK | BAD_INPUT;
+    if(nm & BAD_INPUT) nm |= BAD_OUTPUT;
+    const unsigned char f = cflag[e];
+    if(f == 2) nm |= BAD_OUTPUT | BAD_CONV;
+    else if(f == 1) nm |= OK_CONV;
+    const float ov = O[id];
+    nm |= afterMaskF(ov, a.tH, a.tL);
     mask[id] = nm;
     convF[id] = v;
-    diffF[id] = (nm & BAD_OUTPUT) ? 1e-30f : (v * convFactor - o) * finalFactor;
+    diffF[id] = (nm & BAD_OUTPUT) ? 1e-30f : (v * convFactor - ov) * finalFactor;
   }
 }
 
@@ -1594,13 +1882,11 @@ void convSubMixed(xb_ctx* c, double* dKernSum) {
   a.tL = (float)c->p.threshLow;
   const int xSteps = (c->w + g.fK - 1) / g.fK, ySteps = (c->h + g.fK - 1) / g.fK;
   a.xSteps = xSteps;
-  double* blockXY = nullptr;
-  if(!c->p.convPerPixel) {
-    blockXY = buf<double>(c, "conv_block_xy", (size_t)(xSteps + ySteps));
-    k_block_centres<<<(xSteps + ySteps + 127) / 128, 128, 0, c->stream>>>(c->w, c->h, g.fK, xSteps,
-                                                                        ySteps, blockXY);
-    XB_LAUNCHED(c);
-  }
+  // (the last CTA of a row reads up to seven centres past the columns)
+  double* blockXY = buf<double>(c, "conv_block_xy", (size_t)(xSteps + ySteps + 8));
+  k_block_centres<<<(xSteps + ySteps + 127) / 128, 128, 0, c->stream>>>(c->w, c->h, g.fK, xSteps,
+                                                                      ySteps, blockXY);
+  XB_LAUNCHED(c);
   auto launch = [&](int variant) {
     const float *Ii = (const float*)c->img[I], *Oi = (const float*)c->img[O];
     switch(variant) {
@@ -1620,17 +1906,12 @@ void convSubMixed(xb_ctx* c, double* dKernSum) {
     XB_LAUNCHED(c);
   };
   if(c->p.convPerPixel) {
-    const int nC2 = g.nComp2, nk = g.fK * g.fK;
-    const size_t smemPP = (size_t)nC2 * nk * sizeof(float);
-    int optin = 0;
-    XB_CUDA(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, c->device));
-    if(c->p.kernelOrder > MAX_KORDER || smemPP + 16 * 1024 > (size_t)optin)
-      throw XbError{XB_ERR_UNSUPPORTED, "per-pixel kernel: kernel order too large"};
-    XB_CUDA(allowMaxDynamicSmem((const void*)k_conv_sub_pp_f32<21, 2>, c->device));
+    XB_CUDA(allowMaxDynamicSmem((const void*)k_conv_sub_pp_f32<21, 6>, c->device));
     KT_SCOPE(c, "conv_sub");
-    k_conv_sub_pp_f32<21, 2><<<dim3((xSteps + 1) / 2, ySteps), 2 * 63, smemPP, c->stream>>>(
-        (const float*)c->img[I], (const float*)c->img[O], c->dSol, Kt, dKernSum, a, c->inputMask,
-        c->mask, c->convF, c->diffF);
+    k_conv_sub_pp_f32<21, 6><<<dim3((xSteps + 5) / 6, ySteps), 6 * 21,
+                               ConvTilePP<21, 6>::bytes(g.nComp2), c->stream>>>(
+        (const float*)c->img[I], (const float*)c->img[O], c->dSol, Kt, blockXY, dKernSum, a,
+        c->inputMask, c->mask, c->convF, c->diffF);
     XB_LAUNCHED(c);
   } else {
     // blocks per CTA: 4 (default), 6 or 8; the three give identical images
