@@ -58,9 +58,22 @@ __device__ __forceinline__ double roundToFloat(double t) {
   return __longlong_as_double((b + 0x0FFFFFFFll + ((b >> 29) & 1)) & ~0x1FFFFFFFll);
 }
 
-// Copies of 8 bytes to shared memory that complete asynchronously, in groups.
+// Copies of 4, 8 or 16 bytes to shared memory that complete asynchronously, in
+// groups.
+__device__ __forceinline__ void cpAsync4(void* dst, const void* src) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(
+                   (unsigned)__cvta_generic_to_shared(dst)),
+               "l"(src)
+               : "memory");
+}
 __device__ __forceinline__ void cpAsync8(void* dst, const void* src) {
   asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(
+                   (unsigned)__cvta_generic_to_shared(dst)),
+               "l"(src)
+               : "memory");
+}
+__device__ __forceinline__ void cpAsync16(void* dst, const void* src) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(
                    (unsigned)__cvta_generic_to_shared(dst)),
                "l"(src)
                : "memory");

@@ -705,24 +705,31 @@ __global__ void __launch_bounds__(LUB_THREADS)
 // makeKernelCoeffs + makeKernel + sumKernel (cd.cl:354-442): kernel image at
 // (x, y) and its sum; tree=1 sums in 32-wide groups like sumKernel, tree=0
 // sequentially like the CPU makeKernel (bachUtil.cpp:532-538).
-__global__ void k_kernel_sum(const double* __restrict__ sol, const double* __restrict__ vec,
+// One tap per thread, the terms' loads ahead of the ordered sums; the groups of
+// the tree sum run side by side (two rounds of taps from dependent loads and
+// one lane's serial sum took 40 us; now 23 to 37).
+constexpr int KS_THREADS = 512;
+__global__ void __launch_bounds__(KS_THREADS)
+    k_kernel_sum(const double* __restrict__ sol, const double* __restrict__ vec,
                              int nPSF, int kOrder, int fK, double xf, double yf, int tree,
                              double* __restrict__ out) {
   __shared__ double coeff[MAX_NPSF];
-  __shared__ double kern[MAX_FK * MAX_FK];
+  __shared__ double kern[MAX_FK * MAX_FK + 16];
   __shared__ double part[64];
   const int tid = threadIdx.x, nk = fK * fK;
-  for(int i = tid; i < nPSF; i += blockDim.x) {
+  const int nC2 = (kOrder + 1) * (kOrder + 2) / 2;
+  for(int i = tid; i < nPSF; i += KS_THREADS) {
     double c = 0.0;
     if(i == 0) {
       c = sol[1];
     } else {
-      int k = 2 + (i - 1) * ((kOrder + 1) * (kOrder + 2) / 2);
+      const double* p = sol + 2 + (size_t)(i - 1) * nC2;
       double aX = 1.0;
       for(int x = 0; x <= kOrder; x++) {
         double aY = 1.0;
+#pragma unroll 4
         for(int y = 0; y <= kOrder - x; y++) {
-          c += sol[k++] * aX * aY;
+          c += *p++ * aX * aY;
           aY *= yf;
         }
         aX *= xf;
@@ -731,35 +738,50 @@ __global__ void k_kernel_sum(const double* __restrict__ sol, const double* __res
     coeff[i] = c;
   }
   __syncthreads();
-  for(int p = tid; p < nk; p += blockDim.x) {
+  for(int p = tid; p < nk; p += KS_THREADS) {
     double k0 = 0.0;
-    for(int q = 0; q < nPSF; q++) k0 += coeff[q] * vec[(size_t)q * nk + p];
+    int q = 0;
+    for(; q + 8 <= nPSF; q += 8) {
+      double v[8];
+#pragma unroll
+      for(int u = 0; u < 8; u++) v[u] = vec[(size_t)(q + u) * nk + p];
+#pragma unroll
+      for(int u = 0; u < 8; u++) k0 += coeff[q + u] * v[u];
+    }
+    for(; q < nPSF; q++) k0 += coeff[q] * vec[(size_t)q * nk + p];
     kern[p] = k0;
   }
+  if(tid < 16) kern[nk + tid] = 0.0;
   __syncthreads();
-  if(tid == 0) {
-    double s = 0.0;
-    if(!tree) {
-      for(int p = 0; p < nk; p++) s += kern[p];
-    } else {
-      int count = nk;
-      double* cur = kern;
-      while(count > 1) {
-        int groups = (count + 31) / 32;
-        for(int g = 0; g < groups; g++) {
-          double a = 0.0;
-          int lc = min(32, count - g * 32);
-          for(int l = 0; l < lc; l++) a += cur[g * 32 + l];
-          part[g] = a;
-        }
-        for(int g = 0; g < groups; g++) kern[g] = part[g];
-        cur = kern;
-        count = groups;
+  if(!tree) {
+    if(tid == 0) {
+      double s = 0.0;
+      for(int p = 0; p < nk; p += 8) {  // the zeros past nk leave the sum as it is
+        double v[8];
+#pragma unroll
+        for(int u = 0; u < 8; u++) v[u] = kern[p + u];
+#pragma unroll
+        for(int u = 0; u < 8; u++) s += v[u];
       }
-      s = kern[0];
+      *out = s;
     }
-    *out = s;
+    return;
   }
+  for(int count = nk; count > 1;) {
+    const int groups = (count + 31) / 32;
+    if(tid < groups) {
+      double a = 0.0;
+      const int lc = min(32, count - tid * 32);
+#pragma unroll 8
+      for(int l = 0; l < lc; l++) a += kern[tid * 32 + l];
+      part[tid] = a;
+    }
+    __syncthreads();
+    if(tid < groups) kern[tid] = part[tid];
+    __syncthreads();
+    count = groups;
+  }
+  if(tid == 0) *out = kern[0];
 }
 
 // --------------------------------------------------------------- chi^2 ----
@@ -1155,7 +1177,7 @@ static void computeSigs(xb_ctx* c, int si, const int* dList, int nList, const do
 
 void kernelSumLaunch(xb_ctx* c, const double* dSol, double xf, double yf, int tree, double* dOut) {
   { KT_SCOPE(c, "kernel_sum");
-  k_kernel_sum<<<1, 256, 0, c->stream>>>(dSol, c->dVec, c->g.nPSF, c->p.kernelOrder, c->g.fK, xf, yf,
+  k_kernel_sum<<<1, KS_THREADS, 0, c->stream>>>(dSol, c->dVec, c->g.nPSF, c->p.kernelOrder, c->g.fK, xf, yf,
                                          tree, dOut);
   XB_LAUNCHED(c);
   }

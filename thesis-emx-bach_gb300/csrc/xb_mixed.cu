@@ -108,7 +108,9 @@ __global__ void __launch_bounds__(MX_THREADS)
   }
 }
 
-// convStampOdd and convStampBg on the hi + lo pair; pads the background rows.
+// convStampOdd and convStampBg on the hi + lo pair, one row of W per CTA (one
+// CTA per stamp took 65 us for its dependent passes over L2); pads the
+// background rows.
 __global__ void __launch_bounds__(MX_THREADS)
     k_fill_finish_f32(const int* __restrict__ list, const int* __restrict__ liveN,
                       const int* __restrict__ count,
@@ -117,53 +119,42 @@ __global__ void __launch_bounds__(MX_THREADS)
                       const int2* __restrict__ bgXY, int nBG, int hSS, int w, int h, int wRows,
                       int ldW, float* __restrict__ W, float* __restrict__ Wlo) {
   if(liveN && (int)blockIdx.x >= *liveN) return;
-  const int s = list[blockIdx.x], tid = threadIdx.x;
+  const int s = list[blockIdx.x], n = 1 + blockIdx.y, tid = threadIdx.x;
   const int fSS = 2 * hSS + 1, wCols = fSS * fSS;
   float* Ws = W + (size_t)s * wRows * ldW;
   float* Wl = Wlo + (size_t)s * wRows * ldW;
-  const bool live = cur[s] < count[s];
-  // W[n] -= W[0] for the even/even rows: each thread takes its pixels
-  // through all such rows (independent loads in flight, not one pass per row)
-  __shared__ short evenRows[MAX_NPSF];
-  __shared__ int nEven;
-  if(tid == 0) {
-    int m = 0;
-    for(int n = 1; n < nPSF; n++)
-      if(kx[n] % 2 == 0 && ky[n] % 2 == 0) evenRows[m++] = (short)n;
-    nEven = m;
-  }
-  __syncthreads();
-  const int ne = nEven;
-  for(int p = tid; p < wCols; p += MX_THREADS) {
-    const float bh = Ws[p], bl = Wl[p];
+  if(n < nPSF) {  // W[n] -= W[0] for the even/even rows
+    if(kx[n] % 2 != 0 || ky[n] % 2 != 0) return;
 #pragma unroll 4
-    for(int e = 0; e < ne; e++) {
-      const size_t i = (size_t)evenRows[e] * ldW + p;
+    for(int p = tid; p < wCols; p += MX_THREADS) {
+      const size_t i = (size_t)n * ldW + p;
       float hi, lo;
-      dfSub(Ws[i], Wl[i], bh, bl, hi, lo);
+      dfSub(Ws[i], Wl[i], Ws[p], Wl[p], hi, lo);
       Ws[i] = hi;
       Wl[i] = lo;
     }
+    return;
   }
+  const int b = n - nPSF;
+  const bool live = cur[s] < count[s];
   int2 c = make_int2(0, 0);
   if(live) c = ssxy[(size_t)s * maxSS + cur[s]];
-  for(int b = 0; b < nBG; b++)
-    for(int p = tid; p < ldW; p += MX_THREADS) {
-      double a = 0.0;
-      if(live && p < wCols) {
-        // the reference's form: float-normalised coordinates, FP64 powers
-        const double xf = (double)floatNormF(c.x - hSS + p % fSS, w);
-        const double yf = (double)floatNormF(c.y - hSS + p / fSS, h);
-        double ax = 1.0, ay = 1.0;
-        for(int i = 0; i < bgXY[b].x; i++) ax *= xf;
-        for(int i = 0; i < bgXY[b].y; i++) ay *= yf;
-        a = ax * ay;
-      }
-      float hi, lo;
-      splitF64(a, hi, lo);
-      Ws[(size_t)(nPSF + b) * ldW + p] = hi;
-      Wl[(size_t)(nPSF + b) * ldW + p] = lo;
+  for(int p = tid; p < ldW; p += MX_THREADS) {
+    double a = 0.0;
+    if(live && p < wCols) {
+      // the reference's form: float-normalised coordinates, FP64 powers
+      const double xf = (double)floatNormF(c.x - hSS + p % fSS, w);
+      const double yf = (double)floatNormF(c.y - hSS + p / fSS, h);
+      double ax = 1.0, ay = 1.0;
+      for(int i = 0; i < bgXY[b].x; i++) ax *= xf;
+      for(int i = 0; i < bgXY[b].y; i++) ay *= yf;
+      a = ax * ay;
     }
+    float hi, lo;
+    splitF64(a, hi, lo);
+    Ws[(size_t)(nPSF + b) * ldW + p] = hi;
+    Wl[(size_t)(nPSF + b) * ldW + p] = lo;
+  }
 }
 
 // ------------------------------------------------------------------ Gram ---
@@ -172,84 +163,165 @@ __global__ void __launch_bounds__(MX_THREADS)
 // kernel).  Each W element hi + lo is exact in FP64; the normal matrices are
 // ill-conditioned (cond ~1e14), and an FP32 accumulation moves the fitted
 // kernel sum by up to 9 %.  Each stamp's lower triangle is split over
-// gridDim.y CTAs; k_gram_scatter then fills Q (createQ), B (createB) and the
-// global-matrix dot table.
-constexpr int GM_KT = 32, GM_SPLIT = 6;
-template <class T>
-__global__ void __launch_bounds__(MX_THREADS)
+// gridDim.y CTAs of NT threads with EN entries each; k_gram_scatter then fills Q
+// (createQ), B (createB) and the global-matrix dot table.
+//
+// Bound by FP64, one warp instruction per 19 cycles and SM: one product per
+// entry and pixel, and one sum per element to form hi + lo (the floats widened
+// on their bits, two conversions less).  256 threads with five entries make
+// that sum 6 % of a full list's work; a refill of a few stamps takes 64
+// threads with one entry, which spreads a stamp over ~36 SMs.  hi and lo are
+// staged one tile ahead.  (256 entries per CTA, each CTA converting every
+// row for itself: 2.87 ms for 390 stamps of 67 rows, 0.22 ms for one; now
+// 1.96 ms and 0.14 ms.)
+constexpr int GM_KT = 32;
+// f in FP64 for a normal or zero f; odd is set for any other f
+__device__ __forceinline__ double widen(float f, bool& odd) {
+  const unsigned b = __float_as_uint(f), m = b & 0x7FFFFFFFu;
+  odd |= m != 0u && m - 0x00800000u >= 0x7F000000u;
+  const unsigned hi = m ? (b & 0x80000000u) | ((m >> 3) + (896u << 20)) : 0u;
+  return __hiloint2double((int)hi, (int)(b << 29));
+}
+inline size_t gmSmemBytes(int R) {
+  return (size_t)R * (GM_KT + 1) * sizeof(double) + (size_t)4 * R * GM_KT * sizeof(float);
+}
+template <class T, int NT, int EN>
+__global__ void __launch_bounds__(NT)
     k_gram_mixed(const T* __restrict__ other, const T* __restrict__ conv, int w, int h,
-                 const int* __restrict__ list,
-                 const int* __restrict__ liveN, const int* __restrict__ count, const int* __restrict__ cur,
+                 const int* __restrict__ list, int nList, const int* __restrict__ liveN,
+                 const int* __restrict__ count, const int* __restrict__ cur,
                  const int2* __restrict__ ssxy, int maxSS, int hSS, int wRows, int ldW,
                  const float* __restrict__ W, const float* __restrict__ Wlo,
-                 double* __restrict__ Gout, int weighted, double invGain, double rn2x2) {
-  extern __shared__ double gm_s[];
+                 double* __restrict__ Gout, bool staged, int weighted, double invGain, double rn2x2) {
+  extern __shared__ __align__(16) double gm_s[];
   __shared__ double omT[GM_KT];  // pixel weights of the tile (weighted fit)
-  if(liveN && (int)blockIdx.x >= *liveN) return;
-  const int t = blockIdx.x, s = list[t], tid = threadIdx.x;
+  const int nLive = liveN ? min(*liveN, nList) : nList;
+  if((int)blockIdx.x >= nLive) return;
+  const int tid = threadIdx.x;
   const int fSS = 2 * hSS + 1, wCols = fSS * fSS, R = wRows + 1;
   const int nEnt = R * (R + 1) / 2;
-  const int per = (nEnt + gridDim.y - 1) / gridDim.y, e0 = blockIdx.y * per;
-  double* tile = gm_s;  // R x (GM_KT + 1)
-  const float* Ws = W + (size_t)s * wRows * ldW;
-  const float* Wl = Wlo + (size_t)s * wRows * ldW;
-  const bool live = cur[s] < count[s];
-  int2 c = make_int2(0, 0);
-  if(live) c = ssxy[(size_t)s * maxSS + cur[s]];
-  int ei = -1, ej = 0;
-  const int idx = e0 + tid;
-  if(tid < per && idx < nEnt) {
-    int i = (int)((sqrtf(8.f * idx + 1.f) - 1.f) * 0.5f);
+  auto rowOf = [](int idx) {
+    int i = (int)((sqrtf(8.f * (float)idx + 1.f) - 1.f) * 0.5f);
     while((i + 1) * (i + 2) / 2 <= idx) i++;
     while(i * (i + 1) / 2 > idx) i--;
-    ei = i;
-    ej = idx - i * (i + 1) / 2;
+    return i;
+  };
+  const int e0 = blockIdx.y * NT * EN;
+  const int rows = rowOf(min(e0 + NT * EN, nEnt) - 1) + 1;  // rows this CTA's entries need
+  float* stage = (float*)gm_s;  // 2 x [hi, lo] x R x GM_KT, when staged
+  double* tile = gm_s + (staged ? (size_t)2 * R * GM_KT : 0);  // rows x (GM_KT + 1)
+  int oa[EN], ob[EN];
+#pragma unroll
+  for(int u = 0; u < EN; u++) {
+    const int idx = e0 + u * NT + tid;
+    const int i = idx < nEnt ? rowOf(idx) : 0, jj = idx < nEnt ? idx - i * (i + 1) / 2 : 0;
+    oa[u] = i * (GM_KT + 1);
+    ob[u] = jj * (GM_KT + 1);
   }
-  double acc = 0.0;
-  for(int k0 = 0; k0 < wCols; k0 += GM_KT) {
-    const int kt = min(GM_KT, wCols - k0);
-    for(int i = tid; i < R * GM_KT; i += MX_THREADS) {
-      const int r = i / GM_KT, kk = i % GM_KT;
-      double v = 0.0;
-      if(kk < kt) {
-        if(r < wRows) {
-          v = (double)Ws[(size_t)r * ldW + k0 + kk] + (double)Wl[(size_t)r * ldW + k0 + kk];
-        } else if(live) {
-          const int k = k0 + kk;
-          const int gx = min(max(c.x - hSS + k % fSS, 0), w - 1);
-          const int gy = min(max(c.y - hSS + k / fSS, 0), h - 1);
-          v = (double)(float)other[(size_t)gx + (size_t)gy * w];
+  const int wr = min(rows, wRows), nT = (wCols + GM_KT - 1) / GM_KT;
+  for(int t = blockIdx.x; t < nLive; t += gridDim.x) {
+    const int s = list[t];
+    const float* Ws = W + (size_t)s * wRows * ldW;
+    const float* Wl = Wlo + (size_t)s * wRows * ldW;
+    const bool live = cur[s] < count[s];
+    int2 c = make_int2(0, 0);
+    if(live) c = ssxy[(size_t)s * maxSS + cur[s]];
+    auto pixel = [&](int k) {
+      const int gx = min(max(c.x - hSS + k % fSS, 0), w - 1);
+      const int gy = min(max(c.y - hSS + k / fSS, 0), h - 1);
+      return (size_t)gx + (size_t)gy * w;
+    };
+    auto fetch = [&](int q) {  // tile q's floats (past wCols: the rows' zero padding)
+      float* sh = stage + (size_t)(q & 1) * 2 * R * GM_KT;
+      float* sl = sh + (size_t)R * GM_KT;
+      const int k4 = 4 * (tid & 7), k0 = q * GM_KT;  // ldW is a multiple of 4 floats
+      if(k0 + k4 < ldW)
+        for(int r = tid >> 3; r < wr; r += NT / 8) {
+          cpAsync16(sh + r * GM_KT + k4, Ws + (size_t)r * ldW + k0 + k4);
+          cpAsync16(sl + r * GM_KT + k4, Wl + (size_t)r * ldW + k0 + k4);
+        }
+      if(rows > wRows && tid < GM_KT) {
+        sh[wRows * GM_KT + tid] = live && k0 + tid < wCols ? (float)other[pixel(k0 + tid)] : 0.f;
+        sl[wRows * GM_KT + tid] = 0.f;
+      }
+      cpAsyncCommit();
+    };
+    double acc[EN];
+#pragma unroll
+    for(int u = 0; u < EN; u++) acc[u] = 0.0;
+    if(staged) fetch(0);
+    for(int q = 0; q < nT; q++) {
+      const int kt = min(GM_KT, wCols - q * GM_KT);
+      cpAsyncWaitGroup<0>();
+      __syncthreads();  // the floats are there, and the tile before is used up
+      if(staged) {
+        const float* sh = stage + (size_t)(q & 1) * 2 * R * GM_KT;
+        const float* sl = sh + (size_t)R * GM_KT;
+        constexpr int B = 8;  // elements in flight per thread
+        const int kk = tid & 31;
+        for(int r0 = tid >> 5; r0 < rows; r0 += B * (NT / 32)) {
+          float vh[B], vl[B];
+          double v[B];
+          bool odd = false;
+#pragma unroll
+          for(int u = 0; u < B; u++) {
+            const int r = r0 + u * (NT / 32);
+            const bool in = r < rows && kk < kt;
+            vh[u] = in ? sh[r * GM_KT + kk] : 0.f;
+            vl[u] = in ? sl[r * GM_KT + kk] : 0.f;
+          }
+#pragma unroll
+          for(int u = 0; u < B; u++) v[u] = widen(vh[u], odd) + widen(vl[u], odd);
+          // a vote, so that the conversions of the FP64 unit stay out of the usual case
+          if(__any_sync(0xffffffffu, odd))
+#pragma unroll
+            for(int u = 0; u < B; u++) v[u] = (double)vh[u] + (double)vl[u];
+#pragma unroll
+          for(int u = 0; u < B; u++)
+            if(r0 + u * (NT / 32) < rows) tile[(r0 + u * (NT / 32)) * (GM_KT + 1) + kk] = v[u];
+        }
+      } else {
+        for(int i = tid; i < rows * GM_KT; i += NT) {
+          const int r = i / GM_KT, kk = i % GM_KT, k = q * GM_KT + kk;
+          double v = 0.0;
+          if(kk < kt) {
+            if(r < wRows) v = (double)Ws[(size_t)r * ldW + k] + (double)Wl[(size_t)r * ldW + k];
+            else if(live) v = (double)(float)other[pixel(k)];
+          }
+          tile[r * (GM_KT + 1) + kk] = v;
         }
       }
-      tile[r * (GM_KT + 1) + kk] = v;
-    }
-    if(weighted && tid < GM_KT) {
-      double v = 0.0;
-      if(tid < kt && live) {
-        const int k = k0 + tid;
-        const int gx = min(max(c.x - hSS + k % fSS, 0), w - 1);
-        const int gy = min(max(c.y - hSS + k / fSS, 0), h - 1);
-        const size_t id = (size_t)gx + (size_t)gy * w;
-        v = fitWeight((double)conv[id], (double)other[id], invGain, rn2x2);
+      if(weighted && tid < GM_KT) {
+        double v = 0.0;
+        if(tid < kt && live) {
+          const size_t id = pixel(q * GM_KT + tid);
+          v = fitWeight((double)conv[id], (double)other[id], invGain, rn2x2);
+        }
+        omT[tid] = v;
       }
-      omT[tid] = v;
-    }
-    __syncthreads();
-    if(ei >= 0) {
-      const double* a = tile + ei * (GM_KT + 1);
-      const double* b = tile + ej * (GM_KT + 1);
+      if(staged && q + 1 < nT) fetch(q + 1);
+      __syncthreads();
       if(weighted) {
-        for(int kk = 0; kk < kt; kk++) acc = fma(a[kk], b[kk] * omT[kk], acc);
+        for(int kk = 0; kk < kt; kk++)
+#pragma unroll
+          for(int u = 0; u < EN; u++)
+            acc[u] = fma(tile[oa[u] + kk], tile[ob[u] + kk] * omT[kk], acc[u]);
       } else {
-        for(int kk = 0; kk < kt; kk++) acc = fma(a[kk], b[kk], acc);
+#pragma unroll 4
+        for(int kk = 0; kk < kt; kk++)
+#pragma unroll
+          for(int u = 0; u < EN; u++) acc[u] = fma(tile[oa[u] + kk], tile[ob[u] + kk], acc[u]);
       }
     }
-    __syncthreads();
-  }
-  if(ei >= 0) {
     double* G = Gout + (size_t)t * R * R;
-    G[ei * R + ej] = acc;
-    G[ej * R + ei] = acc;
+#pragma unroll
+    for(int u = 0; u < EN; u++)
+      if(e0 + u * NT + tid < nEnt) {
+        const int a = oa[u] / (GM_KT + 1), b = ob[u] / (GM_KT + 1);
+        G[a * R + b] = acc[u];
+        G[b * R + a] = acc[u];
+      }
+    __syncthreads();  // the next stamp's floats replace this one's
   }
 }
 
@@ -1699,7 +1771,7 @@ void fillStampsMixed(xb_ctx* c, int si, const int* dList, int nList, int imgConv
   }
   {
     KT_SCOPE(c, "fill_finish");
-    k_fill_finish_f32<<<nList, MX_THREADS, 0, c->stream>>>(
+    k_fill_finish_f32<<<dim3(nList, g.nPSF - 1 + g.nBG), MX_THREADS, 0, c->stream>>>(
         dList, liveN, S.count, S.cur, S.ssxy, g.maxSS, c->dKx, c->dKy, g.nPSF, buf<int2>(c, "bgXY", g.nBG),
         g.nBG, g.hSS, c->w, c->h, g.wRows, ldW, S.Wf, S.Wlo);
     XB_LAUNCHED(c);
@@ -1707,23 +1779,36 @@ void fillStampsMixed(xb_ctx* c, int si, const int* dList, int nList, int imgConv
   {
     KT_SCOPE(c, "gram");
     const int R = g.wRows + 1;
-    const size_t smem = (size_t)R * (GM_KT + 1) * sizeof(double);
-    // one Gram entry per thread of the split CTAs
-    const int split = std::max(GM_SPLIT, (R * (R + 1) / 2 + MX_THREADS - 1) / MX_THREADS);
+    const int nEnt = R * (R + 1) / 2;
     double* G = buf<double>(c, "gram_scratch", (size_t)nList * R * R);
-    dim3 grid(nList, split);
+    // a refill's list is short (its bound is not): spread each stamp
+    const bool refill = liveN && liveN != S.dN;
+    const bool spread = refill || (long long)nList * nEnt < 4ll * 256 * c->smCount;
+    int optin = 0;
+    XB_CUDA(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, c->device));
+    const size_t full = gmSmemBytes(R);
+    const bool staged = full + 1024 <= (size_t)optin;
+    const size_t smem = staged ? full : (size_t)R * (GM_KT + 1) * sizeof(double);
+    auto gram = [&](auto* img, auto kernel, int per, int nt) {
+      XB_CUDA(allowMaxDynamicSmem((const void*)kernel, c->device));
+      const int nY = (nEnt + per - 1) / per;
+      // a refill launches what the SMs hold at once and loops over its stamps
+      const int fit = (int)std::max<size_t>(1, (size_t)optin / (smem + 2048)) * c->smCount;
+      const int nX = refill ? std::min(nList, std::max(1, fit / nY)) : nList;
+      kernel<<<dim3(nX, nY), nt, smem, c->stream>>>(
+          img, (decltype(img))c->img[imgConv], c->w, c->h, dList, nList, liveN, S.count, S.cur,
+          S.ssxy, g.maxSS, g.hSS, g.wRows, ldW, S.Wf, S.Wlo, G, staged, c->p.fitWeighted,
+          noiseInvGain(c->p), noiseRn2x2(c->p));
+    };
     if(!c->p.fitWeighted && gramTensorCores(c, si, dList, nList, other, G, liveN)) {
       // exact tensor-core Gram (xb_gram_tc.cu)
-    } else if(c->imgIsF64)
-      k_gram_mixed<double><<<grid, MX_THREADS, smem, c->stream>>>(
-          (const double*)c->img[other], (const double*)c->img[imgConv], c->w, c->h, dList, liveN,
-          S.count, S.cur, S.ssxy, g.maxSS, g.hSS, g.wRows, ldW, S.Wf, S.Wlo, G, c->p.fitWeighted,
-          noiseInvGain(c->p), noiseRn2x2(c->p));
-    else
-      k_gram_mixed<float><<<grid, MX_THREADS, smem, c->stream>>>(
-          (const float*)c->img[other], (const float*)c->img[imgConv], c->w, c->h, dList, liveN,
-          S.count, S.cur, S.ssxy, g.maxSS, g.hSS, g.wRows, ldW, S.Wf, S.Wlo, G, c->p.fitWeighted,
-          noiseInvGain(c->p), noiseRn2x2(c->p));
+    } else if(c->imgIsF64) {
+      if(spread) gram((const double*)c->img[other], k_gram_mixed<double, 64, 1>, 64, 64);
+      else gram((const double*)c->img[other], k_gram_mixed<double, 256, 5>, 1280, 256);
+    } else {
+      if(spread) gram((const float*)c->img[other], k_gram_mixed<float, 64, 1>, 64, 64);
+      else gram((const float*)c->img[other], k_gram_mixed<float, 256, 5>, 1280, 256);
+    }
     XB_LAUNCHED(c);
     k_gram_scatter<<<nList, MX_THREADS, 0, c->stream>>>(dList, liveN, S.count, S.cur, g.wRows,
                                                         g.nPSF, g.nBG, g.qCount, G, S.Q, S.B,

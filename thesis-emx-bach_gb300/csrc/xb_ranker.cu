@@ -33,6 +33,7 @@
 
 #include <cuda_bf16.h>
 
+#include "xb_device.cuh"
 #include "xb_internal.h"
 
 namespace xb {
@@ -93,15 +94,6 @@ __device__ __forceinline__ int rwIndex(int q) {
   return RW_H + q - O_HW;  // head weights, then its bias
 }
 
-__device__ __forceinline__ void cpAsync4(float* dst, const float* src) {
-  asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(
-                   (unsigned)__cvta_generic_to_shared(dst)),
-               "l"(src)
-               : "memory");
-}
-__device__ __forceinline__ void cpAsyncWait() {
-  asm volatile("cp.async.wait_all;" ::: "memory");
-}
 // Barrier of the two warps of sample slot s.
 __device__ __forceinline__ void pairSync(int s) {
   asm volatile("bar.sync %0, 64;" ::"r"(s + 1) : "memory");
@@ -128,7 +120,8 @@ __device__ float rfSample(const float* __restrict__ Wt, const float* __restrict_
     }
   }
   const float st = lane < RK_NS ? stats[lane] : 0.f;
-  cpAsyncWait();
+  cpAsyncCommit();
+  cpAsyncWaitGroup<0>();
   pairSync(s);
   if(lane < 2 * RK_S1) {
     const int y = lane >> 1, h = lane & 1;
