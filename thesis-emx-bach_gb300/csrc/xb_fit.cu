@@ -71,6 +71,18 @@ __device__ __forceinline__ void pivotCombine(double& v, int& i, double ov, int o
   }
 }
 
+// Both stamp sets of cd in one launch (grid dimension y, or x of a one-CTA
+// kernel): n bounds a set's kept stamps, liveN, when set, counts them on the
+// device.
+struct CdSets {
+  const double* Q[2];
+  const double* B[2];
+  int n[2];
+  const int* liveN[2];
+  double* ks[2];
+  int* testIdx[2];
+};
+
 // ------------------------------------------------------ per-stamp test fit --
 // createTestVec/createTestMat (cd.cl:15-44), GPU ludcmp (bach.cl:1-87, no
 // zero-row check) and lubksb, saveKernelSums (cd.cl:46-52).  The Crout
@@ -78,10 +90,14 @@ __device__ __forceinline__ void pivotCombine(double& v, int& i, double ov, int o
 // the same products in the same order, so the factors are identical.
 constexpr int LU_THREADS = 128;
 __global__ void __launch_bounds__(LU_THREADS)
-    k_stamp_test_fit(const double* __restrict__ Q, const double* __restrict__ B, int qc,
-                     const int* __restrict__ liveN, double* __restrict__ kernelSums) {
+    k_stamp_test_fit(const __grid_constant__ CdSets sets, int qc) {
   extern __shared__ double lu_s[];
-  if(liveN && (int)blockIdx.x >= *liveN) return;
+  const int set = blockIdx.y;
+  const int* liveN = sets.liveN[set];
+  if((int)blockIdx.x >= sets.n[set] || (liveN && (int)blockIdx.x >= *liveN)) return;
+  const double* __restrict__ Q = sets.Q[set];
+  const double* __restrict__ B = sets.B[set];
+  double* __restrict__ kernelSums = sets.ks[set];
   const int s = blockIdx.x, tid = threadIdx.x, n = qc - 1;
   double* a = lu_s;                 // qc * qc
   double* b = a + qc * qc;          // qc
@@ -180,50 +196,86 @@ __global__ void __launch_bounds__(LU_THREADS)
 // L^T x = b and z = L^-1 b, the last row of L^T x = D^-1 z is x_n = z_n / d_n):
 // no back substitution.  A zero pivot becomes 1e-20, as in the reference's LU.
 // Warps (stamps) per CTA: 4 (variant 0), 2 or 8; identical results.
+//
+// Bound by FP64, one warp instruction per 19 cycles and SM.  A lane per row
+// spent 1700 of them on the 640 warp instructions' worth of entries, and
+// waited for each entry's loads; so the entries of the trailing triangle (and
+// of the right-hand side) go to the lanes one by one, from a table in the order
+// of falling columns, of which every step takes a prefix, four per lane at a
+// time.  Both sets of 256 stamps of 49 unknowns in one launch: 82 us (two
+// launches of a row per lane: 371).
+constexpr int TF_MAXN = 127;  // the table's fields hold 7 bits of row and column
+inline size_t tfEntries(int n) { return (size_t)(n - 1) * n / 2 + (n - 1); }
+inline size_t tfSmemBytes(int n, int warps) {
+  return ((size_t)(n + 1) * (n | 1) + n) * warps * sizeof(double) + tfEntries(n) * sizeof(unsigned);
+}
 template <int TF_WARPS>
 __global__ void __launch_bounds__(TF_WARPS * 32)
-    k_stamp_test_fit_ldl(const double* __restrict__ Q, const double* __restrict__ B, int qc,
-                         int nStamps, const int* __restrict__ liveN,
-                         double* __restrict__ kernelSums) {
+    k_stamp_test_fit_ldl(const __grid_constant__ CdSets sets, int qc) {
   extern __shared__ double tf_s[];
+  const int set = blockIdx.y, nStamps = sets.n[set];
+  const int* liveN = sets.liveN[set];
+  const double* __restrict__ Q = sets.Q[set];
+  const double* __restrict__ B = sets.B[set];
+  double* __restrict__ kernelSums = sets.ks[set];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int s = blockIdx.x * TF_WARPS + warp;
   const int nLive = liveN ? min(nStamps, *liveN) : nStamps;
-  if(s >= nLive) return;  // whole warps only; the kernel has no block barrier
-  const int n = qc - 1, ld = n + 1;  // unknowns; row stride (column n = the RHS)
-  double* a = tf_s + (size_t)warp * n * ld;
+  if((int)blockIdx.x * TF_WARPS >= nLive) return;
+  const int n = qc - 1, ld = n | 1;  // unknowns; row stride (row n = the RHS)
+  const int perWarp = (n + 1) * ld + n;
+  double* a = tf_s + (size_t)warp * perWarp;
+  double* l = a + (n + 1) * ld;
+  unsigned* tab = (unsigned*)(tf_s + (size_t)TF_WARPS * perWarp);  // dst << 14 | i << 7 | j
+  for(int j = 1 + threadIdx.x; j < n; j += TF_WARPS * 32) {
+    const int m = n - 1 - j;
+    unsigned* t = tab + m * (m + 1) / 2 + m;
+    *t++ = (unsigned)(n * ld + j) << 14 | j << 7 | n;
+    for(int i = j; i < n; i++) *t++ = (unsigned)(i * ld + j) << 14 | i << 7 | j;
+  }
+  __syncthreads();
+  if(s >= nLive) return;  // whole warps only; no block barrier from here on
   const double* Qs = Q + (size_t)s * qc * qc;
   // unknown order: 2, 3, ..., n, then 1 (the kernel sum)
   auto unk = [&](int p) { return p < n - 1 ? p + 2 : 1; };
-  for(int e = lane; e < n * ld; e += 32) {
-    const int p = e / ld, q = e % ld, u = unk(p);
-    double v;
-    if(q == n) {
-      v = B[(size_t)s * qc + u];
-    } else {
-      const int t = unk(q);
-      v = Qs[(size_t)max(u, t) * qc + min(u, t)];
+  for(int q = lane; q < n; q += 32) {
+    const int t = unk(q);
+#pragma unroll 8
+    for(int p = 0; p < n; p++) {
+      const int u = unk(p);
+      a[p * ld + q] = Qs[(size_t)max(u, t) * qc + min(u, t)];
     }
-    a[e] = v;
+    a[n * ld + q] = B[(size_t)s * qc + t];
   }
   __syncwarp();
-  for(int k = 0; k < n; k++) {
+  for(int k = 0; k < n - 1; k++) {
     double d = a[k * ld + k];
     if(d == 0.0) d = 1.0e-20;
     const double rd = 1.0 / d;
-    const double bk = a[k * ld + n];
-    for(int i = k + 1 + lane; i < n; i += 32) {
-      double* ai = a + i * ld;
-      const double li = ai[k] * rd;
-      for(int j = k + 1; j <= i; j++) ai[j] = fma(-li, a[j * ld + k], ai[j]);
-      ai[n] = fma(-li, bk, ai[n]);
+    for(int i = k + 1 + lane; i < n; i += 32) l[i] = a[i * ld + k] * rd;
+    __syncwarp();
+    const int m = n - 1 - k, cnt = m * (m + 1) / 2 + m;
+    for(int e = lane; e < cnt; e += 128) {
+      double c[4], x[4], y[4];
+      unsigned t[4];
+#pragma unroll
+      for(int v = 0; v < 4; v++) t[v] = tab[min(e + 32 * v, cnt - 1)];
+#pragma unroll
+      for(int v = 0; v < 4; v++) {
+        c[v] = a[t[v] >> 14];
+        x[v] = l[t[v] >> 7 & 127];
+        y[v] = a[(t[v] & 127) * ld + k];
+      }
+#pragma unroll
+      for(int v = 0; v < 4; v++)
+        if(e + 32 * v < cnt) a[t[v] >> 14] = fma(-x[v], y[v], c[v]);
     }
     __syncwarp();
   }
   if(lane == 0) {
     double d = a[(n - 1) * ld + n - 1];
     if(d == 0.0) d = 1.0e-20;
-    kernelSums[s] = a[(n - 1) * ld + n] / d;
+    kernelSums[s] = a[n * ld + n - 1] / d;
   }
 }
 
@@ -231,10 +283,17 @@ __global__ void __launch_bounds__(TF_WARPS * 32)
 // sigmaClip of the kernel sums (10 iterations, cdkscUtil.cpp:74-76) and
 // genCdTestStamps (cd.cl:54-94) in ascending order.
 __global__ void __launch_bounds__(256)
-    k_cd_select(const double* __restrict__ ks, int n, const int* __restrict__ liveN, double alpha,
-                double sigKernFit, uint8_t* flags, double* cs, double* cs2,
-                int* __restrict__ testIdx, int* __restrict__ nTest, double* __restrict__ stats) {
-  if(liveN) n = *liveN;
+    k_cd_select(const __grid_constant__ CdSets sets, int nMax, double alpha, double sigKernFit,
+                uint8_t* flags, double* cs, double* cs2, int* __restrict__ nTest,
+                double* __restrict__ stats) {
+  const int set = blockIdx.x, n = sets.liveN[set] ? *sets.liveN[set] : sets.n[set];
+  const double* __restrict__ ks = sets.ks[set];
+  int* __restrict__ testIdx = sets.testIdx[set];
+  flags += (size_t)set * nMax;
+  cs += (size_t)set * nMax;
+  cs2 += (size_t)set * nMax;
+  nTest += set;
+  stats += 2 * set;
   __shared__ double sMean, sStd;
   __shared__ int sh[4];
   __shared__ int warpTot[8];
@@ -1047,9 +1106,9 @@ static FitBuffers fitBuffers(xb_ctx* c, int nMax) {
   f.singular = buf<int>(c, "fit_singular", 1);
   f.sig = buf<double>(c, "fit_sig", std::max(nMax, 1));
   f.scratchD = buf<double>(c, "fit_clipdata", std::max(nMax, 1));
-  f.flags = buf<uint8_t>(c, "fit_flags", std::max(nMax, 1));
-  f.cs = buf<double>(c, "fit_cs", std::max(nMax, 1));
-  f.cs2 = buf<double>(c, "fit_cs2", std::max(nMax, 1));
+  f.flags = buf<uint8_t>(c, "fit_flags", 2 * std::max(nMax, 1));  // cd clips both sets at once
+  f.cs = buf<double>(c, "fit_cs", 2 * std::max(nMax, 1));
+  f.cs2 = buf<double>(c, "fit_cs2", 2 * std::max(nMax, 1));
   return f;
 }
 
@@ -1187,34 +1246,66 @@ void kernelSumLaunch(xb_ctx* c, const double* dSol, double xf, double yf, int tr
 // tuned number of warps (stamps) per CTA among those whose factors fit in
 // shared memory (8 warps of a 61-row system do not); systems too large for
 // two warps take the one-CTA-per-stamp LU of the plain path.
-static void testFitLdl(xb_ctx* c, const StampSetDev& S, int qc, const int* liveN, double* ks) {
+static void testFitLdl(xb_ctx* c, const CdSets& sets, int qc) {
   int optin = 0;
   XB_CUDA(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, c->device));
-  const size_t perWarp = (size_t)(qc - 1) * qc * sizeof(double);
-  if(2 * perWarp > (size_t)optin) {
+  const int n = std::max(sets.n[0], sets.n[1]);
+  if(qc - 1 > TF_MAXN || tfSmemBytes(qc - 1, 2) > (size_t)optin) {
     const size_t smemLU = ((size_t)qc * qc + 3 * qc) * sizeof(double) + qc * sizeof(int);
     if(smemLU > (size_t)optin) throw XbError{XB_ERR_UNSUPPORTED, "test fit: system too large"};
     XB_CUDA(allowMaxDynamicSmem((const void*)k_stamp_test_fit, c->device));
-    k_stamp_test_fit<<<S.n, LU_THREADS, smemLU, c->stream>>>(S.Q, S.B, qc, liveN, ks);
+    k_stamp_test_fit<<<dim3(n, 2), LU_THREADS, smemLU, c->stream>>>(sets, qc);
     XB_LAUNCHED(c);
     return;
   }
   // variants: 0 = 4 warps, 1 = 2 warps, 2 = 8 warps
-  const int nVar = 8 * perWarp <= (size_t)optin ? 3 : 2;
+  const int nVar = tfSmemBytes(qc - 1, 8) <= (size_t)optin ? 3 : 2;
   auto launch = [&](int v) {
-    if(v == 0 && 4 * perWarp > (size_t)optin) v = 1;
+    if(v == 0 && tfSmemBytes(qc - 1, 4) > (size_t)optin) v = 1;
     const int W = v == 1 ? 2 : (v == 2 ? 8 : 4);
-    const size_t smem = (size_t)W * (qc - 1) * qc * sizeof(double);
-    const int grid = (S.n + W - 1) / W;
-    if(W == 2) k_stamp_test_fit_ldl<2><<<grid, 64, smem, c->stream>>>(S.Q, S.B, qc, S.n, liveN, ks);
-    else if(W == 8) k_stamp_test_fit_ldl<8><<<grid, 256, smem, c->stream>>>(S.Q, S.B, qc, S.n, liveN, ks);
-    else k_stamp_test_fit_ldl<4><<<grid, 128, smem, c->stream>>>(S.Q, S.B, qc, S.n, liveN, ks);
+    const size_t smem = tfSmemBytes(qc - 1, W);
+    const dim3 grid((n + W - 1) / W, 2);
+    if(W == 2) k_stamp_test_fit_ldl<2><<<grid, 64, smem, c->stream>>>(sets, qc);
+    else if(W == 8) k_stamp_test_fit_ldl<8><<<grid, 256, smem, c->stream>>>(sets, qc);
+    else k_stamp_test_fit_ldl<4><<<grid, 128, smem, c->stream>>>(sets, qc);
     XB_LAUNCHED(c);
   };
   XB_CUDA(allowMaxDynamicSmem((const void*)k_stamp_test_fit_ldl<2>, c->device));
   XB_CUDA(allowMaxDynamicSmem((const void*)k_stamp_test_fit_ldl<4>, c->device));
   XB_CUDA(allowMaxDynamicSmem((const void*)k_stamp_test_fit_ldl<8>, c->device));
   launch(tunedVariant(c, "stamp_test_fit_ldl", (long long)qc, nVar, launch));
+}
+
+// Test fits, clipping and test lists of both sets (cdkscUtil.cpp:44-120); live:
+// the kept counts are on the device (frame graphs).
+static void cdTestStamps(xb_ctx* c, const FitBuffers& f, int nMax, double* const ks[2],
+                         int* const testIdx[2], int* nTest, double* stats, bool live) {
+  CdSets sets{};
+  for(int si = 0; si < 2; si++) {
+    const StampSetDev& S = c->set[si];
+    sets.Q[si] = S.Q;
+    sets.B[si] = S.B;
+    sets.n[si] = S.n;
+    sets.liveN[si] = live ? S.dN : nullptr;
+    sets.ks[si] = ks[si];
+    sets.testIdx[si] = testIdx[si];
+  }
+  const int qc = c->g.qCount, n = std::max(sets.n[0], sets.n[1]);
+  if(n > 0) {
+    KT_SCOPE(c, "stamp_test_fit");
+    if(mixedMode(c)) {
+      testFitLdl(c, sets, qc);
+    } else {
+      const size_t smemLU = ((size_t)qc * qc + 3 * qc) * sizeof(double) + qc * sizeof(int);
+      XB_CUDA(allowMaxDynamicSmem((const void*)k_stamp_test_fit, c->device));
+      k_stamp_test_fit<<<dim3(n, 2), LU_THREADS, smemLU, c->stream>>>(sets, qc);
+      XB_LAUNCHED(c);
+    }
+  }
+  KT_SCOPE(c, "cd_select");
+  k_cd_select<<<2, 256, 0, c->stream>>>(sets, nMax, c->p.sigClipAlpha, c->p.sigKernFit, f.flags,
+                                        f.cs, f.cs2, nTest, stats);
+  XB_LAUNCHED(c);
 }
 
 void stageCd(xb_ctx* c) {
@@ -1228,28 +1319,7 @@ void stageCd(xb_ctx* c) {
   double* dSolCd = buf<double>(c, "cd_sol", 2 * (size_t)std::max(g.nSol, g.matSize + 1));
   double* kMean = buf<double>(c, "cd_kmean", 2);
   double* merit = buf<double>(c, "cd_merit", 2);
-  const int qc = g.qCount;
-  const size_t smemLU = ((size_t)qc * qc + 3 * qc) * sizeof(double) + qc * sizeof(int);
-  for(int si = 0; si < 2; si++) {
-    StampSetDev& S = c->set[si];
-    if(S.n > 0) {
-      { KT_SCOPE(c, "stamp_test_fit");
-      if(mixedMode(c)) {
-        testFitLdl(c, S, qc, nullptr, ks[si]);
-      } else {
-        XB_CUDA(allowMaxDynamicSmem((const void*)k_stamp_test_fit, c->device));
-        k_stamp_test_fit<<<S.n, LU_THREADS, smemLU, c->stream>>>(S.Q, S.B, qc, nullptr, ks[si]);
-        XB_LAUNCHED(c);
-      }
-      }
-    }
-    { KT_SCOPE(c, "cd_select");
-    k_cd_select<<<1, 256, 0, c->stream>>>(ks[si], S.n, nullptr, c->p.sigClipAlpha, c->p.sigKernFit,
-                                          f.flags, f.cs, f.cs2, testIdx[si], nTest + si,
-                                          stats + 2 * si);
-    XB_LAUNCHED(c);
-    }
-  }
+  cdTestStamps(c, f, nMax, ks, testIdx, nTest, stats, false);
   std::vector<int> hT = toHost(c, nTest, 2);
   const int solStride = std::max(g.nSol, g.matSize + 1);
   for(int si = 0; si < 2; si++) {
@@ -1361,22 +1431,7 @@ void stageCdGraph(xb_ctx* c, long long lCd[2]) {
   double* dSolCd = buf<double>(c, "cd_sol", 2 * (size_t)std::max(g.nSol, g.matSize + 1));
   double* kMean = buf<double>(c, "cd_kmean", 2);
   double* merit = buf<double>(c, "cd_merit", 2);
-  const int qc = g.qCount;
-  const size_t smemLU = ((size_t)qc * qc + 3 * qc) * sizeof(double) + qc * sizeof(int);
-  for(int si = 0; si < 2; si++) {
-    StampSetDev& S = c->set[si];
-    if(mixedMode(c)) {
-      testFitLdl(c, S, qc, S.dN, ks[si]);
-    } else {
-      XB_CUDA(allowMaxDynamicSmem((const void*)k_stamp_test_fit, c->device));
-      k_stamp_test_fit<<<S.n, LU_THREADS, smemLU, c->stream>>>(S.Q, S.B, qc, S.dN, ks[si]);
-      XB_LAUNCHED(c);
-    }
-    k_cd_select<<<1, 256, 0, c->stream>>>(ks[si], S.n, S.dN, c->p.sigClipAlpha, c->p.sigKernFit,
-                                          f.flags, f.cs, f.cs2, testIdx[si], nTest + si,
-                                          stats + 2 * si);
-    XB_LAUNCHED(c);
-  }
+  cdTestStamps(c, f, nMax, ks, testIdx, nTest, stats, true);
   const int solStride = std::max(g.nSol, g.matSize + 1);
   for(int si = 0; si < 2; si++) {
     double* sol = dSolCd + (size_t)si * solStride;
