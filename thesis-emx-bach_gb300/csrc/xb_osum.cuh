@@ -1,5 +1,5 @@
 // xb_osum.cuh — left-to-right FP64 sums of nonnegative terms, bit for bit,
-// 32 terms per step of one warp.
+// 32 terms (or a multiple) per step of one warp.
 //
 // The reference forms its sigma-clip sums on the host as one serial FP64
 // loop over the per-work-item partial sums (bachUtil.cpp:34-128), and every
@@ -57,17 +57,15 @@ __host__ __device__ inline double fromBits(long long b) {
 // normal running sum
 __host__ __device__ inline Grid onGrid(double x, int sE) {
   const long long xb = bitsOf(x);
-  if(xb < 0) return {0, false};  // negative, or -0.0
-  const int xE = (int)(xb >> 52);
-  if(xE > sE) return {0, false};  // x >= 2^(E+1), infinite or NaN
-  // x = mant * 2^(max(xE,1) - 1075), so x/u = mant * 2^-(sh)
-  const long long mant = (xb & kFrac) | (xE ? (1ll << 52) : 0);
-  const int sh = sE - (xE ? xE : 1);
-  if(sh <= 0) return {mant, true};
-  if(sh >= 54) return {0, true};  // x/u < 1/2
-  const long long q = mant >> sh, rem = mant & ((1ll << sh) - 1), half = 1ll << (sh - 1);
-  if(rem == half) return {0, false};
-  return {q + (rem > half ? 1 : 0), true};
+  const int xE = (int)((unsigned long long)xb >> 52);  // sign and exponent
+  if(xb == 0) return {0, true};
+  if(xE > sE || xE == 0) return {0, false};  // negative, too large, infinite, NaN or subnormal
+  // x = mant * 2^(xE - 1075), so x/u = mant * 2^-sh
+  const long long mant = (xb & kFrac) | (1ll << 52);
+  const int sh = sE - xE < 54 ? sE - xE : 54;  // x/u < 1/2 from 54 on
+  if(sh == 0) return {mant, true};
+  const long long r = mant + (1ll << (sh - 1));
+  return {r >> sh, (r & ((1ll << sh) - 1)) != 0};  // a tie: no bits left
 }
 
 // a float term, from its bits (no FP64 operation)
@@ -149,12 +147,17 @@ inline double orderedSumHost(const double* c, int n) {
 // All 32 lanes of a warp call it with the same n and term(i), the i-th term
 // as a double or as a float (whose grid steps need no FP64 operation);
 // every lane returns the sum.  term is best a shared-memory read (one
-// dependent read per step).
-template <class F>
+// dependent read per step).  A step takes V terms per lane: a step's latency
+// grows less than V, so long sums take two.  The first 32 terms double the sum
+// again and again, so they are added serially.  (1047 terms: 17.6k cycles with
+// two terms per lane and 19.6k with one; every addition serially 75k.)
+template <int V = 1, class F>
 __device__ inline double warpOrderedSumOf(int n, F term) {
   const int lane = threadIdx.x & 31;
   double s = 0.0;
   int i = 0;
+#pragma unroll 8
+  for(; i < min(n, 32); i++) s = s + (double)term(i);
   while(i < n) {
     int sE;
     long long S0;
@@ -178,19 +181,57 @@ __device__ inline double warpOrderedSumOf(int n, F term) {
       i++;
       continue;
     }
-    const int len = min(32, n - i);
-    Grid g = {0, false};
-    if(lane < len) g = onGrid(term(i + lane), sE);
-    long long P = g.n;  // inclusive prefix over the lanes
+    const int len = min(32 * V, n - i);
+    Grid g[V];
+    long long P[V];  // inclusive prefix within the lane, then over the lanes
+    bool ok = true;
+#pragma unroll
+    for(int v = 0; v < V; v++) {
+      const int k = lane * V + v;
+      g[v] = onGrid(term(i + (k < len ? k : 0)), sE);
+      if(k >= len) g[v] = {0, true};
+      ok = ok && g[v].ok;
+    }
+#pragma unroll
+    for(int v = 0; v < V; v++) P[v] = g[v].n + (v ? P[v - 1] : 0);
+    // usually every term is accepted: the total from three 26-bit pieces of
+    // the lanes' sums (below 2^53 V) decides it
+    if(__all_sync(0xffffffffu, ok)) {
+      const unsigned long long p = (unsigned long long)P[V - 1];
+      const long long all = ((long long)__reduce_add_sync(0xffffffffu, (unsigned)(p >> 52)) << 52) +
+                            ((long long)__reduce_add_sync(0xffffffffu, (unsigned)(p >> 26) & 0x3FFFFFFu) << 26) +
+                            (long long)__reduce_add_sync(0xffffffffu, (unsigned)p & 0x3FFFFFFu);
+      if(S0 + all < (1ll << 53)) {
+        s = fromBits(((long long)sE << 52) | (S0 + all - (1ll << 52)));
+        i += len;
+        continue;
+      }
+    }
+#pragma unroll
+    for(int v = 0; v < V; v++)
+      if(lane * V + v >= len) g[v].ok = false;
+    long long T = P[V - 1];
 #pragma unroll
     for(int o = 1; o < 32; o <<= 1) {
-      const long long t = __shfl_up_sync(0xffffffffu, P, o);
-      if(lane >= o) P += t;
+      const long long t = __shfl_up_sync(0xffffffffu, T, o);
+      if(lane >= o) T += t;
     }
-    const bool ok = lane < len && g.ok && S0 + P < (1ll << 53);
-    const unsigned bad = __ballot_sync(0xffffffffu, !ok);
-    const int j = bad ? __ffs(bad) - 1 : 32;  // terms accepted
-    const long long Pj = __shfl_sync(0xffffffffu, P, j > 0 ? j - 1 : 0);
+    const long long before = T - P[V - 1];  // of the lanes below
+    int first = V;                          // the lane's first term that is not accepted
+#pragma unroll
+    for(int v = V - 1; v >= 0; v--) {
+      P[v] += before;
+      if(!(g[v].ok && S0 + P[v] < (1ll << 53))) first = v;
+    }
+    const unsigned bad = __ballot_sync(0xffffffffu, first < V);
+    const int b = bad ? __ffs(bad) - 1 : 31;
+    const int fb = __shfl_sync(0xffffffffu, first, b);
+    const int j = bad ? b * V + fb : 32 * V;  // terms accepted
+    long long mine = before;  // the sum of the accepted terms, in lane b
+#pragma unroll
+    for(int v = 0; v < V; v++)
+      if(v < first) mine = P[v];
+    const long long Pj = __shfl_sync(0xffffffffu, mine, b);
     if(j > 0) {
       s = fromBits(((long long)sE << 52) | (S0 + Pj - (1ll << 52)));
       i += j;
@@ -202,8 +243,9 @@ __device__ inline double warpOrderedSumOf(int n, F term) {
   }
   return s;
 }
+template <int V = 1>
 __device__ inline double warpOrderedSum(const double* c, int n) {
-  return warpOrderedSumOf(n, [c](int i) { return c[i]; });
+  return warpOrderedSumOf<V>(n, [c](int i) { return c[i]; });
 }
 #endif
 

@@ -12,6 +12,7 @@
 #include <algorithm>
 #include <climits>
 #include <cmath>
+#include <type_traits>
 
 #include "xb_device.cuh"
 #include "xb_internal.h"
@@ -22,8 +23,6 @@ namespace xb {
 namespace {
 
 constexpr int NSAMPLES = 100, PADDED = 128;
-constexpr int ST_THREADS = 256;
-constexpr int ST_CHUNKS_SMEM = 1280;  // chunk sums kept in shared memory (stamps <= 40960 px)
 
 __device__ __forceinline__ int satFloorToInt(double v) {
   double f = floor(v);
@@ -38,12 +37,12 @@ __device__ __forceinline__ int satFloorToInt(double v) {
 struct Ran1 {
   long long ix1, ix2, ix3;
   int idum, iff;
-  __host__ __device__ void init(int seed) {
+  __host__ __device__ constexpr void init(int seed) {
     idum = seed;
     iff = 0;
     ix1 = ix2 = ix3 = 0;
   }
-  __host__ __device__ double next(double* r) {
+  __host__ __device__ constexpr double next(double* r) {
     const long long M1 = 259200, IA1 = 7141, IC1 = 54773;
     const long long M2 = 134456, IA2 = 8121, IC2 = 28411;
     const long long M3 = 243000, IA3 = 4561, IC3 = 51349;
@@ -78,8 +77,9 @@ struct Ran1 {
 // bach.cl:129-184) and createHistogram (sss.cl:190-324).
 //
 // Every stamp seeds ran1 with -666, so all stamps draw the same sequence:
-// with `draws` (that sequence, precomputed on the host) the 32 candidates of
-// a sampling round are formed in parallel; without it lane 0 runs ran1.
+// with `draws` (that sequence, precomputed on the host; without it, the
+// sequence's first 1024 numbers from a constant table) the 32 candidates of a
+// sampling round are formed in parallel; beyond the table one lane runs ran1.
 // The clip test |v - m| * inv > alpha is monotone in v on each side of m, so
 // each clip round first finds the exact thresholds v_lo < m < v_hi where it
 // turns true (a 32-ary search of one warp over the ordered doubles) and then
@@ -119,13 +119,25 @@ __device__ __forceinline__ bool clipOut(double v, double m, double inv, double a
 
 // One warp: the key of the first double (walking away from m, upwards when
 // up, downwards otherwise) at which clipOut turns true; `none` when it never
-// does.  clipOut is false at m and monotone along the walk.
-__device__ unsigned long long clipEdge(double m, double inv, double alpha, bool up, bool* none) {
+// does.  clipOut is false at m and monotone along the walk.  sd = 1/inv up to
+// rounding: the edge is usually among the doubles around m +- alpha sd, which
+// the lanes test first.
+__device__ unsigned long long clipEdge(double m, double inv, double sd, double alpha, bool up,
+                                       bool* none) {
   const int lane = threadIdx.x & 31;
   const unsigned long long kEnd = dKey(up ? INFINITY : -INFINITY);
   unsigned long long lo = dKey(m), hi = kEnd;  // clipOut(lo) false, clipOut(hi) true
   *none = !clipOut(up ? INFINITY : -INFINITY, m, inv, alpha);
   if(*none) return kEnd;
+  {
+    const unsigned long long k0 = dKey(up ? m + alpha * sd : m - alpha * sd);
+    const unsigned long long k = up ? k0 - 16 + lane : k0 + 16 - lane;
+    const bool valid = up ? k > lo && k <= hi : k < lo && k >= hi;
+    const bool p = valid && clipOut(keyD(k), m, inv, alpha);
+    const unsigned bal = __ballot_sync(0xffffffffu, p);
+    if(__all_sync(0xffffffffu, valid) && !(bal & 1u) && bal)
+      return __shfl_sync(0xffffffffu, k, __ffs(bal) - 1);
+  }
   for(int guard = 0; guard < 40; guard++) {
     const unsigned long long span = up ? hi - lo : lo - hi;
     if(span <= 1) break;
@@ -151,8 +163,54 @@ __device__ unsigned long long clipEdge(double m, double inv, double alpha, bool 
   return hi;
 }
 
-template <class T>
-__global__ void __launch_bounds__(ST_THREADS, 3)
+// The first draws of ran1(-666), for callers without a table of their own
+// (the serial generator takes 110 us for a stamp's usual 256 draws).
+constexpr int RAN1_DRAWS = 1024;
+struct Ran1Table {
+  double v[RAN1_DRAWS];
+};
+constexpr Ran1Table ran1Table() {
+  Ran1Table t{};
+  Ran1 rng{};
+  double r[98] = {};
+  rng.init(-666);
+  for(int i = 0; i < RAN1_DRAWS; i++) t.v[i] = rng.next(r);
+  return t;
+}
+__device__ const Ran1Table kRan1 = ran1Table();
+
+// An FP32 good pixel (positive, not NaN, normal or infinite) in FP64, on its
+// bits: conversions run on the FP64 unit.
+__device__ __forceinline__ double widenGood(float f) {
+  const unsigned b = __float_as_uint(f);
+  return __hiloint2double((int)((b >> 3) + ((b >= 0x7F800000u ? 1792u : 896u) << 20)), (int)(b << 29));
+}
+__device__ __forceinline__ double widenGood(double v) { return v; }
+
+// Shared memory of a stamp's chunks: sums, live bits, changed list and (SM)
+// the good pixels, 33 words per chunk so that a chunk per lane reads without
+// bank conflicts.
+constexpr int ST_CHUNKS_SMEM = 1280;  // chunk sums of the other form kept in shared memory
+inline size_t statsSmemBytes(int maxChunks, bool sm) {
+  if(!sm) return maxChunks <= ST_CHUNKS_SMEM ? (size_t)maxChunks * 16 : 0;
+  return (size_t)maxChunks * (16 + 4 + 2) + 4 + (size_t)maxChunks * 33 * 4;
+}
+
+// One CTA per stamp: NW warps for the pixels and one that draws and sorts the
+// samples meanwhile (they are needed for the histogram only).
+//
+// SM: the good pixels (FP32) stay in shared memory; else they go to the scratch
+// slice, chunk-interleaved.  Bound by FP64, one warp instruction per 19 cycles
+// and SM, and by its serial chains: a pixel's part of a chunk's sum of squares
+// is one FP64 instruction (an FP32 pixel's square is exact in FP64, so the
+// fused multiply-add rounds as the sum does); the plain sums are exact whenever
+// the pixels' total fits 53 bits of their common quantum, and then they are
+// integers and need no order; only chunks that lost a pixel are summed again.
+// Both images, 256 stamps of 107 px: 206 us, 400 of 183 px: 745 us (the
+// good pixels and a byte flag each in global memory, four FP64 instructions per
+// pixel, the samples first: 662 and 1909 us).
+template <class T, bool SM, int NW>
+__global__ void __launch_bounds__(NW * 32 + 32, NW > 8 ? 1 : 3)
     k_stamp_stats(const T* __restrict__ img, uint16_t* __restrict__ mask,
                   const int4* __restrict__ geom, int w, int h, int fSW,
                   T* __restrict__ good, uint8_t* __restrict__ clip,
@@ -163,6 +221,8 @@ __global__ void __launch_bounds__(ST_THREADS, 3)
   const int4 gm = geom[s];  // cx, cy, sx, sy
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   constexpr bool F32 = sizeof(T) == 4;
+  constexpr int NT = NW * 32;  // threads on the pixels
+  static_assert(F32 || !SM, "the pixels in shared memory are floats");
   // A stamp must have the form of the reference's grid (createStampBounds,
   // cl_kern/sss.cl:19-40): its origin inside the image and its size the full
   // stamp width clipped by the image edge.  Its histogram is then taken over
@@ -179,17 +239,19 @@ __global__ void __launch_bounds__(ST_THREADS, 3)
     }
     return;
   }
+  extern __shared__ __align__(16) unsigned char st_s[];
   __shared__ double samples[PADDED];
   __shared__ double rtab[98];
   __shared__ int cand[32];
   __shared__ int sCount;
-  __shared__ int warpTot[ST_THREADS / 32];
-  __shared__ int sTotal;
+  __shared__ int warpGood[2][NW];
+  __shared__ unsigned sKMin, sKMax;
+  __shared__ unsigned long long sTot;  // exact sum of the unclipped pixels, in quanta
   __shared__ double sMean, sStd, sInv, sSum, sSum2;
-  __shared__ int sPrev, sCurr, sClip, sDone;
+  __shared__ int sPrev, sCurr, sClip, sDone, sChanged, sNan;
   __shared__ int bins[256];
-  __shared__ long long hC[257], hCE[257];  // prefix sums of the bin counts (and of index * count)
-  __shared__ int okCount;
+  __shared__ int hC[257];         // prefix sums of the bin counts
+  __shared__ long long hCE[257];  // and of index * count
   __shared__ double hLower, hUpper, hSky, hBinSize, hLowerBinVal;
   __shared__ int hState;  // 0 continue, 1 stop (setFwhm), 2 stop (no fwhm)
   __shared__ double tLo, tHi;          // clip thresholds of the current round
@@ -197,17 +259,17 @@ __global__ void __launch_bounds__(ST_THREADS, 3)
   __shared__ int tNoLo, tNoHi, tDirect;
   __shared__ float bLbv, bInv, bDelta;  // FP32 bin estimate of the current pass
   __shared__ int bExact;
+  __shared__ double bRec;
+  auto pixSync = [] { asm volatile("bar.sync 1, %0;" ::"n"(NT) : "memory"); };
 
-  // ---- phase A: random sampling (warp 0) ----
-  if(tid < 32) {
+  // ---- phase A: random sampling (the last warp) ----
+  if(warp == NW) {
     Ran1 rng;
-    if(lane == 0) {
-      rng.init(-666);
-      sCount = 0;
-    }
+    if(lane == 0) rng.init(-666);
     const int numPix = gm.z * gm.w;
-    // with the draws, the candidates of the first PRE rounds (32 each) are
-    // read together
+    const double* dr = draws ? draws : kRan1.v;
+    const int nDr = draws ? numPix : min(numPix, RAN1_DRAWS / 2);  // candidates with draws
+    // the candidates of the first PRE rounds (32 each) are read together
     constexpr int PRE = 4;
     double preV[PRE];
     bool preOk[PRE];
@@ -215,46 +277,53 @@ __global__ void __launch_bounds__(ST_THREADS, 3)
     for(int r = 0; r < PRE; r++) {
       preV[r] = 0.0;
       preOk[r] = false;
-      if(draws && r * 32 + lane < numPix) {
-        const int rx = (int)floor(draws[2 * (r * 32 + lane)] * (int)gm.z);
-        const int ry = (int)floor(draws[2 * (r * 32 + lane) + 1] * (int)gm.w);
-        const int idx = (rx + gm.x) + (ry + gm.y) * w;
+      if(r * 32 + lane < numPix) {
+        const int rx = (int)floor(dr[2 * (r * 32 + lane)] * (int)gm.z);
+        const int ry = (int)floor(dr[2 * (r * 32 + lane) + 1] * (int)gm.w);
+        const size_t idx = (size_t)(rx + gm.x) + (size_t)(ry + gm.y) * w;
         preV[r] = (double)img[idx];
         preOk[r] = !(mask[idx] > 0 || fabs(preV[r]) <= 1e-10);
       }
     }
-    int cnt = 0, iter = 0;
+    int cnt = 0, iter = 0, drawn = 0;  // drawn: candidates the generator has passed
     while(cnt < NSAMPLES && iter < numPix) {
-      int b = min(32, numPix - iter);
-      int idx = 0;
+      const int b = min(32, numPix - iter);
       const int round = iter / 32;
-      if(draws && round < PRE) {
-        // taken from preV / preOk below
-      } else if(draws) {
-        if(lane < b) {
-          const int rx = (int)floor(draws[2 * (iter + lane)] * (int)gm.z);
-          const int ry = (int)floor(draws[2 * (iter + lane) + 1] * (int)gm.w);
-          idx = (rx + gm.x) + (ry + gm.y) * w;
-        }
-      } else {
-        if(lane == 0) {
-          for(int k = 0; k < b; k++) {
-            int rx = (int)floor(rng.next(rtab) * (int)gm.z);
-            int ry = (int)floor(rng.next(rtab) * (int)gm.w);
-            cand[k] = (rx + gm.x) + (ry + gm.y) * w;
-          }
-        }
-        __syncwarp();
-        if(lane < b) idx = cand[lane];
-      }
       bool ok = false;
       double v = 0.0;
-      if(draws && round < PRE) {
+      if(round < PRE) {
         v = round == 0 ? preV[0] : round == 1 ? preV[1] : round == 2 ? preV[2] : preV[3];
         ok = round == 0 ? preOk[0] : round == 1 ? preOk[1] : round == 2 ? preOk[2] : preOk[3];
-      } else if(lane < b) {
-        v = (double)img[idx];
-        ok = !(mask[idx] > 0 || fabs(v) <= 1e-10);
+      } else {
+        size_t idx = 0;
+        if(iter + b <= nDr) {
+          if(lane < b) {
+            const int rx = (int)floor(dr[2 * (iter + lane)] * (int)gm.z);
+            const int ry = (int)floor(dr[2 * (iter + lane) + 1] * (int)gm.w);
+            idx = (size_t)(rx + gm.x) + (size_t)(ry + gm.y) * w;
+          }
+        } else {
+          // beyond the table: one lane runs the generator
+          if(lane == 0) {
+            for(; drawn < iter; drawn++) {
+              rng.next(rtab);
+              rng.next(rtab);
+            }
+            for(int k = 0; k < b; k++) {
+              const int rx = (int)floor(rng.next(rtab) * (int)gm.z);
+              const int ry = (int)floor(rng.next(rtab) * (int)gm.w);
+              cand[k] = rx | ry << 16;
+            }
+            drawn = iter + b;
+          }
+          __syncwarp();
+          if(lane < b)
+            idx = (size_t)((cand[lane] & 0xFFFF) + gm.x) + (size_t)((cand[lane] >> 16) + gm.y) * w;
+        }
+        if(lane < b) {
+          v = (double)img[idx];
+          ok = !(mask[idx] > 0 || fabs(v) <= 1e-10);
+        }
       }
       unsigned bal = __ballot_sync(0xffffffffu, ok);
       int pos = cnt + __popc(bal & ((1u << lane) - 1u));
@@ -286,24 +355,30 @@ __global__ void __launch_bounds__(ST_THREADS, 3)
         }
         __syncwarp();
       }
+    __syncthreads();  // meets the pixel warps before phase D
+    return;
   }
-  __syncthreads();
 
   // ---- phase B: ordered compaction of good pixels (maskStamp) ----
-  // warp w owns a contiguous range of the stamp's pixel indices and reads it
-  // 32 consecutive pixels at a time; ballots keep the ascending order inside
-  // the warp and one block scan over the warp totals orders the warps.  The
-  // good pixels are kept as read (FP32 pixels stay FP32).
-  // The list is stored chunk-interleaved: entry q (chunk q/32, position
-  // q%32) at slot(q), so that the chunk passes, one chunk per thread, read
-  // 32 consecutive chunks' entries at one position with one coalesced load.
-  // A stamp's slice is fSW^2 rounded up to a multiple of 1024 (statsSlice).
+  // The stamp's pixels go through in ascending order, NT * BB at a time: each
+  // warp takes 32 * BB consecutive ones, ballots order them inside the warp
+  // and the warps' counts order the warps.  The good pixels are kept as read
+  // (FP32 pixels stay FP32).
+  // In a scratch slice the list is chunk-interleaved: entry q (chunk q/32,
+  // position q%32) at listSlot(q), so that the chunk passes, one chunk per
+  // thread, read 32 consecutive chunks' entries at one position with one
+  // coalesced load.  A stamp's slice is fSW^2 rounded up to a multiple of 1024
+  // (statsSlice).
   T* gd = good + (size_t)s * statsSlice(fSW);
-  uint8_t* cl = clip + (size_t)s * statsSlice(fSW);
+  const bool chunksInSmem = SM || maxChunks <= ST_CHUNKS_SMEM;
+  double* cS = chunksInSmem ? (double*)st_s : chunkBuf + (size_t)s * 2 * maxChunks;
+  double* cS2 = cS + maxChunks;
+  unsigned* cm = SM ? (unsigned*)(cS2 + maxChunks)  // a chunk's unclipped pixels
+                    : (unsigned*)(clip + (size_t)s * statsSlice(fSW));
+  float* list = (float*)(cm + maxChunks);                                   // SM only
+  uint16_t* changed = (uint16_t*)(list + (size_t)33 * maxChunks);            // SM only
   const int nPixS = fSW * fSW;
-  constexpr int NWARP = ST_THREADS / 32;
-  const int perW = ((nPixS + NWARP - 1) / NWARP + 31) & ~31;
-  const int w0 = min(warp * perW, nPixS), w1 = min(w0 + perW, nPixS);
+  const unsigned magic = fSW > 1 ? 0xFFFFFFFFu / (unsigned)fSW + 1u : 0u;
   // v <= 1e-10 of the reference: for an FP32 pixel the same test as f <= fTiny,
   // the largest float not above 1e-10
   const float fTiny = __double2float_rd(1e-10);
@@ -312,70 +387,86 @@ __global__ void __launch_bounds__(ST_THREADS, 3)
     return (double)v <= 1e-10;
   };
   auto pixelAt = [&](int idxS, size_t* id) -> bool {
-    const int xI = idxS % fSW + gm.x, yI = idxS / fSW + gm.y;
-    *id = (size_t)xI + (size_t)yI * w;
-    return xI < w && yI < h;
+    // idxS / fSW: the rounded-up reciprocal gives it or one more
+    int y = fSW > 1 ? (int)__umulhi((unsigned)idxS, magic) : idxS;
+    if(y * fSW > idxS) y--;
+    const int x = idxS - y * fSW;
+    *id = (size_t)(x + gm.x) + (size_t)(y + gm.y) * w;
+    return idxS < nPixS && x < gm.z && y < gm.w;
   };
-  // each pass loads BB rows of 32 pixels (and their mask words) before it
-  // tests them, in order
+  if(tid == 0) {
+    sKMin = 0xFFFFFFFFu;
+    sKMax = 0u;
+    sTot = 0ull;
+    sNan = 0;
+  }
   constexpr int BB = 8;
-  int wGood = 0;
-  for(int b0 = w0; b0 < w1; b0 += 32 * BB) {
-    T px[BB];
-    uint16_t mk[BB];
-    size_t ids[BB];
-    bool in[BB];
+  int nGood = 0;
+  unsigned kMin = 0xFFFFFFFFu, kMax = 0u;
+  bool sawNan = false;
+  {
+    T px[BB], pn[BB];
+    uint16_t mk[BB], mn[BB];
+    auto fetch = [&](int base, T* v, uint16_t* m) {
 #pragma unroll
-    for(int u = 0; u < BB; u++) {
-      const int idxS = b0 + u * 32 + lane;
-      in[u] = idxS < w1 && pixelAt(idxS, &ids[u]);
-      px[u] = in[u] ? img[ids[u]] : T(0);
-      mk[u] = in[u] ? mask[ids[u]] : (uint16_t)1;
-    }
-#pragma unroll
-    for(int u = 0; u < BB; u++) {
-      bool g = false;
-      if(in[u] && !(mk[u] > 0 || tiny(px[u]))) {
-        if(isnan(px[u])) mask[ids[u]] |= NAN_PIXEL | BAD_INPUT;
-        else g = true;
+      for(int u = 0; u < BB; u++) {
+        size_t id;
+        const bool in = pixelAt(base + (warp * BB + u) * 32 + lane, &id);
+        v[u] = in ? img[id] : T(0);
+        m[u] = in ? mask[id] : (uint16_t)1;
       }
-      wGood += __popc(__ballot_sync(0xffffffffu, g));
+    };
+    fetch(0, px, mk);
+    for(int base = 0, buf = 0; base < nPixS; base += NT * BB, buf ^= 1) {
+      if(base + NT * BB < nPixS) fetch(base + NT * BB, pn, mn);
+      unsigned bal[BB];
+      int cnt = 0;
+#pragma unroll
+      for(int u = 0; u < BB; u++) {
+        const bool cand_ = mk[u] == 0 && !tiny(px[u]);
+        const bool g = cand_ && !isnan(px[u]);
+        sawNan |= cand_ && !g;
+        bal[u] = __ballot_sync(0xffffffffu, g);
+        cnt += __popc(bal[u]);
+      }
+      if(lane == 0) warpGood[buf][warp] = cnt;
+      pixSync();
+      const int wg = lane < NW ? warpGood[buf][lane] : 0;
+      int pos = nGood + __reduce_add_sync(0xffffffffu, lane < warp ? wg : 0);
+      nGood += __reduce_add_sync(0xffffffffu, wg);
+#pragma unroll
+      for(int u = 0; u < BB; u++) {
+        if(bal[u] >> lane & 1u) {
+          const int q = pos + __popc(bal[u] & ((1u << lane) - 1u));
+          if constexpr(SM) list[q + (q >> 5)] = px[u];
+          else gd[listSlot(q)] = px[u];
+          if constexpr(F32) {
+            const unsigned b = __float_as_uint(px[u]);
+            kMin = min(kMin, b);
+            kMax = max(kMax, b);
+          }
+        }
+        pos += __popc(bal[u]);
+      }
+#pragma unroll
+      for(int u = 0; u < BB; u++) {
+        px[u] = pn[u];
+        mk[u] = mn[u];
+      }
     }
   }
-  const int wBase = blockScanExcl(lane == 0 ? wGood : 0, warpTot, &sTotal);
-  const int nGood = sTotal;
-  int pos = __shfl_sync(0xffffffffu, wBase, 0);
-  for(int b0 = w0; b0 < w1; b0 += 32 * BB) {
-    T px[BB];
-    uint16_t mk[BB];
-    bool in[BB];
-#pragma unroll
-    for(int u = 0; u < BB; u++) {
-      const int idxS = b0 + u * 32 + lane;
-      size_t id;
-      in[u] = idxS < w1 && pixelAt(idxS, &id);
-      px[u] = in[u] ? img[id] : T(0);
-      mk[u] = in[u] ? mask[id] : (uint16_t)1;  // NaN pixels carry their mask bits now
-    }
-#pragma unroll
-    for(int u = 0; u < BB; u++) {
-      const bool g = in[u] && !(mk[u] > 0 || tiny(px[u]));
-      const unsigned bal = __ballot_sync(0xffffffffu, g);
-      if(g) {
-        const int q = pos + __popc(bal & ((1u << lane) - 1u));
-        gd[listSlot(q)] = px[u];
-        cl[listSlot(q)] = 0;
-      }
-      pos += __popc(bal);
+  if(F32) {
+    kMin = __reduce_min_sync(0xffffffffu, kMin);
+    kMax = __reduce_max_sync(0xffffffffu, kMax);
+    if(lane == 0) {
+      atomicMin(&sKMin, kMin);
+      atomicMax(&sKMax, kMax);
     }
   }
+  if(sawNan) sNan = 1;
+  pixSync();
 
   // ---- phase C: sigma clip, maxIter 3 (bachUtil.cpp:34-128) ----
-  // the chunk sums, in shared memory when they fit
-  __shared__ double chunkSm[2][ST_CHUNKS_SMEM];
-  const bool chunksInSmem = (nGood + 31) / 32 <= ST_CHUNKS_SMEM;
-  double* cS = chunksInSmem ? chunkSm[0] : chunkBuf + (size_t)s * 2 * maxChunks;
-  double* cS2 = chunksInSmem ? chunkSm[1] : cS + maxChunks;
   if(tid == 0) {
     sPrev = nGood;
     sCurr = 0;
@@ -384,16 +475,19 @@ __global__ void __launch_bounds__(ST_THREADS, 3)
     sStd = 1e10;
     if(nGood == 0) sDone = 1;
   }
-  __syncthreads();
   const int nChunks = (nGood + 31) / 32;
-  // exact clip thresholds for (m, inv) into tLo/tHi (warp 0; all threads call)
+  auto pixel = [&](int c, int l) -> T {
+    if constexpr(SM) return list[c * 33 + l];
+    else return gd[chunkSlot(c, l)];
+  };
+  // exact clip thresholds for (m, inv) into tLo/tHi (warp 0; all pixel threads call)
   // (warp 0 searches the upper edge, warp 1 the lower one)
-  auto thresholds = [&](double m, double inv) {
+  auto thresholds = [&](double m, double inv, double sd) {
     if(warp < 2) {
       const bool direct = !isfinite(m) || isnan(inv);
       if(!direct) {
         bool none;
-        const unsigned long long k = clipEdge(m, inv, sigClipAlpha, warp == 0, &none);
+        const unsigned long long k = clipEdge(m, inv, sd, sigClipAlpha, warp == 0, &none);
         if(lane == 0) {
           const double t = keyD(k);
           if(warp == 0) {
@@ -409,54 +503,83 @@ __global__ void __launch_bounds__(ST_THREADS, 3)
       }
       if(warp == 0 && lane == 0) tDirect = direct;
     }
-    __syncthreads();
+    pixSync();
   };
-  auto isClipped = [&](double v, double m, double inv) -> bool {
-    if(tDirect) return clipOut(v, m, inv, sigClipAlpha);
-    if(F32) {
-      const float f = (float)v;  // exact: v came from a float pixel
-      return (!tNoHi && f >= fHi) || (!tNoLo && f <= fLo);
-    }
-    return (!tNoHi && v >= tHi) || (!tNoLo && v <= tLo);
+  // A pixel against the thresholds (no FP64 operation for FP32 pixels); an
+  // absent threshold is NaN, which no pixel passes.
+  struct Clip {
+    bool direct;
+    T lo, hi;
   };
-  // the same for a pixel as read (no FP64 conversion for FP32 pixels)
-  auto isClippedPix = [&](T pv, double m, double inv) -> bool {
-    if(tDirect) return clipOut((double)pv, m, inv, sigClipAlpha);
-    if(F32) {
-      const float f = (float)pv;
-      return (!tNoHi && f >= fHi) || (!tNoLo && f <= fLo);
-    }
-    return isClipped((double)pv, m, inv);
+  auto clipNow = [&]() -> Clip {
+    const T nan_ = (T)__int_as_float(0x7fffffff);
+    if(F32) return {tDirect != 0, tNoLo ? nan_ : (T)fLo, tNoHi ? nan_ : (T)fHi};
+    return {tDirect != 0, tNoLo ? nan_ : (T)tLo, tNoHi ? nan_ : (T)tHi};
   };
-  // chunk sums of the unclipped pixels: 32 consecutive good pixels each, in
-  // order (all pixels at first; then fused with each round's clip pass, for
-  // the next round).  A chunk's pixels and flags are loaded before its sums
-  // start; entries past the list's end count as clipped (adding 0.0 leaves a
-  // sum unchanged).
-  // sums of a chunk's unclipped pixels, 16 loads issued at a time
-  auto chunkSums = [&](int c, int lc, bool all) {
+  // The plain sums as integers: each FP32 good pixel is a multiple of 2^(eMin -
+  // 150), eMin the smallest exponent field; while the total stays below 2^53
+  // quanta every partial sum of the reference's order is exact.  (Bits beyond
+  // 62 of a total are excluded first.)
+  const int eMin = (int)(sKMin >> 23), eMax = (int)(sKMax >> 23);
+  bool exact = F32 && nGood > 0 && eMin > 0 && eMax < 255 &&
+               24 + eMax - eMin + (32 - __clz(nGood)) <= 62;
+  auto quanta = [&](float f) -> long long {
+    const unsigned b = __float_as_uint(f);
+    return (long long)((unsigned long long)((b & 0x7FFFFFu) | 0x800000u) << ((int)(b >> 23) - eMin));
+  };
+  // Sums of a chunk's unclipped pixels (bits of m) in order, 16 loads issued
+  // at a time: squares always, the pixels themselves as the mode says.
+  enum { SQUARES, WITH_TOTAL, WITH_SUM };
+  long long tot = 0;
+  auto chunkSums = [&](int c, unsigned m, auto mode) {
     double a = 0.0, a2 = 0.0;
 #pragma unroll
-    for(int h = 0; h < 32; h += 16) {
+    for(int h0 = 0; h0 < 32; h0 += 16) {
       T v[16];
-      bool on[16];
+#pragma unroll
+      for(int l = 0; l < 16; l++) v[l] = (SM || (m >> (h0 + l) & 1u)) ? pixel(c, h0 + l) : T(0);
 #pragma unroll
       for(int l = 0; l < 16; l++) {
-        const int at = chunkSlot(c, h + l);
-        on[l] = h + l < lc && (all || cl[at] == 0);
-        v[l] = h + l < lc ? gd[at] : T(0);
-      }
-#pragma unroll
-      for(int l = 0; l < 16; l++) {
-        const double d = on[l] ? (double)v[l] : 0.0;
-        a += d;
-        a2 += d * d;
+        const bool on = m >> (h0 + l) & 1u;
+        const double d = on ? widenGood(v[l]) : 0.0;
+        if constexpr(F32) {
+          a2 = fma(d, d, a2);
+          if constexpr(mode == WITH_TOTAL) tot += on ? quanta(v[l]) : 0ll;
+        } else {
+          a2 += d * d;
+        }
+        if constexpr(mode == WITH_SUM) a += d;
       }
     }
-    cS[c] = a;
+    if constexpr(mode == WITH_SUM) cS[c] = a;
     cS2[c] = a2;
   };
-  for(int c = tid; c < nChunks; c += ST_THREADS) chunkSums(c, min(32, nGood - c * 32), true);
+  using Squares = std::integral_constant<int, SQUARES>;
+  using Total = std::integral_constant<int, WITH_TOTAL>;
+  using Sum = std::integral_constant<int, WITH_SUM>;
+  auto addTotal = [&](long long t) {  // into sTot, by all pixel threads
+#pragma unroll
+    for(int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
+    if(lane == 0 && t) atomicAdd(&sTot, (unsigned long long)t);
+  };
+  auto allOf = [&](int c) -> unsigned {
+    const int lc = nGood - c * 32;
+    return lc >= 32 ? 0xFFFFFFFFu : (1u << lc) - 1u;
+  };
+  for(int c = tid; c < nChunks; c += NT) {
+    cm[c] = allOf(c);
+    if(exact) chunkSums(c, allOf(c), Total());
+    else chunkSums(c, allOf(c), Sum());
+  }
+  if(exact) {
+    addTotal(tot);
+    pixSync();
+    if(sTot >= 1ull << 53) {
+      exact = false;
+      for(int c = tid; c < nChunks; c += NT) chunkSums(c, allOf(c), Sum());
+    }
+  }
+  pixSync();
   for(int it = 0; it < 3; it++) {
     if(sDone || sCurr == sPrev) break;
     if(sPrev <= 1) {
@@ -466,21 +589,25 @@ __global__ void __launch_bounds__(ST_THREADS, 3)
       }
       break;
     }
-    __syncthreads();
-    if(tid == 0) sCurr = sPrev;
-    __syncthreads();
+    pixSync();
     // the two sequential chunk sums (the reference's serial FP64 loops, bit
     // for bit) on two warps
     if(warp == 0) {
-      const double sum = osum::warpOrderedSum(cS, nChunks);
+      const double sum2 = osum::warpOrderedSum<2>(cS2, nChunks);
+      if(lane == 0) {
+        sSum2 = sum2;
+        sCurr = sPrev;
+      }
+    } else if(warp == 1 && !exact) {
+      const double sum = osum::warpOrderedSum<2>(cS, nChunks);
       if(lane == 0) sSum = sum;
-    } else if(warp == 1) {
-      const double sum2 = osum::warpOrderedSum(cS2, nChunks);
-      if(lane == 0) sSum2 = sum2;
     }
-    __syncthreads();
+    pixSync();
     if(tid == 0) {
-      const double sum = sSum, sum2 = sSum2;
+      const double sum = exact ? (double)(long long)sTot *
+                                     __longlong_as_double((long long)(eMin - 150 + 1023) << 52)
+                               : sSum;
+      const double sum2 = sSum2;
       double n = (double)sCurr;
       double m = sum / n;
       double sd = sqrt((sum2 - n * m * m) / (double)(sCurr - 1));
@@ -488,44 +615,73 @@ __global__ void __launch_bounds__(ST_THREADS, 3)
       sStd = sd;
       sInv = 1.0 / sd;
       sClip = 0;
+      sChanged = 0;
     }
-    __syncthreads();
+    pixSync();
     const double m = sMean, inv = sInv;
-    thresholds(m, inv);
+    thresholds(m, inv, sStd);
+    const Clip k = clipNow();
     int myClip = 0;
-    for(int c = tid; c < nChunks; c += ST_THREADS) {
-      const int lc = min(32, nGood - c * 32);
+    tot = 0;
+    for(int c = tid; c < nChunks; c += NT) {
       // a chunk none of whose pixels is clipped in this round keeps its sums
       // (the same terms in the same order)
-      bool changed = false;
+      const unsigned live = cm[c];
+      unsigned out = 0;
 #pragma unroll
-      for(int h = 0; h < 32; h += 16) {
+      for(int h0 = 0; h0 < 32; h0 += 16) {
         T v[16];
-        uint8_t fl[16];
 #pragma unroll
-        for(int l = 0; l < 16; l++) {
-          v[l] = h + l < lc ? gd[chunkSlot(c, h + l)] : T(0);
-          fl[l] = h + l < lc ? cl[chunkSlot(c, h + l)] : (uint8_t)1;
-        }
+        for(int l = 0; l < 16; l++) v[l] = (SM || (live >> (h0 + l) & 1u)) ? pixel(c, h0 + l) : T(0);
+        if(k.direct) {
 #pragma unroll
-        for(int l = 0; l < 16; l++) {
-          if(fl[l] == 0 && isClippedPix(v[l], m, inv)) {
-            cl[chunkSlot(c, h + l)] = 1;
-            myClip++;
-            changed = true;
-          }
+          for(int l = 0; l < 16; l++)
+            if(clipOut((double)v[l], m, inv, sigClipAlpha)) out |= 1u << (h0 + l);
+        } else {
+#pragma unroll
+          for(int l = 0; l < 16; l++)
+            if(v[l] >= k.hi || v[l] <= k.lo) out |= 1u << (h0 + l);
         }
       }
-      if(changed) chunkSums(c, lc, false);
+      out &= live;
+      if(out) {
+        cm[c] = live & ~out;
+        myClip += __popc(out);
+        if constexpr(F32)
+          if(exact)
+            for(unsigned o = out; o; o &= o - 1) tot -= quanta(pixel(c, __ffs(o) - 1));
+        if constexpr(SM) {
+          changed[atomicAdd(&sChanged, 1)] = (uint16_t)c;
+        } else {
+          if(exact) chunkSums(c, live & ~out, Squares());
+          else chunkSums(c, live & ~out, Sum());
+        }
+      }
     }
-    if(myClip) atomicAdd(&sClip, myClip);
-    __syncthreads();
+    myClip = __reduce_add_sync(0xffffffffu, myClip);
+    if(lane == 0 && myClip) atomicAdd(&sClip, myClip);
+    if(exact) addTotal(tot);
+    pixSync();
     if(tid == 0) sPrev = sCurr - sClip;
-    __syncthreads();
+    if constexpr(SM)
+      for(int i = tid; i < sChanged; i += NT) {
+        const int c = changed[i];
+        if(exact) chunkSums(c, cm[c], Squares());
+        else chunkSums(c, cm[c], Sum());
+      }
+    pixSync();
   }
-  __syncthreads();
+  pixSync();
   const double mean = sMean, invStd = 1.0 / sStd;
-  thresholds(mean, invStd);
+  thresholds(mean, invStd, sStd);
+  const Clip clipEnd = clipNow();
+  __syncthreads();  // the samples are sorted
+  // NaN pixels get their mask bits now that the samples have been taken
+  if(sNan)
+    for(int i = tid; i < nPixS; i += NT) {
+      size_t id;
+      if(pixelAt(i, &id) && mask[id] == 0 && isnan(img[id])) mask[id] |= NAN_PIXEL | BAD_INPUT;
+    }
 
   // ---- phase D: histogram sky / robust sigma (sss.cl:190-324) ----
   if(tid == 0) {
@@ -537,15 +693,14 @@ __global__ void __launch_bounds__(ST_THREADS, 3)
     hLower = hUpper = hSky = 0.0;
     hState = 0;
   }
-  __syncthreads();
+  pixSync();
   for(int attempts = 0;; attempts++) {
     if(attempts >= 5) {
       if(tid == 0) hState = 2;
       break;
     }
-    for(int i = tid; i < 256; i += ST_THREADS) bins[i] = 0;
+    for(int i = tid; i < 256; i += NT) bins[i] = 0;
     if(tid == 0) {
-      okCount = 0;
       // FP32 estimate q' of q = (v - lbv) / bs: |q' - q| <= delta for |q| <= 512
       // (lbv and 1/bs rounded to float, one FP32 rounding each in the
       // subtraction and the product; the FP64 q itself is within 2^-51 |q|)
@@ -554,98 +709,102 @@ __global__ void __launch_bounds__(ST_THREADS, 3)
       const bool ok = F32 && bs > 0.0 && isfinite(bs) && isfinite(lbv) && delta < 0.125;
       bExact = ok ? 0 : 1;
       bLbv = (float)lbv;
-      bInv = (float)(1.0 / bs);
+      bRec = 1.0 / bs;
+      bInv = (float)bRec;
       bDelta = (float)delta;
     }
-    __syncthreads();
+    pixSync();
     const double lbv = hLowerBinVal, bs = hBinSize;
     const bool exactAll = bExact != 0;
-    const float fl = bLbv, fi = bInv, fd = bDelta;
-    int myOk = 0;
+    const float fl = bLbv, fi = bInv, half = 0.5f - bDelta;
+    const double rbs = bRec;
     // the pixels of createHistogram (mask 0, above 1e-10, not clipped) are
     // the good list of phase B (the kernel changes no other mask bit of the
-    // stamp) less the final clip; a warp-uniform trip count lets the lanes of
-    // a warp that land in the same bin (most pixels sit in a few sky bins)
-    // add to it with one atomic
+    // stamp) less the final clip
     constexpr int HB = 8;  // list entries loaded ahead per thread
-    // (the counts do not depend on the order: the slots are read in storage
-    // order, coalesced, each standing for list entry listEntry(slot))
-    const int nSlots = (nGood + 1023) & ~1023;
-    for(int base0 = 0; base0 < nSlots; base0 += ST_THREADS * HB) {
+    // (the counts do not depend on the order: the slots of a scratch slice are
+    // read in storage order, coalesced, each standing for listEntry(slot))
+    const int nSlots = SM ? nGood : (nGood + 1023) & ~1023;
+    for(int base0 = 0; base0 < nSlots; base0 += NT * HB) {
       T pvs[HB];
       bool in[HB];
 #pragma unroll
       for(int u = 0; u < HB; u++) {
-        const int k = base0 + u * ST_THREADS + tid;
-        in[u] = k < nSlots && listEntry(k) < nGood;
-        pvs[u] = in[u] ? gd[k] : T(0);
+        const int k = base0 + u * NT + tid;
+        if constexpr(SM) {
+          in[u] = k < nGood;
+          pvs[u] = in[u] ? list[k + (k >> 5)] : 0.f;
+        } else {
+          in[u] = k < nSlots && listEntry(k) < nGood;
+          pvs[u] = in[u] ? gd[k] : T(0);
+        }
       }
+      unsigned rest = 0;  // entries whose bin the FP32 estimate leaves open
 #pragma unroll
       for(int u = 0; u < HB; u++) {
-        int index = -1;
-        if(in[u]) {
-          const T pv = pvs[u];
-          if(!isClippedPix(pv, mean, invStd)) {
-            if(!exactAll) {
-              const float q = ((float)pv - fl) * fi;
-              if(q > 300.f) {
-                index = 255;
-              } else if(q < -50.f) {
-                index = 0;
-              } else {
-                const float f0 = floorf(q), fr = q - f0;
-                if(fr > fd && fr < 1.f - fd) index = min(max((int)f0 + 1, 0), 255);
-              }
-            }
-            if(index < 0) {
-              const double v = (double)pv;
-              index = satFloorToInt((v - lbv) / bs);
-              index = index == INT_MAX ? INT_MAX : index + 1;
-              index = min(max(index, 0), 255);
-            }
-          }
-        }
-        const unsigned grp = __match_any_sync(0xffffffffu, index);
-        if(index >= 0) {
-          myOk++;
-          if(lane == __ffs(grp) - 1) atomicAdd(&bins[index], __popc(grp));
+        const T pv = pvs[u];
+        const bool out = clipEnd.direct ? clipOut((double)pv, mean, invStd, sigClipAlpha)
+                                        : pv >= clipEnd.hi || pv <= clipEnd.lo;
+        const float q = fminf(fmaxf(((float)pv - fl) * fi, -50.f), 300.f);
+        const float f0 = floorf(q), fr = q - f0;
+        const bool open = exactAll || (fabsf(fr - 0.5f) >= half && q > -50.f && q < 300.f);
+        if(in[u] && !out) {
+          if(open) rest |= 1u << u;
+          else atomicAdd(&bins[min(max((int)f0 + 1, 0), 255)], 1);
         }
       }
+      if(__any_sync(0xffffffffu, rest))
+#pragma unroll
+        for(int u = 0; u < HB; u++)
+          if(rest >> u & 1u) {
+            // floor of the quotient from the reciprocal, whose product is within
+            // 2^-40 of it below 2^10; at a bin's edge the division decides
+            const double v = (double)pvs[u], q = (v - lbv) * rbs, f0 = floor(q);
+            int index;
+            if(fabs(q) < 1024.0 && fabs(q - f0 - 0.5) < 0.5 - 0x1p-40) {
+              index = (int)f0 + 1;
+            } else {
+              index = satFloorToInt((v - lbv) / bs);
+              index = index == INT_MAX ? INT_MAX : index + 1;
+            }
+            atomicAdd(&bins[min(max(index, 0), 255)], 1);
+          }
     }
-    if(myOk) atomicAdd(&okCount, myOk);
-    __syncthreads();
+    pixSync();
     if(warp == 0) {
-      const int ok = okCount;
       const double binSize = hBinSize, lowerBinVal = hLowerBinVal;
+      // The reference walks the bins serially (createHistogram,
+      // sss.cl:190-324); every quantity it forms is a prefix sum of the
+      // counts, so one warp scans the 256 bins once and finds each walk's
+      // stopping point by binary search, all of them side by side.
+      // The running sums of bin counts (sumBins, sumExpect) are FP64 in the
+      // reference but hold integers below 2^53, so they are integers here;
+      // S < x for an integer S and a double x is S < ceil(x).
+      int c8[8], tc = 0;
+      long long e8[8], te = 0;
+#pragma unroll
+      for(int k = 0; k < 8; k++) {
+        const int i = 8 * lane + k;
+        tc += bins[i];
+        te += (long long)i * bins[i];
+        c8[k] = tc;
+        e8[k] = te;
+      }
+      int pc = tc;
+      long long pe = te;  // inclusive scan of the lane totals
+#pragma unroll
+      for(int o = 1; o < 32; o <<= 1) {
+        const int uc = __shfl_up_sync(0xffffffffu, pc, o);
+        const long long ue = __shfl_up_sync(0xffffffffu, pe, o);
+        if(lane >= o) {
+          pc += uc;
+          pe += ue;
+        }
+      }
+      const int ok = __shfl_sync(0xffffffffu, pc, 31);
       if(ok == 0 || binSize == 0.0) {
         if(lane == 0) hState = 2;
       } else {
-        // The reference walks the bins serially (createHistogram,
-        // sss.cl:190-324); every quantity it forms is a prefix sum of the
-        // counts, so one warp scans the 256 bins once and finds each walk's
-        // stopping point by binary search.
-        // The running sums of bin counts (sumBins, sumExpect) are FP64 in the
-        // reference but hold integers below 2^53, so they are int64 here;
-        // S < x for an integer S and a double x is S < ceil(x).
-        long long c8[8], e8[8], tc = 0, te = 0;
-#pragma unroll
-        for(int k = 0; k < 8; k++) {
-          const int i = 8 * lane + k;
-          tc += bins[i];
-          te += (long long)i * bins[i];
-          c8[k] = tc;
-          e8[k] = te;
-        }
-        long long pc = tc, pe = te;  // inclusive scan of the lane totals
-#pragma unroll
-        for(int o = 1; o < 32; o <<= 1) {
-          const long long uc = __shfl_up_sync(0xffffffffu, pc, o);
-          const long long ue = __shfl_up_sync(0xffffffffu, pe, o);
-          if(lane >= o) {
-            pc += uc;
-            pe += ue;
-          }
-        }
 #pragma unroll
         for(int k = 0; k < 8; k++) {  // hC[i] = sum of bins[0..i), hCE[i] = sum of j * bins[j]
           hC[8 * lane + k + 1] = pc - tc + c8[k];
@@ -653,12 +812,12 @@ __global__ void __launch_bounds__(ST_THREADS, 3)
         }
         if(lane == 0) hC[0] = hCE[0] = 0;
         __syncwarp();
-        const long long tenth = (long long)ceil(ok / 10.0);
+        const int tenth = (int)((ok + 9u) / 10u);  // ceil of the FP64 quotient
         // first i in [lo, hi] with hC[i] >= target, hi when none
-        auto firstAtLeast = [&](int lo, int hi, long long target) {
+        auto firstAtLeast = [&](int lo, int hi, unsigned target) {
           while(lo < hi) {
             const int mid = (lo + hi) >> 1;
-            if(hC[mid] >= target) hi = mid;
+            if((unsigned)hC[mid] >= target) hi = mid;
             else lo = mid + 1;
           }
           return lo;
@@ -667,7 +826,8 @@ __global__ void __launch_bounds__(ST_THREADS, 3)
         // window for lower index L ends at U(L) = the first U in [L+1, 255]
         // with hC[U] - hC[L] >= tenth (255 when none; U(L) never decreases,
         // so this is where the two-pointer walk stands), and the walk visits
-        // L = 1, 2, ... while the previous window ended below 255.  The
+        // L = 1, 2, ... while the previous window ended below 255, that is
+        // while a bin count up to 254 had reached its target.  The
         // reference compares the FP64 quotients S / (U - L); both are integer
         // over integer (sums of counts < 2^31, widths 1..254), and two
         // different such fractions differ by more than 2^-47 relative, so
@@ -675,11 +835,31 @@ __global__ void __launch_bounds__(ST_THREADS, 3)
         // S / D > S' / D'  <=>  S * D' > S' * D, exact in 64-bit integers.
         // The walk keeps the first L of the largest density (strict >), from
         // maxDens = 0.
+        int lo[8], hi[8];
+        unsigned goal[8];  // counts stay below 2^31
+#pragma unroll
+        for(int k = 0; k < 8; k++) {
+          goal[k] = (unsigned)hC[1 + lane + 32 * k] + tenth;
+          lo[k] = 2 + lane + 32 * k;
+          hi[k] = 255;
+        }
+#pragma unroll
+        for(int step = 0; step < 8; step++)
+#pragma unroll
+          for(int k = 0; k < 8; k++) {
+            const int mid = (lo[k] + hi[k]) >> 1;
+            if(lo[k] < hi[k]) {
+              if((unsigned)hC[mid] >= goal[k]) hi[k] = mid;
+              else lo[k] = mid + 1;
+            }
+          }
         long long bN = 0, bD = 1;
         int bL = -1;
-        for(int L = 1 + lane; L <= 254; L += 32) {
-          if(L > 1 && firstAtLeast(L, 255, hC[L - 1] + tenth) >= 255) continue;
-          const int U = firstAtLeast(L + 1, 255, hC[L] + tenth);
+#pragma unroll
+        for(int k = 0; k < 8; k++) {
+          const int L = 1 + lane + 32 * k;
+          if(L > 254 || (L > 1 && (unsigned)hC[254] < (unsigned)hC[L - 1] + tenth)) continue;
+          const int U = lo[k];
           const long long S = hC[U] - hC[L], D = U - L;
           if(S * bD > bN * D) {
             bN = S;
@@ -699,20 +879,22 @@ __global__ void __launch_bounds__(ST_THREADS, 3)
             bL = oL;
           }
         }
+        // Lane 0: the mode's walk from maxIndex adds bins while below a tenth.
+        // Lanes 1 and 2: the quartile walks from bin 0 (hC[256] = ok bounds
+        // both, and the upper one ends no earlier than the lower one); a quarter
+        // of a count is exact in FP64, so its ceiling is the integer one.
+        const int maxIndex = bL < 0 ? 0 : bL;
+        const double part = ok * (lane == 2 ? 0.75 : 0.25);
+        const int iEnd = lane == 0 ? firstAtLeast(maxIndex + 1, 255, (unsigned)hC[maxIndex] + tenth)
+                                   : firstAtLeast(0, 256, (unsigned)(((lane == 2 ? 3ll : 1ll) * ok + 3) / 4));
+        const double num = lane == 0 ? (double)(hCE[iEnd] - hCE[maxIndex]) : (double)hC[iEnd] - part;
+        const int den = lane == 0 ? hC[iEnd] - hC[maxIndex] : bins[max(iEnd, 1) - 1];
+        const double quot = num / (double)den;
+        const double value = lane == 0 ? quot + 0.5 : iEnd - quot;
+        const double lower = __shfl_sync(0xffffffffu, value, 1);
+        const double upper = __shfl_sync(0xffffffffu, value, 2);
         if(lane == 0) {
-          const int maxIndex = bL < 0 ? 0 : bL;
-          // the mode's walk from maxIndex adds bins while below a tenth
-          const int iEnd = firstAtLeast(maxIndex + 1, 255, hC[maxIndex] + tenth);
-          const long long S = hC[iEnd] - hC[maxIndex], E = hCE[iEnd] - hCE[maxIndex];
-          double modeBin = (double)E / (double)S + 0.5;
-          double skyEst = lowerBinVal + binSize * (modeBin - 1.0);
-          double lower = ok * 0.25, upper = ok * 0.75;
-          const long long lowerCeil = (long long)ceil(lower), upperCeil = (long long)ceil(upper);
-          // the quartile walks from bin 0 (hC[256] = ok bounds both)
-          const int i1 = firstAtLeast(0, 256, lowerCeil);
-          lower = i1 - ((double)hC[i1] - lower) / bins[i1 - 1];
-          const int i2 = firstAtLeast(i1, 256, upperCeil);
-          upper = i2 - ((double)hC[i2] - upper) / bins[i2 - 1];
+          const double skyEst = lowerBinVal + binSize * (value - 1.0);
           hSky = skyEst;
           hLower = lower;
           hUpper = upper;
@@ -728,13 +910,42 @@ __global__ void __launch_bounds__(ST_THREADS, 3)
         }
       }
     }
-    __syncthreads();
+    pixSync();
     if(hState != 0) break;
   }
   if(tid == 0) {
     fwhmOut[s] = hState == 1 ? hBinSize * (hUpper - hLower) / iqRange : 0.0;
     skyOut[s] = hSky;
   }
+}
+
+// Launches the statistics of n stamps.  FP32 stamps whose pixels fit in shared
+// memory keep them there (up to about 214 px on a side), with 16 warps where
+// only one CTA fits on an SM; larger ones and FP64 images use the scratch.
+template <class T>
+cudaError_t launchStampStats(const T* img, uint16_t* mask, const int4* geom, int n, int w, int h,
+                             int fSW, T* good, uint8_t* clip, double* chunkBuf, double alpha,
+                             double iqRange, double* sky, double* fwhm, const double* draws,
+                             int device, cudaStream_t stream) {
+  const int maxChunks = (int)(((long long)fSW * fSW + 31) / 32);
+  int optin = 0;
+  cudaError_t e = cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, device);
+  if(e != cudaSuccess) return e;
+  auto go = [&](auto kernel, int threads, size_t smem) -> cudaError_t {
+    if(smem > 32 * 1024) {
+      const cudaError_t a = allowMaxDynamicSmem((const void*)kernel, device);
+      if(a != cudaSuccess) return a;
+    }
+    kernel<<<n, threads, smem, stream>>>(img, mask, geom, w, h, fSW, good, clip, chunkBuf, maxChunks,
+                                         alpha, iqRange, sky, fwhm, draws);
+    return cudaSuccess;
+  };
+  if constexpr(sizeof(T) == 4) {
+    const size_t smem = statsSmemBytes(maxChunks, true), fixed = 8192;  // static and reserved
+    if(2 * (smem + fixed) <= (size_t)optin) return go(k_stamp_stats<T, true, 8>, 288, smem);
+    if(smem + fixed <= (size_t)optin) return go(k_stamp_stats<T, true, 16>, 544, smem);
+  }
+  return go(k_stamp_stats<T, false, 8>, 288, statsSmemBytes(maxChunks, false));
 }
 
 // Mask access shared by the substamp search: volatile 16-bit loads (other
@@ -1630,21 +1841,17 @@ static const double* ran1Draws(xb_ctx* c, int n) {
 static void sssPass(xb_ctx* c, int* nKept) {
   const Geo& g = c->g;
   const int fSW = c->fStampWidth, nAll = c->nAll;
-  const int maxChunks = (fSW * fSW + 31) / 32;
   double* chunkBuf = c->dWork;  // sized by stageSss
   const double* draws = ran1Draws(c, 2 * fSW * fSW);
   for(int im = 0; im < 2; im++) {
     { KT_SCOPE(c, "stamp_stats");
-    if(c->imgIsF64)
-      k_stamp_stats<double><<<nAll, ST_THREADS, 0, c->stream>>>(
-          (const double*)c->img[im], c->mask, c->geomAll, c->w, c->h, fSW,
-          c->goodScratch, c->clipScratch, chunkBuf, maxChunks, c->p.sigClipAlpha,
-          c->p.iqRange, c->skyAll[im], c->fwhmAll[im], draws);
-    else
-      k_stamp_stats<float><<<nAll, ST_THREADS, 0, c->stream>>>(
-          (const float*)c->img[im], c->mask, c->geomAll, c->w, c->h, fSW,
-          reinterpret_cast<float*>(c->goodScratch), c->clipScratch, chunkBuf, maxChunks, c->p.sigClipAlpha,
-          c->p.iqRange, c->skyAll[im], c->fwhmAll[im], draws);
+    auto stats = [&](auto* img, auto* good) {
+      XB_CUDA(launchStampStats(img, c->mask, c->geomAll, nAll, c->w, c->h, fSW, good, c->clipScratch,
+                               chunkBuf, c->p.sigClipAlpha, c->p.iqRange, c->skyAll[im],
+                               c->fwhmAll[im], draws, c->device, c->stream));
+    };
+    if(c->imgIsF64) stats((const double*)c->img[im], c->goodScratch);
+    else stats((const float*)c->img[im], reinterpret_cast<float*>(c->goodScratch));
     XB_LAUNCHED(c);
     }
   }
@@ -1913,12 +2120,14 @@ extern "C" int xb_stamp_stats_noalloc(const float* dImg, uint16_t* dMask, int w,
   // Nothing needs clearing: within one launch every scratch byte the kernel
   // reads is written first (clip flags and good pixels during the
   // compaction, chunk sums before they are summed).
-  xb::k_stamp_stats<float><<<nStamps, xb::ST_THREADS, 0, (cudaStream_t)stream>>>(
-      dImg, dMask, reinterpret_cast<const int4*>(dGeom), w, h, fStampWidth,
-      reinterpret_cast<float*>(good), clip, chunks,
-      maxChunks, sigClipAlpha, iqRange, dSky, dFwhm, nullptr);
+  cudaError_t e = xb::launchStampStats(
+      dImg, dMask, reinterpret_cast<const int4*>(dGeom), nStamps, w, h, fStampWidth,
+      reinterpret_cast<float*>(good), clip, chunks, sigClipAlpha, iqRange, dSky, dFwhm,
+      (const double*)nullptr, dev, (cudaStream_t)stream);
+  if(e != cudaSuccess) cudaGetLastError();  // not left pending for the caller
+  if(e != cudaSuccess) return noallocFail(err, errCap, XB_ERR_CUDA, cudaGetErrorString(e));
   // no error was pending before the launch, so any error now is the launch's
-  cudaError_t e = cudaGetLastError();
+  e = cudaGetLastError();
   if(e != cudaSuccess) return noallocFail(err, errCap, XB_ERR_CUDA, cudaGetErrorString(e));
   return XB_OK;
 }
@@ -1926,7 +2135,7 @@ extern "C" int xb_stamp_stats_noalloc(const float* dImg, uint16_t* dMask, int w,
 namespace xb {
 namespace {
 __global__ void k_ordered_sum(const double* __restrict__ c, int n, double* __restrict__ out) {
-  const double s = osum::warpOrderedSum(c, n);
+  const double s = osum::warpOrderedSum<2>(c, n);
   if(threadIdx.x == 0) *out = s;
 }
 __global__ void k_ordered_sum_f32(const float* __restrict__ c, int n, double* __restrict__ out) {
