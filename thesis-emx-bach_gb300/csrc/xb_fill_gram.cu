@@ -1,5 +1,6 @@
 // xb_fill_gram.cu — the mixed path's substamp fill and its exact tensor-core
-// Gram matrix in one kernel, one CTA per stamp.
+// Gram matrix in one kernel, one CTA per stamp, or a cluster of four for the few
+// stamps of a refill, whose latency is the frame's.
 //
 // For the common shapes it replaces three launches (k_fill_w_f32 ->
 // k_fill_finish_f32 -> k_gram_tc) that passed W through HBM: the separate
@@ -23,7 +24,8 @@
 //      Steps 2-3 run in passes of at most FG_GP Y filters (the pass holding
 //      basis function 0 first; the default basis has 21 distinct Y filters,
 //      so 3 passes), so that the Y outputs of one pass fit beside everything
-//      else in ~85 KB;
+//      else in ~85 KB (a cluster's CTA has a quarter of the output rows and
+//      takes all filters in one pass);
 //   4. the exact sliced Gram of xb_tc.cuh: each thread loads its units of the
 //      CTA's own W back from L2 chunk by chunk, slices them with the row
 //      exponents into BF16 digits, one thread multiplies them by tcgen05.mma
@@ -56,28 +58,38 @@ constexpr int FG_R8 = 8;    // outputs per thread item (rows of the Y pass, pixe
 constexpr int FG_GP = 7;    // Y filters per pass
 constexpr int FG_MAXPASS = 4;
 constexpr int FG_MAXG = FG_MAXPASS * FG_GP;
+constexpr int FG_CL = 4, FG_NTS = 512;  // CTAs and threads for a stamp of a short list
 
-// Shared-memory layout of the fill (steps 1-3); the Gram (step 4) and the
-// epilogue reuse the same area from offset 0.
+// Shared-memory layout of the fill (steps 1-3) for a CTA's nr output rows; the
+// Gram (step 4) and the epilogue reuse the same area from offset 0.
 struct FgLayout {
-  int tw, fSS, ldWin, winRows, ldY;
+  int tw, th, fSS, nr, ldWin, winRows, ldY;
   size_t oWin, oF, oW0, oY, fill, total;
 };
-__host__ __device__ inline FgLayout fgLayout(int hSS, int hK, int nGroups, int nPSF) {
+// output rows per CTA of a stamp of fSS rows over cl CTAs: whole blocks of FG_R8
+__host__ __device__ inline int fgRows(int fSS, int cl) {
+  const int nRB = (fSS + FG_R8 - 1) / FG_R8, rows = (nRB + cl - 1) / cl * FG_R8;
+  return rows < fSS ? rows : fSS;
+}
+// Y filters per pass
+__host__ __device__ inline int fgPerPass(int cl) { return cl > 1 ? FG_MAXG : FG_GP; }
+__host__ __device__ inline FgLayout fgLayout(int hSS, int hK, int nGroups, int nPSF, int cl) {
   FgLayout L;
   L.fSS = 2 * hSS + 1;
+  L.nr = fgRows(L.fSS, cl);
   L.tw = L.fSS + 2 * hK;
+  L.th = L.nr + 2 * hK;
   L.ldWin = (L.tw + 3 + 3) / 4 * 4;   // TMA box width: 16-byte rows, room for the x offset
-  L.winRows = L.tw + FG_R8;           // rows past tw are read only by discarded outputs
+  L.winRows = L.th + FG_R8;           // rows past th are read only by discarded outputs
   L.ldY = L.tw + FG_R8;               // odd stride: the X items' rows fall on distinct banks
   if(L.ldY % 2 == 0) L.ldY++;
-  const int fK = 2 * hK + 1, gp = nGroups < FG_GP ? nGroups : FG_GP;
+  const int fK = 2 * hK + 1, gp = nGroups < fgPerPass(cl) ? nGroups : fgPerPass(cl);
   auto al = [](size_t v) { return (v + 127) / 128 * 128; };
   L.oWin = 0;
   L.oF = al(L.oWin + (size_t)L.ldWin * L.winRows * 4);
   L.oW0 = al(L.oF + (size_t)2 * (nPSF + nGroups) * fK * 4);
-  L.oY = al(L.oW0 + (size_t)2 * L.fSS * L.fSS * 4);
-  L.fill = al(L.oY + (size_t)gp * L.fSS * L.ldY * 4);
+  L.oY = al(L.oW0 + (size_t)2 * L.nr * L.fSS * 4);
+  L.fill = al(L.oY + (size_t)gp * L.nr * L.ldY * 4);
   size_t m = L.fill;
   if((size_t)2 * tc::OPBUF > m) m = 2 * tc::OPBUF;
   if((size_t)tc::EPI2_BYTES > m) m = tc::EPI2_BYTES;
@@ -159,8 +171,10 @@ __device__ __forceinline__ void maxBits(unsigned* slot, float m) {
   atomicMax(slot, __float_as_uint(m));  // m >= 0: the bit patterns are ordered
 }
 
-template <int NT>
-__global__ void __launch_bounds__(NT, 2)
+// CL CTAs (a cluster) share a stamp by output rows; they exchange the row
+// maxima before slicing and their exact sums at the end.
+template <int NT, int CL>
+__global__ void __launch_bounds__(NT, NT > 384 ? 1 : 2)
     k_fill_gram(const __grid_constant__ CUtensorMap tmap, const __grid_constant__ FillGramArgs a) {
   using namespace tc;
   constexpr int HK = FG_HK, FK = 2 * HK + 1;
@@ -171,26 +185,32 @@ __global__ void __launch_bounds__(NT, 2)
   __shared__ unsigned char evenRow[MAX_NPSF];
   __shared__ unsigned long long bars[4];  // two operand buffers, the window copy, the test stall
   __shared__ uint32_t tmemBase;
-  if(a.liveN && (int)blockIdx.x >= *a.liveN) return;  // before any barrier or TMEM allocation
-  const int t = blockIdx.x, s = a.list[t], tid = threadIdx.x, warp = tid >> 5;
-  const int fSS = 2 * a.hSS + 1, K = fSS * fSS, R = a.wRows + 1, nPSF = a.nPSF;
+  const int t = blockIdx.x / CL, rank = blockIdx.x % CL;
+  if(a.liveN && t >= *a.liveN) return;  // the whole cluster, before any barrier or TMEM allocation
+  const int s = a.list[t], tid = threadIdx.x, warp = tid >> 5;
+  const int fSS = 2 * a.hSS + 1, R = a.wRows + 1, nPSF = a.nPSF;
   const int ldW = a.ldW;
   float* Ws = a.W + (size_t)s * a.wRows * ldW;
   float* Wl = a.Wlo + (size_t)s * a.wRows * ldW;
   double* Gs = a.G + (size_t)t * R * R;
   if(!(a.cur[s] < a.count[s])) {
     // no substamp left: W and G are zero (what the separate kernels give)
-    for(int i = tid; i < a.wRows * ldW; i += NT) {
+    for(int i = rank * NT + tid; i < a.wRows * ldW; i += CL * NT) {
       Ws[i] = 0.f;
       Wl[i] = 0.f;
     }
-    for(int i = tid; i < R * R; i += NT) Gs[i] = 0.0;
+    for(int i = rank * NT + tid; i < R * R; i += CL * NT) Gs[i] = 0.0;
     return;
   }
   const unsigned long long deadline = timerNs() + WAIT_NS;
   unsigned char* buf = (unsigned char*)(((uintptr_t)fg_s + 1023) & ~(uintptr_t)1023);
-  const FgLayout L = fgLayout(a.hSS, HK, a.nGroups, nPSF);
-  const int tw = L.tw, ldWin = L.ldWin, ldY = L.ldY;
+  const FgLayout L = fgLayout(a.hSS, HK, a.nGroups, nPSF, CL);
+  const int tw = L.tw, th = L.th, ldWin = L.ldWin, ldY = L.ldY, ldR = L.nr;
+  // this CTA's output rows rBase .. rBase + nr and its K pixels, a part of the
+  // rows of W that starts at a multiple of eight
+  const int rBase = min(rank * ldR, fSS), nr = min(ldR, fSS - rBase), K = nr * fSS;
+  Ws += rBase * fSS;
+  Wl += rBase * fSS;
   float* win = (float*)(buf + L.oWin);
   float* fxh = (float*)(buf + L.oF);
   float* fxl = fxh + nPSF * FK;
@@ -201,8 +221,11 @@ __global__ void __launch_bounds__(NT, 2)
   float* ytmp = (float*)(buf + L.oY);
 
   const int2 c = a.ssxy[(size_t)s * a.maxSS + a.cur[s]];
-  const int xHalf = a.hSS + HK, wx0 = c.x - xHalf, wy0 = c.y - xHalf;
-  const bool tma = a.useTma && wx0 >= 0 && wy0 >= 0 && wx0 + tw <= a.w && wy0 + tw <= a.h;
+  const int xHalf = a.hSS + HK, wx0 = c.x - xHalf, wy0 = c.y - xHalf + rBase;
+  // (a box that ends below the window or the frame brings rows that only
+  // discarded outputs read)
+  const bool tma = a.useTma && nr > 0 && wx0 >= 0 && wy0 >= 0 && wx0 + tw <= a.w &&
+                   wy0 + nr + 2 * HK <= a.h;
   const int x0 = wx0 & ~3;              // 16-byte aligned start of the TMA box
   const int dx = tma ? wx0 - x0 : 0;    // window column 0 in the staged rows
   const uint32_t winBar = smemU32(&bars[2]);
@@ -213,7 +236,7 @@ __global__ void __launch_bounds__(NT, 2)
     barInit(smemU32(&bars[3]), 1);  // nothing arrives here (test option testStall)
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     if(tma) {
-      const uint32_t bytes = (uint32_t)(ldWin * tw * 4);
+      const uint32_t bytes = (uint32_t)(ldWin * th * 4);
       asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(winBar), "r"(bytes)
                    : "memory");
       asm volatile(
@@ -229,7 +252,7 @@ __global__ void __launch_bounds__(NT, 2)
     evenRow[n] = (n > 0 && a.kx[n] % 2 == 0 && a.ky[n] % 2 == 0) ? 1 : 0;
   if(tid < RB) rowMax[tid] = 0u;
   if(!tma) {
-    for(int i = tid; i < tw * tw; i += NT) {
+    for(int i = tid; i < tw * th; i += NT) {
       const int gx = min(max(wx0 + i % tw, 0), a.w - 1);
       const int gy = min(max(wy0 + i / tw, 0), a.h - 1);
       win[(i / tw) * ldWin + i % tw] = a.conv[(size_t)gx + (size_t)gy * a.w];
@@ -246,18 +269,18 @@ __global__ void __launch_bounds__(NT, 2)
     ok = __syncthreads_or(late) == 0;
   }
 
-  const int nRB = (fSS + FG_R8 - 1) / FG_R8;  // row blocks of the Y pass
+  const int nRB = (nr + FG_R8 - 1) / FG_R8;   // row blocks of the Y pass
   const int nXB = (fSS + FG_R8 - 1) / FG_R8;  // pixel blocks of the X pass
-  const int yPer = nRB * tw, xPer = fSS * nXB;
+  const int yPer = nRB * tw, xPer = nr * nXB;
   // Y item i of filter g: rows block i / tw, window column i % tw
   auto yItem = [&](int g, int i) {
     const int r0 = (i / tw) * FG_R8, col = i % tw;
     float v[FG_R8];
     yPass8<FK>(win + r0 * ldWin + col + dx, ldWin, fyh + g * FK, fyl + g * FK, v);
-    float* yo = ytmp + ((size_t)a.slot[g] * fSS + r0) * ldY + col;
+    float* yo = ytmp + ((size_t)a.slot[g] * ldR + r0) * ldY + col;
 #pragma unroll
     for(int j = 0; j < FG_R8; j++)
-      if(r0 + j < fSS) yo[j * ldY] = v[j];
+      if(r0 + j < nr) yo[j * ldY] = v[j];
   };
   // stores 8 outputs of row n starting at pixel p0 (nv of them valid) and
   // folds their largest |hi| into the row maximum
@@ -277,7 +300,7 @@ __global__ void __launch_bounds__(NT, 2)
     const int row = i / nXB, ii0 = (i % nXB) * FG_R8;
     const int nv = min(FG_R8, fSS - ii0), p0 = row * fSS + ii0;
     float hi[FG_R8], lo[FG_R8];
-    xPass8<FK>(ytmp + ((size_t)a.slot[a.groupOf[n]] * fSS + row) * ldY + ii0, fxh + n * FK,
+    xPass8<FK>(ytmp + ((size_t)a.slot[a.groupOf[n]] * ldR + row) * ldY + ii0, fxh + n * FK,
                fxl + n * FK, hi, lo);
     if(n == 0) {
 #pragma unroll
@@ -300,7 +323,7 @@ __global__ void __launch_bounds__(NT, 2)
     const int row = i / nXB, ii0 = (i % nXB) * FG_R8;
     const int nv = min(FG_R8, fSS - ii0), p0 = row * fSS + ii0;
     const int ex = a.bgXY[b].x, ey = a.bgXY[b].y;
-    const float yf = df::floatNormF(c.y - a.hSS + row, a.h);
+    const float yf = df::floatNormF(c.y - a.hSS + rBase + row, a.h);
     float hi[FG_R8], lo[FG_R8];
 #pragma unroll
     for(int j = 0; j < FG_R8; j++) {
@@ -320,7 +343,7 @@ __global__ void __launch_bounds__(NT, 2)
   auto imgItem = [&](int i) {
     const int row = i / nXB, ii0 = (i % nXB) * FG_R8;
     const int nv = min(FG_R8, fSS - ii0), p0 = row * fSS + ii0;
-    const int gy = min(max(c.y - a.hSS + row, 0), a.h - 1);
+    const int gy = min(max(c.y - a.hSS + rBase + row, 0), a.h - 1);
     float m = 0.f;
     for(int j = 0; j < nv; j++) {
       const int gx = min(max(c.x - a.hSS + ii0 + j, 0), a.w - 1);
@@ -346,9 +369,9 @@ __global__ void __launch_bounds__(NT, 2)
       else if(it < n2) bgItem((it - n1) / xPer, (it - n1) % xPer);
       else imgItem(it - n2);
     }
-    const int padW = ldW - K, nChunkK = (K + KC - 1) / KC * KC;
-    for(int i = tid; i < a.wRows * padW; i += NT) {
-      const size_t o = (size_t)(i / padW) * ldW + K + i % padW;
+    const int padW = ldW - fSS * fSS, nChunkK = (K + KC - 1) / KC * KC;
+    for(int i = rank * NT + tid; i < a.wRows * padW; i += CL * NT) {
+      const size_t o = (size_t)(i / padW) * ldW + (fSS - rBase) * fSS + i % padW;
       Ws[o] = 0.f;
       Wl[o] = 0.f;
     }
@@ -369,17 +392,28 @@ __global__ void __launch_bounds__(NT, 2)
   }
   // the CTA's W stores before its own reads of them (step 4)
   __syncthreads();
-  if(tid < RB) expo[tid] = tid < R ? rowExponent(__uint_as_float(rowMax[tid])) : 0;
+  if(CL > 1) clusterSync();  // every CTA's row maxima
+  if(tid < RB) {
+    unsigned m = rowMax[tid];
+    if constexpr(CL > 1) {
+#pragma unroll
+      for(int q = 0; q < CL; q++) m = max(m, peerLoad32(peerAddr(smemU32(&rowMax[tid]), q)));
+    }
+    expo[tid] = tid < R ? rowExponent(__uint_as_float(m)) : 0;
+  }
+  // (no CTA waits for another one while it holds TMEM)
   if(warp == 0) tmemAlloc512(&tmemBase);
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
   const uint32_t tmem = tmemBase;
-  if(!gramChunksDirect<NT>(Ws, Wl, a.wRows, ldW, R, K, imgRow, expo, buf, bars, tmem, deadline,
-                           a.testStall ? &bars[3] : nullptr))
+  if(K > 0 && !gramChunksDirect<NT>(Ws, Wl, a.wRows, ldW, R, K, imgRow, expo, buf, bars, tmem, deadline,
+                                    a.testStall ? &bars[3] : nullptr))
     ok = false;
-  epilogueAtomic(tmem, (long long*)buf, expo, R, Gs);
+  epilogueAtomic<CL>(tmem, (long long*)buf, expo, R, Gs, rank, K > 0);
   if(tid == 0 && !ok) atomicOr(a.timeout, 1);
+  __syncwarp();
+  if(CL > 1) clusterSync();  // the others have read this CTA's sums
 }
 
 // cuTensorMapEncodeTiled through the runtime's driver entry point, so the
@@ -414,7 +448,7 @@ bool fillGramFits(const xb_ctx* c) {
   if(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, c->device) != cudaSuccess)
     return false;
   // the static arrays of the kernel take ~5 KB beside the dynamic area
-  return fgLayout(g.hSS, g.hK, nGroups, g.nPSF).total + 8 * 1024 <= (size_t)optin;
+  return fgLayout(g.hSS, g.hK, nGroups, g.nPSF, 1).total + 8 * 1024 <= (size_t)optin;
 }
 
 void fillGramLaunch(xb_ctx* c, int si, const int* dList, int nList, int imgConv, double* G,
@@ -423,7 +457,16 @@ void fillGramLaunch(xb_ctx* c, int si, const int* dList, int nList, int imgConv,
   const Basis& bs = c->basis;
   StampSetDev& S = c->set[si];
   const int nGroups = (int)bs.yGroupStart.size() - 1;
-  const FgLayout L = fgLayout(g.hSS, g.hK, nGroups, g.nPSF);
+  int optin = 0;
+  XB_CUDA(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, c->device));
+  // A refill's few stamps (its bound is not: the count is on the device) and short
+  // lists leave most SMs idle: four CTAs share each of them.  Four stamps take 76
+  // us so and 240 us on a CTA each; 256 stamps 556 and 437 us, so up to half an
+  // SM count of stamps, where four waves of the first meet the second, are split.
+  const bool split = ((liveN && liveN != S.dN) || nList * 2 <= c->smCount) &&
+                     fgLayout(g.hSS, g.hK, nGroups, g.nPSF, FG_CL).total + 8 * 1024 <= (size_t)optin;
+  const int cl = split ? FG_CL : 1, perPass = fgPerPass(cl);
+  const FgLayout L = fgLayout(g.hSS, g.hK, nGroups, g.nPSF, cl);
   FillGramArgs a{};
   a.conv = (const float*)c->img[imgConv];
   a.other = (const float*)c->img[1 - imgConv];
@@ -458,16 +501,16 @@ void fillGramLaunch(xb_ctx* c, int si, const int* dList, int nList, int imgConv,
   order.push_back(groupOf[0]);
   for(int gi = 0; gi < nGroups; gi++)
     if(gi != groupOf[0]) order.push_back(gi);
-  a.nPass = (nGroups + FG_GP - 1) / FG_GP;
+  a.nPass = (nGroups + perPass - 1) / perPass;
   int nr = 0;
   for(int p = 0; p < a.nPass; p++) {
-    a.gBeg[p] = p * FG_GP;
+    a.gBeg[p] = p * perPass;
     a.rBeg[p] = nr;
-    const int gEnd = std::min(nGroups, (p + 1) * FG_GP);
-    for(int k = p * FG_GP; k < gEnd; k++) {
+    const int gEnd = std::min(nGroups, (p + 1) * perPass);
+    for(int k = p * perPass; k < gEnd; k++) {
       const int gi = order[k];
       a.gOrder[k] = (unsigned char)gi;
-      a.slot[gi] = (unsigned char)(k - p * FG_GP);
+      a.slot[gi] = (unsigned char)(k - p * perPass);
       for(int m = bs.yGroupStart[gi]; m < bs.yGroupStart[gi + 1]; m++)
         if(bs.yGroupMembers[m] != 0) a.rows[nr++] = (unsigned char)bs.yGroupMembers[m];
     }
@@ -476,7 +519,7 @@ void fillGramLaunch(xb_ctx* c, int si, const int* dList, int nList, int imgConv,
   a.rBeg[a.nPass] = nr;
   for(int n = 0; n < g.nPSF; n++) a.groupOf[n] = (unsigned char)groupOf[n];
   // the window's tile copy: rows of the frame in 16-byte multiples, box
-  // ldWin x tw floats (its x start is rounded down to 4 floats in the kernel)
+  // ldWin x th floats (its x start is rounded down to 4 floats in the kernel)
   CUtensorMap tm;
   memset(&tm, 0, sizeof(tm));
   a.useTma = 0;
@@ -484,20 +527,37 @@ void fillGramLaunch(xb_ctx* c, int si, const int* dList, int nList, int imgConv,
   if(enc && c->w % 4 == 0 && ((uintptr_t)a.conv & 15) == 0) {
     const cuuint64_t dims[2] = {(cuuint64_t)c->w, (cuuint64_t)c->h};
     const cuuint64_t strides[1] = {(cuuint64_t)c->w * 4};
-    const cuuint32_t box[2] = {(cuuint32_t)L.ldWin, (cuuint32_t)L.tw};
+    const cuuint32_t box[2] = {(cuuint32_t)L.ldWin, (cuuint32_t)L.th};
     const cuuint32_t es[2] = {1, 1};
     if(enc(&tm, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 2, (void*)a.conv, dims, strides, box, es,
            CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE,
            CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS)
       a.useTma = c->fillGramTma;
   }
+  if(split) {
+    XB_CUDA(allowMaxDynamicSmem((const void*)k_fill_gram<FG_NTS, FG_CL>, c->device));
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(nList * FG_CL);
+    cfg.blockDim = dim3(FG_NTS);
+    cfg.dynamicSmemBytes = L.total;
+    cfg.stream = c->stream;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = FG_CL;
+    attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    XB_CUDA(cudaLaunchKernelEx(&cfg, k_fill_gram<FG_NTS, FG_CL>, tm, a));
+    XB_LAUNCHED(c);
+    return;
+  }
   // threads per CTA: 384 (variant 0) or 256; both keep two CTAs per SM and
   // give the same W and G bit for bit (every output's arithmetic is per item)
-  XB_CUDA(allowMaxDynamicSmem((const void*)k_fill_gram<384>, c->device));
-  XB_CUDA(allowMaxDynamicSmem((const void*)k_fill_gram<256>, c->device));
+  XB_CUDA(allowMaxDynamicSmem((const void*)k_fill_gram<384, 1>, c->device));
+  XB_CUDA(allowMaxDynamicSmem((const void*)k_fill_gram<256, 1>, c->device));
   auto launch = [&](int v) {
-    if(v == 1) k_fill_gram<256><<<nList, 256, L.total, c->stream>>>(tm, a);
-    else k_fill_gram<384><<<nList, 384, L.total, c->stream>>>(tm, a);
+    if(v == 1) k_fill_gram<256, 1><<<nList, 256, L.total, c->stream>>>(tm, a);
+    else k_fill_gram<384, 1><<<nList, 384, L.total, c->stream>>>(tm, a);
     XB_LAUNCHED(c);
   };
   launch(tunedVariant(c, "fill_gram", (long long)g.fSS * 100000 + g.nPSF * 100 + g.nBG, 2, launch));

@@ -437,13 +437,20 @@ __device__ __forceinline__ bool gramChunksDirect(const float* __restrict__ Ws,
                                                  const unsigned long long* stallBar = nullptr) {
   static_assert(2 * NT >= RB * (KC / 8), "two units per thread cover a chunk");
   const int tid = threadIdx.x;
-  const int nChunk = (K + KC - 1) / KC, nUnits = R * (KC / 8);
+  const int nChunk = (K + KC - 1) / KC;
+  // units: eight rows fastest, so that a warp's 16-byte operand rows fall on
+  // distinct banks (units of one row fastest put eight on the same ones) and its
+  // loads still take whole 128-byte lines; rows R..R8-1 are zeros
+  const int R8 = (R + 7) / 8 * 8, nUnits = R8 * (KC / 8);
+  auto rowOf = [](int u) { return (u >> 6) * 8 + (u & 7); };
+  auto groupOf = [](int u) { return (u >> 3) & 7; };
+  static_assert(KC / 8 == 8, "eight K groups per chunk");
   bool ok = true;
-  // rows R..RB-1 stay zero in both buffers
-  for(int u = tid; u < 2 * (RB - R) * (KC / 8); u += NT) {
-    const int bsel = u / ((RB - R) * (KC / 8)), v = u % ((RB - R) * (KC / 8));
+  // rows R8..RB-1 stay zero in both buffers
+  for(int u = tid; u < 2 * (RB - R8) * (KC / 8); u += NT) {
+    const int bsel = u / ((RB - R8) * (KC / 8)), v = u % ((RB - R8) * (KC / 8));
     const uint32_t zero[NS][4] = {};
-    storeSlices(buf + bsel * OPBUF, R + v / (KC / 8), v % (KC / 8), zero);
+    storeSlices(buf + bsel * OPBUF, R8 + v / (KC / 8), v % (KC / 8), zero);
   }
   for(int ch = 0; ch < nChunk; ch++) {
     const int b = ch & 1;
@@ -452,12 +459,12 @@ __device__ __forceinline__ bool gramChunksDirect(const float* __restrict__ Ws,
 #pragma unroll
     for(int i = 0; i < 2; i++) {
       const int u = tid + i * NT;
-      const int r = u / (KC / 8), kg = u % (KC / 8), k0 = ch * KC + kg * 8;
+      const int r = rowOf(u), kg = groupOf(u), k0 = ch * KC + kg * 8;
 #pragma unroll
       for(int e = 0; e < 8; e++) xh[i][e] = xl[i][e] = 0.f;
-      if(u < nUnits) {
+      if(u < nUnits && r < R) {
         if(r < wRows) {
-          if(k0 < ldW) {  // ldW is a multiple of 8: a unit is wholly inside or past it
+          if(k0 < K) {  // ldW is a multiple of 8, so the unit lies inside the row
             const float4* ph = (const float4*)(Ws + (size_t)r * ldW + k0);
             const float4* pl = (const float4*)(Wl + (size_t)r * ldW + k0);
             const float4 h0 = ph[0], h1 = ph[1], l0 = pl[0], l1 = pl[1];
@@ -481,10 +488,9 @@ __device__ __forceinline__ bool gramChunksDirect(const float* __restrict__ Ws,
     for(int i = 0; i < 2; i++) {
       const int u = tid + i * NT;
       if(u < nUnits) {
-        const int r = u / (KC / 8), kg = u % (KC / 8);
         uint32_t q[NS][4];
-        slice8(xh[i], xl[i], expo[r], q);
-        storeSlices(B, r, kg, q);
+        slice8(xh[i], xl[i], expo[rowOf(u)], q);
+        storeSlices(B, rowOf(u), groupOf(u), q);
       }
     }
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
@@ -509,9 +515,35 @@ __device__ __forceinline__ bool gramChunksDirect(const float* __restrict__ Ws,
 // likewise SB; every entry of G then follows from its own (a, b), and the
 // two triangles agree because A and B are symmetric exact integers.  TMEM
 // columns come four at a time.  Frees the TMEM (warp 0).
+//
+// CL > 1: the CTAs of a cluster hold the sums of their parts of K (one that
+// has none, any = false, adds nothing); they are added, exactly as every other
+// sum here, from each other's shared memory, and each CTA writes its share of G.
+// The caller keeps the cluster together after it (clusterSync).
 constexpr int EPI2_BYTES = 2 * RB * ELD * 8;
+__device__ __forceinline__ void clusterSync() {
+  asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+  asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+// the address in CTA rank's shared memory of this CTA's address a
+__device__ __forceinline__ uint32_t peerAddr(uint32_t a, int rank) {
+  uint32_t r;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(rank));
+  return r;
+}
+__device__ __forceinline__ long long peerLoad64(uint32_t a) {
+  long long v;
+  asm volatile("ld.shared::cluster.b64 %0, [%1];" : "=l"(v) : "r"(a) : "memory");
+  return v;
+}
+__device__ __forceinline__ unsigned peerLoad32(uint32_t a) {
+  unsigned v;
+  asm volatile("ld.shared::cluster.b32 %0, [%1];" : "=r"(v) : "r"(a) : "memory");
+  return v;
+}
+template <int CL>
 __device__ __forceinline__ void epilogueAtomic(uint32_t tmem, long long* sums, const int* expo,
-                                               int R, double* G) {
+                                               int R, double* G, int rank, bool any) {
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nWarps = blockDim.x >> 5;
   unsigned long long* SA = (unsigned long long*)sums;
   unsigned long long* SB = SA + RB * ELD;
@@ -521,6 +553,7 @@ __device__ __forceinline__ void epilogueAtomic(uint32_t tmem, long long* sums, c
   const int a = 32 * (q & 1) + lane;
   const int t1 = q >> 1, t2 = 2 + (q >> 1);
   const uint32_t lanes = (uint32_t)(32 * q) << 16;
+  if(any)
   for(int b0 = 4 * part; b0 < RB; b0 += 4 * nParts) {
     long long xa[4] = {0, 0, 0, 0}, xb[4] = {0, 0, 0, 0}, ya[4] = {0, 0, 0, 0},
               yb[4] = {0, 0, 0, 0};
@@ -570,10 +603,22 @@ __device__ __forceinline__ void epilogueAtomic(uint32_t tmem, long long* sums, c
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
   if(warp == 0) tmemFree512(tmem);
-  for(int e = tid; e < R * R; e += blockDim.x) {
+  if(CL > 1) clusterSync();
+  for(int e = rank * (int)blockDim.x + tid; e < R * R; e += CL * blockDim.x) {
     const int ra = e / R, rb = e % R;
-    const long long A = (long long)SA[ra * ELD + rb];
-    const long long B = (long long)SB[ra * ELD + rb];
+    long long A, B;
+    if constexpr(CL > 1) {
+      A = B = 0;
+      const uint32_t at = smemU32(&SA[ra * ELD + rb]);
+#pragma unroll
+      for(int c = 0; c < CL; c++) {
+        A += peerLoad64(peerAddr(at, c));
+        B += peerLoad64(peerAddr(at + RB * ELD * 8, c));
+      }
+    } else {
+      A = (long long)SA[ra * ELD + rb];
+      B = (long long)SB[ra * ELD + rb];
+    }
     const double v = (double)A * 0x1p28 + (double)B;
     const int ex = expo[ra] + expo[rb] - 63;
     G[e] = v * __longlong_as_double((long long)(1023 + ex) << 52);
