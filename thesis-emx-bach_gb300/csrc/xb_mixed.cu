@@ -1508,11 +1508,26 @@ __global__ void k_kernel_terms(const double* __restrict__ sol, const double* __r
 __global__ void k_border_f32(const float* __restrict__ O, int w, int h, int hK, float tH, float tL,
                              const uint8_t* __restrict__ inMask, uint16_t* __restrict__ mask, float* __restrict__ convF,
                              float* __restrict__ diffF) {
-  const long long n = (long long)w * h;
-  for(long long id = (long long)blockIdx.x * blockDim.x + threadIdx.x; id < n;
-      id += (long long)gridDim.x * blockDim.x) {
-    const int x = (int)(id % w), y = (int)(id / w);
-    if(x >= hK && x < w - hK && y >= hK && y < h - hK) continue;
+  // the border's pixels only: whole rows above and below, then both sides of
+  // the rows between
+  const int top = min(hK, h), bottom = max(h - hK, top), left = min(hK, w), right = max(w - hK, left);
+  const int side = left + w - right;
+  const long long nRows = (long long)(top + h - bottom) * w, n = nRows + (long long)(bottom - top) * side;
+  for(long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n;
+      i += (long long)gridDim.x * blockDim.x) {
+    int x, y;
+    if(i < nRows) {
+      y = (int)(i / w);
+      x = (int)(i - (long long)y * w);
+      if(y >= top) y += bottom - top;
+    } else {
+      const long long k = i - nRows;
+      y = (int)(k / side);
+      x = (int)(k - (long long)y * side);
+      if(x >= left) x += right - left;
+      y += top;
+    }
+    const size_t id = (size_t)y * w + x;
     mask[id] |= afterMaskF(O[id], tH, tL);
     if(inMask && inMask[id]) mask[id] |= INPUT_MASK | BAD_INPUT | BAD_OUTPUT;
     convF[id] = 1e-30f;
