@@ -58,7 +58,7 @@ constexpr int FG_R8 = 8;    // outputs per thread item (rows of the Y pass, pixe
 constexpr int FG_GP = 7;    // Y filters per pass
 constexpr int FG_MAXPASS = 4;
 constexpr int FG_MAXG = FG_MAXPASS * FG_GP;
-constexpr int FG_CL = 4, FG_NTS = 512;  // CTAs and threads for a stamp of a short list
+constexpr int FG_CL = 4;  // CTAs for a stamp of a short list
 
 // Shared-memory layout of the fill (steps 1-3) for a CTA's nr output rows; the
 // Gram (step 4) and the epilogue reuse the same area from offset 0.
@@ -534,21 +534,28 @@ void fillGramLaunch(xb_ctx* c, int si, const int* dList, int nList, int imgConv,
            CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS)
       a.useTma = c->fillGramTma;
   }
+  const long long shape = (long long)g.fSS * 100000 + g.nPSF * 100 + g.nBG;
   if(split) {
-    XB_CUDA(allowMaxDynamicSmem((const void*)k_fill_gram<FG_NTS, FG_CL>, c->device));
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(nList * FG_CL);
-    cfg.blockDim = dim3(FG_NTS);
-    cfg.dynamicSmemBytes = L.total;
-    cfg.stream = c->stream;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeClusterDimension;
-    attr[0].val.clusterDim.x = FG_CL;
-    attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = 1;
-    XB_CUDA(cudaLaunchKernelEx(&cfg, k_fill_gram<FG_NTS, FG_CL>, tm, a));
-    XB_LAUNCHED(c);
+    // threads per CTA: 512 (variant 0) or 256
+    XB_CUDA(allowMaxDynamicSmem((const void*)k_fill_gram<512, FG_CL>, c->device));
+    XB_CUDA(allowMaxDynamicSmem((const void*)k_fill_gram<256, FG_CL>, c->device));
+    auto launch = [&](int v) {
+      cudaLaunchConfig_t cfg = {};
+      cfg.gridDim = dim3(nList * FG_CL);
+      cfg.blockDim = dim3(v == 1 ? 256 : 512);
+      cfg.dynamicSmemBytes = L.total;
+      cfg.stream = c->stream;
+      cudaLaunchAttribute attr[1];
+      attr[0].id = cudaLaunchAttributeClusterDimension;
+      attr[0].val.clusterDim.x = FG_CL;
+      attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+      cfg.attrs = attr;
+      cfg.numAttrs = 1;
+      if(v == 1) XB_CUDA(cudaLaunchKernelEx(&cfg, k_fill_gram<256, FG_CL>, tm, a));
+      else XB_CUDA(cudaLaunchKernelEx(&cfg, k_fill_gram<512, FG_CL>, tm, a));
+      XB_LAUNCHED(c);
+    };
+    launch(tunedVariant(c, "fill_gram", FG_CL * 1000000000ll + shape, 2, launch));
     return;
   }
   // threads per CTA: 384 (variant 0) or 256; both keep two CTAs per SM and
@@ -560,7 +567,7 @@ void fillGramLaunch(xb_ctx* c, int si, const int* dList, int nList, int imgConv,
     else k_fill_gram<384, 1><<<nList, 384, L.total, c->stream>>>(tm, a);
     XB_LAUNCHED(c);
   };
-  launch(tunedVariant(c, "fill_gram", (long long)g.fSS * 100000 + g.nPSF * 100 + g.nBG, 2, launch));
+  launch(tunedVariant(c, "fill_gram", shape, 2, launch));
 }
 
 }  // namespace xb
