@@ -202,6 +202,9 @@ int xb_ctx_destroy(xb_ctx* c) {
   for(auto& kv : c->pool)
     if(kv.second.p) cudaFree(kv.second.p);
   if(c->stream) cudaStreamDestroy(c->stream);
+  if(c->sideStream) cudaStreamDestroy(c->sideStream);
+  if(c->sideFork) cudaEventDestroy(c->sideFork);
+  if(c->sideJoin) cudaEventDestroy(c->sideJoin);
   delete c;
   return XB_OK;
 }

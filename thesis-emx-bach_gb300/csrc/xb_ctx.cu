@@ -172,6 +172,39 @@ void* poolGet(xb_ctx* c, const char* name, size_t bytes) {
   return p;
 }
 
+SideWork::SideWork(xb_ctx* c) : c_(c), main_(c->stream) {
+  if(!c->sideStream) XB_CUDA(cudaStreamCreateWithFlags(&c->sideStream, cudaStreamNonBlocking));
+  if(!c->sideFork) XB_CUDA(cudaEventCreateWithFlags(&c->sideFork, cudaEventDisableTiming));
+  if(!c->sideJoin) XB_CUDA(cudaEventCreateWithFlags(&c->sideJoin, cudaEventDisableTiming));
+  XB_CUDA(cudaEventRecord(c->sideFork, main_));
+}
+void SideWork::enter() {
+  XB_CUDA(cudaStreamWaitEvent(c_->sideStream, c_->sideFork, 0));
+  c_->stream = c_->sideStream;
+  c_->lane = 1;
+  in_ = used_ = true;
+}
+void SideWork::leave() {
+  c_->stream = main_;
+  c_->lane = 0;
+  in_ = false;
+}
+void SideWork::join() {
+  if(in_) leave();
+  if(used_ && !joined_) {
+    joined_ = true;
+    XB_CUDA(cudaEventRecord(c_->sideJoin, c_->sideStream));
+    XB_CUDA(cudaStreamWaitEvent(main_, c_->sideJoin, 0));
+  }
+}
+SideWork::~SideWork() {
+  if(in_) leave();
+  if(used_ && !joined_) {  // an error on the way: the main stream still waits
+    cudaEventRecord(c_->sideJoin, c_->sideStream);
+    cudaStreamWaitEvent(main_, c_->sideJoin, 0);
+  }
+}
+
 cudaEvent_t ktEvent(xb_ctx* c) {
   if(!c->kt.pool.empty()) {
     cudaEvent_t e = c->kt.pool.back();

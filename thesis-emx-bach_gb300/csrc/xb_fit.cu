@@ -1097,18 +1097,18 @@ static FitBuffers fitBuffers(xb_ctx* c, int nMax) {
   const Geo& g = c->g;
   FitBuffers f{};
   const int ld = g.matSize + 1;
-  f.list = buf<int>(c, "fit_list", std::max(nMax, 1));
-  f.wts = buf<double>(c, "fit_wts", mixedMode(c) ? 1 : (size_t)std::max(nMax, 1) * (g.nComp2 + 1) * (g.nComp2 + 1));
+  f.list = buf<int>(c, laneName(c, "fit_list", "fit_list_side"), std::max(nMax, 1));
+  f.wts = buf<double>(c, laneName(c, "fit_wts", "fit_wts_side"), mixedMode(c) ? 1 : (size_t)std::max(nMax, 1) * (g.nComp2 + 1) * (g.nComp2 + 1));
   f.stride = plainDotStride(g);
-  f.M = buf<double>(c, "fit_M", (size_t)ld * ld);
-  f.rhs = buf<double>(c, "fit_rhs", std::max(g.nSol, ld));
-  f.piv = buf<int>(c, "fit_piv", ld);
-  f.singular = buf<int>(c, "fit_singular", 1);
-  f.sig = buf<double>(c, "fit_sig", std::max(nMax, 1));
-  f.scratchD = buf<double>(c, "fit_clipdata", std::max(nMax, 1));
-  f.flags = buf<uint8_t>(c, "fit_flags", 2 * std::max(nMax, 1));  // cd clips both sets at once
-  f.cs = buf<double>(c, "fit_cs", 2 * std::max(nMax, 1));
-  f.cs2 = buf<double>(c, "fit_cs2", 2 * std::max(nMax, 1));
+  f.M = buf<double>(c, laneName(c, "fit_M", "fit_M_side"), (size_t)ld * ld);
+  f.rhs = buf<double>(c, laneName(c, "fit_rhs", "fit_rhs_side"), std::max(g.nSol, ld));
+  f.piv = buf<int>(c, laneName(c, "fit_piv", "fit_piv_side"), ld);
+  f.singular = buf<int>(c, laneName(c, "fit_singular", "fit_singular_side"), 1);
+  f.sig = buf<double>(c, laneName(c, "fit_sig", "fit_sig_side"), std::max(nMax, 1));
+  f.scratchD = buf<double>(c, laneName(c, "fit_clipdata", "fit_clipdata_side"), std::max(nMax, 1));
+  f.flags = buf<uint8_t>(c, laneName(c, "fit_flags", "fit_flags_side"), 2 * std::max(nMax, 1));  // cd clips both sets at once
+  f.cs = buf<double>(c, laneName(c, "fit_cs", "fit_cs_side"), 2 * std::max(nMax, 1));
+  f.cs2 = buf<double>(c, laneName(c, "fit_cs2", "fit_cs2_side"), 2 * std::max(nMax, 1));
   return f;
 }
 
@@ -1116,7 +1116,7 @@ static int2* kernelPowers(xb_ctx* c) {
   const Geo& g = c->g;
   std::vector<int2> kp(g.nComp2);
   for(int k = 0; k < g.nComp2; k++) kp[k] = make_int2(c->basis.kpX[k], c->basis.kpY[k]);
-  int2* d = buf<int2>(c, "kernelPowers", g.nComp2);
+  int2* d = buf<int2>(c, laneName(c, "kernelPowers", "kernelPowers_side"), g.nComp2);
   toDevice(c, d, kp);
   return d;
 }
@@ -1308,6 +1308,17 @@ static void cdTestStamps(xb_ctx* c, const FitBuffers& f, int nMax, double* const
   XB_LAUNCHED(c);
 }
 
+// What the fits of both sets read and one of them would fill in first.
+static void cdTables(xb_ctx* c) {
+  if(!mixedMode(c)) return;
+  mixedTables(c);
+  deviceStatus(c);
+}
+
+// The two sets' global test fits are chains of small kernels on a few SMs each
+// (the mixed solve takes 16), so they run side by side: one fit's time less
+// (0.4 ms of a 2048 x 2048 mixed frame's 5.2, 3.5 ms of a plain 437 x 611 one's
+// 16.9).
 void stageCd(xb_ctx* c) {
   const Geo& g = c->g;
   const int nMax = std::max(std::max(c->set[0].n, c->set[1].n), 1);
@@ -1322,29 +1333,40 @@ void stageCd(xb_ctx* c) {
   cdTestStamps(c, f, nMax, ks, testIdx, nTest, stats, false);
   std::vector<int> hT = toHost(c, nTest, 2);
   const int solStride = std::max(g.nSol, g.matSize + 1);
-  for(int si = 0; si < 2; si++) {
+  FitBuffers fb[2] = {f, f};
+  auto fit = [&](int si) {  // the global test fit of set si up to its merit
     double* sol = dSolCd + (size_t)si * solStride;
-    if(c->trace) c->put("kernel_sums" + std::to_string(si), toHost(c, ks[si], c->set[si].n));
-    if(hT[si] == 0) {
-      c->merit[si] = 666;
-      continue;
-    }
-    solveGlobal(c, si, f, testIdx[si], hT[si], nullptr, 1 - si, false, sol);
+    solveGlobal(c, si, fb[si], testIdx[si], hT[si], nullptr, 1 - si, false, sol);
     kernelSumLaunch(c, sol, (0 - 0.5 * c->w) / (0.5 * c->w), (0 - 0.5 * c->h) / (0.5 * c->h), 1,
                     kMean + si);
-    computeSigs(c, si, testIdx[si], hT[si], sol, si, f.sig);
-    { KT_SCOPE(c, "cd_merit");
-    k_cd_merit<<<1, 256, 0, c->stream>>>(f.sig, hT[si], nullptr, kMean + si, c->p.sigClipAlpha,
-                                         f.scratchD, f.flags, f.cs, f.cs2, merit + si);
+    computeSigs(c, si, testIdx[si], hT[si], sol, si, fb[si].sig);
+    KT_SCOPE(c, "cd_merit");
+    k_cd_merit<<<1, 256, 0, c->stream>>>(fb[si].sig, hT[si], nullptr, kMean + si,
+                                         c->p.sigClipAlpha, fb[si].scratchD, fb[si].flags, fb[si].cs,
+                                         fb[si].cs2, merit + si);
     XB_LAUNCHED(c);
-    }
-    std::vector<double> m = toHost(c, merit + si, 1);
-    c->merit[si] = m[0];
-    if(c->trace) {
+  };
+  if(hT[0] > 0 && hT[1] > 0) {
+    cdTables(c);
+    SideWork side(c);
+    side.enter();
+    fb[1] = fitBuffers(c, nMax);
+    fit(1);
+    side.leave();
+    fit(0);
+    side.join();
+  } else {
+    for(int si = 0; si < 2; si++)
+      if(hT[si] > 0) fit(si);
+  }
+  for(int si = 0; si < 2; si++) {
+    if(c->trace) c->put("kernel_sums" + std::to_string(si), toHost(c, ks[si], c->set[si].n));
+    c->merit[si] = hT[si] > 0 ? toHost(c, merit + si, 1)[0] : 666;
+    if(c->trace && hT[si] > 0) {
       const std::string sfx = std::to_string(si);
       c->put("cd_test" + sfx, toHost(c, testIdx[si], hT[si]));
-      c->put("cd_solution" + sfx, toHost(c, sol, g.nSol));
-      c->put("cd_sig" + sfx, toHost(c, f.sig, hT[si]));
+      c->put("cd_solution" + sfx, toHost(c, dSolCd + (size_t)si * solStride, g.nSol));
+      c->put("cd_sig" + sfx, toHost(c, fb[si].sig, hT[si]));
       c->scalars["cd_kernel_mean" + sfx] = toHost(c, kMean + si, 1)[0];
     }
   }
@@ -1433,21 +1455,30 @@ void stageCdGraph(xb_ctx* c, long long lCd[2]) {
   double* merit = buf<double>(c, "cd_merit", 2);
   cdTestStamps(c, f, nMax, ks, testIdx, nTest, stats, true);
   const int solStride = std::max(g.nSol, g.matSize + 1);
-  for(int si = 0; si < 2; si++) {
+  FitBuffers fb[2] = {f, f};
+  auto fit = [&](int si) {
     double* sol = dSolCd + (size_t)si * solStride;
     const int bound = c->set[si].n;
     graphSetDouble(c, merit + si, 666.0);
     lCd[si] = graphIfPositive(c, nTest + si, 1, [&] {
-      solveGlobal(c, si, f, testIdx[si], bound, nTest + si, 1 - si, false, sol);
+      solveGlobal(c, si, fb[si], testIdx[si], bound, nTest + si, 1 - si, false, sol);
       kernelSumLaunch(c, sol, (0 - 0.5 * c->w) / (0.5 * c->w), (0 - 0.5 * c->h) / (0.5 * c->h), 1,
                       kMean + si);
-      computeSigs(c, si, testIdx[si], bound, sol, si, f.sig, nTest + si);
-      k_cd_merit<<<1, 256, 0, c->stream>>>(f.sig, bound, nTest + si, kMean + si,
-                                           c->p.sigClipAlpha, f.scratchD, f.flags, f.cs, f.cs2,
-                                           merit + si);
+      computeSigs(c, si, testIdx[si], bound, sol, si, fb[si].sig, nTest + si);
+      k_cd_merit<<<1, 256, 0, c->stream>>>(fb[si].sig, bound, nTest + si, kMean + si,
+                                           c->p.sigClipAlpha, fb[si].scratchD, fb[si].flags,
+                                           fb[si].cs, fb[si].cs2, merit + si);
       XB_LAUNCHED(c);
     });
-  }
+  };
+  cdTables(c);
+  SideWork side(c);
+  side.enter();
+  fb[1] = fitBuffers(c, nMax);
+  fit(1);
+  side.leave();
+  fit(0);
+  side.join();
 }
 
 // ksc as a frame graph captures it: the reject-and-refit loop is a WHILE

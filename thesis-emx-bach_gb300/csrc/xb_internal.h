@@ -112,6 +112,11 @@ struct xb_ctx {
   int device = 0;
   int smCount = 0;
   cudaStream_t stream = nullptr;
+  // a second stream for work beside the first one's (SideWork), with buffers of
+  // its own where both write: lane is 1 while launches go there
+  cudaStream_t sideStream = nullptr;
+  cudaEvent_t sideFork = nullptr, sideJoin = nullptr;
+  int lane = 0;
   int w = 0, h = 0;
   int imgIsF64 = 0;
   void* img[2] = {nullptr, nullptr};
@@ -323,6 +328,7 @@ void convSubMixed(xb_ctx* c, double* dKernSum);
 // (xf, yf) is sum_t xf^i yf^j Kt[t], t over the (i, j) of the kernel
 // polynomial, x power outer.
 double* kernelTermsLaunch(xb_ctx* c);
+void mixedTables(xb_ctx* c);  // the build's tables (uploaded once per context)
 void buildSystemMixed(xb_ctx* c, int si, const int* dList, int nList, int bgBase, double* M,
                       double* rhs, const int* liveN = nullptr);
 
@@ -330,12 +336,34 @@ void buildSystemMixed(xb_ctx* c, int si, const int* dList, int nList, int bgBase
 // solve, pivoted LU when a pivot fails.  M is kept; rhs becomes the solution.
 void globalSolveMixed(xb_ctx* c, const double* M, int n, double* rhs, int* piv, int* singular);
 // Device status words of the mixed path: [0] bit 0 = an LDL^T pivot failed
-// (per solve), [1] bit 0 = a bounded device-side wait ran out (sticky until
-// checkSolveTimeout reports it).  Zeroed when first allocated.
+// (per solve; [2] for a solve on the side stream), [1] bit 0 = a bounded
+// device-side wait ran out (sticky until checkSolveTimeout reports it).  Zeroed
+// when first allocated.
 int* deviceStatus(xb_ctx* c);
 // Throws XB_ERR_DEVICE_TIMEOUT when a bounded wait of the cluster solve or
 // the tensor-core Gram ran out since the last call (synchronises the stream).
 void checkSolveTimeout(xb_ctx* c);
+// Work beside the context stream's: between enter() and leave() launches go to
+// the side stream, after everything issued before the object was made; join()
+// (at the latest its end) makes the context stream wait for them.  Captures
+// into a graph as parallel branches.
+class SideWork {
+ public:
+  explicit SideWork(xb_ctx* c);
+  ~SideWork();
+  void enter();
+  void leave();
+  void join();
+
+ private:
+  xb_ctx* c_;
+  cudaStream_t main_;
+  bool in_ = false, used_ = false, joined_ = false;
+};
+// The name of a buffer that both lanes write.
+inline const char* laneName(const xb_ctx* c, const char* first, const char* side) {
+  return c->lane ? side : first;
+}
 // Autotuner (xb_tune.cpp): the variant of a tunable kernel to launch for
 // (kernel, device, shape); times all nVariants through `launch` on first use.
 int tunedVariant(xb_ctx* c, const char* kernel, long long shape, int nVariants,

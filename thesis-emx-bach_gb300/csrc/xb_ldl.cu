@@ -567,25 +567,25 @@ cudaError_t launchCluster(xb_ctx* c, Kern kernel, int CL, int threads, size_t sm
 
 int* deviceStatus(xb_ctx* c) {
   const bool fresh = c->pool.find("ldl_status") == c->pool.end();
-  int* status = buf<int>(c, "ldl_status", 2);
+  int* status = buf<int>(c, "ldl_status", 3);
   if(fresh) {
-    const int zero[2] = {0, 0};
+    const int zero[3] = {0, 0, 0};
     if(c->capturing) uploadNow(c, status, zero, sizeof(zero));
-    else XB_CUDA(cudaMemsetAsync(status, 0, 2 * sizeof(int), c->stream));
+    else XB_CUDA(cudaMemsetAsync(status, 0, 3 * sizeof(int), c->stream));
   }
   return status;
 }
 
 void globalSolveMixed(xb_ctx* c, const double* M, int n, double* rhs, int* piv, int* singular) {
   const int ld = n + 1;
-  int* status = deviceStatus(c);
+  int* status = deviceStatus(c) + (c->lane ? 2 : 0);
   XB_CUDA(cudaMemsetAsync(status, 0, sizeof(int), c->stream));
   // 16-CTA clusters where the device allows them and the context asks for
   // them, else 8 (the same bits)
   static std::atomic<int> clusterSize{0};
   {
     KT_SCOPE(c, "global_ldl");
-    double* Yg = buf<double>(c, "ldl_y", (size_t)(LS_P + 1) * lsLayout(n, 16).nPad);
+    double* Yg = buf<double>(c, laneName(c, "ldl_y", "ldl_y_side"), (size_t)(LS_P + 1) * lsLayout(n, 16).nPad);
     auto launch = [&](auto kernel, int CL) -> cudaError_t {
       const LsLayout lay = lsLayout(n, CL);
       if(lay.nr + 1 > LS_OWN) return cudaErrorInvalidConfiguration;
@@ -604,7 +604,7 @@ void globalSolveMixed(xb_ctx* c, const double* M, int n, double* rhs, int* piv, 
     }
     XB_LAUNCHED(c);
   }
-  luFallbackSolve(c, M, buf<double>(c, "ldl_F", (size_t)ld * ld), n, rhs, piv, singular, status);
+  luFallbackSolve(c, M, buf<double>(c, laneName(c, "ldl_F", "ldl_F_side"), (size_t)ld * ld), n, rhs, piv, singular, status);
 }
 
 void checkSolveTimeout(xb_ctx* c) {

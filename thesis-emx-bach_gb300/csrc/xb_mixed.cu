@@ -1903,16 +1903,9 @@ void luFallbackSolve(xb_ctx* c, const double* M, double* F, int n, double* rhs, 
   }
 }
 
-// Global matrix and RHS of the mixed path for the stamps list[0..nList) of
-// set si (weights from the current substamps, W dots per stamp).
-void buildSystemMixed(xb_ctx* c, int si, const int* dList, int nList, int bgBase, double* M,
-                      double* rhs, const int* liveN) {
+void mixedTables(xb_ctx* c) {
   const Geo& g = c->g;
-  StampSetDev& S = c->set[si];
-  const int K = c->p.kernelOrder, monoDim = 2 * K + 1;
-  const int nMono = triNum(2 * K + 1);
-  if(nMono + 1 > MXB_MAXC)
-    throw XbError{XB_ERR_UNSUPPORTED, "kernel order too high for the mixed build"};
+  const int K = c->p.kernelOrder, monoDim = 2 * K + 1, nMono = triNum(2 * K + 1);
   // monomial exponents, their index table and the kernel powers: fixed by
   // the parameters, uploaded once per context
   int2* dExp = buf<int2>(c, "mx_exp", nMono);
@@ -1933,14 +1926,30 @@ void buildSystemMixed(xb_ctx* c, int si, const int* dList, int nList, int bgBase
     toDevice(c, dKp, kp);
     c->mxTables = 1;
   }
+}
+
+// Global matrix and RHS of the mixed path for the stamps list[0..nList) of
+// set si (weights from the current substamps, W dots per stamp).
+void buildSystemMixed(xb_ctx* c, int si, const int* dList, int nList, int bgBase, double* M,
+                      double* rhs, const int* liveN) {
+  const Geo& g = c->g;
+  StampSetDev& S = c->set[si];
+  const int K = c->p.kernelOrder, monoDim = 2 * K + 1;
+  const int nMono = triNum(2 * K + 1);
+  if(nMono + 1 > MXB_MAXC)
+    throw XbError{XB_ERR_UNSUPPORTED, "kernel order too high for the mixed build"};
+  mixedTables(c);
+  int2* dExp = buf<int2>(c, "mx_exp", nMono);
+  int* dIdx = buf<int>(c, "mx_idx", (size_t)monoDim * monoDim);
+  int2* dKp = buf<int2>(c, "mx_kp", g.nComp2);
   const int stride = mixedDotStride(g);
   const int nQP = (g.nComp1 + 1) * (g.nComp1 + 2) / 2 - 1;
   const int nRows = nQP + 1 + stride + g.nComp1 + 1;
   const int nSplit = (nList + MXB_T - 1) / MXB_T;
-  double* P = buf<double>(c, "mx_partials", (size_t)std::max(nSplit, 1) * nRows * (nMono + 1));
+  double* P = buf<double>(c, laneName(c, "mx_partials", "mx_partials_side"), (size_t)std::max(nSplit, 1) * nRows * (nMono + 1));
   if(nSplit > 0) {
     KT_SCOPE(c, "mx_build");
-    float2* Ytab = buf<float2>(c, "mx_mono", (size_t)nList * (nMono + 1));
+    float2* Ytab = buf<float2>(c, laneName(c, "mx_mono", "mx_mono_side"), (size_t)nList * (nMono + 1));
     k_mx_mono<<<std::min((nList * (nMono + 1) + 255) / 256, c->smCount * 4), 256, 0, c->stream>>>(
         dList, nList, liveN, S.count, S.cur, S.ssxy, g.maxSS, dExp, nMono, c->w, c->h, Ytab);
     XB_LAUNCHED(c);
