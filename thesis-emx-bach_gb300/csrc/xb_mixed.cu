@@ -712,6 +712,15 @@ __global__ void __launch_bounds__(1024)
 // kernel rows (broadcast float4 reads), 441 FMAs per 27 + 18 shared loads.
 // BX (4, 6 or 8) is chosen by the autotuner; the three give identical
 // images.
+//
+// Bound by FP32: 441 FMAs a pixel of three registers each, which issue at 0.7 of
+// the rate (0.3 ms at 4096^2), beside the halo's loads, the kernels' FP64 terms
+// and the output.  The tile comes a row per warp with its bad bits from the same
+// registers, the background is a polynomial in y per column, and seven rows of
+// the other image are loaded ahead; 72 to 75 registers keep 24 to 28 warps on an
+// SM.  4096^2 with BX = 4, 6, 8: 0.58, 0.52, 0.57 ms (0.70 ms with BX = 4 and a
+// division per tile pixel, ballots from shared memory, all background terms and
+// one load per row; 0.65, 0.57, 0.74 ms at 121 registers).
 struct ConvArgsF {
   int w, h, hK, fK, nPSF, kOrder, bgOrder, nComp, scaleConv;
   float tH, tL;
@@ -756,7 +765,8 @@ template <int FK, int BX>
 struct ConvTileF {
   static constexpr int HK = FK / 2, NK = FK * FK, PX = 7, RY = 3;
   static constexpr int TPB = (FK / PX) * (FK / RY);  // threads per kernel block
-  static constexpr int NT = BX * TPB;
+  static constexpr int RW = BX * TPB;                // threads with a tile = output columns
+  static constexpr int NT = (RW + 31) / 32 * 32;     // and the lanes that fill the last warp
   static constexpr int TW = BX * FK + 2 * HK, TH = FK + 2 * HK;
   static constexpr int S = TW + (BX == 2 ? 13 : BX == 4 ? 3 : BX == 6 ? 25 : 15);
   static constexpr int NW = (TW + 31) / 32 + 1;  // bad-flag words per tile row (+1: 64-bit reads)
@@ -807,7 +817,7 @@ __device__ __forceinline__ void convBlockKernels(const double* __restrict__ Kt,
 // The rounding order of each output is the reference's tap order: over
 // kernel rows jj, then columns ii, one FP32 FMA per tap.
 template <int FK, int BX>
-__global__ void __launch_bounds__(BX * 21, BX == 8 ? 2 : 1)
+__global__ void __launch_bounds__(ConvTileF<FK, BX>::NT, BX == 4 ? 7 : BX == 6 ? 6 : 4)
     k_conv_sub_f32(const float* __restrict__ I, const float* __restrict__ O,
                    const double* __restrict__ sol, const double* __restrict__ Kt,
                    const double* __restrict__ blockXY, const double* __restrict__ kernSumPtr,
@@ -817,7 +827,7 @@ __global__ void __launch_bounds__(BX * 21, BX == 8 ? 2 : 1)
   using L = ConvTileF<FK, BX>;
   static_assert(FK % L::PX == 0 && FK % L::RY == 0 && L::TPB == 21, "tiling");
   constexpr int HK = L::HK, NK = L::NK, S = L::S, TW = L::TW, TH = L::TH, NW = L::NW, KS = L::KS;
-  constexpr int NT = L::NT, NFULL = NT / 32;  // full warps (ballots, |k| sums)
+  constexpr int NT = L::NT, RW = L::RW, NWARP = NT / 32;
   extern __shared__ __align__(16) unsigned char cv_smem[];
   float* tile = (float*)cv_smem;
   float* kern = (float*)(cv_smem + L::OFF_KERN);
@@ -828,10 +838,38 @@ __global__ void __launch_bounds__(BX * 21, BX == 8 ? 2 : 1)
   const int xB0 = blockIdx.x * BX, yB = blockIdx.y;
   const int x0 = xB0 * FK, y0 = yB * FK;  // tile origin; block pixels start at +HK
   const int K = a.kOrder;
-  for(int i = tid; i < TH * TW; i += NT) {
-    const int ly = i / TW, lx = i - ly * TW;
-    const int gx = min(x0 + lx, a.w - 1), gy = min(y0 + ly, a.h - 1);
-    tile[ly * S + lx] = I[(size_t)gx + (size_t)gy * a.w];
+  // the tile, a row per warp (two in flight), and its bad-input flags as bits
+  // (word c/32 of a row, bit c%32; the last word of a row is zero)
+  for(int l0 = warp; l0 < TH; l0 += 2 * NWARP) {
+    float v[2][NW - 1];
+    bool bd[2][NW - 1];
+#pragma unroll
+    for(int u = 0; u < 2; u++) {
+      const size_t row = (size_t)min(y0 + l0 + u * NWARP, a.h - 1) * a.w;
+#pragma unroll
+      for(int wc = 0; wc < NW - 1; wc++) {
+        const int c = wc * 32 + lane;
+        const size_t id = row + min(x0 + c, a.w - 1);
+        const bool in = c < TW && l0 + u * NWARP < TH;
+        v[u][wc] = in ? I[id] : 0.f;
+        bd[u][wc] = in && inMask && inMask[id];
+      }
+    }
+#pragma unroll
+    for(int u = 0; u < 2; u++) {
+      const int ly = l0 + u * NWARP;
+      if(ly >= TH) break;
+#pragma unroll
+      for(int wc = 0; wc < NW - 1; wc++) {
+        const int c = wc * 32 + lane;
+        const float f = v[u][wc];
+        if(c < TW) tile[ly * S + c] = f;
+        const bool bad = bd[u][wc] || f == 0.f || f >= a.tH || f <= a.tL;
+        const unsigned m = __ballot_sync(0xffffffffu, c < TW && bad);
+        if(lane == 0) bits[ly * NW + wc] = m;
+      }
+      if(lane == 0) bits[ly * NW + NW - 1] = 0u;
+    }
   }
   // kernel of each block (conv(), src/bach.cpp:339-350)
   {
@@ -844,37 +882,19 @@ __global__ void __launch_bounds__(BX * 21, BX == 8 ? 2 : 1)
     }
   }
   __syncthreads();
-  if(warp < NFULL) {
-    // bad-input flags of the tile as bits (word c/32 of a row, bit c%32; the
-    // last word of a row is zero), one row per warp at a time
-    for(int ly = warp; ly < TH; ly += NFULL) {
-      const int gy = min(y0 + ly, a.h - 1);
+  // sum of |k| of each block: lane-strided partial sums, then a butterfly
+  for(int b = warp; b < BX; b += NWARP) {
+    float s = 0.f;
+    for(int p = lane; p < NK; p += 32) s += fabsf(kern[(b * FK + p / FK) * KS + p % FK]);
 #pragma unroll
-      for(int wc = 0; wc < NW; wc++) {
-        const int c = wc * 32 + lane;
-        bool bd = false;
-        if(c < TW) {
-          bd = convMaskF(tile[ly * S + c], a.tH, a.tL) & BAD_INPUT;
-          if(inMask) bd |= inMask[(size_t)min(x0 + c, a.w - 1) + (size_t)gy * a.w] != 0;
-        }
-        const unsigned m = __ballot_sync(0xffffffffu, bd);
-        if(lane == 0) bits[ly * NW + wc] = m;
-      }
-    }
-    // sum of |k| of each block: lane-strided partial sums, then a butterfly
-    for(int b = warp; b < BX; b += NFULL) {
-      float s = 0.f;
-      for(int p = lane; p < NK; p += 32) s += fabsf(kern[(b * FK + p / FK) * KS + p % FK]);
-#pragma unroll
-      for(int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-      if(lane == 0) aks[b] = s;
-    }
+    for(int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+    if(lane == 0) aks[b] = s;
   }
   const int nBgC = (a.bgOrder + 1) * (a.bgOrder + 2) / 2;
   if(tid < nBgC) bgc[tid] = (float)sol[a.nComp + 2 + tid];
-  __syncthreads();
   // thread -> (block b, column group k, row group g): 7 columns x 3 rows
-  const int b = tid / L::TPB, r = tid - b * L::TPB, kq = r / 7, g = r - kq * 7;
+  // (the lanes beyond the last tile repeat it and store nothing)
+  const int ct = min(tid, RW - 1), b = ct / L::TPB, r = ct - b * L::TPB, kq = r / 7, g = r - kq * 7;
   const int ly0 = L::RY * g, lx0 = b * FK + L::PX * kq;
   const float* kb = kern + b * FK * KS;
   float acc[3][7];
@@ -948,7 +968,7 @@ __global__ void __launch_bounds__(BX * 21, BX == 8 ? 2 : 1)
   __syncthreads();  // every thread is done with the kernel rows
   float* sv = kern;  // conv sums of the CTA's pixels, row-major (FK rows x BX*FK)
   unsigned char* cflag = cv_smem + L::OFF_FLAG;  // 0: window clean, 1: OK_CONV, 2: BAD_CONV
-  constexpr int RW = BX * FK;
+  if(tid < RW)
 #pragma unroll
   for(int o = 0; o < 3; o++)
 #pragma unroll
@@ -968,42 +988,62 @@ __global__ void __launch_bounds__(BX * 21, BX == 8 ? 2 : 1)
   const float invKernMult = a.scaleConv ? 1.f / kernSum : 1.f;
   const float convFactor = a.scaleConv ? kernSum : 1.f;
   const float finalFactor = a.scaleConv ? -(1.f / kernSum) : 1.f;
-  static_assert(NT == RW, "one output column per thread");
+  static_assert(RW == BX * FK, "one output column per thread");
   const int x = x0 + HK + tid;
-  if(x >= a.w - HK) return;
+  if(tid >= RW || x >= a.w - HK) return;
   // background polynomial (getBackground, cd.cl:444-467) in FP32: the terms
-  // are O(1e3) ADU, so FP32 rounding moves a pixel by ~1e-4 ADU
+  // are O(1e3) ADU, so FP32 rounding moves a pixel by ~1e-4 ADU; this column's
+  // polynomial in y first, then Horner per pixel
   const float bxf = ((float)x - hxF) * ihxF;
-  for(int ly = 0; ly < FK; ly++) {
-    const int y = y0 + HK + ly;
-    if(y >= a.h - HK) break;
-    const int e = ly * RW + tid;
-    const float byf = ((float)y - hyF) * ihyF;
-    float bgv = 0.f, ax = 1.f;
+  float cy[5] = {0.f, 0.f, 0.f, 0.f, 0.f};
+  {
+    float ax = 1.f;
     int k = 0;
-    for(int i = 0; i <= a.bgOrder; i++) {
-      float ay = 1.f;
-      for(int j = 0; j <= a.bgOrder - i; j++) {
-        bgv = fmaf(bgc[k++], ax * ay, bgv);
-        ay *= byf;
-      }
+#pragma unroll
+    for(int i = 0; i < 5; i++) {
+#pragma unroll
+      for(int j = 0; j < 5; j++)
+        if(i + j <= a.bgOrder) cy[j] = fmaf(bgc[k++], ax, cy[j]);
       ax *= bxf;
     }
-    const float v = (sv[e] + bgv) * invKernMult;
-    const size_t id = (size_t)x + (size_t)y * a.w;
-    const float tc = tile[(ly + HK) * S + tid + HK];
-    uint16_t cm = convMaskF(tc, a.tH, a.tL);
-    if(inMask && inMask[id]) cm |= INPUT_MASK | BAD_INPUT;
-    uint16_t nm = cm;
-    if(cm & BAD_INPUT) nm |= BAD_OUTPUT;
-    const unsigned char f = cflag[e];
-    if(f == 2) nm |= BAD_OUTPUT | BAD_CONV;
-    else if(f == 1) nm |= OK_CONV;
-    const float ov = O[id];
-    nm |= afterMaskF(ov, a.tH, a.tL);
-    mask[id] = nm;
-    convF[id] = v;
-    diffF[id] = (nm & BAD_OUTPUT) ? 1e-30f : (v * convFactor - ov) * finalFactor;
+  }
+  const int nRow = min(FK, a.h - HK - (y0 + HK));
+  constexpr int U = 7;  // rows whose loads go ahead together
+  static_assert(FK % U == 0, "whole groups of rows");
+  const size_t id0 = (size_t)x + (size_t)(y0 + HK) * a.w;
+#pragma unroll 1
+  for(int l0 = 0; l0 < nRow; l0 += U) {
+    float ovs[U];
+    bool im[U];
+#pragma unroll
+    for(int u = 0; u < U; u++) {
+      const size_t id = id0 + (size_t)min(l0 + u, nRow - 1) * a.w;
+      ovs[u] = O[id];
+      im[u] = inMask && inMask[id];
+    }
+#pragma unroll
+    for(int u = 0; u < U; u++) {
+      const int ly = l0 + u;
+      if(ly >= nRow) break;
+      const int e = ly * RW + tid;
+      const float byf = ((float)(y0 + HK + ly) - hyF) * ihyF;
+      const float bgv = fmaf(fmaf(fmaf(fmaf(cy[4], byf, cy[3]), byf, cy[2]), byf, cy[1]), byf, cy[0]);
+      const float v = (sv[e] + bgv) * invKernMult;
+      const size_t id = id0 + (size_t)ly * a.w;
+      const float tc = tile[(ly + HK) * S + tid + HK];
+      uint16_t cm = convMaskF(tc, a.tH, a.tL);
+      if(im[u]) cm |= INPUT_MASK | BAD_INPUT;
+      uint16_t nm = cm;
+      if(cm & BAD_INPUT) nm |= BAD_OUTPUT;
+      const unsigned char f = cflag[e];
+      if(f == 2) nm |= BAD_OUTPUT | BAD_CONV;
+      else if(f == 1) nm |= OK_CONV;
+      const float ov = ovs[u];
+      nm |= afterMaskF(ov, a.tH, a.tL);
+      mask[id] = nm;
+      convF[id] = v;
+      diffF[id] = (nm & BAD_OUTPUT) ? 1e-30f : (v * convFactor - ov) * finalFactor;
+    }
   }
 }
 
@@ -1098,7 +1138,7 @@ __global__ void __launch_bounds__(BX * 21, 3)
   using L = ConvTileF<FK, BX>;
   using P = ConvTilePP<FK, BX>;
   constexpr int HK = L::HK, NK = L::NK, S = L::S, TW = L::TW, TH = L::TH, NW = L::NW, KS = L::KS;
-  constexpr int NT = L::NT, NFULL = NT / 32, TMAX = P::TMAX, RW = BX * FK;
+  constexpr int NT = L::RW, NFULL = NT / 32, TMAX = P::TMAX, RW = BX * FK;
   extern __shared__ __align__(16) unsigned char cv_smem[];
   float* tile = (float*)cv_smem;
   float* kern = (float*)(cv_smem + L::OFF_KERN);
@@ -2000,15 +2040,15 @@ void convSubMixed(xb_ctx* c, double* dKernSum) {
     const float *Ii = (const float*)c->img[I], *Oi = (const float*)c->img[O];
     switch(variant) {
       case 0:
-        k_conv_sub_f32<21, 4><<<dim3((xSteps + 3) / 4, ySteps), 4 * 21, ConvTileF<21, 4>::BYTES, c->stream>>>(
+        k_conv_sub_f32<21, 4><<<dim3((xSteps + 3) / 4, ySteps), ConvTileF<21, 4>::NT, ConvTileF<21, 4>::BYTES, c->stream>>>(
             Ii, Oi, c->dSol, Kt, blockXY, dKernSum, a, c->inputMask, c->mask, c->convF, c->diffF);
         break;
       case 1:
-        k_conv_sub_f32<21, 6><<<dim3((xSteps + 5) / 6, ySteps), 6 * 21, ConvTileF<21, 6>::BYTES, c->stream>>>(
+        k_conv_sub_f32<21, 6><<<dim3((xSteps + 5) / 6, ySteps), ConvTileF<21, 6>::NT, ConvTileF<21, 6>::BYTES, c->stream>>>(
             Ii, Oi, c->dSol, Kt, blockXY, dKernSum, a, c->inputMask, c->mask, c->convF, c->diffF);
         break;
       default:
-        k_conv_sub_f32<21, 8><<<dim3((xSteps + 7) / 8, ySteps), 8 * 21, ConvTileF<21, 8>::BYTES, c->stream>>>(
+        k_conv_sub_f32<21, 8><<<dim3((xSteps + 7) / 8, ySteps), ConvTileF<21, 8>::NT, ConvTileF<21, 8>::BYTES, c->stream>>>(
             Ii, Oi, c->dSol, Kt, blockXY, dKernSum, a, c->inputMask, c->mask, c->convF, c->diffF);
         break;
     }
