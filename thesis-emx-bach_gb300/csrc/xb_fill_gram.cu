@@ -131,37 +131,63 @@ struct FillGramArgs {
   int* timeout;
 };
 
+// Taps per turn of the loops below: the window values slide through registers,
+// one new load per tap, and the code stays small enough for the instruction
+// cache.  (Issue-bound: of 111 instructions a tap and eight outputs, ten were
+// loads; with three, and one FP32 operation less per step, 256 stamps take 363 us
+// instead of 437, 400 stamps 518 instead of 637.)
+constexpr int FG_U = 7;
 // Y pass, 8 consecutive output rows of one window column: v[j] is the
 // reference's float accumulation over taps t = 0..FK-1 (window row j + t,
-// filter entry FK-1-t), in that order.  The tap loop is not unrolled (eight
-// independent chains per tap keep the FP32 pipe busy; small code keeps the
-// instruction cache warm); ld is the window's row stride.
+// filter entry FK-1-t), in that order; eight independent chains per tap keep
+// the FP32 pipe busy.  f holds the filter's float pairs; ld is the window's row
+// stride.
 template <int FK>
-__device__ __forceinline__ void yPass8(const float* wp, int ld, const float* fh, const float* fl,
-                                       float (&v)[FG_R8]) {
+__device__ __forceinline__ void yPass8(const float* wp, int ld, const float2* f, float (&v)[FG_R8]) {
+  static_assert(FK % FG_U == 0, "whole turns");
+  float x[FG_R8 + FG_U - 1];
 #pragma unroll
   for(int j = 0; j < FG_R8; j++) v[j] = 0.f;
-#pragma unroll 1
-  for(int t = 0; t < FK; t++) {
-    const float h = fh[FK - 1 - t], l = fl[FK - 1 - t];
-    const float* p = wp + t * ld;
 #pragma unroll
-    for(int j = 0; j < FG_R8; j++) v[j] = df::refStepY(v[j], p[j * ld], h, l);
+  for(int j = 0; j < FG_R8 - 1; j++) x[j] = wp[j * ld];
+#pragma unroll 1
+  for(int t0 = 0; t0 < FK; t0 += FG_U) {
+    const float* p = wp + (t0 + FG_R8 - 1) * ld;
+#pragma unroll
+    for(int u = 0; u < FG_U; u++) x[FG_R8 - 1 + u] = p[u * ld];
+#pragma unroll
+    for(int u = 0; u < FG_U; u++) {
+      const float2 h = f[FK - 1 - t0 - u];
+#pragma unroll
+      for(int j = 0; j < FG_R8; j++) v[j] = df::refStepY(v[j], x[u + j], h.x, h.y);
+    }
+#pragma unroll
+    for(int j = 0; j < FG_R8 - 1; j++) x[j] = x[FG_U + j];
   }
 }
 // X pass, 8 consecutive output pixels of one row: the double-float sum over
 // taps t = 0..FK-1 (Y-pass value j + t, filter entry FK-1-t), in that order.
 template <int FK>
-__device__ __forceinline__ void xPass8(const float* yp, const float* fh, const float* fl,
-                                       float (&hi)[FG_R8], float (&lo)[FG_R8]) {
-  float sh[FG_R8], sl[FG_R8];
+__device__ __forceinline__ void xPass8(const float* yp, const float2* f, float (&hi)[FG_R8],
+                                       float (&lo)[FG_R8]) {
+  float sh[FG_R8], sl[FG_R8], x[FG_R8 + FG_U - 1];
 #pragma unroll
   for(int j = 0; j < FG_R8; j++) sh[j] = sl[j] = 0.f;
-#pragma unroll 1
-  for(int t = 0; t < FK; t++) {
-    const float h = fh[FK - 1 - t], l = fl[FK - 1 - t];
 #pragma unroll
-    for(int j = 0; j < FG_R8; j++) df::dfAccum(sh[j], sl[j], yp[t + j], h, l);
+  for(int j = 0; j < FG_R8 - 1; j++) x[j] = yp[j];
+#pragma unroll 1
+  for(int t0 = 0; t0 < FK; t0 += FG_U) {
+    const float* p = yp + t0 + FG_R8 - 1;
+#pragma unroll
+    for(int u = 0; u < FG_U; u++) x[FG_R8 - 1 + u] = p[u];
+#pragma unroll
+    for(int u = 0; u < FG_U; u++) {
+      const float2 h = f[FK - 1 - t0 - u];
+#pragma unroll
+      for(int j = 0; j < FG_R8; j++) df::dfAccum(sh[j], sl[j], x[u + j], h.x, h.y);
+    }
+#pragma unroll
+    for(int j = 0; j < FG_R8 - 1; j++) x[j] = x[FG_U + j];
   }
 #pragma unroll
   for(int j = 0; j < FG_R8; j++) df::dfNorm(sh[j], sl[j], hi[j], lo[j]);
@@ -212,10 +238,8 @@ __global__ void __launch_bounds__(NT, NT > 384 ? 1 : 2)
   Ws += rBase * fSS;
   Wl += rBase * fSS;
   float* win = (float*)(buf + L.oWin);
-  float* fxh = (float*)(buf + L.oF);
-  float* fxl = fxh + nPSF * FK;
-  float* fyh = fxl + nPSF * FK;
-  float* fyl = fyh + a.nGroups * FK;
+  float2* fx = (float2*)(buf + L.oF);
+  float2* fy = fx + nPSF * FK;
   float* w0h = (float*)(buf + L.oW0);
   float* w0l = w0h + K;
   float* ytmp = (float*)(buf + L.oY);
@@ -246,8 +270,13 @@ __global__ void __launch_bounds__(NT, NT > 384 ? 1 : 2)
           : "memory");
     }
   }
-  // the filters as float pairs: X [nPSF][FK] hi, lo; Y [group][FK] hi, lo
-  for(int i = tid; i < 2 * (nPSF + a.nGroups) * FK; i += NT) fxh[i] = a.fSplit[i];
+  // the filters as float pairs, X [nPSF][FK] then Y [group][FK] (hi and lo apart in
+  // global memory)
+  for(int i = tid; i < nPSF * FK; i += NT) fx[i] = make_float2(a.fSplit[i], a.fSplit[nPSF * FK + i]);
+  for(int i = tid; i < a.nGroups * FK; i += NT) {
+    const float* g = a.fSplit + 2 * nPSF * FK;
+    fy[i] = make_float2(g[i], g[a.nGroups * FK + i]);
+  }
   for(int n = tid; n < nPSF; n += NT)
     evenRow[n] = (n > 0 && a.kx[n] % 2 == 0 && a.ky[n] % 2 == 0) ? 1 : 0;
   if(tid < RB) rowMax[tid] = 0u;
@@ -276,7 +305,7 @@ __global__ void __launch_bounds__(NT, NT > 384 ? 1 : 2)
   auto yItem = [&](int g, int i) {
     const int r0 = (i / tw) * FG_R8, col = i % tw;
     float v[FG_R8];
-    yPass8<FK>(win + r0 * ldWin + col + dx, ldWin, fyh + g * FK, fyl + g * FK, v);
+    yPass8<FK>(win + r0 * ldWin + col + dx, ldWin, fy + g * FK, v);
     float* yo = ytmp + ((size_t)a.slot[g] * ldR + r0) * ldY + col;
 #pragma unroll
     for(int j = 0; j < FG_R8; j++)
@@ -300,8 +329,7 @@ __global__ void __launch_bounds__(NT, NT > 384 ? 1 : 2)
     const int row = i / nXB, ii0 = (i % nXB) * FG_R8;
     const int nv = min(FG_R8, fSS - ii0), p0 = row * fSS + ii0;
     float hi[FG_R8], lo[FG_R8];
-    xPass8<FK>(ytmp + ((size_t)a.slot[a.groupOf[n]] * ldR + row) * ldY + ii0, fxh + n * FK,
-               fxl + n * FK, hi, lo);
+    xPass8<FK>(ytmp + ((size_t)a.slot[a.groupOf[n]] * ldR + row) * ldY + ii0, fx + n * FK, hi, lo);
     if(n == 0) {
 #pragma unroll
       for(int j = 0; j < FG_R8; j++)
@@ -460,8 +488,9 @@ void fillGramLaunch(xb_ctx* c, int si, const int* dList, int nList, int imgConv,
   int optin = 0;
   XB_CUDA(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, c->device));
   // A refill's few stamps (its bound is not: the count is on the device) and short
-  // lists leave most SMs idle: four CTAs share each of them.  Four stamps take 76
-  // us so and 240 us on a CTA each; 256 stamps 556 and 437 us, so up to half an
+  // lists leave most SMs idle: four CTAs share each of them.  Four stamps take 70
+  // us so and about 200 us on a CTA each; 256 stamps 556 and 437 us (both before
+  // the passes' last step), so up to half an
   // SM count of stamps, where four waves of the first meet the second, are split.
   const bool split = ((liveN && liveN != S.dN) || nList * 2 <= c->smCount) &&
                      fgLayout(g.hSS, g.hK, nGroups, g.nPSF, FG_CL).total + 8 * 1024 <= (size_t)optin;
