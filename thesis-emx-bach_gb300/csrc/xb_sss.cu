@@ -1334,12 +1334,11 @@ __global__ void __launch_bounds__(FM_THREADS)
 // ------------------------------------------- substamp search in shared memory --
 // The decisions of k_find_substamps_maps for FP32 images, with the stamp in
 // shared memory at 6.4 bytes per pixel (pixel, flags, row winner, two bit
-// maps), so that stamps up to ~190 px fit and two 107-px ones share an SM:
+// maps), so that stamps up to ~188 px fit and two 107-px ones share an SM:
 //   * a candidate's window maximum (the largest key, ties to the first in
-//     raster order) is found when the scan reaches the candidate, by one warp:
-//     a lane per row of the window reads that row's winner (hx, the maximum
-//     over the 2 hSS + 1 columns around the candidate's) and one reduction
-//     finds the first largest;
+//     raster order) is found when the scan reaches the candidate, by one thread
+//     from the window rows' winners (hx, the maximum over the 2 hSS + 1 columns
+//     around the candidate's);
 //   * the window conditions "holds a bad pixel" and "holds a pixel above the
 //     stamp's threshold" are bit maps dilated by the window, so a lookup each;
 //     an acceptance turns its window bad, which ORs one rectangle into the
@@ -1349,21 +1348,35 @@ __global__ void __launch_bounds__(FM_THREADS)
 // !((v - sky) * (1/fwhm) < tKF), monotone in v, become compares against their
 // exact thresholds, found once per stamp by a warp search over the ordered
 // doubles; so does the pass threshold v > lim.
+// A pass lists its candidates in raster order, 2048 at a time; a thread takes
+// one, and the first that passes is the next substamp.
 // Two-dimensional maps of the winners and conditions by block scans, rebuilt
 // around every acceptance (15 bytes per pixel, one CTA per SM, stamps above
 // 123 px from global memory), took 0.55 ms for 2 x 256 stamps of 107 px and
-// 3.77 ms for 2 x 400 of 183; now
-// 0.38 and 0.88 ms.
+// 3.77 ms for 2 x 400 of 183; these forms with a warp per candidate, a load at a
+// time and the thresholds searched over all doubles 0.38 and 0.88 ms; now 0.20
+// and 0.53 ms.
 constexpr int FS_T = 512;
 constexpr uint8_t FS_BAD = 0x80;  // in the flags byte
 constexpr int FS_MAXN = 255;      // row winners are bytes, 0xFF none
 constexpr int FS_SEG = 8;         // columns per task of the row winners
+constexpr int FS_LIST = 2048;     // candidates listed at a time
 
 // One warp: smallest key in (lo, hi] at which pred turns true, given
 // pred(lo) false and pred(hi) true (pred monotone between them).
+// The key is usually among the doubles around `guess`, which the lanes test
+// first.
 template <class P>
-__device__ unsigned long long warpFirstTrue(unsigned long long lo, unsigned long long hi, P pred) {
+__device__ unsigned long long warpFirstTrue(unsigned long long lo, unsigned long long hi,
+                                            double guess, P pred) {
   const int lane = threadIdx.x & 31;
+  if(isfinite(guess)) {
+    const unsigned long long k = dKey(guess) - 16 + lane;
+    const bool valid = k > lo && k <= hi;
+    const unsigned bal = __ballot_sync(0xffffffffu, valid && pred(keyD(k)));
+    if(__all_sync(0xffffffffu, valid) && !(bal & 1u) && bal)
+      return __shfl_sync(0xffffffffu, k, __ffs(bal) - 1);
+  }
   for(int guard = 0; guard < 40; guard++) {
     const unsigned long long span = hi - lo;
     if(span <= 1) break;
@@ -1442,8 +1455,10 @@ __global__ void __launch_bounds__(FS_T, 2)
   uint32_t* dPred = dTmp + n * nw;
   __shared__ int2 locXY[MAX_MAXSS];
   __shared__ double locVal[MAX_MAXSS];
-  __shared__ int sBest, sM;
-  __shared__ double rA[NW], rB[NW];
+  __shared__ int sBest[2], sM, sTotal, sScan[NW];
+  __shared__ uint16_t list[FS_LIST];
+  __shared__ double rA[NW];
+  __shared__ unsigned rB[NW];
   __shared__ double sSum;
   __shared__ float sfP, sfK, sfLim;
   __shared__ int sDirect;
@@ -1451,20 +1466,32 @@ __global__ void __launch_bounds__(FS_T, 2)
   // warps 2.. load the stamp while warps 0 and 1 search the exact
   // thresholds of the two static predicates; the window conditions cover
   // the pixels inside the frame (x < sx, y < sy)
-  if(warp >= 2)
-    for(int ly = warp - 2; ly < n; ly += NW - 2)
-      for(int j = 0; j < nw; j++) {
+  if(warp >= 2) {
+    // whole rows (at most eight words) ahead of their tests
+    for(int ly = warp - 2; ly < n; ly += NW - 2) {
+      float v[8];
+      uint16_t mk[8];
+      const size_t row = (size_t)cx + (size_t)(cy + ly) * w;
+#pragma unroll
+      for(int j = 0; j < 8; j++) {
         const int lx = 32 * j + lane;
-        bool b = false;
+        v[j] = lx < n ? img[row + lx] : 0.f;
+        mk[j] = lx < n ? ldMask(mask, row + lx) : (uint16_t)0;
+      }
+#pragma unroll
+      for(int j = 0; j < 8; j++) {
+        if(j >= nw) break;
+        const int lx = 32 * j + lane;
+        const bool b = (mk[j] & badMask) != 0;
         if(lx < n) {
-          const size_t a = (size_t)(cx + lx) + (size_t)(cy + ly) * w;
-          V[ly * n + lx] = img[a];
-          b = (ldMask(mask, a) & badMask) != 0;
+          V[ly * n + lx] = v[j];
           F[ly * n + lx] = b ? FS_BAD : 0;
         }
         const uint32_t m = __ballot_sync(0xffffffffu, b && lx < sx && ly < sy);
         if(lane == 0) dTmp[ly * nw + j] = m;
       }
+    }
+  }
   if(warp < 2) {
     auto pr = [&](double v) { return (v - sky) / fwhm > tKF; };
     auto kq = [&](double v) { return !((v - sky) * invFwhm < tKF); };
@@ -1473,10 +1500,10 @@ __global__ void __launch_bounds__(FS_T, 2)
     if(!direct) {
       const unsigned long long kLo = dKey(-INFINITY), kHi = dKey(INFINITY);
       if(warp == 0) {
-        const unsigned long long kP = warpFirstTrue(kLo, kHi, pr);
+        const unsigned long long kP = warpFirstTrue(kLo, kHi, sky + tKF * fwhm, pr);
         if(lane == 0) sfP = __double2float_ru(keyD(kP));  // pr(v) <=> v >= sfP for a float v
       } else {
-        const unsigned long long kK = warpFirstTrue(kLo, kHi, kq);
+        const unsigned long long kK = warpFirstTrue(kLo, kHi, sky + tKF * fwhm, kq);
         if(lane == 0) sfK = __double2float_ru(keyD(kK));
       }
     }
@@ -1529,6 +1556,7 @@ __global__ void __launch_bounds__(FS_T, 2)
   dilateColumns(dTmp, dBad);
   dilateColumns(dPred, dTmp);
   const uint32_t* dOk = dTmp;
+  uint32_t* cands = dPred;  // free from here on
   auto bitAt = [&](const uint32_t* d, int y, int x) { return (d[y * nw + (x >> 5)] >> (x & 31)) & 1u; };
 
   // A key is the float bit pattern of a qualifying pixel (0: none).
@@ -1604,29 +1632,31 @@ __global__ void __launch_bounds__(FS_T, 2)
     __syncthreads();
   };
   rowWinners(0, n - 1, 0, n - 1);
-  const int W = 2 * hSS + 1;
   // The pixel a candidate stands for: its window's first largest key, or
-  // itself where the window has none.  One warp.
-  auto windowMax = [&](int p) -> int {
-    const int ly = p / n, lx = p - ly * n;
+  // itself where the window has none.
+  auto windowMax = [&](int p, int ly, int lx) -> int {
+    const int y1 = min(ly + hSS, n - 1);
     uint32_t bk = 0;
     int m = p;
-    for(int b = 0; b < W; b += 32) {
-      const int y = ly - hSS + b + lane;
-      uint32_t k = 0;
-      int q = p;
-      if(b + lane < W && y >= 0 && y < n) {
-        const int h = hx[y * n + lx];
-        if(h != 0xFF) {
-          q = y * n + h;
-          k = __float_as_uint(V[q]);
+    for(int y = max(ly - hSS, 0); y <= y1; y += 8) {
+      int q[8];
+      uint32_t k[8];
+#pragma unroll
+      for(int u = 0; u < 8; u++) q[u] = y + u <= y1 ? hx[(y + u) * n + lx] : 0xFF;
+#pragma unroll
+      for(int u = 0; u < 8; u++) {
+        k[u] = 0;
+        if(q[u] != 0xFF) {
+          q[u] += (y + u) * n;
+          k[u] = __float_as_uint(V[q[u]]);
         }
       }
-      const uint32_t kb = __reduce_max_sync(0xffffffffu, k);
-      if(kb > bk) {
-        bk = kb;
-        m = __shfl_sync(0xffffffffu, q, __ffs(__ballot_sync(0xffffffffu, k == kb)) - 1);
-      }
+#pragma unroll
+      for(int u = 0; u < 8; u++)
+        if(k[u] > bk) {
+          bk = k[u];
+          m = q[u];
+        }
     }
     return m;
   };
@@ -1640,33 +1670,74 @@ __global__ void __launch_bounds__(FS_T, 2)
     if(tid == 0) sfLim = __double2float_rd(lim);    // v > lim <=> v > sfLim for a float v
     __syncthreads();
     const float fLim = sfLim;
-    int start = 0;
-    while(cnt < maxSS && start < N) {
-      int mine = INT_MAX, mineM = 0;
-      for(int p0 = start; p0 < N && mine == INT_MAX; p0 += 4 * FS_T) {
-        for(int k = 0; k < 4 && mine == INT_MAX; k++) {
-          const int pw = p0 + k * FS_T + warp * 32, p = pw + lane;
-          const bool cand = p < N && (F[p] & (FS_BAD | FL_KFQ)) == FL_KFQ && V[p] > fLim;
-          for(unsigned c = __ballot_sync(0xffffffffu, cand); c; c &= c - 1) {
-            const int pc = pw + __ffs(c) - 1, m = windowMax(pc);
+    // this pass's candidates: bits, then lists in raster order
+    for(int ly = warp; ly < n; ly += NW) {
+      uint8_t f[8];
+      float v[8];
+#pragma unroll
+      for(int j = 0; j < 8; j++) {
+        const int lx = 32 * j + lane, p = ly * n + lx;
+        f[j] = lx < n ? F[p] : (uint8_t)0;
+        v[j] = lx < n ? V[p] : 0.f;
+      }
+#pragma unroll
+      for(int j = 0; j < 8; j++) {
+        if(j >= nw) break;
+        const uint32_t c = __ballot_sync(0xffffffffu, (f[j] & (FS_BAD | FL_KFQ)) == FL_KFQ && v[j] > fLim);
+        if(lane == 0) cands[ly * nw + j] = c;
+      }
+    }
+    if(tid < 2) sBest[tid] = INT_MAX;
+    __syncthreads();
+    int from = 0, at = 0, nList = 0, turn = 0;  // list of the candidates from `from` on
+    while(cnt < maxSS) {
+      int mine = INT_MAX;  // index in the list
+      while(mine == INT_MAX) {
+        if(at >= nList) {
+          if(from >= N) break;
+          const int ys = from / n, xs = from - ys * n, e0 = ys * nw + (xs >> 5);
+          nList = 0;
+          for(int eb = e0; eb < n * nw && nList < FS_LIST; eb += FS_T) {
+            const int e = eb + tid, y = e / nw;
+            unsigned c = e < n * nw ? cands[e] : 0u;
+            if(e == e0) c &= 0xFFFFFFFFu << (xs & 31);
+            int k = nList + blockScanExcl(__popc(c), sScan, &sTotal);
+            for(; c && k < FS_LIST; c &= c - 1, k++)
+              list[k] = (uint16_t)(y * n + 32 * (e - y * nw) + __ffs(c) - 1);
+            nList += sTotal;
+            __syncthreads();
+          }
+          from = N;
+          if(nList > FS_LIST) {
+            nList = FS_LIST;
+            from = list[FS_LIST - 1] + 1;
+          }
+          at = 0;
+          if(nList == 0) break;
+        }
+        // a candidate per thread
+        const int k = at + tid;
+        int m = 0;
+        if(k < nList) {
+          const int pc = list[k], ly = pc / n;
+          if(!(F[pc] & FS_BAD)) {  // not in an accepted window since
+            m = windowMax(pc, ly, pc - ly * n);
             const int my = m / n, mx = m - my * n;
-            if(!bitAt(dBad, my, mx) && bitAt(dOk, my, mx)) {
-              mine = pc;
-              mineM = m;
-              break;
-            }
+            if(!bitAt(dBad, my, mx) && bitAt(dOk, my, mx)) mine = k;
           }
         }
-        if(tid == 0) sBest = INT_MAX;
+        const int own = mine, best = __reduce_min_sync(0xffffffffu, mine);
+        if(lane == 0 && best != INT_MAX) atomicMin(&sBest[turn], best);
         __syncthreads();
-        if(lane == 0 && mine != INT_MAX) atomicMin(&sBest, mine);
+        mine = sBest[turn];
+        if(own != INT_MAX && own == mine) sM = m;
+        if(tid == 0) sBest[turn ^ 1] = INT_MAX;
         __syncthreads();
-        if(lane == 0 && mine != INT_MAX && mine == sBest) sM = mineM;
-        mine = sBest;
-        __syncthreads();
+        turn ^= 1;
+        at = mine == INT_MAX ? at + FS_T : mine + 1;
       }
       if(mine == INT_MAX) break;
-      const int p = mine, m = sM;
+      const int m = sM;
       const int mx = cx + m % n, my = cy + m / n;
       const int u0 = max(mx - hSS, cx), v0 = max(my - hSS, cy);
       const int u1 = min(mx + hSS, cx + sx - 1), v1 = min(my + hSS, cy + sy - 1);
@@ -1678,40 +1749,35 @@ __global__ void __launch_bounds__(FS_T, 2)
       // any order; otherwise warp 0 forms the serial sum bit for bit (osum;
       // a pixel below the threshold adds +0.0, which changes nothing).
       double part = 0.0;
-      float amin = INFINITY;
+      unsigned amin = 0x7F800000u;  // bits of the smallest magnitude
       bool nonpos = false;
       for(int i = tid; i < un; i += FS_T) {
         const int q = (v0 + i / uw - cy) * n + (u0 + i % uw - cx);
         const uint8_t fl = F[q];
         if(fl & FL_PRED) {
           part += (double)V[q];
-          amin = fminf(amin, fabsf(V[q]));
+          amin = min(amin, __float_as_uint(V[q]) & 0x7FFFFFFFu);
           nonpos |= (fl & FL_NONPOS) != 0;
         }
       }
 #pragma unroll
-      for(int o = 16; o > 0; o >>= 1) {
-        part += __shfl_xor_sync(0xffffffffu, part, o);
-        amin = fminf(amin, __shfl_xor_sync(0xffffffffu, amin, o));
-      }
+      for(int o = 16; o > 0; o >>= 1) part += __shfl_xor_sync(0xffffffffu, part, o);
+      amin = __reduce_min_sync(0xffffffffu, amin);
       if(lane == 0) {
         rA[warp] = part;
-        rB[warp] = (double)amin;
+        rB[warp] = amin;
       }
       nonpos = __syncthreads_or(nonpos);
       if(warp == 0) {
-        double t = lane < NW ? rA[lane] : 0.0, mn = lane < NW ? rB[lane] : INFINITY;
+        double t = lane < NW ? rA[lane] : 0.0;
 #pragma unroll
-        for(int o = 16; o > 0; o >>= 1) {
-          t += __shfl_xor_sync(0xffffffffu, t, o);
-          mn = fmin(mn, __shfl_xor_sync(0xffffffffu, mn, o));
-        }
-        bool exact = false;
-        if(!nonpos && mn > 0.0 && mn < INFINITY) {
-          int e;
-          frexp(mn, &e);  // mn in [2^(e-1), 2^e)
-          exact = t < ldexp(1.0, e - 1 - 23 + 52);
-        }
+        for(int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
+        const unsigned mn = __reduce_min_sync(0xffffffffu, lane < NW ? rB[lane] : 0x7F800000u);
+        // smallest in [2^(e-127), 2^(e-126)), so every pixel is a multiple of
+        // 2^(e-150), and the sum must stay below 2^(e-98)
+        const int e = (int)(mn >> 23);
+        const bool exact = !nonpos && e > 0 && e < 255 &&
+                           __double_as_longlong(t) < (long long)(e - 98 + 1023) << 52;
         if(!exact)
           t = osum::warpOrderedSumOf(un, [&](int i) {
             const int q = (v0 + i / uw - cy) * n + (u0 + i % uw - cx);
@@ -1721,7 +1787,6 @@ __global__ void __launch_bounds__(FS_T, 2)
       }
       __syncthreads();
       const double ret = sSum;
-      start = p + 1;
       if(ret == 0.0) continue;
       if(tid == 0) {
         locXY[cnt] = make_int2(mx, my);
@@ -1863,7 +1928,7 @@ static void sssPass(xb_ctx* c, int* nKept) {
   // else maps in global memory
   int optin = 0;
   XB_CUDA(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, c->device));
-  const bool inShared = !c->imgIsF64 && fSW <= FS_MAXN && fsSmem + 1024 <= (size_t)optin;
+  const bool inShared = !c->imgIsF64 && fSW <= FS_MAXN && fsSmem + 6 * 1024 <= (size_t)optin;
   // global-memory maps only for the kernel that uses them
   unsigned char* scratch =
       inShared ? nullptr : buf<unsigned char>(c, "fm_scratch", (size_t)2 * nAll * perCta);
