@@ -95,17 +95,23 @@ __device__ __forceinline__ void maskOr(uint16_t* m, size_t i, uint16_t bits) {
 
 // sigmaClip of src/bachUtil.cpp:34-128 for one CTA: data[0..n) in global
 // memory, sums in 32-element chunks (sequential inside a chunk,
-// cl_kern/bach.cl:135-170) added sequentially (bachUtil.cpp:103-104); the
-// clipped flags live in `flags` (n bytes), chunk sums in cs/cs2.  The result
+// cl_kern/bach.cl:135-170) added sequentially (bachUtil.cpp:103-104).  Up to
+// SC_CAP values stay in shared memory, their squares beside them: one warp sums
+// the chunks, one their squares, a lane per chunk, and two threads add the
+// chunks; bound by those chains (with every operand from global memory and one
+// thread for both sums a check of 256 stamps took 20 us, now 15).  More values:
+// clipped flags in `flags` (n bytes), chunk sums in cs/cs2.  The result
 // is written to *outMean / *outStd (shared) by thread 0; all threads must
 // call it.
+constexpr int SC_CAP = 1024, SC_PER = 4;
 __device__ inline void blockSigmaClip(const double* data, int n, int maxIter, double alpha,
                                       uint8_t* flags, double* cs, double* cs2,
                                       double* outMean, double* outStd, int* sh) {
   // sh[0] = prev, sh[1] = curr, sh[2] = clip, sh[3] = stop
   const int tid = threadIdx.x, nt = blockDim.x;
   __shared__ double sInv;
-  for(int k = tid; k < n; k += nt) flags[k] = 0;
+  if(n > SC_CAP || nt * SC_PER < SC_CAP)
+    for(int k = tid; k < n; k += nt) flags[k] = 0;
   if(tid == 0) {
     sh[0] = n;
     sh[1] = 0;
@@ -116,6 +122,80 @@ __device__ inline void blockSigmaClip(const double* data, int n, int maxIter, do
   }
   __syncthreads();
   const int nChunks = (n + 31) / 32;
+  if(n <= SC_CAP && nt * SC_PER >= SC_CAP) {
+    // value k at k + k / 32: a lane's chunk meets no bank conflicts
+    __shared__ double sv[SC_CAP + SC_CAP / 32], sq[SC_CAP + SC_CAP / 32];
+    __shared__ double sc[2][SC_CAP / 32], sSums[2];
+    const int lane = tid & 31, warp = tid >> 5;
+    double d[SC_PER];
+    unsigned live = 0;
+#pragma unroll
+    for(int u = 0; u < SC_PER; u++) {
+      const int k = tid + u * nt;
+      d[u] = 0.0;
+      if(k < n) {
+        d[u] = data[k];
+        live |= 1u << u;
+        sv[k + (k >> 5)] = d[u];
+        sq[k + (k >> 5)] = d[u] * d[u];
+      }
+    }
+    for(int it = 0; it < maxIter; it++) {
+      if(sh[3] || sh[1] == sh[0]) break;
+      if(sh[0] <= 1) {
+        __syncthreads();
+        if(tid == 0) {
+          *outMean = 0.0;
+          *outStd = 1e10;
+        }
+        break;
+      }
+      __syncthreads();
+      if(tid == 0) sh[1] = sh[0];
+      if(warp < 2 && lane < nChunks) {
+        const double* v = (warp ? sq : sv) + 33 * lane;
+        const int lc = min(32, n - 32 * lane);
+        double a = 0.0;
+#pragma unroll 8
+        for(int l = 0; l < lc; l++) a += v[l];
+        sc[warp][lane] = a;
+      }
+      __syncthreads();
+      if(warp < 2 && lane == 0) {
+        double a = 0.0;
+#pragma unroll 4
+        for(int c = 0; c < nChunks; c++) a += sc[warp][c];
+        sSums[warp] = a;
+      }
+      __syncthreads();
+      if(tid == 0) {
+        const double nn = (double)sh[1];
+        const double m = sSums[0] / nn;
+        const double sd = sqrt((sSums[1] - nn * m * m) / (double)(sh[1] - 1));
+        *outMean = m;
+        *outStd = sd;
+        sInv = 1.0 / sd;
+        sh[2] = 0;
+      }
+      __syncthreads();
+      const double m = *outMean, inv = sInv;
+      int myClip = 0;
+#pragma unroll
+      for(int u = 0; u < SC_PER; u++)
+        if((live >> u & 1u) && fabs(d[u] - m) * inv > alpha) {
+          const int k = tid + u * nt;
+          live &= ~(1u << u);
+          sv[k + (k >> 5)] = sq[k + (k >> 5)] = 0.0;
+          myClip++;
+        }
+      if(myClip) atomicAdd(&sh[2], myClip);
+      __syncthreads();
+      if(tid == 0) sh[0] = sh[1] - sh[2];
+      __syncthreads();
+    }
+    __syncthreads();
+    return;
+  }
   for(int it = 0; it < maxIter; it++) {
     if(sh[3] || sh[1] == sh[0]) break;
     if(sh[0] <= 1) {
