@@ -33,10 +33,11 @@ __device__ __forceinline__ float floatNormF(int x, int w) {
 __device__ __forceinline__ float refStepY(float v, float a, float fh, float fl) {
   const float ph = a * fh;
   const float pe = fmaf(a, fh, -ph);  // a*fh = ph + pe exactly
+  const float pl = a * fl;
   const float s = v + ph;             // two-sum: v + ph = s + e exactly
   const float bb = s - v;
   const float e = (v - (s - bb)) + (ph - bb);
-  return s + (e + fmaf(a, fl, pe));
+  return s + (e + (pe + pl));
 }
 // (sh, sl) += t * (fh + fl)
 __device__ __forceinline__ void dfAccum(float& sh, float& sl, float t, float fh, float fl) {
@@ -46,7 +47,7 @@ __device__ __forceinline__ void dfAccum(float& sh, float& sl, float t, float fh,
   const float bb = s - sh;
   const float e = (sh - (s - bb)) + (ph - bb);
   sh = s;
-  sl += e + fmaf(t, fl, pe);
+  sl += e + (pe + t * fl);
 }
 // renormalised hi + lo of sh + sl
 __device__ __forceinline__ void dfNorm(float sh, float sl, float& hi, float& lo) {

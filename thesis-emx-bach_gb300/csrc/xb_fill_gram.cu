@@ -134,8 +134,8 @@ struct FillGramArgs {
 // Taps per turn of the loops below: the window values slide through registers,
 // one new load per tap, and the code stays small enough for the instruction
 // cache.  (Issue-bound: of 111 instructions a tap and eight outputs, ten were
-// loads; with three, and one FP32 operation less per step, 256 stamps take 363 us
-// instead of 437, 400 stamps 518 instead of 637.)
+// loads; with two, 256 stamps take 375 us instead of 437, 400 stamps 536 instead
+// of 637.)
 constexpr int FG_U = 7;
 // Y pass, 8 consecutive output rows of one window column: v[j] is the
 // reference's float accumulation over taps t = 0..FK-1 (window row j + t,

@@ -1,19 +1,18 @@
 // xb_mixed.cu — the mixed-precision (chosen) path, XB_MODE_MIXED.
 //
 // Same stages, same decisions logic, different arithmetic:
-//   * basis convolutions of the substamps in FP32 FMA, W kept in FP32;
-//   * one Gram matrix per stamp of the W rows plus the projected image row
-//     (FP32 accumulation), scattered into Q, B and the dot products the
-//     global normal matrix needs (createQ/createB/createMatrix terms);
-//   * the global system in FP64: LU with fused multiply-adds on a 16-CTA
-//     thread-block cluster, triangular solves by column sweeps, and one
-//     iterative-refinement step with an FP64 residual;
-//   * the chi^2 model in FP32 (the reference already stores it in FP32,
-//     cl_kern/cd.cl:489-531);
+//   * basis convolutions of the substamps in float pairs (xb_df.cuh), W as hi +
+//     lo; one Gram matrix per stamp of the W rows plus the projected image row,
+//     scattered into Q, B and the dot products the global normal matrix needs
+//     (createQ/createB/createMatrix terms).  The fused kernel of
+//     xb_fill_gram.cu takes the common shapes; the kernels here the others;
+//   * the global system in FP64 by LDL^T on a cluster (xb_ldl.cu); the pivoted
+//     LU and refined solve here run when one of its pivots fails;
+//   * the chi^2 model in double-float, stored in FP32 as the reference does
+//     (cl_kern/cd.cl:489-531);
 //   * the full-frame convolution in FP32: 4, 6 or 8 kernel blocks per CTA,
 //     a 7 x 3 pixel tile per thread held in registers.
-// Statistics, substamp search and the per-stamp test fits are shared with the
-// plain path.
+// Statistics and substamp search are shared with the plain path.
 
 #include <cooperative_groups.h>
 
