@@ -1,5 +1,5 @@
 """The stamp statistics against the FP64 oracle over stamp sizes (good pixels in
-shared memory with 8 or 16 warps, in the scratch slice with chunk sums in shared
+shared memory, in the scratch slice with chunk sums in shared
 memory and without) and pixel contents: sky and sources, a constant, a dynamic
 range whose plain sums are not exact in 53 bits, pixels around zero, NaN pixels
 and mostly masked stamps.  Sky, width and mask are identical."""

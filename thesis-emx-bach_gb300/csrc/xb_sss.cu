@@ -88,22 +88,11 @@ struct Ran1 {
 // only pixels within that bound of a bin edge redo it in FP64.  All decisions
 // and sums are those of the reference's order.
 
-// The good-pixel list of a stamp, chunk-interleaved: entry q lives at
-// slot ((q >> 10) << 10) | ((q & 31) << 5) | ((q >> 5) & 31) of the stamp's
-// slice, whose length is fSW^2 rounded up to a multiple of 1024.
+// A stamp's slice of the good-pixel scratch: fSW^2 rounded up to a multiple of
+// 1024 elements.
 __host__ __device__ __forceinline__ size_t statsSlice(int fSW) {
   return ((size_t)fSW * fSW + 1023) & ~(size_t)1023;
 }
-__device__ __forceinline__ int listSlot(int q) {
-  return ((q >> 10) << 10) | ((q & 31) << 5) | ((q >> 5) & 31);
-}
-__device__ __forceinline__ int chunkSlot(int c, int l) {  // entry c * 32 + l
-  return ((c >> 5) << 10) | (l << 5) | (c & 31);
-}
-__device__ __forceinline__ int listEntry(int slot) {  // inverse of listSlot
-  return ((slot >> 10) << 10) | ((slot & 31) << 5) | ((slot >> 5) & 31);
-}
-
 // Order-preserving map of doubles (no NaN) to 64-bit keys and back.
 __device__ __forceinline__ unsigned long long dKey(double x) {
   const unsigned long long b = (unsigned long long)__double_as_longlong(x);
@@ -200,17 +189,17 @@ inline size_t statsSmemBytes(int maxChunks, bool sm) {
 // samples meanwhile (they are needed for the histogram only).
 //
 // SM: the good pixels (FP32) stay in shared memory; else they go to the scratch
-// slice, chunk-interleaved.  Bound by FP64, one warp instruction per 19 cycles
+// slice.  Bound by FP64, one warp instruction per 19 cycles
 // and SM, and by its serial chains: a pixel's part of a chunk's sum of squares
 // is one FP64 instruction (an FP32 pixel's square is exact in FP64, so the
 // fused multiply-add rounds as the sum does); the plain sums are exact whenever
 // the pixels' total fits 53 bits of their common quantum, and then they are
 // integers and need no order; only chunks that lost a pixel are summed again.
-// Both images, 256 stamps of 107 px: 206 us, 400 of 183 px: 745 us (the
+// Both images, 256 stamps of 107 px: 206 us, 400 of 183 px: 529 us (the
 // good pixels and a byte flag each in global memory, four FP64 instructions per
 // pixel, the samples first: 662 and 1909 us).
 template <class T, bool SM, int NW>
-__global__ void __launch_bounds__(NW * 32 + 32, NW > 8 ? 1 : 3)
+__global__ void __launch_bounds__(NW * 32 + 32, sizeof(T) == 8 ? 2 : 3)
     k_stamp_stats(const T* __restrict__ img, uint16_t* __restrict__ mask,
                   const int4* __restrict__ geom, int w, int h, int fSW,
                   T* __restrict__ good, uint8_t* __restrict__ clip,
@@ -364,11 +353,8 @@ __global__ void __launch_bounds__(NW * 32 + 32, NW > 8 ? 1 : 3)
   // warp takes 32 * BB consecutive ones, ballots order them inside the warp
   // and the warps' counts order the warps.  The good pixels are kept as read
   // (FP32 pixels stay FP32).
-  // In a scratch slice the list is chunk-interleaved: entry q (chunk q/32,
-  // position q%32) at listSlot(q), so that the chunk passes, one chunk per
-  // thread, read 32 consecutive chunks' entries at one position with one
-  // coalesced load.  A stamp's slice is fSW^2 rounded up to a multiple of 1024
-  // (statsSlice).
+  // A scratch slice holds them in order; a chunk pass, one chunk per thread, reads
+  // its 32 in 16-byte loads, whose lines the L1 keeps for the following ones.
   T* gd = good + (size_t)s * statsSlice(fSW);
   const bool chunksInSmem = SM || maxChunks <= ST_CHUNKS_SMEM;
   double* cS = chunksInSmem ? (double*)st_s : chunkBuf + (size_t)s * 2 * maxChunks;
@@ -439,7 +425,7 @@ __global__ void __launch_bounds__(NW * 32 + 32, NW > 8 ? 1 : 3)
         if(bal[u] >> lane & 1u) {
           const int q = pos + __popc(bal[u] & ((1u << lane) - 1u));
           if constexpr(SM) list[q + (q >> 5)] = px[u];
-          else gd[listSlot(q)] = px[u];
+          else gd[q] = px[u];
           if constexpr(F32) {
             const unsigned b = __float_as_uint(px[u]);
             kMin = min(kMin, b);
@@ -478,7 +464,30 @@ __global__ void __launch_bounds__(NW * 32 + 32, NW > 8 ? 1 : 3)
   const int nChunks = (nGood + 31) / 32;
   auto pixel = [&](int c, int l) -> T {
     if constexpr(SM) return list[c * 33 + l];
-    else return gd[chunkSlot(c, l)];
+    else return gd[c * 32 + l];
+  };
+  // 16 pixels of a chunk from l on (what lies past the list is garbage)
+  auto pixels16 = [&](int c, int l, T (&v)[16]) {
+    if constexpr(SM) {
+#pragma unroll
+      for(int k = 0; k < 16; k++) v[k] = list[c * 33 + l + k];
+    } else if constexpr(F32) {
+#pragma unroll
+      for(int k = 0; k < 4; k++) {
+        const float4 q = ((const float4*)(gd + c * 32 + l))[k];
+        v[4 * k] = q.x;
+        v[4 * k + 1] = q.y;
+        v[4 * k + 2] = q.z;
+        v[4 * k + 3] = q.w;
+      }
+    } else {
+#pragma unroll
+      for(int k = 0; k < 8; k++) {
+        const double2 q = ((const double2*)(gd + c * 32 + l))[k];
+        v[2 * k] = q.x;
+        v[2 * k + 1] = q.y;
+      }
+    }
   };
   // exact clip thresholds for (m, inv) into tLo/tHi (warp 0; all pixel threads call)
   // (warp 0 searches the upper edge, warp 1 the lower one)
@@ -536,8 +545,7 @@ __global__ void __launch_bounds__(NW * 32 + 32, NW > 8 ? 1 : 3)
 #pragma unroll
     for(int h0 = 0; h0 < 32; h0 += 16) {
       T v[16];
-#pragma unroll
-      for(int l = 0; l < 16; l++) v[l] = (SM || (m >> (h0 + l) & 1u)) ? pixel(c, h0 + l) : T(0);
+      pixels16(c, h0, v);
 #pragma unroll
       for(int l = 0; l < 16; l++) {
         const bool on = m >> (h0 + l) & 1u;
@@ -631,8 +639,7 @@ __global__ void __launch_bounds__(NW * 32 + 32, NW > 8 ? 1 : 3)
 #pragma unroll
       for(int h0 = 0; h0 < 32; h0 += 16) {
         T v[16];
-#pragma unroll
-        for(int l = 0; l < 16; l++) v[l] = (SM || (live >> (h0 + l) & 1u)) ? pixel(c, h0 + l) : T(0);
+        pixels16(c, h0, v);
         if(k.direct) {
 #pragma unroll
           for(int l = 0; l < 16; l++)
@@ -722,22 +729,15 @@ __global__ void __launch_bounds__(NW * 32 + 32, NW > 8 ? 1 : 3)
     // the good list of phase B (the kernel changes no other mask bit of the
     // stamp) less the final clip
     constexpr int HB = 8;  // list entries loaded ahead per thread
-    // (the counts do not depend on the order: the slots of a scratch slice are
-    // read in storage order, coalesced, each standing for listEntry(slot))
-    const int nSlots = SM ? nGood : (nGood + 1023) & ~1023;
-    for(int base0 = 0; base0 < nSlots; base0 += NT * HB) {
+    for(int base0 = 0; base0 < nGood; base0 += NT * HB) {
       T pvs[HB];
       bool in[HB];
 #pragma unroll
       for(int u = 0; u < HB; u++) {
         const int k = base0 + u * NT + tid;
-        if constexpr(SM) {
-          in[u] = k < nGood;
-          pvs[u] = in[u] ? list[k + (k >> 5)] : 0.f;
-        } else {
-          in[u] = k < nSlots && listEntry(k) < nGood;
-          pvs[u] = in[u] ? gd[k] : T(0);
-        }
+        in[u] = k < nGood;
+        if constexpr(SM) pvs[u] = in[u] ? list[k + (k >> 5)] : 0.f;
+        else pvs[u] = in[u] ? gd[k] : T(0);
       }
       unsigned rest = 0;  // entries whose bin the FP32 estimate leaves open
 #pragma unroll
@@ -919,9 +919,12 @@ __global__ void __launch_bounds__(NW * 32 + 32, NW > 8 ? 1 : 3)
   }
 }
 
-// Launches the statistics of n stamps.  FP32 stamps whose pixels fit in shared
-// memory keep them there (up to about 214 px on a side), with 16 warps where
-// only one CTA fits on an SM; larger ones and FP64 images use the scratch.
+// Launches the statistics of n stamps.  FP32 stamps of which three fit on an SM
+// keep their pixels in shared memory (up to about 119 px on a side); larger ones
+// and FP64 images use the scratch, also three CTAs to an SM, which overlap each
+// other's serial chains (an image's 390 stamps of 132 px in shared memory, two to an
+// SM, 190 us, in the scratch 147; 400 of 183 px, one of 16 warps to an SM, 372
+// and 264).
 template <class T>
 cudaError_t launchStampStats(const T* img, uint16_t* mask, const int4* geom, int n, int w, int h,
                              int fSW, T* good, uint8_t* clip, double* chunkBuf, double alpha,
@@ -942,8 +945,7 @@ cudaError_t launchStampStats(const T* img, uint16_t* mask, const int4* geom, int
   };
   if constexpr(sizeof(T) == 4) {
     const size_t smem = statsSmemBytes(maxChunks, true), fixed = 8192;  // static and reserved
-    if(2 * (smem + fixed) <= (size_t)optin) return go(k_stamp_stats<T, true, 8>, 288, smem);
-    if(smem + fixed <= (size_t)optin) return go(k_stamp_stats<T, true, 16>, 544, smem);
+    if(3 * (smem + fixed) <= (size_t)optin) return go(k_stamp_stats<T, true, 8>, 288, smem);
   }
   return go(k_stamp_stats<T, false, 8>, 288, statsSmemBytes(maxChunks, false));
 }
