@@ -1,6 +1,7 @@
 """The substamp search with far more candidates per stamp than one list of it
-holds (csrc/xb_sss.cu, 2048 at a time), most of them with a bad window, against
-the FP64 oracle: substamps, values and mask are identical."""
+holds (csrc/xb_sss.cu, 2048 at a time, 512 in the largest stamps), most of them
+with a bad window, against the FP64 oracle: substamps, values and mask are
+identical."""
 import numpy as np
 import pytest
 
@@ -8,7 +9,7 @@ pytestmark = pytest.mark.gpu
 
 
 @pytest.mark.parametrize("size,stamps,dens,clean", [(420, 3, 0.2, 60), (560, 3, 0.15, 60), (400, 2, 0.2, 50),
-                                                    (300, 2, 0.22, 60)])
+                                                    (300, 2, 0.22, 60), (630, 3, 0.15, 60), (633, 3, 0.15, 60)])
 def test_many_candidates_equal_the_oracle(oracle, size, stamps, dens, clean):
     import xbach
     rng = np.random.default_rng(size + clean)

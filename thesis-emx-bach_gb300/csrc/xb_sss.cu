@@ -1336,7 +1336,7 @@ __global__ void __launch_bounds__(FM_THREADS)
 // ------------------------------------------- substamp search in shared memory --
 // The decisions of k_find_substamps_maps for FP32 images, with the stamp in
 // shared memory at 6.4 bytes per pixel (pixel, flags, row winner, two bit
-// maps), so that stamps up to ~188 px fit and two 107-px ones share an SM:
+// maps), so that stamps up to 190 px fit and two 107-px ones share an SM:
 //   * a candidate's window maximum (the largest key, ties to the first in
 //     raster order) is found when the scan reaches the candidate, by one thread
 //     from the window rows' winners (hx, the maximum over the 2 hSS + 1 columns
@@ -1350,8 +1350,8 @@ __global__ void __launch_bounds__(FM_THREADS)
 // !((v - sky) * (1/fwhm) < tKF), monotone in v, become compares against their
 // exact thresholds, found once per stamp by a warp search over the ordered
 // doubles; so does the pass threshold v > lim.
-// A pass lists its candidates in raster order, 2048 at a time; a thread takes
-// one, and the first that passes is the next substamp.
+// A pass lists its candidates in raster order, 2048 at a time (512 in the largest
+// stamps); a thread takes one, and the first that passes is the next substamp.
 // Two-dimensional maps of the winners and conditions by block scans, rebuilt
 // around every acceptance (15 bytes per pixel, one CTA per SM, stamps above
 // 123 px from global memory), took 0.55 ms for 2 x 256 stamps of 107 px and
@@ -1362,7 +1362,7 @@ constexpr int FS_T = 512;
 constexpr uint8_t FS_BAD = 0x80;  // in the flags byte
 constexpr int FS_MAXN = 255;      // row winners are bytes, 0xFF none
 constexpr int FS_SEG = 8;         // columns per task of the row winners
-constexpr int FS_LIST = 2048;     // candidates listed at a time
+constexpr int FS_LIST = 2048;     // candidates listed at a time, FS_T where more do not fit
 
 // One warp: smallest key in (lo, hi] at which pred turns true, given
 // pred(lo) false and pred(hi) true (pred monotone between them).
@@ -1434,7 +1434,7 @@ __global__ void __launch_bounds__(FS_T, 2)
                         const double* __restrict__ sky1, const double* __restrict__ fwhm1,
                         int2* __restrict__ xy0, double* __restrict__ val0, int* __restrict__ cnt0,
                         int2* __restrict__ xy1, double* __restrict__ val1, int* __restrict__ cnt1,
-                        int w, int fSW, int hSS, int maxSS, double tH, double tKF) {
+                        int w, int fSW, int hSS, int maxSS, double tH, double tKF, int cap) {
   extern __shared__ __align__(16) unsigned char fs_s[];
   const int s = blockIdx.x, im = blockIdx.y, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   constexpr int NW = FS_T / 32;
@@ -1455,10 +1455,10 @@ __global__ void __launch_bounds__(FS_T, 2)
   uint32_t* dBad = (uint32_t*)(fs_s + (((size_t)N * 6 + 3) & ~(size_t)3));  // n x nw bit rows
   uint32_t* dTmp = dBad + n * nw;
   uint32_t* dPred = dTmp + n * nw;
+  uint16_t* list = (uint16_t*)(dPred + n * nw);  // cap candidates
   __shared__ int2 locXY[MAX_MAXSS];
   __shared__ double locVal[MAX_MAXSS];
   __shared__ int sBest[2], sM, sTotal, sScan[NW];
-  __shared__ uint16_t list[FS_LIST];
   __shared__ double rA[NW];
   __shared__ unsigned rB[NW];
   __shared__ double sSum;
@@ -1699,20 +1699,20 @@ __global__ void __launch_bounds__(FS_T, 2)
           if(from >= N) break;
           const int ys = from / n, xs = from - ys * n, e0 = ys * nw + (xs >> 5);
           nList = 0;
-          for(int eb = e0; eb < n * nw && nList < FS_LIST; eb += FS_T) {
+          for(int eb = e0; eb < n * nw && nList < cap; eb += FS_T) {
             const int e = eb + tid, y = e / nw;
             unsigned c = e < n * nw ? cands[e] : 0u;
             if(e == e0) c &= 0xFFFFFFFFu << (xs & 31);
             int k = nList + blockScanExcl(__popc(c), sScan, &sTotal);
-            for(; c && k < FS_LIST; c &= c - 1, k++)
+            for(; c && k < cap; c &= c - 1, k++)
               list[k] = (uint16_t)(y * n + 32 * (e - y * nw) + __ffs(c) - 1);
             nList += sTotal;
             __syncthreads();
           }
           from = N;
-          if(nList > FS_LIST) {
-            nList = FS_LIST;
-            from = list[FS_LIST - 1] + 1;
+          if(nList > cap) {
+            nList = cap;
+            from = list[cap - 1] + 1;
           }
           at = 0;
           if(nList == 0) break;
@@ -1930,17 +1930,18 @@ static void sssPass(xb_ctx* c, int* nKept) {
   // else maps in global memory
   int optin = 0;
   XB_CUDA(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, c->device));
-  const bool inShared = !c->imgIsF64 && fSW <= FS_MAXN && fsSmem + 6 * 1024 <= (size_t)optin;
+  const bool inShared = !c->imgIsF64 && fSW <= FS_MAXN && fsSmem + 2 * FS_T + 1024 <= (size_t)optin;
+  const int cap = fsSmem + 2 * FS_LIST + 1024 <= (size_t)optin ? FS_LIST : FS_T;
   // global-memory maps only for the kernel that uses them
   unsigned char* scratch =
       inShared ? nullptr : buf<unsigned char>(c, "fm_scratch", (size_t)2 * nAll * perCta);
   if(inShared) {
     XB_CUDA(allowMaxDynamicSmem((const void*)k_find_substamps_sm, c->device));
-    k_find_substamps_sm<<<grid, FS_T, fsSmem, c->stream>>>(
+    k_find_substamps_sm<<<grid, FS_T, fsSmem + 2 * cap, c->stream>>>(
         (const float*)c->img[0], (const float*)c->img[1], c->mask, c->geomAll, c->skyAll[0],
         c->fwhmAll[0], c->skyAll[1], c->fwhmAll[1], c->ssxyAll[0], c->ssvalAll[0], c->cntAll[0],
         c->ssxyAll[1], c->ssvalAll[1], c->cntAll[1], c->w, fSW, g.hSS, g.maxSS, c->p.threshHigh,
-        c->p.threshKernFit);
+        c->p.threshKernFit, cap);
   } else if(c->imgIsF64)
     k_find_substamps_maps<double><<<grid, FM_THREADS, 0, c->stream>>>(
         (const double*)c->img[0], (const double*)c->img[1], c->mask, c->geomAll,
