@@ -1709,8 +1709,10 @@ __global__ void __launch_bounds__(FS_T, 2)
             nList += sTotal;
             __syncthreads();
           }
+          // a full list, also one that filled exactly, goes on behind its last
+          // candidate: words may be left that no step has looked at
           from = N;
-          if(nList > cap) {
+          if(nList >= cap) {
             nList = cap;
             from = list[cap - 1] + 1;
           }
