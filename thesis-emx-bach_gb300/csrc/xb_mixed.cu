@@ -766,7 +766,11 @@ struct ConvArgsF {
 
 // Normalised centres of the fK x fK kernel blocks, xf of the xSteps block
 // columns then yf of the block rows: (centre - w/2) / (w/2) in FP64, the
-// coordinates of the spatial kernel terms (conv(), src/bach.cpp:339-350).
+// coordinates of the spatial kernel terms (conv(), src/bach.cpp:339-350).  The
+// last CTA of a row reads up to BLOCK_SPARE centres past the columns, for blocks
+// that lie past the frame and store nothing: the rows' centres, and zeros behind
+// them.
+constexpr int BLOCK_SPARE = 8;
 __global__ void k_block_centres(int w, int h, int fK, int xSteps, int ySteps,
                                 double* __restrict__ xy) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
@@ -777,6 +781,8 @@ __global__ void k_block_centres(int w, int h, int fK, int xSteps, int ySteps,
   } else if(i < xSteps + ySteps) {
     const double hy = 0.5 * h;
     xy[i] = ((i - xSteps) * fK + 2 * hK - hy) / hy;
+  } else if(i < xSteps + ySteps + BLOCK_SPARE) {
+    xy[i] = 0.0;
   }
 }
 
@@ -1432,12 +1438,14 @@ __global__ void __launch_bounds__(BX * 21, 3)
       }
     }
     const float ak = aks[b], et = eTot[b];
+    // output pixels of this thread's tile (the others store nothing)
+    const int nX = a.w - 2 * HK - x0 - lx0, nY = a.h - 2 * HK - y0 - ly0;
     const unsigned lanes = (warp + 1) * 32 <= NT ? 0xffffffffu : (1u << (NT & 31)) - 1u;
 #pragma unroll
     for(int o = 0; o < 3; o++)
 #pragma unroll
       for(int q = 0; q < 7; q++) {
-        const bool hit = ((orw[o] >> q) & WIN) != 0ull;
+        const bool hit = q < nX && o < nY && ((orw[o] >> q) & WIN) != 0ull;
         int f = 0;
         if(hit) {
           if((sk[o][q] + se[o][q]) < (0.01f - 1e-4f) * (ak - et)) f = 1;
@@ -2068,10 +2076,9 @@ void convSubMixed(xb_ctx* c, double* dKernSum) {
   a.tL = (float)c->p.threshLow;
   const int xSteps = (c->w + g.fK - 1) / g.fK, ySteps = (c->h + g.fK - 1) / g.fK;
   a.xSteps = xSteps;
-  // (the last CTA of a row reads up to seven centres past the columns)
-  double* blockXY = buf<double>(c, "conv_block_xy", (size_t)(xSteps + ySteps + 8));
-  k_block_centres<<<(xSteps + ySteps + 127) / 128, 128, 0, c->stream>>>(c->w, c->h, g.fK, xSteps,
-                                                                      ySteps, blockXY);
+  const int nXY = xSteps + ySteps + BLOCK_SPARE;
+  double* blockXY = buf<double>(c, "conv_block_xy", (size_t)nXY);
+  k_block_centres<<<(nXY + 127) / 128, 128, 0, c->stream>>>(c->w, c->h, g.fK, xSteps, ySteps, blockXY);
   XB_LAUNCHED(c);
   auto launch = [&](int variant) {
     const float *Ii = (const float*)c->img[I], *Oi = (const float*)c->img[O];
