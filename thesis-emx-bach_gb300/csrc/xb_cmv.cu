@@ -278,7 +278,7 @@ __global__ void __launch_bounds__(NT)
 // projections: 961 chained sums of 62 cycles, so spreading a stamp over CTAs is
 // what shortens it (one CTA per stamp, the projections after the products and
 // from dependent global loads, took 0.46 ms for 256 stamps; now 0.27 ms, 0.09 ms for one stamp).
-constexpr int DOT_THREADS = 64, DOT_KT = 32, DOT_MAX = 1024;
+constexpr int DOT_THREADS = 64, DOT_KT = 32;
 struct DotPair {
   int ra, rb, oi;  // rows of W and output index; ra < 0: none
 };
@@ -481,8 +481,6 @@ void stageCmv(xb_ctx* c) {
   const Geo& g = c->g;
   if((g.qCount - 1) * (g.qCount) / 2 > GQ_MAXENT)
     throw XbError{XB_ERR_UNSUPPORTED, "too many basis functions for the Gram kernel"};
-  if(!mixedMode(c) && g.nComp1 * g.nBG + g.nBG + g.nBG * g.nBG > DOT_MAX)
-    throw XbError{XB_ERR_UNSUPPORTED, "too many basis and background terms for the dot kernel"};
   // basis tables (host-built once per context) and background exponents
   std::vector<int2> bg(g.nBG);
   for(int b = 0; b < g.nBG; b++) bg[b] = make_int2(c->basis.bgX[b], c->basis.bgY[b]);

@@ -1133,6 +1133,11 @@ static void solveGlobal(xb_ctx* c, int si, const FitBuffers& f, const int* list,
   if(mixed) {  // forms its spatial weights itself; its dots are filled by the Gram kernel
     buildSystemMixed(c, si, list, nList, bgBase, f.M, dSol, liveN);
   } else {
+    // xb_cd and xb_ksc take at most this many products per stamp; xb_cmv, whose
+    // results can be read by themselves, has no such bound
+    constexpr int MAX_PRODUCTS = 1024;
+    if(nList > 0 && g.nComp1 * g.nBG + g.nBG + g.nBG * g.nBG > MAX_PRODUCTS)
+      throw XbError{XB_ERR_UNSUPPORTED, "too many basis and background terms for the plain fit"};
     const int2* kp = kernelPowers(c);
     const int n1 = g.nComp2 + 1;
     { KT_SCOPE(c, "weights");
