@@ -440,7 +440,10 @@ void fillStamps(xb_ctx* c, int si, const int* dList, int nList, int imgConv, con
   const size_t smemGram = (std::max((size_t)2 * (g.qCount - 1) * (GQ_KT + 1), (size_t)g.wCols) +
                            (omega ? (size_t)g.wCols : 0)) * sizeof(double);
   const int nEnt = (g.qCount - 1) * g.qCount / 2;
-  // 128 entries per CTA where the list fills the SMs, else 64
+  // 128 entries per CTA where the list fills the SMs, else 64: of 50 rows, 64 and
+  // 128 entries take 148 and 151 us for 20 stamps, 204 and 219 for 36, 269 and 290
+  // for 47, 416 and 361 for 60, 412 and 403 for 70, 452 and 477 for 83, 580 and 574
+  // for 106, 726 and 651 for 122; the line is at 61 stamps
   auto gram = [&](auto* img, auto kernel, int nt) {
     XB_CUDA(allowMaxDynamicSmem((const void*)kernel, c->device));
     kernel<<<dim3(nList, (nEnt + nt - 1) / nt + 1), nt, smemGram, c->stream>>>(

@@ -356,7 +356,9 @@ void stageInitMask(xb_ctx* c) {
   const int spreadWidth = (int)(c->p.hKernelWidth * c->p.inSpreadMaskFactor);
   const int r = spreadWidth / 2;
   if(r > 0) {
-    // wider spreads than this build's first kernel held in 48 KB are refused still
+    // spreads of more than 78 pixels are refused, by the interface: the kernel has no
+    // bound of its own (a byte per pixel of a 64 x 16 tile with its halo, and of the
+    // halo's rows, within 48 KB)
     if((64ll + 2 * r) * (16 + 2 * r) + (16ll + 2 * r) * 64 > 48 * 1024)
       throw XbError{XB_ERR_CUDA, "input mask spread too wide"};
     KT_SCOPE(c, "spread_mask");

@@ -488,10 +488,12 @@ void fillGramLaunch(xb_ctx* c, int si, const int* dList, int nList, int imgConv,
   int optin = 0;
   XB_CUDA(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, c->device));
   // A refill's few stamps (its bound is not: the count is on the device) and short
-  // lists leave most SMs idle: four CTAs share each of them.  Four stamps take 70
-  // us so and about 200 us on a CTA each; 256 stamps 556 and 437 us (both before
-  // the passes' last step), so up to half an
-  // SM count of stamps, where four waves of the first meet the second, are split.
+  // lists leave most SMs idle: four CTAs share each of them.  A split list takes
+  // about 60 us per round of SMs / 4 stamps, a CTA per stamp 200 us up to two per
+  // SM: 63 and 198 us for 9 stamps, 65 and 202 for 36, 121 and 202 for 60, 123 and
+  // 202 for 70, 177 and 202 for 83, 180 and 203 for 106, 235 and 204 for 122.
+  // Lists up to half an SM count are split, well on the safe side of the
+  // crossing near 110.
   const bool split = ((liveN && liveN != S.dN) || nList * 2 <= c->smCount) &&
                      fgLayout(g.hSS, g.hK, nGroups, g.nPSF, FG_CL).total + 8 * 1024 <= (size_t)optin;
   const int cl = split ? FG_CL : 1, perPass = fgPerPass(cl);

@@ -340,8 +340,9 @@ void globalSolveMixed(xb_ctx* c, const double* M, int n, double* rhs, int* piv, 
 // device-side wait ran out (sticky until checkSolveTimeout reports it).  Zeroed
 // when first allocated.
 int* deviceStatus(xb_ctx* c);
-// Throws XB_ERR_DEVICE_TIMEOUT when a bounded wait of the cluster solve or
+// Throws XB_ERR_DEVICE_TIMEOUT when a bounded wait of the fused fill + Gram or
 // the tensor-core Gram ran out since the last call (synchronises the stream).
+// (The cluster solve waits at hardware cluster barriers only.)
 void checkSolveTimeout(xb_ctx* c);
 // Work beside the context stream's: between enter() and leave() launches go to
 // the side stream, after everything issued before the object was made; join()

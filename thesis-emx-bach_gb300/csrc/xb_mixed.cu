@@ -750,9 +750,9 @@ __global__ void __launch_bounds__(1024)
 // BX (4, 6 or 8) is chosen by the autotuner; the three give identical
 // images.
 //
-// Bound by FP32: 441 FMAs a pixel of three registers each, which issue at 0.7 of
-// the rate (0.3 ms at 4096^2), beside the halo's loads, the kernels' FP64 terms
-// and the output.  The tile comes a row per warp with its bad bits from the same
+// Bound by instruction issue (66 % of the slots, FP32 pipe 43 %): 441 FMAs a pixel
+// (0.19 ms at 4096^2 at the FP32 peak) beside the halo's loads, the kernels' FP64
+// terms (pipe 19 %) and the output.  The tile comes a row per warp with its bad bits from the same
 // registers, the background is a polynomial in y per column, and seven rows of
 // the other image are loaded ahead; 72 to 75 registers keep 24 to 28 warps on an
 // SM.  4096^2 with BX = 4, 6, 8: 0.58, 0.52, 0.57 ms (0.70 ms with BX = 4 and a
@@ -1101,9 +1101,11 @@ __global__ void __launch_bounds__(ConvTileF<FK, BX>::NT, BX == 4 ? 7 : BX == 6 ?
 // One convolution per spatial term, two at a time over the same 7 x 3 pixel
 // tile per thread as k_conv_sub_f32: a row of 27 window values feeds three
 // rows of two kernels, 882 FMAs per 27 + 36 shared loads (the term kernels are
-// the same for every block).  Bound by FP32 (0.28 ms at 2048^2 for six terms);
-// seven pixels of one row per thread and, for every pixel with a bad one under
-// its window, its own kernel tap by tap took 5.2 ms, this form 0.94 ms.
+// the same for every block).  Bound by instruction issue (53 % of the slots, FP32
+// pipe 41 %; its FMAs alone are 0.28 ms at 2048^2 for six terms) at twelve warps an
+// SM, 161 registers and code that misses the instruction cache; seven pixels of
+// one row per thread and, for every pixel with a bad one under its window, its own
+// kernel tap by tap took 5.2 ms, this form 0.88 ms.
 //
 // The 0.99 |kernel| rule of such a pixel: with E = sum_t max|dP_t| |Kt[t]| the
 // largest change of a tap's kernel within the block, the bad taps' sum is
@@ -1111,7 +1113,8 @@ __global__ void __launch_bounds__(ConvTileF<FK, BX>::NT, BX == 4 ? 7 : BX == 6 ?
 // total of E, which decides most pixels; the others take their own kernel's
 // bad taps and the whole sum to first order in dP.  Those whose bounds still
 // straddle 0.99 (with 1e-4 for the rounding of the FP32 sums) sum their own
-// kernel, a warp per pixel.  (All of them a lane per pixel: 2.3 ms, the CTA
+// kernel, a warp per pixel.  Only output pixels take the rule (those past the
+// frame, with a bad edge copied into their windows, cost another 0.3 ms).  (All of them a lane per pixel: 2.3 ms, the CTA
 // waiting for it; the first bound alone before that sum: 1.3 ms.)
 template <int FK, int BX>
 struct ConvTilePP {

@@ -924,7 +924,7 @@ __global__ void __launch_bounds__(NW * 32 + 32, sizeof(T) == 8 ? 2 : 3)
 // and FP64 images use the scratch, also three CTAs to an SM, which overlap each
 // other's serial chains (an image's 390 stamps of 132 px in shared memory, two to an
 // SM, 190 us, in the scratch 147; 400 of 183 px, one of 16 warps to an SM, 372
-// and 264).
+// and 264).  The limit of a block, 227 KB, stands in for an SM's 228 KB.
 template <class T>
 cudaError_t launchStampStats(const T* img, uint16_t* mask, const int4* geom, int n, int w, int h,
                              int fSW, T* good, uint8_t* clip, double* chunkBuf, double alpha,
