@@ -1113,7 +1113,9 @@ __global__ void __launch_bounds__(ConvTileF<FK, BX>::NT, BX == 4 ? 7 : BX == 6 ?
 // total of E, which decides most pixels; the others take their own kernel's
 // bad taps and the whole sum to first order in dP.  Those whose bounds still
 // straddle 0.99 (with 1e-4 for the rounding of the FP32 sums) sum their own
-// kernel, a warp per pixel.  Only output pixels take the rule (those past the
+// kernel, a warp per pixel, and within 6e-5 of 0.99 in the order of the taps, whose
+// FP32 rounding then decides (the warp's sums alone put one pixel on the other
+// side in four of 24 frames of 2048^2).  Only output pixels take the rule (those past the
 // frame, with a bad edge copied into their windows, cost another 0.3 ms).  (All of them a lane per pixel: 2.3 ms, the CTA
 // waiting for it; the first bound alone before that sum: 1.3 ms.)
 template <int FK, int BX>
@@ -1486,7 +1488,11 @@ __global__ void __launch_bounds__(BX * 21, 3)
             else if((bs - eps) > (0.01f + 1e-4f) * (lin + cTot[b] + eps)) f = 2;
           }
         }
-        // undecided: the warp sums that pixel's own kernel, 14 taps per lane
+        // undecided: the warp sums that pixel's own kernel, 14 taps per lane.  The
+        // reference sums the taps one after the other; in FP32 that sum is within
+        // 440 * 2^-24 of its value and the warp's within 20 * 2^-24, so their
+        // ratios differ by less than TIE.
+        constexpr float TIE = 6e-5f;
         for(unsigned u = __ballot_sync(lanes, hit && f == 0); u; u &= u - 1) {
           const int src = __ffs(u) - 1, st = warp * 32 + src;
           const int sb = st / L::TPB, sr = st - sb * L::TPB, sk7 = sr / 7;
@@ -1498,15 +1504,22 @@ __global__ void __launch_bounds__(BX * 21, 3)
                 (float)(xpow[i * RW + px] * ypow[(lane - t0) * FK + py] - poly[sb * TMAX + lane]);
           }
           __syncwarp(lanes);
-          float av = 0.f, uv = 0.f;
-          for(int p = lane; p < NK; p += __popc(lanes)) {
+          const int nl = __popc(lanes);
+          auto tap = [&](int p, bool& good) -> float {  // |kernel| of a tap
             const int jj = p / FK, ii = p - jj * FK;
             const int at = (FK - 1 - jj) * KS + FK - 1 - ii;
             float kv = kern[sb * FK * KS + at];
             for(int tt = 1; tt < nC2; tt++)
               kv = fmaf(sDP[warp][tt], term[(tt - 1) * FK * KS + at], kv);
-            av += fabsf(kv);
-            if(!((bits[(py + jj) * NW + ((px + ii) >> 5)] >> ((px + ii) & 31)) & 1u)) uv += fabsf(kv);
+            good = !((bits[(py + jj) * NW + ((px + ii) >> 5)] >> ((px + ii) & 31)) & 1u);
+            return fabsf(kv);
+          };
+          float av = 0.f, uv = 0.f;
+          for(int p = lane; p < NK; p += nl) {
+            bool good;
+            const float v = tap(p, good);
+            av += v;
+            if(good) uv += v;
           }
 #pragma unroll
           for(int d = 16; d > 0; d >>= 1) {
@@ -1516,7 +1529,25 @@ __global__ void __launch_bounds__(BX * 21, 3)
               uv += u2;
             }
           }
-          const int fs = (__shfl_sync(lanes, uv, 0) / __shfl_sync(lanes, av, 0)) < 0.99f ? 2 : 1;
+          float ratio = __shfl_sync(lanes, uv, 0) / __shfl_sync(lanes, av, 0);
+          // within reach of the rounding of both sums: the taps in the order of conv.cl
+          if(!(fabsf(ratio - 0.99f) > TIE)) {
+            av = uv = 0.f;
+            for(int p0 = 0; p0 < NK; p0 += nl) {
+              bool good = false;
+              const float v = p0 + lane < NK ? tap(p0 + lane, good) : 0.f;
+              const unsigned gm = __ballot_sync(lanes, good);
+              const int cnt = min(nl, NK - p0);
+#pragma unroll 6
+              for(int l = 0; l < cnt; l++) {
+                const float x = __shfl_sync(lanes, v, l);
+                av += x;
+                if((gm >> l) & 1u) uv += x;
+              }
+            }
+            ratio = uv / av;
+          }
+          const int fs = ratio < 0.99f ? 2 : 1;
           if(lane == src) f = fs;
           __syncwarp(lanes);
         }
