@@ -1103,9 +1103,9 @@ __global__ void __launch_bounds__(ConvTileF<FK, BX>::NT, BX == 4 ? 7 : BX == 6 ?
 // rows of two kernels, 882 FMAs per 27 + 36 shared loads (the term kernels are
 // the same for every block).  Bound by instruction issue (53 % of the slots, FP32
 // pipe 41 %; its FMAs alone are 0.28 ms at 2048^2 for six terms) at twelve warps an
-// SM, 161 registers and code that misses the instruction cache; seven pixels of
+// SM, 162 registers and code that misses the instruction cache; seven pixels of
 // one row per thread and, for every pixel with a bad one under its window, its own
-// kernel tap by tap took 5.2 ms, this form 0.88 ms.
+// kernel tap by tap took 5.2 ms, this form 0.91 ms.
 //
 // The 0.99 |kernel| rule of such a pixel: with E = sum_t max|dP_t| |Kt[t]| the
 // largest change of a tap's kernel within the block, the bad taps' sum is
@@ -1115,9 +1115,10 @@ __global__ void __launch_bounds__(ConvTileF<FK, BX>::NT, BX == 4 ? 7 : BX == 6 ?
 // straddle 0.99 (with 1e-4 for the rounding of the FP32 sums) sum their own
 // kernel, a warp per pixel, and within 6e-5 of 0.99 in the order of the taps, whose
 // FP32 rounding then decides (the warp's sums alone put one pixel on the other
-// side in four of 24 frames of 2048^2).  Only output pixels take the rule (those past the
-// frame, with a bad edge copied into their windows, cost another 0.3 ms).  (All of them a lane per pixel: 2.3 ms, the CTA
-// waiting for it; the first bound alone before that sum: 1.3 ms.)
+// side in four of 24 frames of 2048^2).  Only output pixels take the rule (those past
+// the frame, with a bad edge copied into their windows, cost up to 0.3 ms).  (All
+// undecided ones a lane per pixel: 2.3 ms, the CTA waiting for it; the first bound
+// alone before that sum: 1.3 ms.)
 template <int FK, int BX>
 struct ConvTilePP {
   using L = ConvTileF<FK, BX>;
