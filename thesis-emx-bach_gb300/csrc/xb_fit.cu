@@ -12,7 +12,6 @@
 #include <cooperative_groups.h>
 
 #include <algorithm>
-#include <atomic>
 #include <climits>
 
 #include "xb_device.cuh"
@@ -1170,7 +1169,6 @@ static void solveGlobal(xb_ctx* c, int si, const FitBuffers& f, const int* list,
   }
   // 16 CTAs where the device allows that cluster, else 8 (the same products
   // in the same order either way)
-  static std::atomic<int> clusterSize{0};
   auto launchLu = [&](auto kernel, int CL) -> cudaError_t {
     cudaError_t e = allowMaxDynamicSmem((const void*)kernel, c->device);
     if(e == cudaSuccess && CL > 8)
@@ -1191,15 +1189,9 @@ static void solveGlobal(xb_ctx* c, int si, const FitBuffers& f, const int* list,
     return cudaLaunchKernelEx(&cfg, kernel, f.M, n, dSol, f.singular);
   };
   { KT_SCOPE(c, "global_lu");
-  cudaError_t e = cudaErrorUnknown;
-  if(clusterSize.load() != 8) {
-    e = launchLu(k_global_lu<16>, 16);
-    if(e == cudaSuccess) clusterSize = 16;
-    else cudaGetLastError();
-  }
-  if(e != cudaSuccess) {
+  if(launchLu(k_global_lu<16>, 16) != cudaSuccess) {
+    cudaGetLastError();
     XB_CUDA(launchLu(k_global_lu<8>, 8));
-    clusterSize = 8;
   }
   XB_LAUNCHED(c);
   }
